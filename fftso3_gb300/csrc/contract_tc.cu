@@ -44,6 +44,7 @@
 #include "../../include/fftso3_gb300.h"
 #include "common.cuh"
 #include "contract.cuh"
+#include "direct_dft.cuh"
 #include "fused.cuh"
 #include "tc.cuh"
 #include "tc_ptx.cuh"
@@ -1117,6 +1118,7 @@ struct TCState {
     long long total_rows = 0;
     __nv_bfloat16* d_tab[3] = {nullptr, nullptr, nullptr};
     float2* d_work = nullptr;     // FFT work grid [fn][k][p][q] (two-pass and generic-N FFTs)
+    bool direct = false;          // generic N: the FFT passes as direct DFTs (direct_dft.cu)
     bool fused_fft = false;       // SO(3), N = 64..512: both FFT passes in one launch through an L2 ring
     float2* d_ring = nullptr;     // fused FFT: ring of beta-slice chunks
     size_t ring_elems = 0;
@@ -1353,13 +1355,14 @@ int tc_create(TCState** out, int L, int N, int batch, const double* d_table_fp64
     {
         const char* ev = getenv("FFTSO3_TWO_PASS_FFT");
         s->fused_fft = !s2 && fft_grid_fused_supported(N) && !(ev && ev[0] == '1');
+        s->direct = !fft_fast_supported(N) && direct_dft_supported(N);
     }
     if (s->fused_fft) {
         s->ring_elems = fft_grid_fused_ring_elems(N);
         if ((rc = tc_alloc(s, (void**)&s->d_ring, sizeof(float2) * s->ring_elems, err))) return bail(rc);
         if ((rc = tc_alloc(s, (void**)&s->d_fctl, sizeof(int) * fft_grid_fused_ctl_ints(batch, N), err)))
             return bail(rc);
-    } else if (!(s2 && fft_fast_supported(N))) {
+    } else if (!(s2 && (fft_fast_supported(N) || s->direct))) {
         if ((rc = tc_alloc(s, (void**)&s->d_work, sizeof(float2) * gridel, err))) return bail(rc);
     }
     // refinement: the residual buffer follows the pencils in one allocation, so that together they hold one
@@ -1450,7 +1453,7 @@ int tc_create(TCState** out, int L, int N, int batch, const double* d_table_fp64
         err = std::string("tensor-core kernel attributes: ") + cudaGetErrorString(e);
         return bail(FFTSO3_ERR_CUDA);
     }
-    if (autotune && !fft_fast_supported(N))
+    if (autotune && !fft_fast_supported(N) && !s->direct)
         if ((rc = autotune_fft(s, err))) return bail(rc);
     if (autotune && !simt && s->ntiles > 1)
         if ((rc = autotune_cluster(s, err))) return bail(rc);
@@ -1776,6 +1779,20 @@ static int fft_forward(TCState* s, const void* grid, cudaStream_t st, StageTimer
         }
         return FFTSO3_SUCCESS;
     }
+    if (s->direct) {
+        T->begin(ST_FFT_ROWS, st);
+        if (s->s2)
+            TCK(launch_direct_s2_pass(grid, s->d_pencil, s->batch, s->N, 1, s->real, s->d_tw, st));
+        else
+            TCK(launch_direct_grid_pass(grid, s->d_work, s->batch, s->N, 1, s->real, s->d_tw, st));
+        T->end(st);
+        if (!s->s2) {
+            T->begin(ST_FFT_COLS, st);
+            TCK(launch_direct_grid_pass(s->d_work, s->d_pencil, s->batch, s->N, 2, s->real, s->d_tw, st));
+            T->end(st);
+        }
+        return FFTSO3_SUCCESS;
+    }
     T->begin(ST_FFT_ROWS, st);
     TCK(launch_fft_lines(fft_launch(s, grid, s->d_work, false, s->real, false), st));
     T->end(st);
@@ -1816,6 +1833,20 @@ static int fft_inverse(TCState* s, void* grid, cudaStream_t st, StageTimer* T, s
         T->end(st);
         T->begin(ST_FFT_ROWS, st);
         TCK(launch_fft_grid_pass(s->d_work, grid, s->batch, s->N, -1, s->d_tw, st, s->real));
+        T->end(st);
+        return FFTSO3_SUCCESS;
+    }
+    if (s->direct) {
+        if (!s->s2) {
+            T->begin(ST_FFT_COLS, st);
+            TCK(launch_direct_grid_pass(s->d_pencil, s->d_work, s->batch, s->N, -2, s->real, s->d_tw, st));
+            T->end(st);
+        }
+        T->begin(ST_FFT_ROWS, st);
+        if (s->s2)
+            TCK(launch_direct_s2_pass(s->d_pencil, grid, s->batch, s->N, -1, s->real, s->d_tw, st));
+        else
+            TCK(launch_direct_grid_pass(s->d_work, grid, s->batch, s->N, -1, s->real, s->d_tw, st));
         T->end(st);
         return FFTSO3_SUCCESS;
     }
@@ -1865,12 +1896,11 @@ static int tc_forward_once(TCState* s, const void* grid, float2* F, cudaStream_t
     return FFTSO3_SUCCESS;
 }
 
-// real_in (S^2 real kinds): read the real coefficients straight into the GEMM input instead of F.
-static int tc_inverse_once(TCState* s, const float2* F, void* grid, cudaStream_t st, StageTimer* T,
-                           std::string& err, const void* real_in = nullptr)
+// The pencils of the Nyquist bins, which no coefficient maps to (the direct DFT's passes take them as zero themselves).
+static cudaError_t zero_nyquist_pencils(TCState* s, cudaStream_t st)
 {
     const long long N = s->N;
-    T->begin(ST_NYQUIST, st);
+    if (s->direct) return cudaSuccess;
     if (s->s2) {
         const long long tot = (long long)s->batch * N;
         s2_zero_nyquist_pencils_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(s->d_pencil, (int)N, s->batch);
@@ -1878,8 +1908,18 @@ static int tc_inverse_once(TCState* s, const float2* F, void* grid, cudaStream_t
         const long long tot = (long long)s->batch * 2 * N * N;
         zero_nyquist_pencils_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(s->d_pencil, (int)N, s->batch);
     }
-    TCK(cudaGetLastError());
-    T->end(st);
+    return cudaGetLastError();
+}
+
+// real_in (S^2 real kinds): read the real coefficients straight into the GEMM input instead of F.
+static int tc_inverse_once(TCState* s, const float2* F, void* grid, cudaStream_t st, StageTimer* T,
+                           std::string& err, const void* real_in = nullptr)
+{
+    if (!s->direct) {
+        T->begin(ST_NYQUIST, st);
+        TCK(zero_nyquist_pencils(s, st));
+        T->end(st);
+    }
     T->begin(ST_BASIS, st);
     if (real_in)
         TCK(launch_s2_real_to_group(real_in, s->d_fg, s->d_goff2, s->L, s->batch, st));
@@ -2103,12 +2143,9 @@ int tc_forward_finish(TCState* s, void* coeffs, cudaStream_t st, StageTimer* T, 
 int tc_inverse_prepare(TCState* s, const void* coeffs, cudaStream_t st, StageTimer* T, std::string& err)
 {
     const float2* Fc = (const float2*)coeffs;
-    const long long N = s->N;
     T->begin(ST_BASIS, st);
     if (s->real && s->s2) {
-        const long long tot = (long long)s->batch * N;
-        s2_zero_nyquist_pencils_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(s->d_pencil, (int)N, s->batch);
-        TCK(cudaGetLastError());
+        TCK(zero_nyquist_pencils(s, st));
         TCK(launch_s2_real_to_group(coeffs, s->d_fg, s->d_goff2, s->L, s->batch, st));
         T->end(st);
         return FFTSO3_SUCCESS;
@@ -2120,14 +2157,11 @@ int tc_inverse_prepare(TCState* s, const void* coeffs, cudaStream_t st, StageTim
             TCK(launch_so3_r2c(coeffs, s->d_fc, false, s->L, s->batch, st));
         Fc = s->d_fc;
     }
+    TCK(zero_nyquist_pencils(s, st));
     if (s->s2) {
-        const long long tot = (long long)s->batch * N;
-        s2_zero_nyquist_pencils_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(s->d_pencil, (int)N, s->batch);
         s2_packed_to_group_kernel<<<dim3(s->ngroups, s->batch), 128, 0, st>>>(Fc, s->d_fg, s->d_goff2, s->L,
                                                                              coeffs_per_fn(s));
     } else {
-        const long long tot = (long long)s->batch * 2 * N * N;
-        zero_nyquist_pencils_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(s->d_pencil, (int)N, s->batch);
         packed_to_group_tiled<<<ptile_grid(s->L, s->batch), 256, 0, st>>>(Fc, s->d_fg, s->d_goff2, s->L,
                                                                           coeffs_per_fn(s), s->batch);
     }
