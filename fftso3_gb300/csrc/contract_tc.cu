@@ -44,6 +44,7 @@
 #include "../../include/fftso3_gb300.h"
 #include "common.cuh"
 #include "contract.cuh"
+#include "dft_tc.cuh"
 #include "direct_dft.cuh"
 #include "fused.cuh"
 #include "tc.cuh"
@@ -1119,6 +1120,8 @@ struct TCState {
     __nv_bfloat16* d_tab[3] = {nullptr, nullptr, nullptr};
     float2* d_work = nullptr;     // FFT work grid [fn][k][p][q] (two-pass and generic-N FFTs)
     bool direct = false;          // generic N: the FFT passes as direct DFTs (direct_dft.cu)
+    bool dft_tc = false;          // ... on the tensor cores (dft_tc.cu)
+    void* d_dft = nullptr;        // ... the DFT matrices of either
     bool fused_fft = false;       // SO(3), N = 64..512: both FFT passes in one launch through an L2 ring
     float2* d_ring = nullptr;     // fused FFT: ring of beta-slice chunks
     size_t ring_elems = 0;
@@ -1196,7 +1199,7 @@ void tc_destroy(TCState* s)
     if (!s) return;
     for (int p = 0; p < 3; ++p)
         if (s->d_tab[p]) cudaFree(s->d_tab[p]);
-    void* ptrs[] = {s->d_tab32, s->d_wf, s->d_work, s->d_ring, s->d_fctl, s->d_pencil, s->d_coef2, s->d_fc, s->d_grow0, s->d_goff2, s->d_fg,
+    void* ptrs[] = {s->d_tab32, s->d_wf, s->d_work, s->d_dft, s->d_ring, s->d_fctl, s->d_pencil, s->d_coef2, s->d_fc, s->d_grow0, s->d_goff2, s->d_fg,
                     s->d_items_fwd, s->d_items_inv, s->d_iaux_fwd, s->d_iaux_inv, s->d_err};
     for (void* q : ptrs)
         if (q) cudaFree(q);
@@ -1355,7 +1358,13 @@ int tc_create(TCState** out, int L, int N, int batch, const double* d_table_fp64
     {
         const char* ev = getenv("FFTSO3_TWO_PASS_FFT");
         s->fused_fft = !s2 && fft_grid_fused_supported(N) && !(ev && ev[0] == '1');
-        s->direct = !fft_fast_supported(N) && direct_dft_supported(N);
+        // the direct DFT from half a million samples (S^2: a million; smaller batches are bound by launch latencies, where
+        // the line FFT's simpler kernels win: l_max 16, 4 functions, 0.16 M samples, 76 against 81 us both directions;
+        // l_max 38, 0.47 M, 125 against 119 us; l_max 30, 32 functions, 7.6 M, 524 against 361 us; S^2 l_max 47, 8 signals,
+        // 51 against 53 us, l_max 200, 8 signals, 1.3 M, equal, l_max 100, 64 signals, 2.6 M, 219 against 124 us;
+        // l_max 39, 0.51 M, on the tensor cores 125 against 107 us)
+        s->direct = !fft_fast_supported(N) && direct_dft_supported(N) && gridel >= (s2 ? 1000000 : 500000);
+        s->dft_tc = s->direct && !s2 && !simt && dft_tc_supported(N);
     }
     if (s->fused_fft) {
         s->ring_elems = fft_grid_fused_ring_elems(N);
@@ -1364,6 +1373,14 @@ int tc_create(TCState** out, int L, int N, int batch, const double* d_table_fp64
             return bail(rc);
     } else if (!(s2 && (fft_fast_supported(N) || s->direct))) {
         if ((rc = tc_alloc(s, (void**)&s->d_work, sizeof(float2) * gridel, err))) return bail(rc);
+    }
+    if (s->direct) {
+        if ((rc = tc_alloc(s, &s->d_dft, s->dft_tc ? dft_tc_table_bytes(N) : direct_dft_table_bytes(N), err))) return bail(rc);
+        const cudaError_t e = s->dft_tc ? dft_tc_build_table(s->d_dft, N, d_tw, 0) : direct_dft_build_table(s->d_dft, N, d_tw, 0);
+        if (e != cudaSuccess) {
+            err = std::string("DFT matrices: ") + cudaGetErrorString(e);
+            return bail(FFTSO3_ERR_CUDA);
+        }
     }
     // refinement: the residual buffer follows the pencils in one allocation, so that together they hold one
     // 16-byte (double-float) element per pencil place for the exact inverse
@@ -1752,6 +1769,12 @@ static int launch_gemm(TCState* s, bool fwd, cudaStream_t st, std::string& err, 
 static long long coeffs_per_fn(const TCState* s) { return s->s2 ? (long long)s->B * s->B : so3_off(s->B); }
 static long long grid_per_fn(const TCState* s) { return (long long)s->N * s->N * (s->s2 ? 1 : s->N); }
 
+static cudaError_t direct_pass(TCState* s, const void* in, void* out, int pass, cudaStream_t st)
+{
+    return s->dft_tc ? launch_dft_tc_grid_pass(in, out, s->batch, s->N, pass, s->real, s->d_dft, s->d_err, st)
+                     : launch_direct_grid_pass(in, out, s->batch, s->N, pass, s->real, s->d_dft, st);
+}
+
 // grid -> k-contiguous pencils (SO(3): [fn][p][q][k], S^2: [fn][p][k]); grid is
 // float2, or float when s->real.
 static int fft_forward(TCState* s, const void* grid, cudaStream_t st, StageTimer* T, std::string& err)
@@ -1782,13 +1805,13 @@ static int fft_forward(TCState* s, const void* grid, cudaStream_t st, StageTimer
     if (s->direct) {
         T->begin(ST_FFT_ROWS, st);
         if (s->s2)
-            TCK(launch_direct_s2_pass(grid, s->d_pencil, s->batch, s->N, 1, s->real, s->d_tw, st));
+            TCK(launch_direct_s2_pass(grid, s->d_pencil, s->batch, s->N, 1, s->real, s->d_dft, st));
         else
-            TCK(launch_direct_grid_pass(grid, s->d_work, s->batch, s->N, 1, s->real, s->d_tw, st));
+            TCK(direct_pass(s, grid, s->d_work, 1, st));
         T->end(st);
         if (!s->s2) {
             T->begin(ST_FFT_COLS, st);
-            TCK(launch_direct_grid_pass(s->d_work, s->d_pencil, s->batch, s->N, 2, s->real, s->d_tw, st));
+            TCK(direct_pass(s, s->d_work, s->d_pencil, 2, st));
             T->end(st);
         }
         return FFTSO3_SUCCESS;
@@ -1839,14 +1862,14 @@ static int fft_inverse(TCState* s, void* grid, cudaStream_t st, StageTimer* T, s
     if (s->direct) {
         if (!s->s2) {
             T->begin(ST_FFT_COLS, st);
-            TCK(launch_direct_grid_pass(s->d_pencil, s->d_work, s->batch, s->N, -2, s->real, s->d_tw, st));
+            TCK(direct_pass(s, s->d_pencil, s->d_work, -2, st));
             T->end(st);
         }
         T->begin(ST_FFT_ROWS, st);
         if (s->s2)
-            TCK(launch_direct_s2_pass(s->d_pencil, grid, s->batch, s->N, -1, s->real, s->d_tw, st));
+            TCK(launch_direct_s2_pass(s->d_pencil, grid, s->batch, s->N, -1, s->real, s->d_dft, st));
         else
-            TCK(launch_direct_grid_pass(s->d_work, grid, s->batch, s->N, -1, s->real, s->d_tw, st));
+            TCK(direct_pass(s, s->d_work, grid, -1, st));
         T->end(st);
         return FFTSO3_SUCCESS;
     }

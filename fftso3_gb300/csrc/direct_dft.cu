@@ -6,8 +6,10 @@
 // register tile of products per thread, outputs straight from registers (unit-contiguous side: 128-byte runs) or
 // through the folded buffer (line-contiguous side).  The next tile's lines are requested into L2 while the products
 // run, and two CTAs share an SM where the shared memory allows, so one loads while the other multiplies.
-// What bounds it: N / 2 packed-pair FMAs a complex sample (37 T FMA/s measured with fma.rn.f32x2; 25 T with scalar
-// fma, whose three register operands meet in the register banks), so HBM below N of about 200 and FP32 above.
+// What bounds it: N / 2 packed FMAs a complex sample (35 T FMA/s measured with fma.rn.f32x2; 25 T with scalar fma, whose
+// three register operands meet in the register banks), and that a CTA's loads and products take turns: at N = 194, 16
+// functions, a pass takes 1.1 to 1.2 ms, 0.3 of it the bytes, 0.5 the products (0.35 at the FMA rate), the rest loading and
+// folding.  SO(3) passes of N = 80 to 222 run on the tensor cores instead (dft_tc.cu).
 #include <algorithm>
 
 #include "common.cuh"
@@ -27,11 +29,18 @@ struct Shape {
 };
 static size_t smem_bytes(const Fold& f, int LT)
 {
-    return sizeof(float) * mat_floats(f) + sizeof(float2) * f.H * (4 * LT + 2) + 3 * 2 * sizeof(long long) * LT + 16;
+    return sizeof(float2) * mat_elems(f) + sizeof(float4) * f.H * (2 * LT + 1) + 3 * 2 * sizeof(long long) * LT + 16;
 }
+__global__ void build_table_kernel(float2* M, int N, const double2* tw)
+{
+    const Fold f = fold_of(N);
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e < mat_elems(f)) M[e] = mat_entry(f, e, tw);
+}
+
 // The shape with the fewest idle lanes among those of at least four warps; two CTAs of up to eight warps an SM (one loads while the other
-// multiplies) before one.
-static Shape shape_of(int N)
+// multiplies) before one, and (few units) tiles for every SM.
+static Shape shape_of(int N, unsigned nu = 0x7fffffffu, int nsm = 1)
 {
     Shape s = {};
     s.f = fold_of(N);
@@ -41,7 +50,8 @@ static Shape shape_of(int N)
             const int qw = (s.f.nb + ql - 1) / ql, warps = qw * ub, lt = ub * 128 / ql;
             const size_t b = smem_bytes(s.f, lt);
             if (32 * warps > MAXT || b > 227 * 1024) continue;
-            const double sc = (double)s.f.nb / (ql * qw) * (b <= 113 * 1024 && warps <= 8 ? 1.0 : 0.6) * (warps >= 4 ? 1.0 : warps / 4.0) +
+            const double sc = (double)s.f.nb / (ql * qw) * (b <= 113 * 1024 && warps <= 8 ? 1.0 : 0.6) * (warps >= 4 ? 1.0 : warps / 4.0) *
+                                  std::min(1.0, (double)((nu + lt - 1) / lt) / nsm) +
                               0.01 * warps;
             if (sc > best) {
                 best = sc;
@@ -57,9 +67,10 @@ static Shape shape_of(int N)
 
 struct Args {
     DirectPass p;
-    const double2* tw;
+    const float4* table;
     int LT, UB;
     unsigned nu, ntiles;
+    int nsm;
 };
 
 __device__ __forceinline__ void l2_prefetch(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
@@ -71,13 +82,15 @@ __global__ void __launch_bounds__(MAXT, 1) direct_dft_kernel(const __grid_consta
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const DirectPass& p = a.p;
     const Fold f = fold_of(p.N);
-    const int N = f.N, P = f.P, H = f.H, LT = a.LT, US = LT;
-    // an odd number of 16-byte chunks from one t to the next: the folding stores' lanes (consecutive t) then spread
-    // over the banks
-    const int TS = 4 * LT + 2;
-    float* M = reinterpret_cast<float*>(smem_raw);
-    float2* V = reinterpret_cast<float2*>(M + mat_floats(f));  // [t] (TS apart) [four folded terms][LT]
+    const int N = f.N, P = f.P, H = f.H, LT = a.LT, HU = LT / 2;
+    // odd, so that the folding stores of consecutive t meet distinct banks
+    const int TS = 2 * LT + 1;
+    float2* M = reinterpret_cast<float2*>(smem_raw);
+    // folded units [t] (TS apart) [parity][even units, then odd ones]: a pair of units is HU apart, so that a thread
+    // owns adjacent units (16-byte global accesses) and reads them without bank conflicts
+    float4* V = reinterpret_cast<float4*>(M + mat_elems(f));
     long long* tab = reinterpret_cast<long long*>(V + H * TS);  // [2 buffers][in, out, mirror][LT]
+    constexpr bool REAL = KIND != DIRECT_COMPLEX;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
 
     // offsets of a tile's units: input (-1: past the last unit), output, mirrored output (-1: none)
@@ -99,12 +112,12 @@ __global__ void __launch_bounds__(MAXT, 1) direct_dft_kernel(const __grid_consta
         }
     };
     auto put = [&](int t, int u, const Folded& r) {
-        float2* d = V + t * TS + u;
-#pragma unroll
-        for (int j = 0; j < 4; ++j, d += US) *d = r.v[j];
+        float4* d = V + t * TS + (u >> 1) + (u & 1) * HU;
+        d[0] = r.even;
+        d[LT] = r.odd;
     };
 
-    build_mats(M, f, a.tw);
+    for (int e = tid; e < mat_elems(f) / 2; e += blockDim.x) reinterpret_cast<float4*>(M)[e] = __ldg(a.table + e);
     int buf = 0;
     if (blockIdx.x < a.ntiles) tables(blockIdx.x, 0);
     __syncthreads();
@@ -113,8 +126,8 @@ __global__ void __launch_bounds__(MAXT, 1) direct_dft_kernel(const __grid_consta
     const int qb = (warp - ub * qw) * QL + lane % QL;
     const bool active = ub < a.UB && qb < f.nb;
     const int par = qb >= f.nbE, qi = active ? (par ? qb - f.nbE : qb) : 0;
-    const int u0 = ub * (128 / QL) + 2 * (lane / QL);
-    constexpr int UO = 64 / QL;
+    constexpr int G = 32 / QL;
+    const int pr = ub * 2 * G + lane / QL;  // first pair of units; the second G further on
     const float2 z = make_float2(0.f, 0.f);
     for (unsigned tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x, buf ^= 1) {
         const long long* ib = tab + buf * 3 * LT;
@@ -125,7 +138,7 @@ __global__ void __launch_bounds__(MAXT, 1) direct_dft_kernel(const __grid_consta
             for (int u = warp; u < LT; u += nw) {
                 const long long b = ib[u];
                 if (b < 0) {
-                    for (int t = lane; t < H; t += 32) put(t, u, Folded{{z, z, z, z}});
+                    for (int t = lane; t < H; t += 32) put(t, u, Folded{make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)});
                     continue;
                 }
                 const float* g0 = reinterpret_cast<const float*>(p.in) + (KIND == DIRECT_REAL_IN ? b : 2 * b);
@@ -137,7 +150,7 @@ __global__ void __launch_bounds__(MAXT, 1) direct_dft_kernel(const __grid_consta
 #pragma unroll 2
                 for (int t = lane; t < H; t += 32) {
                     const int tn = t ? N - t : 0, tq = t ? P + t : P;
-                    put(t, u, fold_line(t, P, at(t), at(tn), at(P - t), at(tq)));
+                    put(t, u, fold_line<REAL>(t, P, at(t), at(tn), at(P - t), at(tq)));
                 }
             }
         } else {
@@ -155,19 +168,15 @@ __global__ void __launch_bounds__(MAXT, 1) direct_dft_kernel(const __grid_consta
                     // f_j = X_0 + (-1)^j X_P + sum 2 Re X_t cos + 2 Im X_t sin: a_t = 2 Re X_t, b_t = 2 Im X_t; X_P = 0
                     const float4 x = at(t), y = t ? at(P - t) : z4;
                     const float c = t ? 2.f : 1.f, s = t ? 2.f : 0.f;
-                    put(t, u, fold_ab(t, P, make_float2(c * x.x, c * x.z), make_float2(s * x.y, s * x.w),
-                                      make_float2(c * y.x, c * y.z), make_float2(s * y.y, s * y.w)));
+                    put(t, u, fold_ab<true>(t, P, make_float2(c * x.x, c * x.z), make_float2(s * x.y, s * x.w),
+                                            make_float2(c * y.x, c * y.z), make_float2(s * y.y, s * y.w)));
                 } else {
                     const float4 x = at(t), xn = at(t ? N - t : 0);
                     const float4 xp = p.nyq && t == 0 ? z4 : at(P - t), xq = t ? at(P + t) : xp;
-                    const Folded r0 = fold_line(t, P, make_float2(x.x, x.y), make_float2(xn.x, xn.y),
-                                                make_float2(xp.x, xp.y), make_float2(xq.x, xq.y));
-                    const Folded r1 = fold_line(t, P, make_float2(x.z, x.w), make_float2(xn.z, xn.w),
-                                                make_float2(xp.z, xp.w), make_float2(xq.z, xq.w));
-                    float2* d = V + t * TS + 2 * u;
-#pragma unroll
-                    for (int j = 0; j < 4; ++j, d += US)
-                        *reinterpret_cast<float4*>(d) = make_float4(r0.v[j].x, r0.v[j].y, r1.v[j].x, r1.v[j].y);
+                    put(t, 2 * u, fold_line<false>(t, P, make_float2(x.x, x.y), make_float2(xn.x, xn.y),
+                                                   make_float2(xp.x, xp.y), make_float2(xq.x, xq.y)));
+                    put(t, 2 * u + 1, fold_line<false>(t, P, make_float2(x.z, x.w), make_float2(xn.z, xn.w),
+                                                       make_float2(xp.z, xp.w), make_float2(xq.z, xq.w)));
                 }
                 t += ti;
                 u += ui;
@@ -208,7 +217,7 @@ __global__ void __launch_bounds__(MAXT, 1) direct_dft_kernel(const __grid_consta
         }
         // ---- products
         Tile acc;
-        if (active) product<QL>(M + 2 * par * f.QS + 4 * qi, V + 2 * par * US + u0, H, f.QS, US, TS, acc);
+        if (active) product<QL>(M + par * f.QS + 4 * qi, V + par * LT + pr, H, f.QS, HU, TS, acc);
         const int q0 = 8 * qi + par;  // outputs q0, q0 + 2, q0 + 4, q0 + 6 (<= P)
         if (!SC) {
             if (active) {
@@ -216,7 +225,7 @@ __global__ void __launch_bounds__(MAXT, 1) direct_dft_kernel(const __grid_consta
                 if (KIND == DIRECT_REAL_IN) {
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
-                        const int u = u0 + (j & 1) + (j >> 1) * UO;
+                        const int u = 2 * (pr + (j >> 1) * G) + (j & 1);
                         if (ib[u] < 0) continue;
                         float2* o = reinterpret_cast<float2*>(p.out) + ob[u];
                         float2* lo = o + q0 * p.o_e;
@@ -225,16 +234,16 @@ __global__ void __launch_bounds__(MAXT, 1) direct_dft_kernel(const __grid_consta
                         for (int i = 0; i < 4; ++i, lo += step, hi -= step) {
                             const int q = q0 + 2 * i;
                             if (q > P) break;
-                            const float2 C = unpack2(acc.C[i][j]), S = unpack2(acc.S[i][j]);
-                            *reinterpret_cast<float4*>(lo) = make_float4(C.x, -S.x, C.y, -S.y);
+                            const float2 A = unpack2(acc.A[i][j]), B = unpack2(acc.B[i][j]);
+                            *reinterpret_cast<float4*>(lo) = make_float4(A.x, -A.y, B.x, -B.y);
                             if (p.full && q > 0 && q < P)
-                                *reinterpret_cast<float4*>(hi) = make_float4(C.x, S.x, C.y, S.y);
+                                *reinterpret_cast<float4*>(hi) = make_float4(A.x, A.y, B.x, B.y);
                         }
                     }
                 } else {
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
-                        const int u = u0 + h * UO;
+                        const int u = 2 * (pr + h * G);
                         if (ib[u] < 0) continue;  // the units come in pairs (nu and ni are even)
                         float2* o = reinterpret_cast<float2*>(p.out) + ob[u];
                         float2* lo = o + q0 * p.o_e;
@@ -245,10 +254,10 @@ __global__ void __launch_bounds__(MAXT, 1) direct_dft_kernel(const __grid_consta
                         for (int i = 0; i < 4; ++i, lo += step, hi -= step) {
                             const int q = q0 + 2 * i;
                             if (q > P) break;
-                            const float2 C0 = unpack2(acc.C[i][2 * h]), S0 = unpack2(acc.S[i][2 * h]);
-                            const float2 C1 = unpack2(acc.C[i][2 * h + 1]), S1 = unpack2(acc.S[i][2 * h + 1]);
-                            const float4 x = make_float4(C0.x + S0.y, C0.y - S0.x, C1.x + S1.y, C1.y - S1.x);
-                            const float4 y = make_float4(C0.x - S0.y, C0.y + S0.x, C1.x - S1.y, C1.y + S1.x);
+                            const float2 A0 = unpack2(acc.A[i][2 * h]), B0 = unpack2(acc.B[i][2 * h]);
+                            const float2 A1 = unpack2(acc.A[i][2 * h + 1]), B1 = unpack2(acc.B[i][2 * h + 1]);
+                            const float4 x = make_float4(A0.x + A0.y, B0.x - B0.y, A1.x + A1.y, B1.x - B1.y);
+                            const float4 y = make_float4(A0.x - A0.y, B0.x + B0.y, A1.x - A1.y, B1.x + B1.y);
                             *reinterpret_cast<float4*>(lo) = x;
                             if (q > 0 && q < P) *reinterpret_cast<float4*>(hi) = y;
                             if (MIR && mir) {
@@ -267,25 +276,25 @@ __global__ void __launch_bounds__(MAXT, 1) direct_dft_kernel(const __grid_consta
             if (active) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    const int u = u0 + (j & 1) + (j >> 1) * UO;
-                    float2* r = V + u * (N + 1);
+                    const int u = 2 * (pr + (j >> 1) * G) + (j & 1);
+                    float2* r = reinterpret_cast<float2*>(V) + u * (N + 1);
                     float* r0 = reinterpret_cast<float*>(V) + 2 * u * (N + 1);
                     float* r1 = r0 + N + 1;
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         const int q = q0 + 2 * i;
                         if (q > P) break;
-                        const float2 C = unpack2(acc.C[i][j]), S = unpack2(acc.S[i][j]);
+                        const float2 A = unpack2(acc.A[i][j]), B = unpack2(acc.B[i][j]);
                         if (KIND == DIRECT_REAL_OUT) {
-                            r0[q] = C.x + S.x;
-                            r1[q] = C.y + S.y;
+                            r0[q] = A.x + A.y;
+                            r1[q] = B.x + B.y;
                             if (q > 0 && q < P) {
-                                r0[N - q] = C.x - S.x;
-                                r1[N - q] = C.y - S.y;
+                                r0[N - q] = A.x - A.y;
+                                r1[N - q] = B.x - B.y;
                             }
                         } else {
-                            r[q] = make_float2(C.x + S.y, C.y - S.x);
-                            if (q > 0 && q < P) r[N - q] = make_float2(C.x - S.y, C.y + S.x);
+                            r[q] = make_float2(A.x + A.y, B.x - B.y);
+                            if (q > 0 && q < P) r[N - q] = make_float2(A.x - A.y, B.x + B.y);
                         }
                     }
                 }
@@ -300,11 +309,12 @@ __global__ void __launch_bounds__(MAXT, 1) direct_dft_kernel(const __grid_consta
                     for (int j = lane; j < N; j += 32) o[j] = r[i * (N + 1) + j];
                 }
             } else {
+                const float2* r = reinterpret_cast<const float2*>(V);
                 for (int u = warp; u < LT; u += nw) {
                     if (ib[u] < 0) continue;
                     float2* o = reinterpret_cast<float2*>(p.out) + ob[u];
 #pragma unroll 4
-                    for (int j = lane; j < N; j += 32) o[j] = V[u * (N + 1) + j];
+                    for (int j = lane; j < N; j += 32) o[j] = r[u * (N + 1) + j];
                 }
             }
             __syncthreads();
@@ -318,12 +328,9 @@ static cudaError_t run_ql(const Args& a, const Shape& s, cudaStream_t st)
     auto kern = direct_dft_kernel<KIND, LC, SC, MIR, QL>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
     if (e != cudaSuccess) return e;
-    int dev = 0, nsm = 0, per = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, s.threads, s.smem);
-    if (e != cudaSuccess) return e;
-    const unsigned nblk = std::min(a.ntiles, (unsigned)(nsm * std::max(per, 1)));
+    // CTAs an SM holds (the runtime's occupancy query costs more than a small pass): shared memory, and 128 registers a thread
+    const int per = std::max(1, std::min((int)(228 * 1024 / (s.smem + 1024)), 512 / s.threads));
+    const unsigned nblk = std::min(a.ntiles, (unsigned)(a.nsm * per));
     kern<<<nblk, s.threads, s.smem, st>>>(a);
     return cudaGetLastError();
 }
@@ -338,6 +345,14 @@ static cudaError_t run(const Args& a, const Shape& s, cudaStream_t st)
 
 using namespace ddft;
 
+size_t direct_dft_table_bytes(int N) { return sizeof(float2) * mat_elems(fold_of(N)); }
+
+cudaError_t direct_dft_build_table(void* table, int N, const void* tw, cudaStream_t st)
+{
+    build_table_kernel<<<(mat_elems(fold_of(N)) + 255) / 256, 256, 0, st>>>((float2*)table, N, (const double2*)tw);
+    return cudaGetLastError();
+}
+
 bool direct_dft_supported(int N)
 {
     if (N < 2 || N % 2) return false;
@@ -345,17 +360,21 @@ bool direct_dft_supported(int N)
     return s.QL > 0;
 }
 
-cudaError_t launch_direct_dft(const DirectPass& p, const void* tw, cudaStream_t st)
+cudaError_t launch_direct_dft(const DirectPass& p, const void* table, cudaStream_t st)
 {
     if (!direct_dft_supported(p.N) || p.nf < 1 || p.no < 1 || p.ni < 1) return cudaErrorInvalidValue;
     if (p.nf > (0x7fffffffLL / p.no) / p.ni) return cudaErrorInvalidValue;
-    const Shape s = shape_of(p.N);
     Args a;
     a.p = p;
-    a.tw = (const double2*)tw;
+    a.nu = (unsigned)(p.nf * p.no * p.ni);
+    int dev = 0, nsm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    const Shape s = shape_of(p.N, a.nu, nsm);
+    a.table = (const float4*)table;
     a.LT = s.LT;
     a.UB = s.UB;
-    a.nu = (unsigned)(p.nf * p.no * p.ni);
+    a.nsm = nsm;
     a.ntiles = (a.nu + s.LT - 1) / s.LT;
     const bool lc = p.i_e == 1, sc = p.o_e == 1;
     if (p.kind == DIRECT_REAL_IN && lc && !sc) return run<DIRECT_REAL_IN, true, false>(a, s, st);
@@ -368,7 +387,7 @@ cudaError_t launch_direct_dft(const DirectPass& p, const void* tw, cudaStream_t 
 }
 
 cudaError_t launch_direct_grid_pass(const void* in, void* out, long long nf, int N, int pass, bool real,
-                                    const void* tw, cudaStream_t st)
+                                    const void* table, cudaStream_t st)
 {
     const long long n = N, NN = n * n, NNN = NN * n;
     const int B = N / 2;
@@ -421,10 +440,10 @@ cudaError_t launch_direct_grid_pass(const void* in, void* out, long long nf, int
             break;
         default: return cudaErrorInvalidValue;
     }
-    return launch_direct_dft(p, tw, st);
+    return launch_direct_dft(p, table, st);
 }
 
-cudaError_t launch_direct_s2_pass(const void* in, void* out, long long nf, int N, int dir, bool real, const void* tw,
+cudaError_t launch_direct_s2_pass(const void* in, void* out, long long nf, int N, int dir, bool real, const void* table,
                                   cudaStream_t st)
 {
     const long long n = N, NN = n * n;
@@ -456,7 +475,7 @@ cudaError_t launch_direct_s2_pass(const void* in, void* out, long long nf, int N
             p.o_l = n;
         }
     }
-    return launch_direct_dft(p, tw, st);
+    return launch_direct_dft(p, table, st);
 }
 
 }  // namespace fftso3

@@ -7,11 +7,12 @@
 //   C[q] = sum_{t<=P/2} (a_t +/- a_{P-t}) cos,   S[q] = sum_{t<=P/2} (b_t -/+ b_{P-t}) sin:
 // N^2 / 2 FMAs a complex line (P / 2 a real one) whatever N's factors are, all of them independent register-tile work
 // with every operand in shared memory.  A mixed-radix Stockham FFT has fewer operations, but its stages each cross
-// shared memory and a barrier, and a prime factor R costs it R FMAs an element anyway.  Measured on one GB300
-// (DFT stages of both directions, l_max 96, 64 functions, N = 194): see direct_dft.cu.
+// shared memory and a barrier, and a prime factor R costs it R FMAs an element anyway.  Measured on one GB300 (all four
+// passes, 64 complex functions, N = 194): 38.9 ms with the separate transposes as a mixed-radix FFT, 18.5 ms here.
 //
-// Data are held as units of two floats that go through the same products (one packed FMA): the real and imaginary
-// part of a complex line, or the same element of two real lines.
+// A unit is a complex line, or two real lines x, y.  Its folded terms are held as the pairs (a.x, b.y), (a.y, b.x) (real
+// lines: (a.x, b.x), (a.y, b.y)) and the matrices as the pairs (cos, sin), so that one packed FMA advances a cosine sum
+// and a sine sum with no operand to duplicate, and the two halves of an accumulator are what the outputs add and subtract.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -24,12 +25,6 @@ __device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c)
 {
     u64 r;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ u64 dup2(float a)
-{
-    u64 r;
-    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
     return r;
 }
 __device__ __forceinline__ float2 unpack2(u64 a)
@@ -57,100 +52,82 @@ __host__ __device__ inline Fold fold_of(int N)
     f.QS = 4 * f.nbE;  // the odd q are never more than the even ones
     return f;
 }
-// the matrices [t][cos even, sin even, cos odd, sin odd][q index]
-__host__ __device__ inline int mat_floats(const Fold& f) { return 4 * f.H * f.QS; }
+// the matrices [t][parity of q][q index] as (cos, sin)
+__host__ __device__ inline int mat_elems(const Fold& f) { return 2 * f.H * f.QS; }
 
-// cos / sin of 2 pi t q / N from the plan's table W[i] = e^{-2 pi i i / N}, q = 2 i (even) or 2 i + 1; zero past P.
-__device__ __forceinline__ void build_mats(float* M, const Fold& f, const double2* __restrict__ tw)
+// Entry e of the matrices: (cos, sin) of 2 pi t q / N from the plan's table W[i] = e^{-2 pi i i / N}, q = 2 i (even) or
+// 2 i + 1; zero past P.
+__device__ __forceinline__ float2 mat_entry(const Fold& f, int e, const double2* __restrict__ tw)
 {
-    const int row = 2 * f.QS;
-    for (int e = threadIdx.x; e < f.H * row; e += blockDim.x) {
-        const int t = e / row, r = e - t * row, odd = r >= f.QS, i = r - odd * f.QS, q = 2 * i + odd;
-        float c = 0.f, s = 0.f;
-        if (q <= f.P) {
-            const double2 v = __ldg(tw + (t * q) % f.N);
-            c = (float)v.x;
-            s = (float)(-v.y);
-        }
-        float* m = M + (4 * t + 2 * odd) * f.QS + i;
-        m[0] = c;
-        m[f.QS] = s;
-    }
+    const int row = 2 * f.QS, t = e / row, r = e - t * row, odd = r >= f.QS, q = 2 * (r - odd * f.QS) + odd;
+    if (q > f.P) return make_float2(0.f, 0.f);
+    const double2 w = __ldg(tw + (t * q) % f.N);
+    return make_float2((float)w.x, (float)(-w.y));
 }
 
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
 
-// Folded values of t from x_t, x_{N-t}, x_{P-t}, x_{P+t} (t = 0: x_N counts as 0 and x_P once; t = P/2 for even P:
-// the two pairs coincide), in the order of the matrices: even-q cosine and sine terms, odd-q ones.
+// Folded terms of t from x_t, x_{N-t}, x_{P-t}, x_{P+t} (t = 0: x_N counts as 0 and x_P once; t = P/2 for even P: the
+// two pairs coincide), for the even and the odd q, as the pairs described above (REAL: of two real lines).
 struct Folded {
-    float2 v[4];
+    float4 even, odd;
 };
+template <bool REAL>
 __device__ __forceinline__ Folded fold_ab(int t, int P, float2 a, float2 b, float2 ap, float2 bp)
 {
     const float2 z = make_float2(0.f, 0.f);
+    const bool mid = 2 * t == P;
+    const float2 ae = mid ? a : add2(a, ap), be = mid ? z : sub2(b, bp);
+    const float2 ao = mid ? z : sub2(a, ap), bo = mid ? b : add2(b, bp);
     Folded r;
-    if (2 * t == P) {
-        r.v[0] = a;
-        r.v[1] = z;
-        r.v[2] = z;
-        r.v[3] = b;
-    } else {
-        r.v[0] = add2(a, ap);
-        r.v[1] = sub2(b, bp);
-        r.v[2] = sub2(a, ap);
-        r.v[3] = add2(b, bp);
-    }
+    r.even = REAL ? make_float4(ae.x, be.x, ae.y, be.y) : make_float4(ae.x, be.y, ae.y, be.x);
+    r.odd = REAL ? make_float4(ao.x, bo.x, ao.y, bo.y) : make_float4(ao.x, bo.y, ao.y, bo.x);
     return r;
 }
+template <bool REAL>
 __device__ __forceinline__ Folded fold_line(int t, int P, float2 x, float2 xn, float2 xp, float2 xq)
 {
     const float2 z = make_float2(0.f, 0.f);
-    if (t == 0) return fold_ab(t, P, x, z, xp, z);
-    return fold_ab(t, P, add2(x, xn), sub2(x, xn), add2(xp, xq), sub2(xp, xq));
+    if (t == 0) return fold_ab<REAL>(t, P, x, z, xp, z);
+    return fold_ab<REAL>(t, P, add2(x, xn), sub2(x, xn), add2(xp, xq), sub2(xp, xq));
 }
 
 // A thread's register tile: four outputs q of one parity of four units.  Lanes: QL blocks of outputs fastest, then 32 / QL
-// pairs of units; a thread's units are 2 ug, 2 ug + 1 and the same 64 / QL further on.  Adjacent lanes then read the same
-// units: a 16-byte shared-memory read costs max(2, distinct bytes / 128) cycles (measured: 2 for a warp-uniform one, 4 for 32
-// lanes side by side or for eight lanes' addresses repeated in each quarter warp), so a step t costs 12 cycles of the
-// shared-memory pipe for 32 packed FMAs, 48 against the 64 that four warps' FMAs take.
+// units.  Adjacent lanes then read the same units: a 16-byte shared-memory read costs max(2, distinct bytes / 128) cycles
+// (measured: 2 for a warp-uniform one, 4 for 32 lanes side by side or for eight lanes' addresses repeated in each quarter
+// warp), so a step t costs 12 cycles of the shared-memory pipe for 32 packed FMAs, 48 against the 64 that four warps' FMAs
+// take.
 struct Tile {
-    u64 C[4][4], S[4][4];
+    u64 A[4][4], B[4][4];  // [output][unit]: the accumulators of the unit's two pairs
 };
-// m: the block's cosines at t = 0 (sines QS further on, next t 4 QS); v: the thread's first unit of the parity's
-// cosine terms at t = 0 (sine terms US further on, next t TS).
+// m: the block's pairs at t = 0 (next t 2 QS further on); v: the thread's first unit of the parity at t = 0 (next t TS
+// further on), the others 32 / QL, HU, HU + 32 / QL further on.
 template <int QL>
-__device__ __forceinline__ void product(const float* m, const float2* v, int H, int QS, int US, int TS, Tile& a)
+__device__ __forceinline__ void product(const float2* m, const float4* v, int H, int QS, int HU, int TS, Tile& a)
 {
-    constexpr int UO = 64 / QL;
+    constexpr int G = 32 / QL;
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) a.C[i][j] = a.S[i][j] = 0;
-#pragma unroll 1
+        for (int j = 0; j < 4; ++j) a.A[i][j] = a.B[i][j] = 0;
+#pragma unroll 2
     for (int t = 0; t < H; ++t) {
-        const float4 c = *reinterpret_cast<const float4*>(m);
-        const float4 s = *reinterpret_cast<const float4*>(m + QS);
-        const ulonglong2 a0 = *reinterpret_cast<const ulonglong2*>(v);
-        const ulonglong2 a1 = *reinterpret_cast<const ulonglong2*>(v + UO);
-        const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(v + US);
-        const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(v + US + UO);
-        m += 4 * QS;
+        const ulonglong2 m0 = *reinterpret_cast<const ulonglong2*>(m);
+        const ulonglong2 m1 = *reinterpret_cast<const ulonglong2*>(m + 2);
+        const u64 c[4] = {m0.x, m0.y, m1.x, m1.y};
+        const ulonglong2 x[4] = {
+            *reinterpret_cast<const ulonglong2*>(v), *reinterpret_cast<const ulonglong2*>(v + HU),
+            *reinterpret_cast<const ulonglong2*>(v + G), *reinterpret_cast<const ulonglong2*>(v + HU + G)};
+        m += 2 * QS;
         v += TS;
-        const u64 cd[4] = {dup2(c.x), dup2(c.y), dup2(c.z), dup2(c.w)};
-        const u64 sd[4] = {dup2(s.x), dup2(s.y), dup2(s.z), dup2(s.w)};
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            a.C[i][0] = fma2(cd[i], a0.x, a.C[i][0]);
-            a.C[i][1] = fma2(cd[i], a0.y, a.C[i][1]);
-            a.C[i][2] = fma2(cd[i], a1.x, a.C[i][2]);
-            a.C[i][3] = fma2(cd[i], a1.y, a.C[i][3]);
-            a.S[i][0] = fma2(sd[i], b0.x, a.S[i][0]);
-            a.S[i][1] = fma2(sd[i], b0.y, a.S[i][1]);
-            a.S[i][2] = fma2(sd[i], b1.x, a.S[i][2]);
-            a.S[i][3] = fma2(sd[i], b1.y, a.S[i][3]);
-        }
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                a.A[i][j] = fma2(c[i], x[j].x, a.A[i][j]);
+                a.B[i][j] = fma2(c[i], x[j].y, a.B[i][j]);
+            }
     }
 }
 
@@ -180,15 +157,19 @@ struct DirectPass {
 };
 // Even N whose matrices and one tile fit a CTA's shared memory (N <= 400 or so).
 bool direct_dft_supported(int N);
-cudaError_t launch_direct_dft(const DirectPass& p, const void* tw, cudaStream_t st);
+// The matrices of length N in device memory, made once per plan from its twiddle table tw (N double2): built by every CTA
+// of every pass, the FP64 loads and conversions took 10 to 25 us of small passes.
+size_t direct_dft_table_bytes(int N);
+cudaError_t direct_dft_build_table(void* table, int N, const void* tw, cudaStream_t st);
+cudaError_t launch_direct_dft(const DirectPass& p, const void* table, cudaStream_t st);
 // The passes of the SO(3) grid transforms over nf grids of N^3, as launch_fft_grid_pass but with its own layout of
 // the work grid: pass 1 grid [nf][k][j1][j2] -> work [nf][k][q][j1]; 2 work -> pencils [nf][p][q][k]; -2 pencils ->
 // work [nf][j1][q][k]; -1 work -> grid.  real: real samples in / real part out; the work grid then holds q <= N/2
 // only.  The inverse passes take the Nyquist bins p = N/2, q = N/2 as zero without reading them.
 cudaError_t launch_direct_grid_pass(const void* in, void* out, long long nf, int N, int pass, bool real,
-                                    const void* tw, cudaStream_t st);
+                                    const void* table, cudaStream_t st);
 // ... and of nf S^2 grids of N^2: dir 1 grid [nf][k][j] -> pencils [nf][p][k], dir -1 pencils -> grid (bin N/2 zero).
-cudaError_t launch_direct_s2_pass(const void* in, void* out, long long nf, int N, int dir, bool real, const void* tw,
+cudaError_t launch_direct_s2_pass(const void* in, void* out, long long nf, int N, int dir, bool real, const void* table,
                                   cudaStream_t st);
 
 }  // namespace fftso3
