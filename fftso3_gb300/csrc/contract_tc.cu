@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     const uint32_t tmem = *tmem_slot;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---------------- TMA producer of the table tiles
             // The ring holds only STAGES k-steps, so each step's tiles are also
             // prefetched into L2 PF steps ahead (across item boundaries): the
@@ -394,7 +394,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                     mbar_wait(&full[k % STAGES], (k / STAGES) & 1, args.err, 7);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---------------- MMA issuer
             constexpr uint32_t idesc = idesc_bf16(!FWD);
             constexpr uint32_t idesc256 = idesc_bf16(!FWD, 2 * BN);

@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     const uint32_t tmem = *tmem_slot;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---------------- TMA producer: the table digit planes and the coefficients' digit image
             const CUtensorMap* tm[NS] = {&t0, &t1, &t2, &t3};
             int kc = 0;
@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---------------- MMA issuer: A_j x [B_0 .. B_{3-j}] -> levels j..3
             uint32_t idesc[NS];
 #pragma unroll
