@@ -442,6 +442,7 @@ int fftso3_batch_create(fftso3_batch** out, int kind, const int* l_max, int n_fu
             rc = tc_fused_phases(b->fused, g0, c0, err);
             if (rc == FFTSO3_SUCCESS) {
                 b->phases = true;
+                b->bytes += tc_fused_device_bytes(b->fused);
                 b->tuned = true;
                 b->nstreams_used = 1;
             } else if (rc == FFTSO3_ERR_UNSUPPORTED) {

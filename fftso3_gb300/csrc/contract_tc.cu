@@ -2198,6 +2198,10 @@ int tc_inverse_fft(TCState* s, void* grid, cudaStream_t st, StageTimer* T, std::
     return fft_inverse(s, grid, st, T, err);
 }
 
+// Samples from which a batch's DFT passes run on the tensor cores (both directions, complex / real, us, slice FFT -> tensor
+// cores: 0.9 M samples 177 / 163 -> 187 / 172, 5.4 M 472 / 397 -> 404 / 315, 82 M 9297 / 5708 -> 4417 / 3883).
+constexpr long long DFT_BATCH_SAMPLES = 2000000;
+
 struct TCFused {
     std::vector<TCState*> parts;
     GemmSeg* d_segs[2] = {nullptr, nullptr};  // forward, inverse
@@ -2216,6 +2220,11 @@ struct TCFused {
     size_t slice_smem = 0;
     bool real = false;
     bool slice_wide = false;  // 512-thread slice FFT CTAs (FFTSO3_SLICE_WIDE=1)
+    // large batches: the DFT passes on the tensor cores in place of the slice FFT, with their matrices and work grids
+    DftTcBatch dft;
+    unsigned char* d_dft = nullptr;
+    float2* d_dwork = nullptr;
+    long long bytes = 0;
 };
 
 void tc_fused_destroy(TCFused* f)
@@ -2223,6 +2232,9 @@ void tc_fused_destroy(TCFused* f)
     if (!f) return;
     if (f->d_bseg) cudaFree(f->d_bseg);
     if (f->d_cseg) cudaFree(f->d_cseg);
+    dft_tc_batch_destroy(f->dft);
+    if (f->d_dft) cudaFree(f->d_dft);
+    if (f->d_dwork) cudaFree(f->d_dwork);
     for (int d = 0; d < 2; ++d) {
         if (f->d_segs[d]) cudaFree(f->d_segs[d]);
         if (f->d_items[d]) cudaFree(f->d_items[d]);
@@ -2425,6 +2437,56 @@ int tc_fused_phases(TCFused* f, const std::vector<long long>& g0, const std::vec
         err = std::string("fused phases: ") + cudaGetErrorString(e);
         return FFTSO3_ERR_CUDA;
     }
+    // the DFT on the tensor cores
+    long long samples = 0;
+    size_t tab = 0, work = 0;
+    bool dft = true;
+    for (TCState* p : f->parts) {
+        samples += (long long)p->batch * p->N * p->N * p->N;
+        tab += (dft_tc_table_bytes(p->N) + 255) & ~(size_t)255;
+        if (!p->d_work) work += (size_t)p->batch * p->N * p->N * p->N;
+        dft = dft && dft_tc_batch_supported(p->N);
+    }
+    auto drop_dft = [&] {
+        dft_tc_batch_destroy(f->dft);
+        if (f->d_dft) cudaFree(f->d_dft);
+        if (f->d_dwork) cudaFree(f->d_dwork);
+        f->d_dft = nullptr;
+        f->d_dwork = nullptr;
+        f->bytes = 0;
+    };
+    drop_dft();
+    if (dft && samples >= DFT_BATCH_SAMPLES) {
+        // (no memory for the work grids: the slice FFT, which needs none)
+        e = cudaMalloc(&f->d_dft, tab);
+        if (e == cudaSuccess && work) e = cudaMalloc(&f->d_dwork, sizeof(float2) * work);
+        std::vector<DftTcBucket> buckets;
+        size_t to = 0, wo = 0;
+        for (size_t j = n; j-- > 0 && e == cudaSuccess;) {  // ascending N
+            const int i = ord[j];
+            TCState* p = f->parts[i];
+            unsigned char* t = f->d_dft + to;
+            to += (dft_tc_table_bytes(p->N) + 255) & ~(size_t)255;
+            e = dft_tc_build_table(t, p->N, p->d_tw, 0);
+            float2* w = p->d_work;
+            if (!w) {
+                w = f->d_dwork + wo;
+                wo += (size_t)p->batch * p->N * p->N * p->N;
+            }
+            buckets.push_back({p->N, p->batch, p->d_pencil, w, t, g0[i]});
+        }
+        if (e == cudaSuccess) e = dft_tc_batch_create(f->dft, buckets, real);
+        if (e == cudaSuccess) e = cudaDeviceSynchronize();
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            drop_dft();
+        } else if (e != cudaSuccess) {
+            err = std::string("fused phases: ") + cudaGetErrorString(e);
+            return FFTSO3_ERR_CUDA;
+        } else {
+            f->bytes = (long long)(tab + sizeof(float2) * work);
+        }
+    }
     f->nbseg = (int)segs.size();
     f->nblk = blk;
     f->ncblk = cblk;
@@ -2441,7 +2503,10 @@ int tc_fused_forward(TCFused* f, const void* grid, void* coeffs, cudaStream_t st
         return FFTSO3_ERR_CUDA;
     }
     T->begin(ST_FFT_SLICES, st);
-    TCK(launch_slice_fft(f->d_bseg, f->nbseg, f->nblk, f->slice_smem, true, f->real, f->slice_wide, grid, nullptr, st));
+    if (f->dft.segs)
+        TCK(launch_dft_tc_batch(f->dft, true, grid, nullptr, f->d_err, st));
+    else
+        TCK(launch_slice_fft(f->d_bseg, f->nbseg, f->nblk, f->slice_smem, true, f->real, f->slice_wide, grid, nullptr, st));
     T->end(st);
     int rc = tc_fused_gemm(f, true, st, T, err);
     if (rc) return rc;
@@ -2463,10 +2528,15 @@ int tc_fused_inverse(TCFused* f, const void* coeffs, void* grid, cudaStream_t st
     int rc = tc_fused_gemm(f, false, st, T, err);
     if (rc) return rc;
     T->begin(ST_FFT_SLICES, st);
-    TCK(launch_slice_fft(f->d_bseg, f->nbseg, f->nblk, f->slice_smem, false, f->real, f->slice_wide, nullptr, grid, st));
+    if (f->dft.segs)
+        TCK(launch_dft_tc_batch(f->dft, false, nullptr, grid, f->d_err, st));
+    else
+        TCK(launch_slice_fft(f->d_bseg, f->nbseg, f->nblk, f->slice_smem, false, f->real, f->slice_wide, nullptr, grid, st));
     T->end(st);
     return FFTSO3_SUCCESS;
 }
+
+long long tc_fused_device_bytes(const TCFused* f) { return f ? f->bytes : 0; }
 
 int tc_fused_status(TCFused* f)
 {

@@ -59,6 +59,7 @@ int tc_fused_create(TCFused** out, const std::vector<TCState*>& parts, std::stri
 void tc_fused_destroy(TCFused* f);
 int tc_fused_gemm(TCFused* f, bool fwd, cudaStream_t st, StageTimer* T, std::string& err);
 int tc_fused_status(TCFused* f);
+long long tc_fused_device_bytes(const TCFused* f);  // beyond the plans': the tensor-core DFT's matrices and work grids
 // Three launches per direction over SO(3) plans of one kind without refinement (fused.cuh): slice FFT, GEMM,
 // conversion (forward) and the mirror image (inverse).  Plan i's functions sit at element offsets g0[i] / c0[i]
 // of the caller's grids / coefficients.  FFTSO3_ERR_UNSUPPORTED when one beta slice of the largest N does not

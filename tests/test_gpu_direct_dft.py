@@ -68,3 +68,38 @@ def test_s2(gblib, L, batch, real):
 @pytest.mark.parametrize("real", [False, True])
 def test_fp32_precision(gblib, real):
     _round_trip(gblib, 1 if real else 0, real, 21, 7, "fp32", np.tile(so3_coeffs(21, 3, not real), 7))
+
+
+@pytest.mark.parametrize("real", [False, True])
+def test_uneven_batch(gblib, real):
+    """Both passes of every bucket in one launch (two million samples or more): the smallest N, powers of two (whose plans
+    keep no work grid), primes and the largest N of the one-launch form; two calls on different buffers, from graphs."""
+    import torch
+
+    ls = [1, 2, 7, 15, 16, 31, 31, 36, 39, 47, 52, 63] + ([70, 105] if real else [77])
+    kind = 1 if real else 0
+    dt, dt32 = (torch.float64, torch.float32) if real else (torch.complex128, torch.complex64)
+    b = gblib.Batch(kind, ls, "tc_bf16x3", "stable", gblib.FLAG_GRAPH)
+    assert b.grid_elems >= 2000000
+    s = torch.cuda.current_stream().cuda_stream
+    for call in range(2):
+        F = torch.empty(b.coeff_elems, dtype=dt32, device="cuda")
+        for i, L in enumerate(ls):
+            c = torch.from_numpy(so3_coeffs(L, 11 + i + 50 * call, not real)).to(dt32).cuda()
+            F[b.coeff_offset(i):b.coeff_offset(i) + c.numel()] = c
+        g, F2 = torch.empty(b.grid_elems, dtype=dt32, device="cuda"), torch.empty_like(F)
+        b.inverse(F.data_ptr(), g.data_ptr(), s)
+        f = g + 0.1 * g.abs().mean() * torch.randn(g.shape, dtype=dt32, device="cuda")
+        b.forward(f.data_ptr(), F2.data_ptr(), s)
+        b.check()
+        assert b.graph_kernels(0) == 3 and b.graph_kernels(1) == 3
+        for i, L in enumerate(ls):
+            p = gblib.Plan(kind, L, 1, "fp64", "stable")
+            cs, gs = slice(b.coeff_offset(i), b.coeff_offset(i) + p.coeff_elems), slice(b.grid_offset(i), b.grid_offset(i) + p.grid_elems)
+            g64, c64 = torch.empty(p.grid_elems, dtype=dt, device="cuda"), torch.empty(p.coeff_elems, dtype=dt, device="cuda")
+            F64, f64 = F[cs].to(dt), f[gs].to(dt)
+            p.inverse(F64.data_ptr(), g64.data_ptr(), s)
+            p.forward(f64.data_ptr(), c64.data_ptr(), s)
+            torch.cuda.synchronize()
+            for got, ref in ((g[gs], g64), (F2[cs], c64)):
+                assert torch.linalg.vector_norm(got.to(dt) - ref) <= TOL * torch.linalg.vector_norm(ref), (call, L)
