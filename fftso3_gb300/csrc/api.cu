@@ -1045,7 +1045,7 @@ int fftso3_inverse_points(fftso3_plan* plan, const void* coeffs, int index, cons
         e = cudaMemcpyAsync(d_seed, seeds.data(), sizeof(WignerSeeds) * n, cudaMemcpyHostToDevice, st);
         if (e == cudaSuccess)
             e = launch_so3_points(Fc, (const WignerSeeds*)d_seed, d_pts, (const double4*)plan->d_prec, plan->d_psq,
-                                  plan->d_lfact, L, plan->recursion == FFTSO3_RECURSION_STABLE, n, m0b, S, d_part,
+                                  plan->d_lfact, L, plan->recursion == FFTSO3_RECURSION_STABLE, plan->real, n, m0b, S, d_part,
                                   d_out, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // seeds vector must outlive the copy
     } else {
@@ -1053,7 +1053,7 @@ int fftso3_inverse_points(fftso3_plan* plan, const void* coeffs, int index, cons
         for (int i = 0; i < n; ++i) xs[i] = cos(pts[2 * i]);
         e = cudaMemcpyAsync(d_seed, xs.data(), sizeof(double) * n, cudaMemcpyHostToDevice, st);
         if (e == cudaSuccess)
-            e = launch_s2_points(Fc, (const double*)d_seed, d_pts, (const double2*)plan->d_prec, L, n, m0b, S, d_part,
+            e = launch_s2_points(Fc, (const double*)d_seed, d_pts, (const double2*)plan->d_prec, L, plan->real, n, m0b, S, d_part,
                                  d_out, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     }

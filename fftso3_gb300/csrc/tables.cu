@@ -93,21 +93,26 @@ __device__ __forceinline__ double2 block_sum(double2 v)
 // operations on the O(B^3) core only:
 //   * one warp evaluates 32 points (lane = point): the loops over (m0, n0, l) are the same for every
 //     point, so each coefficient load is one broadcast per warp and no lane waits on another;
-//   * the beta-independent factors of the recursion (64) come from a per-plan table (below), so a
-//     recursion step is five multiplies / subtractions instead of two square roots and two divisions;
+//   * the beta-independent factors of the recursion (64), with the sum's factor 2l+1 folded in, come from a
+//     per-plan table (below), so a recursion step is one multiplication and two FMAs instead of two square
+//     roots and two divisions; with the eight FMAs of four complex pairs a degree costs 11 FP64 operations
+//     (15 with the reference's operation order and the factor applied apart: 2048 points at l_max 127, stable
+//     recursion: 63 ms, now 33 ms, the FP64 units at their measured 0.49 T FMA/s);
+//   * real functions take one pair of each two, F(l,-m,-n) being the conjugate up to sign (7 operations);
 //   * the seeds (65)-(68) of all groups of one m0 are the prefixes of one chain over n0 (the
 //     reference's loops over n run from m0 - 1 down to n0), so they cost O(B^2) per point, not O(B^3);
 //   * e^{-i m0 alpha} comes from sincos once per m0, e^{-i n0 alpha} by one complex step per group.
-// The Wigner-d values are the same doubles as the table kernel's (same operations, this unit's
-// -fmad=false), so a reference-recursion plan keeps the reference's underflow near beta = pi.
+// The seeds are the table kernel's doubles, so a reference-recursion plan keeps the reference's underflow near
+// beta = pi; the recursion's values agree with the table's to rounding (explicit FMAs; this unit is -fmad=false).
 // The degrees m0 split into parts of equal work (blockIdx.y) whose partial sums are added in a fixed
 // order by a second kernel.
 
-// beta-independent factors of (64) per (group, l), l = m0 + 1..L, as {a, c, P2, P1}:
-//   a = 1/sqrt((l^2-m^2)(l^2-n^2)),  c = sqrt(((l-1)^2-m^2)((l-1)^2-n^2)) l/(l-1),
-//   P2 = (2l-1) m n/(l-1),  P1 = l(2l-1),  d^l = a ((P1 cos(beta) - P2) d^{l-1} - c d^{l-2}),
-// with the expressions of rec64_faithful and of the stable column (so the same doubles); row (0, 1)
-// is unused (d^1_00 = cos(beta)) and zero.  Group (m0, n0) starts at rec_row0(m0) + (n0 + m0)(L - m0).
+// beta-independent factors of (64) per (group, l), l = m0 + 1..L, as {A, B, C, -}, for the scaled values
+// u^l = (2l+1) d^l that the sums use:
+//   u^l = (A cos(beta) - B) u^{l-1} - C u^{l-2}:  one multiplication and two FMAs,
+//   A = a l(2l-1) s1, B = a s1 (2l-1) m n/(l-1), C = a s2 sqrt(((l-1)^2-m^2)((l-1)^2-n^2)) l/(l-1),
+//   a = 1/sqrt((l^2-m^2)(l^2-n^2)), s1 = (2l+1)/(2l-1), s2 = (2l+1)/(2l-3);
+// row (0, 1) is A = 3 (u^1_00 = 3 cos(beta)).  Group (m0, n0) starts at rec_row0(m0) + (n0 + m0)(L - m0).
 // sq[l (l - 1) + n + l] = sqrt(((l + n) + 1) / (l - n)), 1 <= l <= L + 1, -l <= n < l: the seed factors.
 __host__ __device__ inline long long rec_row0(int m0, int L)
 {
@@ -130,13 +135,13 @@ __global__ void wigner_rec_factors_kernel(double4* __restrict__ rec, double* __r
         double4* row = rec + rec_row0(m0, L) + (long long)(n0 + m0) * (L - m0);
         const double mm = (double)m0 * (double)m0, nn = (double)n0 * (double)n0;
         for (int l = m0 + 1; l <= L; ++l) {
-            double4 f = make_double4(0., 0., 0., 0.);
+            double4 f = make_double4(3., 0., 0., 0.);
             if (l >= 2) {
-                const double ll = (double)l * (double)l, lm1 = (double)l - 1.;
-                f.x = 1. / sqrt((ll - mm) * (ll - nn));
-                f.y = sqrt(fmax((lm1 * lm1 - mm) * (lm1 * lm1 - nn), 0.0)) * (double)l / lm1;
-                f.z = (2. * (double)l - 1.) * (double)m0 * (double)n0 / lm1;
-                f.w = (double)l * (2. * (double)l - 1.);
+                const double ll = (double)l * (double)l, lm1 = (double)l - 1., w = 2. * (double)l + 1.;
+                const double aw = w / sqrt((ll - mm) * (ll - nn));
+                f.x = aw * (double)l;
+                f.y = aw * (double)m0 * (double)n0 / lm1;
+                f.z = aw / (2. * (double)l - 3.) * sqrt(fmax((lm1 * lm1 - mm) * (lm1 * lm1 - nn), 0.0)) * (double)l / lm1;
             }
             row[l - m0 - 1] = f;
         }
@@ -158,11 +163,10 @@ struct PointParts {
 
 constexpr int PW = 4;  // warps (batches of 32 points) per CTA
 
-__device__ __forceinline__ double4 ld_rec(const double4* p)
+__device__ __forceinline__ double3 ld_rec(const double4* p)
 {
-    const double2* q = reinterpret_cast<const double2*>(p);
-    const double2 a = __ldg(q), b = __ldg(q + 1);
-    return make_double4(a.x, a.y, b.x, b.y);
+    const double2 a = __ldg(reinterpret_cast<const double2*>(p));
+    return make_double3(a.x, a.y, __ldg(reinterpret_cast<const double*>(p) + 2));
 }
 
 __device__ __forceinline__ double2 cmul2(double2 a, double2 b)
@@ -170,7 +174,7 @@ __device__ __forceinline__ double2 cmul2(double2 a, double2 b)
     return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 
-template <bool STABLE>
+template <bool STABLE, bool REAL>
 __global__ void __launch_bounds__(32 * PW) so3_points_kernel(const double2* __restrict__ F,
                                                              const WignerSeeds* __restrict__ pseeds,
                                                              const double* __restrict__ pts,
@@ -179,9 +183,6 @@ __global__ void __launch_bounds__(32 * PW) so3_points_kernel(const double2* __re
                                                              const double* __restrict__ lfact, int L, int n,
                                                              const PointParts parts, double2* __restrict__ part)
 {
-    extern __shared__ double wl[];  // wl[l] = 2l + 1
-    for (int l = threadIdx.x; l <= L; l += blockDim.x) wl[l] = (double)(2 * l + 1);
-    __syncthreads();
     const int lane = threadIdx.x & 31;
     const int b = blockIdx.x * PW + (threadIdx.x >> 5);
     if (b * 32 >= n) return;
@@ -203,21 +204,15 @@ __global__ void __launch_bounds__(32 * PW) so3_points_kernel(const double2* __re
         if (m0 == 0) {
             // group (0, 0), both modes: d^0 = 1, d^1 = cos(beta), then (64)
             double2 D = __ldg(&F[0]);
-            if (L >= 1) {
-                const double2 c = __ldg(&F[so3_idx(1, 0, 0)]);
-                D.x = __fma_rn(c.x, wl[1] * cb, D.x);
-                D.y = __fma_rn(c.y, wl[1] * cb, D.y);
-            }
-            double d2 = 1., d1 = cb;
-            for (int l = 2; l <= L; ++l) {
-                const double4 f = ld_rec(&rec[row0 + (l - 1)]);
-                const double v = f.x * ((f.w * cb - f.z) * d1 - f.y * d2);
-                const double wv = wl[l] * v;
+            double u2 = 0., u1 = 1.;
+            for (int l = 1; l <= L; ++l) {
+                const double3 f = ld_rec(&rec[row0 + (l - 1)]);
+                const double u = __fma_rn(__fma_rn(f.x, cb, -f.y), u1, -(f.z * u2));
                 const double2 c = __ldg(&F[so3_idx(l, 0, 0)]);
-                D.x = __fma_rn(c.x, wv, D.x);
-                D.y = __fma_rn(c.y, wv, D.y);
-                d2 = d1;
-                d1 = v;
+                D.x = __fma_rn(c.x, u, D.x);
+                D.y = __fma_rn(c.y, u, D.y);
+                u2 = u1;
+                u1 = u;
             }
             acc.x += D.x;
             acc.y += D.y;
@@ -248,23 +243,27 @@ __global__ void __launch_bounds__(32 * PW) so3_points_kernel(const double2* __re
             }
             const bool four = n0 != m0 && n0 != -m0;
             double2 D0 = make_double2(0., 0.), D1 = D0, D2 = D0, D3 = D0;
-            auto emit = [&](int l, double v) {
-                const double wv = wl[l] * v;
+            // u = (2l+1) d^l
+            auto emit = [&](int l, double u) {
                 const long long o = so3_off(l);
                 const long long w = 2 * l + 1;
                 const double2 c0 = __ldg(&F[o + (m0 + l) + (n0 + l) * w]);
-                const double2 c1 = __ldg(&F[o + (l - m0) + (l - n0) * w]);
-                D0.x = __fma_rn(c0.x, wv, D0.x);
-                D0.y = __fma_rn(c0.y, wv, D0.y);
-                D1.x = __fma_rn(c1.x, wv, D1.x);
-                D1.y = __fma_rn(c1.y, wv, D1.y);
+                D0.x = __fma_rn(c0.x, u, D0.x);
+                D0.y = __fma_rn(c0.y, u, D0.y);
+                if (!REAL) {
+                    const double2 c1 = __ldg(&F[o + (l - m0) + (l - n0) * w]);
+                    D1.x = __fma_rn(c1.x, u, D1.x);
+                    D1.y = __fma_rn(c1.y, u, D1.y);
+                }
                 if (four) {
                     const double2 c2 = __ldg(&F[o + (n0 + l) + (m0 + l) * w]);
-                    const double2 c3 = __ldg(&F[o + (l - n0) + (l - m0) * w]);
-                    D2.x = __fma_rn(c2.x, wv, D2.x);
-                    D2.y = __fma_rn(c2.y, wv, D2.y);
-                    D3.x = __fma_rn(c3.x, wv, D3.x);
-                    D3.y = __fma_rn(c3.y, wv, D3.y);
+                    D2.x = __fma_rn(c2.x, u, D2.x);
+                    D2.y = __fma_rn(c2.y, u, D2.y);
+                    if (!REAL) {
+                        const double2 c3 = __ldg(&F[o + (l - n0) + (l - m0) * w]);
+                        D3.x = __fma_rn(c3.x, u, D3.x);
+                        D3.y = __fma_rn(c3.y, u, D3.y);
+                    }
                 }
             };
             if (STABLE) {
@@ -287,39 +286,47 @@ __global__ void __launch_bounds__(32 * PW) so3_points_kernel(const double2* __re
                         d1 = sgn * exp2(e2 - (double)E);
                     }
                 }
-                double d2 = 0.;
-                emit(m0, (E == 0) ? d1 : ldexp(d1, E));
+                double u2 = 0., u1 = (double)(2 * m0 + 1) * d1;
+                emit(m0, (E == 0) ? u1 : ldexp(u1, E));
                 for (int l = l1; l <= L; ++l) {
-                    const double4 f = ld_rec(&rec[grow + (l - l1)]);
-                    const double v = f.x * ((f.w * cb - f.z) * d1 - f.y * d2);
-                    d2 = d1;
-                    d1 = v;
-                    if (E < 0 && fabs(d1) > 0x1p600) {
-                        d1 = ldexp(d1, -600);
-                        d2 = ldexp(d2, -600);
+                    const double3 f = ld_rec(&rec[grow + (l - l1)]);
+                    const double u = __fma_rn(__fma_rn(f.x, cb, -f.y), u1, -(f.z * u2));
+                    u2 = u1;
+                    u1 = u;
+                    if (E < 0 && fabs(u1) > 0x1p600) {
+                        u1 = ldexp(u1, -600);
+                        u2 = ldexp(u2, -600);
                         E += 600;
                     }
-                    emit(l, (E == 0) ? d1 : ldexp(d1, E));
+                    emit(l, (E == 0) ? u1 : ldexp(u1, E));
                 }
             } else {
                 const double v0g = m0 == 1 ? (n0 == 1 ? s.d111 : (n0 == 0 ? s.d110 : s.d11m1)) : v0;
-                emit(m0, v0g);
+                double u2 = (double)(2 * m0 + 1) * v0g;
+                emit(m0, u2);
                 if (l1 <= L) {
-                    emit(l1, v1);
-                    double d2 = v0g, d1 = v1;
+                    double u1 = (double)(2 * l1 + 1) * v1;
+                    emit(l1, u1);
                     for (int l = l1 + 1; l <= L; ++l) {
-                        const double4 f = ld_rec(&rec[grow + (l - l1)]);
-                        const double v = f.x * ((f.w * cb - f.z) * d1 - f.y * d2);
-                        emit(l, v);
-                        d2 = d1;
-                        d1 = v;
+                        const double3 f = ld_rec(&rec[grow + (l - l1)]);
+                        const double u = __fma_rn(__fma_rn(f.x, cb, -f.y), u1, -(f.z * u2));
+                        emit(l, u);
+                        u2 = u1;
+                        u1 = u;
                     }
                 }
             }
             // p0 (m0, n0), p1 (-m0, -n0) sign (-1)^(m0+n0), p2 (n0, m0) same sign, p3 (-n0, -m0)
             const double sg = ((m0 + n0) & 1) ? -1. : 1.;
             const double2 ph0 = cmul2(Ema, Eng);
-            const double2 t0 = cmul2(D0, ph0), t1 = cmul2(D1, make_double2(ph0.x, -ph0.y));
+            const double2 t0 = cmul2(D0, ph0);
+            if (REAL) {
+                // p1 and p3 are the conjugates of p0 and p2 (the function's value is real; its imaginary part is not formed)
+                acc.x += 2. * t0.x;
+                if (four) acc.x += 2. * sg * cmul2(D2, cmul2(Ena, Emg)).x;
+                continue;
+            }
+            const double2 t1 = cmul2(D1, make_double2(ph0.x, -ph0.y));
             acc.x += t0.x + sg * t1.x;
             acc.y += t0.y + sg * t1.y;
             if (four) {
@@ -348,11 +355,12 @@ __global__ void sum_parts_kernel(const double2* __restrict__ part, int S, int n,
 }
 
 // Degree parts of about equal work ((2 m0 + 1)(L - m0 + 2) per m0 for SO(3), L - m + 2 per order m for
-// S^2), enough of them that the launch has about 16 warps per SM; returns their number S, bounds in m0b[0..S].
+// S^2), enough of them that the launch has about 64 warps per SM (the parts of one launch
+// then end within a few percent of each other); returns their number S, bounds in m0b[0..S].
 int points_parts(bool so3, int L, int n, int nsm, int* m0b)
 {
     const long long nb = ((long long)n + 31) / 32;
-    long long S = (16LL * std::max(nsm, 1) + nb - 1) / nb;
+    long long S = (64LL * std::max(nsm, 1) + nb - 1) / nb;
     S = std::max(1LL, std::min<long long>({S, (long long)MAX_POINT_PARTS, (long long)L + 1}));
     auto work = [&](int m) { return (so3 ? 2.0 * m + 1.0 : 1.0) * (L - m + 2); };
     double total = 0.;
@@ -369,19 +377,17 @@ int points_parts(bool so3, int L, int n, int nsm, int* m0b)
 }
 
 cudaError_t launch_so3_points(const double2* F, const WignerSeeds* pseeds, const double* pts, const double4* rec,
-                              const double* sq, const double* lfact, int L, bool stable, int n, const int* m0b,
-                              int S, double2* part, double2* out, cudaStream_t st)
+                              const double* sq, const double* lfact, int L, bool stable, bool real, int n,
+                              const int* m0b, int S, double2* part, double2* out, cudaStream_t st)
 {
     if (S < 1 || S > MAX_POINT_PARTS) return cudaErrorInvalidValue;
     PointParts P;
     for (int s = 0; s <= S; ++s) P.m0[s] = m0b[s];
     const long long nb = ((long long)n + 31) / 32;
     const dim3 grid((unsigned)((nb + PW - 1) / PW), (unsigned)S);
-    const size_t smem = sizeof(double) * (size_t)(L + 1);
-    if (stable)
-        so3_points_kernel<true><<<grid, 32 * PW, smem, st>>>(F, pseeds, pts, rec, sq, lfact, L, n, P, part);
-    else
-        so3_points_kernel<false><<<grid, 32 * PW, smem, st>>>(F, pseeds, pts, rec, sq, lfact, L, n, P, part);
+    auto kern = stable ? (real ? so3_points_kernel<true, true> : so3_points_kernel<true, false>)
+                       : (real ? so3_points_kernel<false, true> : so3_points_kernel<false, false>);
+    kern<<<grid, 32 * PW, 0, st>>>(F, pseeds, pts, rec, sq, lfact, L, n, P, part);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     sum_parts_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(part, S, n, out);
@@ -393,9 +399,9 @@ cudaError_t launch_so3_points(const double2* F, const WignerSeeds* pseeds, const
 // y(theta,phi) = sum_{l,m} F(l,m) nP(l,m)(cos theta) e^{i m phi} (fdcl_FFTS2.cpp:17-46, :194-230), in the
 // layout of the SO(3) point kernel: one warp per 32 points, the orders m split into parts of equal work.
 // The Legendre recursion of fdcl_FFTS2.cpp:48-100 runs with its beta-independent factors from a per-plan
-// table: step l uses fact(l, m) = sqrt((4l^2 - 1)/(l^2 - m^2)) and 1/fact(l - 1, m) (the reference
+// table: step l uses fact(l, m) = sqrt((4l^2 - 1)/(l^2 - m^2)) and fact(l, m)/fact(l - 1, m) (the reference
 // divides by fact(l - 1, m), so values agree with it to rounding, not bit for bit); the seed pmm(m) keeps
-// the reference's operations, chained over m.  Table: per m, rows l = m + 2..L of {fact, 1/previous
+// the reference's operations, chained over m.  Table: per m, rows l = m + 2..L of {fact, fact/previous
 // fact}, starting at s2_row0(m) (the first previous fact is sqrt(2m + 3)).
 __host__ __device__ inline long long s2_row0(int m, int L)
 {
@@ -413,7 +419,7 @@ __global__ void legendre_rec_factors_kernel(double2* __restrict__ rec, int L)
     double oldfact = sqrt(2.0 * (double)m + 3.0);
     for (int l = m + 2; l <= L; ++l) {
         const double fact = sqrt((4.0 * (double)l * (double)l - 1.0) / (double)(l * l - m * m));
-        row[l - m - 2] = make_double2(fact, 1.0 / oldfact);
+        row[l - m - 2] = make_double2(fact, fact / oldfact);
         oldfact = fact;
     }
 }
@@ -424,6 +430,7 @@ cudaError_t launch_legendre_rec_factors(double2* rec, int L, cudaStream_t st)
     return cudaGetLastError();
 }
 
+template <bool REAL>
 __global__ void __launch_bounds__(32 * PW) s2_points_kernel(const double2* __restrict__ F, const double* __restrict__ xs,
                                                             const double* __restrict__ pts,
                                                             const double2* __restrict__ rec, int L, int n,
@@ -461,7 +468,7 @@ __global__ void __launch_bounds__(32 * PW) s2_points_kernel(const double2* __res
             const double2 a = __ldg(&F[s2_idx(l, m)]);
             Dp.x = __fma_rn(a.x, v, Dp.x);
             Dp.y = __fma_rn(a.y, v, Dp.y);
-            if (m > 0) {
+            if (!REAL && m > 0) {
                 const double2 c = __ldg(&F[s2_idx(l, -m)]);
                 Dn.x = __fma_rn(c.x, v, Dn.x);
                 Dn.y = __fma_rn(c.y, v, Dn.y);
@@ -473,7 +480,7 @@ __global__ void __launch_bounds__(32 * PW) s2_points_kernel(const double2* __res
             emit(m + 1, p1);
             for (int l = m + 2; l <= L; ++l) {
                 const double2 f = __ldg(&rec[row + (l - m - 2)]);
-                const double v = (x * p1 - p0 * f.y) * f.x;
+                const double v = __fma_rn(f.x * x, p1, -(f.y * p0));
                 emit(l, v);
                 p0 = p1;
                 p1 = v;
@@ -482,6 +489,10 @@ __global__ void __launch_bounds__(32 * PW) s2_points_kernel(const double2* __res
         row += (L - m - 1 > 0) ? L - m - 1 : 0;
         double sp, cp;
         sincos((double)m * phi, &sp, &cp);
+        if (REAL) {  // the order -m gives the conjugate; only the real part is formed
+            acc.x += (m > 0 ? 2.0 : 1.0) * (Dp.x * cp - Dp.y * sp);
+            continue;
+        }
         acc.x += Dp.x * cp - Dp.y * sp;  // F(l, m) nP e^{i m phi}
         acc.y += Dp.x * sp + Dp.y * cp;
         if (m > 0) {
@@ -493,15 +504,16 @@ __global__ void __launch_bounds__(32 * PW) s2_points_kernel(const double2* __res
     if (pt < n) part[(long long)blockIdx.y * n + pt] = acc;
 }
 
-cudaError_t launch_s2_points(const double2* F, const double* xs, const double* pts, const double2* rec, int L, int n,
-                             const int* m0b, int S, double2* part, double2* out, cudaStream_t st)
+cudaError_t launch_s2_points(const double2* F, const double* xs, const double* pts, const double2* rec, int L, bool real,
+                             int n, const int* m0b, int S, double2* part, double2* out, cudaStream_t st)
 {
     if (S < 1 || S > MAX_POINT_PARTS) return cudaErrorInvalidValue;
     PointParts P;
     for (int s = 0; s <= S; ++s) P.m0[s] = m0b[s];
     const long long nb = ((long long)n + 31) / 32;
     const dim3 grid((unsigned)((nb + PW - 1) / PW), (unsigned)S);
-    s2_points_kernel<<<grid, 32 * PW, 0, st>>>(F, xs, pts, rec, L, n, P, part);
+    if (real) s2_points_kernel<true><<<grid, 32 * PW, 0, st>>>(F, xs, pts, rec, L, n, P, part);
+    else s2_points_kernel<false><<<grid, 32 * PW, 0, st>>>(F, xs, pts, rec, L, n, P, part);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     sum_parts_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(part, S, n, out);
