@@ -225,6 +225,11 @@ FFTLaunch fft_cols(const fftso3_plan* p, const void* in, void* out, long long no
     return L;
 }
 
+cudaError_t fft64(const FFTLaunch& L, cudaStream_t st)
+{
+    return dft64_supported(L.fac.N) ? launch_dft64(L, st) : launch_fft_lines(L, st);
+}
+
 #define STAGE(id, call)      \
     do {                     \
         T.begin(id, st);     \
@@ -249,18 +254,36 @@ int fp64_inverse(fftso3_plan* p, const void* Fin_, void* gout, int nb, void* wor
             STAGE(ST_BASIS, launch_so3_r2c(Fin_, fc, true, L, nb, st));
             Fin = (const double2*)fc;
         }
-        STAGE(ST_NYQUIST, launch_zero_nyquist_so3(work, true, N, (long long)nb * N, st));
-        STAGE(s_con, launch_so3_inv_fp64(p->d_table, p->d_goff, Fin, (double2*)work, L, N, nb, st));
-        STAGE(s_rows, launch_fft_lines(fft_rows(p, work, work, (long long)nb * N * N, false, false, true), st));
-        STAGE(s_cols, launch_fft_lines(fft_cols(p, work, gout, (long long)nb * N, p->real, true), st));
+        // Nyquist bins: taken as zero by the passes that can, else written
+        const bool direct = dft64_supported(N);
+        if (!direct) STAGE(ST_NYQUIST, launch_zero_nyquist_so3(work, true, N, (long long)nb * N, st));
+        STAGE(s_con, launch_so3_inv_fp64(p->d_table, p->d_goff, Fin, (double2*)work, L, N, nb, p->real, st));
+        // along q, then along p; real: only the rows p < N/2, whose transforms' conjugates are the others'
+        FFTLaunch rows = fft_rows(p, work, work, (long long)nb * N * N, false, false, true);
+        FFTLaunch cols = fft_cols(p, work, gout, (long long)nb * N, p->real, true);
+        rows.inner = N;
+        rows.istride = N;
+        rows.ostride = (long long)N * N;
+        rows.nyq = cols.nyq = 1;
+        rows.skip = N / 2;
+        if (p->real) {
+            rows.nlines = (long long)nb * N * (N / 2);
+            rows.inner = N / 2;
+            rows.skip = -1;
+            cols.herm = 1;
+        }
+        STAGE(s_rows, fft64(rows, st));
+        STAGE(s_cols, fft64(cols, st));
     } else {
         if (p->real) {
             STAGE(ST_BASIS, launch_s2_r2c(Fin_, fc, true, L, nb, st));
             Fin = (const double2*)fc;
         }
-        STAGE(ST_NYQUIST, launch_zero_nyquist_s2(work, true, N, (long long)nb * N, st));
+        FFTLaunch rows = fft_rows(p, work, gout, (long long)nb * N, false, p->real, true);
+        rows.nyq = 1;
+        if (!dft64_supported(N)) STAGE(ST_NYQUIST, launch_zero_nyquist_s2(work, true, N, (long long)nb * N, st));
         STAGE(s_con, launch_s2_inv_fp64(p->d_table, p->d_goff, Fin, (double2*)work, L, N, nb, st));
-        STAGE(s_rows, launch_fft_lines(fft_rows(p, work, gout, (long long)nb * N, false, p->real, true), st));
+        STAGE(s_rows, fft64(rows, st));
     }
     return FFTSO3_SUCCESS;
 }
@@ -396,14 +419,20 @@ int run_forward(fftso3_plan* p, const void* grid, void* coeffs, cudaStream_t st)
         return refine_forward(p, grid, coeffs, st);
     }
     if (p->so3) {
-        STAGE(ST_FFT_ROWS, launch_fft_lines(fft_rows(p, grid, p->d_work, (long long)b * N * N, p->real, false, true), st));
-        STAGE(ST_FFT_COLS, launch_fft_lines(fft_cols(p, p->d_work, p->d_work, (long long)b * N, false, true), st));
+        // along j2, then along j1; real: only the columns q <= N/2
+        FFTLaunch cols = fft_cols(p, p->d_work, p->d_work, (long long)b * N, false, true);
+        if (p->real) {
+            cols.inner = N / 2 + 1;
+            cols.nlines = (long long)b * N * (N / 2 + 1);
+        }
+        STAGE(ST_FFT_ROWS, fft64(fft_rows(p, grid, p->d_work, (long long)b * N * N, p->real, false, true), st));
+        STAGE(ST_FFT_COLS, fft64(cols, st));
         double2* Fout = p->real ? (double2*)p->d_fc : (double2*)coeffs;
         STAGE(ST_FP64_FWD,
-              launch_so3_fwd_fp64(p->d_table, p->d_goff, (const double2*)p->d_work, p->d_w, Fout, L, N, b, st));
+              launch_so3_fwd_fp64(p->d_table, p->d_goff, (const double2*)p->d_work, p->d_w, Fout, L, N, b, p->real, st));
         if (p->real) STAGE(ST_BASIS, launch_so3_c2r(p->d_fc, coeffs, true, L, b, st));
     } else {
-        STAGE(ST_FFT_ROWS, launch_fft_lines(fft_rows(p, grid, p->d_work, (long long)b * N, p->real, false, true), st));
+        STAGE(ST_FFT_ROWS, fft64(fft_rows(p, grid, p->d_work, (long long)b * N, p->real, false, true), st));
         double2* Fout = p->real ? (double2*)p->d_fc : (double2*)coeffs;
         STAGE(ST_FP64_FWD, launch_s2_fwd_fp64(p->d_table, p->d_goff, (const double2*)p->d_work, p->d_w, Fout, L, N,
                                               b, p->real, st));

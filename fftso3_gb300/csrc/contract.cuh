@@ -4,10 +4,11 @@
 
 namespace fftso3 {
 
+// real: Hermitian data -- the forward reads the bins q <= N/2 only, and either forms one of each conjugate pair
 cudaError_t launch_so3_fwd_fp64(const double* table, const long long* goff, const double2* G, const double* w,
-                                double2* F, int L, int N, int batch, cudaStream_t st);
+                                double2* F, int L, int N, int batch, bool real, cudaStream_t st);
 cudaError_t launch_so3_inv_fp64(const double* table, const long long* goff, const double2* F, double2* H, int L,
-                                int N, int batch, cudaStream_t st);
+                                int N, int batch, bool real, cudaStream_t st);
 cudaError_t launch_zero_nyquist_so3(void* H, bool fp64, int N, long long nslices, cudaStream_t st);
 cudaError_t launch_so3_c2r(const void* Fc, void* Fr, bool fp64, int L, int batch, cudaStream_t st);
 cudaError_t launch_so3_r2c(const void* Fr, void* Fc, bool fp64, int L, int batch, cudaStream_t st);

@@ -63,72 +63,94 @@ __device__ __forceinline__ double warp_reduce_scatter4(const double (&v)[4], int
 
 // ------------------------------------------------------------------ SO(3)
 
-template <int NT>
+// REAL: the pairs 0 and 2 only; the transform of real samples is Hermitian, so the others are (-1)^(m+n) times their
+// conjugates (half of the sums).
+template <int NT, bool REAL>
 __global__ void __launch_bounds__(NT) so3_fwd_fp64_kernel(const double* __restrict__ table,
                                                           const long long* __restrict__ goff,
                                                           const double2* __restrict__ G, const double* __restrict__ w,
                                                           double2* __restrict__ F, int L, int N, long long gstride,
                                                           long long cstride)
 {
-    extern __shared__ double2 X[];  // [4][N]
+    constexpr int S = REAL ? 2 : 1, NP = 4 / S;  // pair of slot p: S p
+    extern __shared__ double2 X[];  // [NP][N]
     const int g = blockIdx.x, b = blockIdx.y;
     int m0, n0;
     group_mn(g, m0, n0);
     const GroupPairs P = group_pairs(m0, n0);
+    const int np = (P.np + S - 1) / S;
     const double2* Gb = G + (long long)b * gstride;
     const long long NN = (long long)N * N;
-    for (int i = threadIdx.x; i < P.np * N; i += NT) {
+    for (int i = threadIdx.x; i < np * N; i += NT) {
         int p = i / N, k = i - p * N;
-        int pi = mod_n(-P.m[p], N), qi = mod_n(-P.n[p], N);
+        int pi = mod_n(-P.m[S * p], N), qi = mod_n(-P.n[S * p], N);
+        const bool c = REAL && qi > N / 2;  // read as the conjugate of the mirrored bin
+        if (c) {
+            pi = pi ? N - pi : 0;
+            qi = N - qi;
+        }
         double2 v = Gb[(long long)k * NN + (long long)pi * N + qi];
         double wk = w[k];
-        X[p * N + k] = make_double2(wk * v.x, wk * v.y);
+        X[p * N + k] = make_double2(wk * v.x, c ? -(wk * v.y) : wk * v.y);
     }
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const double* tg = table + goff[g];
     double* Fb = reinterpret_cast<double*>(F + (long long)b * cstride);
-    // after the reduce-scatter lane holds value vi = 2 p + (re, im) of pair p; lanes 4j write
-    const int vi = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1), wp = vi >> 1;
-    const bool writer = (lane & 3) == 0 && wp < P.np;
-    const int wm = wp < P.np ? P.m[wp] : 0, wn = wp < P.np ? P.n[wp] : 0;
-    const double wsign = wp < P.np ? (double)P.sign[wp] : 0.;
+    // after the reduce-scatter lane holds value vi = 2 p + (re, im) of slot p; lanes 4j (REAL: 8j) write
+    const int vi = REAL ? ((lane >> 4) & 1) * 2 + ((lane >> 3) & 1)
+                        : ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+    const int wp = vi >> 1, wq = S * wp;
+    const bool writer = (lane & (REAL ? 7 : 3)) == 0 && wp < np;
+    const int wm = wp < np ? P.m[wq] : 0, wn = wp < np ? P.n[wq] : 0;
+    const double wsign = wp < np ? (double)P.sign[wq] : 0.;
+    // the conjugate partner (-m, -n): (-1)^(m+n) conj
+    const double csign = (((wm + wn) & 1) ? -1. : 1.) * ((vi & 1) ? -1. : 1.);
     for (int l = m0 + warp; l <= L; l += NT / 32) {
         const double* drow = tg + (long long)(l - m0) * N;
-        double v[8] = {0., 0., 0., 0., 0., 0., 0., 0.};
+        double v[2 * NP];
+#pragma unroll
+        for (int j = 0; j < 2 * NP; ++j) v[j] = 0.;
         for (int k = lane; k < N; k += 32) {
             double d = drow[k];
 #pragma unroll
-            for (int p = 0; p < 4; ++p)
-                if (p < P.np) {
+            for (int p = 0; p < NP; ++p)
+                if (p < np) {
                     double2 x = X[p * N + k];
                     v[2 * p] += d * x.x;
                     v[2 * p + 1] += d * x.y;
                 }
         }
-        const double y = warp_reduce_scatter8(v, lane);
-        if (writer) Fb[2 * so3_idx(l, wm, wn) + (vi & 1)] = wsign * y;
+        double y;
+        if constexpr (REAL) y = warp_reduce_scatter4(v, lane);
+        else y = warp_reduce_scatter8(v, lane);
+        if (writer) {
+            Fb[2 * so3_idx(l, wm, wn) + (vi & 1)] = wsign * y;
+            if (REAL && m0 > 0) Fb[2 * so3_idx(l, -wm, -wn) + (vi & 1)] = csign * (wsign * y);
+        }
     }
 }
 
-template <int NT>
+// REAL: the pairs 0 and 2 only; H(-m, -n) = conj H(m, n) for the coefficients of a real function.
+template <int NT, bool REAL>
 __global__ void __launch_bounds__(NT) so3_inv_fp64_kernel(const double* __restrict__ table,
                                                           const long long* __restrict__ goff,
                                                           const double2* __restrict__ F, double2* __restrict__ H,
                                                           int L, int N, long long gstride, long long cstride)
 {
-    extern __shared__ double2 Y[];  // [4][B]
+    constexpr int S = REAL ? 2 : 1, NP = 4 / S;
+    extern __shared__ double2 Y[];  // [NP][B]
     const int g = blockIdx.x, b = blockIdx.y;
     const int B = L + 1;
     int m0, n0;
     group_mn(g, m0, n0);
     const GroupPairs P = group_pairs(m0, n0);
-    const int nl = B - m0;
+    const int nl = B - m0, np = (P.np + S - 1) / S;
     const double2* Fb = F + (long long)b * cstride;
-    for (int i = threadIdx.x; i < P.np * nl; i += NT) {
+    for (int i = threadIdx.x; i < np * nl; i += NT) {
         int p = i / nl, l = m0 + (i - p * nl);
-        double2 c = Fb[so3_idx(l, P.m[p], P.n[p])];
-        double s = (double)(2 * l + 1) * P.sign[p];
+        double2 c = Fb[so3_idx(l, P.m[S * p], P.n[S * p])];
+        double s = (double)(2 * l + 1) * P.sign[S * p];
         Y[p * B + (l - m0)] = make_double2(s * c.x, s * c.y);
     }
     __syncthreads();
@@ -136,22 +158,26 @@ __global__ void __launch_bounds__(NT) so3_inv_fp64_kernel(const double* __restri
     double2* Hb = H + (long long)b * gstride;
     const long long NN = (long long)N * N;
     for (int k = threadIdx.x; k < N; k += NT) {
-        double ar[4] = {0., 0., 0., 0.}, ai[4] = {0., 0., 0., 0.};
+        double ar[NP], ai[NP];
+#pragma unroll
+        for (int p = 0; p < NP; ++p) ar[p] = ai[p] = 0.;
         for (int j = 0; j < nl; ++j) {
             double d = tg[(long long)j * N + k];
 #pragma unroll
-            for (int p = 0; p < 4; ++p)
-                if (p < P.np) {
+            for (int p = 0; p < NP; ++p)
+                if (p < np) {
                     double2 y = Y[p * B + j];
                     ar[p] += d * y.x;
                     ai[p] += d * y.y;
                 }
         }
 #pragma unroll
-        for (int p = 0; p < 4; ++p)
-            if (p < P.np) {
-                int pi = mod_n(P.m[p], N), qi = mod_n(P.n[p], N);
-                Hb[(long long)k * NN + (long long)pi * N + qi] = make_double2(ar[p], ai[p]);
+        for (int p = 0; p < NP; ++p)
+            if (p < np) {
+                const int m = P.m[S * p], n = P.n[S * p];
+                Hb[(long long)k * NN + (long long)mod_n(m, N) * N + mod_n(n, N)] = make_double2(ar[p], ai[p]);
+                if (REAL && m0 > 0)
+                    Hb[(long long)k * NN + (long long)mod_n(-m, N) * N + mod_n(-n, N)] = make_double2(ar[p], -ai[p]);
             }
     }
 }
@@ -187,57 +213,76 @@ __device__ __forceinline__ double2 cmul2(double2 a, double2 b)
 }
 __device__ __forceinline__ double2 conj2(double2 a) { return make_double2(a.x, -a.y); }
 
-// F_r = Re(T F_c T^H) per l (fdcl_FFTSO3.cpp:1169-1181): the real-basis
-// coefficients of a real function from its complex coefficients.
-template <typename CIN, typename ROUT, typename A>
-__global__ void so3_c2r_kernel(const CIN* __restrict__ Fc, ROUT* __restrict__ Fr, int L, long long cstride)
+// The basis changes, F_r = Re(T F_c T^H) per l (fdcl_FFTSO3.cpp:1169-1181) and back, F_c = T^H F_r T (the complex
+// coefficients whose synthesis equals the real synthesis of F_r).  One thread a quadruple (l, +-mu, +-nu), which is closed
+// under both: every coefficient is read and written once.  (One CTA a degree read each four times and left most SMs idle at
+// a batch of one: 0.56 and 0.43 ms at l_max 127 in FP64, now 0.04 and 0.05.)  HERM: the FP64 forward writes exact conjugate pairs.
+__device__ __forceinline__ int quad_off(int l) { return l * (l + 1) * (2 * l + 1) / 6; }
+__device__ __forceinline__ void quad_of(int e, int& l, int& mu, int& nu)
 {
-    const int l = blockIdx.x, b = blockIdx.y;
-    const int W = 2 * l + 1;
-    const CIN* fc = Fc + (long long)b * cstride;
-    ROUT* fr = Fr + (long long)b * cstride;
-    for (int i = threadIdx.x; i < W * W; i += blockDim.x) {
-        int m = i % W - l, n = i / W - l;
-        int am[2] = {-m, m}, bn[2] = {-n, n};
-        int na = (m == 0) ? 1 : 2, nb = (n == 0) ? 1 : 2;
-        A acc = 0;
-        for (int ia = 0; ia < na; ++ia)
-            for (int ib = 0; ib < nb; ++ib) {
-                c2t<A> t1 = tmat_t<A>(m, am[ia]), t2 = conj_t(tmat_t<A>(n, bn[ib]));
-                CIN v = fc[so3_idx(l, am[ia], bn[ib])];
-                c2t<A> c = cmul_t(cmul_t(t1, c2t<A>{(A)v.x, (A)v.y}), t2);
-                acc += c.x;
-            }
-        fr[so3_idx(l, m, n)] = (ROUT)acc;
-    }
+    l = (int)cbrtf(3.f * (float)e);
+    while (l > 0 && quad_off(l) > e) --l;
+    while (quad_off(l + 1) <= e) ++l;
+    const int r = e - quad_off(l);
+    nu = r / (l + 1);
+    mu = r - nu * (l + 1);
 }
 
-// F_c = T^H F_r T per l: the complex coefficients whose synthesis equals the
-// real-basis synthesis sum (2l+1) F_r U (U = Re(conj(T) D T^T), fdcl_FFTSO3.cpp:1010-1022).
-template <typename RIN, typename COUT, typename A>
-__global__ void so3_r2c_kernel(const RIN* __restrict__ Fr, COUT* __restrict__ Fc, int L, long long cstride)
+template <typename CIN, typename ROUT, typename A, bool HERM>
+__global__ void so3_c2r_kernel(const CIN* __restrict__ Fc, ROUT* __restrict__ Fr, int nquad, long long C)
 {
-    const int l = blockIdx.x, b = blockIdx.y;
-    const int W = 2 * l + 1;
-    const RIN* fr = Fr + (long long)b * cstride;
-    COUT* fc = Fc + (long long)b * cstride;
-    for (int i = threadIdx.x; i < W * W; i += blockDim.x) {
-        int m = i % W - l, n = i / W - l;
-        int am[2] = {m, -m}, bn[2] = {n, -n};
-        int na = (m == 0) ? 1 : 2, nb = (n == 0) ? 1 : 2;
-        c2t<A> acc = {(A)0, (A)0};
-        for (int ia = 0; ia < na; ++ia)
-            for (int ib = 0; ib < nb; ++ib) {
-                c2t<A> c = cmul_t(conj_t(tmat_t<A>(am[ia], m)), tmat_t<A>(bn[ib], n));
-                A v = (A)fr[so3_idx(l, am[ia], bn[ib])];
-                acc.x += c.x * v;
-                acc.y += c.y * v;
-            }
-        COUT o;
-        o.x = acc.x;
-        o.y = acc.y;
-        fc[so3_idx(l, m, n)] = o;
-    }
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= nquad) return;
+    int l, mu, nu;
+    quad_of(e, l, mu, nu);
+    const CIN* fc = Fc + (long long)blockIdx.y * C;
+    ROUT* fr = Fr + (long long)blockIdx.y * C;
+    c2t<A> v[2][2];  // [a < 0][b < 0]
+#pragma unroll
+    for (int i = 0; i < (HERM ? 1 : 2); ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const CIN x = fc[so3_idx(l, i ? -mu : mu, j ? -nu : nu)];
+            v[i][j] = {(A)x.x, (A)x.y};
+        }
+    auto at = [&](int a, int b) { return a < 0 ? (b < 0 ? v[1][1] : v[1][0]) : (b < 0 ? v[0][1] : v[0][0]); };
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int m = i ? -mu : mu, n = j ? -nu : nu;
+            if ((i && mu == 0) || (j && nu == 0)) continue;
+            fr[so3_idx(l, m, n)] = (ROUT)real_coefficient<A, HERM>(m, n, at);
+        }
+}
+
+template <typename RIN, typename COUT, typename A>
+__global__ void so3_r2c_kernel(const RIN* __restrict__ Fr, COUT* __restrict__ Fc, int nquad, long long C)
+{
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= nquad) return;
+    int l, mu, nu;
+    quad_of(e, l, mu, nu);
+    const RIN* fr = Fr + (long long)blockIdx.y * C;
+    COUT* fc = Fc + (long long)blockIdx.y * C;
+    A v[2][2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) v[i][j] = (A)fr[so3_idx(l, i ? -mu : mu, j ? -nu : nu)];
+    auto at = [&](int a, int b) { return a < 0 ? (b < 0 ? v[1][1] : v[1][0]) : (b < 0 ? v[0][1] : v[0][0]); };
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int m = i ? -mu : mu, n = j ? -nu : nu;
+            if ((i && mu == 0) || (j && nu == 0)) continue;
+            const c2t<A> x = complex_coefficient<A>(m, n, at);
+            COUT o;
+            o.x = x.x;
+            o.y = x.y;
+            fc[so3_idx(l, m, n)] = o;
+        }
 }
 
 // ------------------------------------------------------------------- S^2
@@ -500,11 +545,11 @@ __global__ void __launch_bounds__(256) s2_real_to_group_kernel(const float* __re
 // ---------------------------------------------------------------- launchers
 
 cudaError_t launch_so3_fwd_fp64(const double* table, const long long* goff, const double2* G, const double* w,
-                                double2* F, int L, int N, int batch, cudaStream_t st)
+                                double2* F, int L, int N, int batch, bool real, cudaStream_t st)
 {
     const int B = L + 1;
-    size_t smem = sizeof(double2) * 4 * N;
-    auto k = so3_fwd_fp64_kernel<256>;
+    size_t smem = sizeof(double2) * (real ? 2 : 4) * N;
+    auto k = real ? so3_fwd_fp64_kernel<256, true> : so3_fwd_fp64_kernel<256, false>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     dim3 grid(B * B, batch);
@@ -513,12 +558,13 @@ cudaError_t launch_so3_fwd_fp64(const double* table, const long long* goff, cons
 }
 
 cudaError_t launch_so3_inv_fp64(const double* table, const long long* goff, const double2* F, double2* H, int L,
-                                int N, int batch, cudaStream_t st)
+                                int N, int batch, bool real, cudaStream_t st)
 {
     const int B = L + 1;
-    size_t smem = sizeof(double2) * 4 * B;
+    size_t smem = sizeof(double2) * (real ? 2 : 4) * B;
     dim3 grid(B * B, batch);
-    so3_inv_fp64_kernel<256><<<grid, 256, smem, st>>>(table, goff, F, H, L, N, (long long)N * N * N, so3_off(B));
+    auto k = real ? so3_inv_fp64_kernel<256, true> : so3_inv_fp64_kernel<256, false>;
+    k<<<grid, 256, smem, st>>>(table, goff, F, H, L, N, (long long)N * N * N, so3_off(B));
     return cudaGetLastError();
 }
 
@@ -535,23 +581,25 @@ cudaError_t launch_zero_nyquist_so3(void* H, bool fp64, int N, long long nslices
 
 cudaError_t launch_so3_c2r(const void* Fc, void* Fr, bool fp64, int L, int batch, cudaStream_t st)
 {
-    dim3 grid(L + 1, batch);
-    long long cs = so3_off(L + 1);
+    const long long C = so3_off(L + 1);
+    const int nq = (L + 1) * (L + 2) * (2 * L + 3) / 6;
+    const dim3 grid((unsigned)((nq + 127) / 128), batch);
     if (fp64)
-        so3_c2r_kernel<double2, double, double><<<grid, 256, 0, st>>>((const double2*)Fc, (double*)Fr, L, cs);
+        so3_c2r_kernel<double2, double, double, true><<<grid, 128, 0, st>>>((const double2*)Fc, (double*)Fr, nq, C);
     else
-        so3_c2r_kernel<float2, float, float><<<grid, 256, 0, st>>>((const float2*)Fc, (float*)Fr, L, cs);
+        so3_c2r_kernel<float2, float, float, false><<<grid, 128, 0, st>>>((const float2*)Fc, (float*)Fr, nq, C);
     return cudaGetLastError();
 }
 
 cudaError_t launch_so3_r2c(const void* Fr, void* Fc, bool fp64, int L, int batch, cudaStream_t st)
 {
-    dim3 grid(L + 1, batch);
-    long long cs = so3_off(L + 1);
+    const long long C = so3_off(L + 1);
+    const int nq = (L + 1) * (L + 2) * (2 * L + 3) / 6;
+    const dim3 grid((unsigned)((nq + 127) / 128), batch);
     if (fp64)
-        so3_r2c_kernel<double, double2, double><<<grid, 256, 0, st>>>((const double*)Fr, (double2*)Fc, L, cs);
+        so3_r2c_kernel<double, double2, double><<<grid, 128, 0, st>>>((const double*)Fr, (double2*)Fc, nq, C);
     else
-        so3_r2c_kernel<float, float2, float><<<grid, 256, 0, st>>>((const float*)Fr, (float2*)Fc, L, cs);
+        so3_r2c_kernel<float, float2, float><<<grid, 128, 0, st>>>((const float*)Fr, (float2*)Fc, nq, C);
     return cudaGetLastError();
 }
 

@@ -365,7 +365,7 @@ template <typename T, typename TIN, bool REAL_IN, bool REAL_OUT>
 __global__ void __launch_bounds__(256) fft_lines_kernel(const TIN* __restrict__ in, void* __restrict__ out, FFTFactors fac,
                                                         long long nlines, int lpb_log2, long long inner, long long ostride,
                                                         long long istride, long long es, const void* __restrict__ twg,
-                                                        int lines_fastest)
+                                                        int lines_fastest, int herm)
 {
     using C = typename V2<T>::t;
     constexpr bool PACK = REAL_IN || REAL_OUT;
@@ -416,8 +416,19 @@ __global__ void __launch_bounds__(256) fft_lines_kernel(const TIN* __restrict__ 
                 j = e - p2 * N;
             }
             if (p2 >= np2) continue;
-            const C a = reinterpret_cast<const C*>(in)[base[2 * p2] + (long long)j * es];
-            const C b = reinterpret_cast<const C*>(in)[base[2 * p2 + 1] + (long long)j * es];
+            C a, b;
+            if (herm && j == N / 2) {  // (FFTLaunch::herm)
+                a = b = V2<T>::mk((T)0, (T)0);
+            } else {
+                const bool c = herm && j > N / 2;
+                const long long o = (long long)(c ? N - j : j) * es;
+                a = reinterpret_cast<const C*>(in)[base[2 * p2] + o];
+                b = reinterpret_cast<const C*>(in)[base[2 * p2 + 1] + o];
+                if (c) {
+                    a.y = -a.y;
+                    b.y = -b.y;
+                }
+            }
             buf0[p2 * LS + j] = V2<T>::mk(a.x - b.y, a.y + b.x);
         }
     } else if (lines_fastest) {
@@ -1141,7 +1152,7 @@ size_t fft_smem_bytes(int N, int lpb, bool fp64)
 template <typename T, typename TIN, bool RI, bool RO>
 static cudaError_t launch_one(const void* in, void* out, const FFTFactors& fac, long long nlines, int lpb,
                               long long inner, long long ostride, long long istride, long long es,
-                              const void* tw, bool lines_fastest, int threads, cudaStream_t st)
+                              const void* tw, bool lines_fastest, int threads, int herm, cudaStream_t st)
 {
     if (threads < 32 || threads > 256 || threads % 32 != 0) return cudaErrorInvalidValue;
     if ((RI || RO) && lpb < 2) lpb = 2;  // real data: lines transformed in pairs
@@ -1156,7 +1167,7 @@ static cudaError_t launch_one(const void* in, void* out, const FFTFactors& fac, 
     if ((1 << lg) != lpb || lpb > 256) return cudaErrorInvalidValue;  // lines per CTA: power of two
     long long nblk = (nlines + lpb - 1) / lpb;
     kern<<<(unsigned)nblk, threads, smem, st>>>(reinterpret_cast<const TIN*>(in), out, fac, nlines, lg, inner, ostride,
-                                            istride, es, tw, lines_fastest ? 1 : 0);
+                                            istride, es, tw, lines_fastest ? 1 : 0, herm);
     return cudaGetLastError();
 }
 
@@ -1165,28 +1176,28 @@ cudaError_t launch_fft_lines(const FFTLaunch& L, cudaStream_t st)
     if (L.df32) {  // double-float complex lines (16 bytes per element), complex in and out only
         if (L.real_in || L.real_out) return cudaErrorInvalidValue;
         return launch_one<df32, dfc32, false, false>(L.in, L.out, L.fac, L.nlines, L.lpb, L.inner, L.ostride,
-                                                     L.istride, L.es, L.tw, L.lines_fastest, L.threads, st);
+                                                     L.istride, L.es, L.tw, L.lines_fastest, L.threads, L.herm, st);
     }
     if (L.fp64) {
         if (L.real_in && L.real_out) return cudaErrorInvalidValue;
         if (L.real_in)
             return launch_one<double, double, true, false>(L.in, L.out, L.fac, L.nlines, L.lpb, L.inner, L.ostride,
-                                                           L.istride, L.es, L.tw, L.lines_fastest, L.threads, st);
+                                                           L.istride, L.es, L.tw, L.lines_fastest, L.threads, L.herm, st);
         if (L.real_out)
             return launch_one<double, double2, false, true>(L.in, L.out, L.fac, L.nlines, L.lpb, L.inner, L.ostride,
-                                                            L.istride, L.es, L.tw, L.lines_fastest, L.threads, st);
+                                                            L.istride, L.es, L.tw, L.lines_fastest, L.threads, L.herm, st);
         return launch_one<double, double2, false, false>(L.in, L.out, L.fac, L.nlines, L.lpb, L.inner, L.ostride,
-                                                         L.istride, L.es, L.tw, L.lines_fastest, L.threads, st);
+                                                         L.istride, L.es, L.tw, L.lines_fastest, L.threads, L.herm, st);
     } else {
         if (L.real_in && L.real_out) return cudaErrorInvalidValue;
         if (L.real_in)
             return launch_one<float, float, true, false>(L.in, L.out, L.fac, L.nlines, L.lpb, L.inner, L.ostride,
-                                                         L.istride, L.es, L.tw, L.lines_fastest, L.threads, st);
+                                                         L.istride, L.es, L.tw, L.lines_fastest, L.threads, L.herm, st);
         if (L.real_out)
             return launch_one<float, float2, false, true>(L.in, L.out, L.fac, L.nlines, L.lpb, L.inner, L.ostride,
-                                                          L.istride, L.es, L.tw, L.lines_fastest, L.threads, st);
+                                                          L.istride, L.es, L.tw, L.lines_fastest, L.threads, L.herm, st);
         return launch_one<float, float2, false, false>(L.in, L.out, L.fac, L.nlines, L.lpb, L.inner, L.ostride,
-                                                       L.istride, L.es, L.tw, L.lines_fastest, L.threads, st);
+                                                       L.istride, L.es, L.tw, L.lines_fastest, L.threads, L.herm, st);
     }
 }
 

@@ -24,6 +24,10 @@ struct FFTLaunch {
     bool real_out;
     bool lines_fastest;   // consecutive lines adjacent in memory (column pass)
     int threads = 256;    // threads per CTA (<= 256)
+    // FP64 synthesis passes (dft64.cu, and the line FFT with real_out): element N/2 is taken as zero (nyq); elements past
+    // N/2 as the conjugates of their mirrors, without reading them (herm, with real_out and nyq); lines i with
+    // i % inner == skip are not written (dft64 only)
+    int nyq = 0, herm = 0, skip = -1;
 };
 
 void make_fft_factors(int N, FFTFactors& f);
@@ -32,6 +36,9 @@ void make_fft_factors(int N, FFTFactors& f);
 void make_fft_factors_prime_first(int N, FFTFactors& f);
 size_t fft_smem_bytes(int N, int lpb, bool fp64);
 cudaError_t launch_fft_lines(const FFTLaunch& L, cudaStream_t st);
+// FP64 passes of short lines as direct DFTs (dft64.cu); one line's arithmetic depends on N only.
+bool dft64_supported(int N);
+cudaError_t launch_dft64(const FFTLaunch& L, cudaStream_t st);
 
 // Double-float (dfc32) FFT along a strided axis of arrays whose innermost index k (N values) is contiguous,
 // in place: line (o, k), o < nouter, has element j at obase(o) + k + j S, obase(o) = (o / oinner) oouter +

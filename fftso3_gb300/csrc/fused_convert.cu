@@ -48,15 +48,6 @@ __device__ __forceinline__ long long gm_offset(int l, int m, int n, int B)
     return block_start(m0, B) + (long long)run_index(m0, n0, pp) * (B - m0) + (l - m0);
 }
 
-// largest l with l (4 l^2 - 1) / 3 <= r (the packed offset of degree l; < 2^31 for l <= 256)
-__device__ __forceinline__ int off32(int l) { return l * (4 * l * l - 1) / 3; }
-__device__ __forceinline__ int degree_of(int r)
-{
-    int l = (int)cbrtf(0.75f * (float)r);
-    while (l > 0 && off32(l) > r) --l;
-    while (off32(l + 1) <= r) ++l;
-    return l;
-}
 
 
 template <bool REAL>
@@ -78,18 +69,10 @@ __global__ void __launch_bounds__(CONVERT_THREADS) fused_group_to_packed_kernel(
         reinterpret_cast<float2*>(out)[S.c0 + u] = fg[gm_offset(l, m, n, B)];
         return;
     }
-    const int am[2] = {-m, m}, bn[2] = {-n, n};
-    const int na = (m == 0) ? 1 : 2, nb = (n == 0) ? 1 : 2;
-    float2 v[2][2];
-    for (int ia = 0; ia < na; ++ia)
-        for (int ib = 0; ib < nb; ++ib) v[ia][ib] = fg[gm_offset(l, am[ia], bn[ib], B)];
-    float acc = 0.f;
-    for (int ia = 0; ia < na; ++ia)
-        for (int ib = 0; ib < nb; ++ib) {
-            const c2t<float> t1 = tmat_t<float>(m, am[ia]), t2 = conj_t(tmat_t<float>(n, bn[ib]));
-            const c2t<float> c = cmul_t(cmul_t(t1, c2t<float>{v[ia][ib].x, v[ia][ib].y}), t2);
-            acc += c.x;
-        }
+    const float acc = real_coefficient<float, false>(m, n, [&](int a, int c) {
+        const float2 v = fg[gm_offset(l, a, c, B)];
+        return c2t<float>{v.x, v.y};
+    });
     reinterpret_cast<float*>(out)[S.c0 + u] = acc;
 }
 
@@ -127,18 +110,7 @@ __global__ void __launch_bounds__(CONVERT_THREADS) fused_packed_to_group_kernel(
         v = reinterpret_cast<const float2*>(in)[S.c0 + (long long)f * C + so3_idx(l, m, n)];
     } else {
         const float* __restrict__ fr = reinterpret_cast<const float*>(in) + S.c0 + (long long)f * C;
-        const int am[2] = {m, -m}, bn[2] = {n, -n};
-        const int na = (m == 0) ? 1 : 2, nb = (n == 0) ? 1 : 2;
-        float x[2][2];
-        for (int ia = 0; ia < na; ++ia)
-            for (int ib = 0; ib < nb; ++ib) x[ia][ib] = fr[so3_idx(l, am[ia], bn[ib])];
-        c2t<float> acc = {0.f, 0.f};
-        for (int ia = 0; ia < na; ++ia)
-            for (int ib = 0; ib < nb; ++ib) {
-                const c2t<float> c = cmul_t(conj_t(tmat_t<float>(am[ia], m)), tmat_t<float>(bn[ib], n));
-                acc.x += c.x * x[ia][ib];
-                acc.y += c.y * x[ia][ib];
-            }
+        const c2t<float> acc = complex_coefficient<float>(m, n, [&](int a, int c) { return fr[so3_idx(l, a, c)]; });
         v = make_float2(acc.x, acc.y);
     }
     const float sc = (float)(2 * l + 1) * (float)psign;

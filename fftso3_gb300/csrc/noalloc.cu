@@ -230,7 +230,7 @@ extern "C" int fftso3_forward_noalloc(int l_max, const void* grid, void* coeffs,
     C.lines_fastest = true;
     if ((e = launch_fft_lines(C, st)) != cudaSuccess) return na_fail(FFTSO3_ERR_CUDA, cudaGetErrorString(e));
     e = launch_so3_fwd_fp64((const double*)(scratch + OFF_TABLE), (const long long*)(scratch + OFF_GOFF), work,
-                            (const double*)(scratch + OFF_W), (double2*)coeffs, l_max, N, 1, st);
+                            (const double*)(scratch + OFF_W), (double2*)coeffs, l_max, N, 1, false, st);
     if (e != cudaSuccess) return na_fail(FFTSO3_ERR_CUDA, cudaGetErrorString(e));
     return FFTSO3_SUCCESS;
 }
