@@ -330,7 +330,7 @@ int refine_forward(fftso3_plan* p, const void* grid, void* coeffs, cudaStream_t 
     return tc_refine_add(p->tc, resid, coeffs, st, &T, g_err);
 }
 
-// The spectral form of the refined forward (SO(3), exact inverse, N = 64..512): the samples' FFT in
+// The spectral form of the refined forward (SO(3), exact inverse, N <= 222, 256 or 512): the samples' FFT in
 // double-float (pencils hi in the plan's pencil buffer, remainders lo in its residual buffer), F0 = the GEMM of
 // hi, then per chunk the residual in the pencil domain, r^ = (hi + lo) - N^2 H(F0) (H: the exact synthesis
 // contraction, whose FFT is N^2 H), written over hi, and F = F0 + the GEMM of r^.  Equal to the grid form
@@ -383,7 +383,7 @@ int refine_forward_spectral(fftso3_plan* p, const void* grid, void* coeffs, cuda
                                        lo + (long long)f0 * G, st, &T, g_err, true)))
                 return rc;
         }
-        return tc_refine_finish_group(p->tc, coeffs, st, &T, g_err);
+        return tc_refine_finish_group(p->tc, coeffs, oz_correction_terms(p->oz), st, &T, g_err);
     }
     int rc = tc_forward_pencils(p->tc, coeffs, st, &T, g_err);
     if (rc) return rc;
@@ -400,7 +400,7 @@ int refine_forward_spectral(fftso3_plan* p, const void* grid, void* coeffs, cuda
                                    g_err)))
             return rc;
     }
-    return tc_refine_add_pencils(p->tc, coeffs, st, &T, g_err);
+    return tc_refine_add_pencils(p->tc, coeffs, oz_correction_terms(p->oz), st, &T, g_err);
 }
 
 bool spectral_refine(const fftso3_plan* p)
@@ -445,7 +445,7 @@ int run_forward(fftso3_plan* p, const void* grid, void* coeffs, cudaStream_t st)
 // tensor cores and a double-float FFT, a contraction chunk of functions at a time, the double-float pencils in
 // the plan's pencil + residual buffers; otherwise the FP64 inverse in chunks of rchunk functions -- rounded once
 // into the FP32 grid.  host (non-null): the grids go to host memory; grid is then device staging for them (unused
-// by the double-float FFT of N = 64..512, which streams pieces through a small device ring instead).
+// by the double-float DFTs of N <= 222, 256 and 512, which stream pieces through a small device ring instead).
 int exact_inverse(fftso3_plan* p, const void* coeffs, void* grid, cudaStream_t st, void* host = nullptr)
 {
     StageTimer& T = p->timer;
@@ -688,10 +688,10 @@ int fftso3_plan_create(fftso3_plan** out, int kind, int l_max, int batch, int pr
             // Chunks of 16 functions (two column tiles, whose items share each table tile through L2, so the
             // digit planes are read once per 16 functions) when the device has room for them with 16 GB to
             // spare after the FP64 table is freed, else 8 (one column tile), else fewer
-            // The spectral form (N = 64..512) needs the double-float pencils only as its FFT's work space
+            // The spectral form (N <= 222, 256 or 512) needs the double-float pencils only as its FFT's work space
             // (pen_fns = up to 8 functions at a time), so its contraction chunks grow to 32 functions (four column
             // tiles sharing each table tile; the digit planes read once per 32 functions).
-            const bool spectral = fft_df32_k_supported(N);
+            const bool spectral = oz_spectral_supported(N);
             const size_t pen_fn = 16 * (size_t)p->grid_elems;
             const size_t planes = 4 * 2 * (size_t)(p->table_elems / N) * (size_t)((N + 63) / 64 * 64);
             const size_t tab64 = sizeof(double) * (size_t)p->table_elems;
@@ -893,7 +893,7 @@ int fftso3_forward_host(fftso3_plan* plan, const void* grid_host, void* coeffs_h
     return FFTSO3_SUCCESS;
 }
 
-// The exact inverse into host memory (SO(3), N = 64..512), pipelined in chunks of up to 8 functions (one column
+// The exact inverse into host memory (SO(3), N <= 222, 256 or 512), pipelined in chunks of up to 8 functions (one column
 // tile of the exact contraction): each chunk's coefficients are copied in, contracted and transformed, and its
 // grids stream out through the device ring on the copy stream, so the copies out (the host link bounds the call)
 // start after the first chunk instead of after the whole batch.

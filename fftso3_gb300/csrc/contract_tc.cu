@@ -2028,16 +2028,17 @@ int tc_gemm_forward_group(TCState* s, cudaStream_t st, StageTimer* T, std::strin
     return FFTSO3_SUCCESS;
 }
 
-int tc_refine_finish_group(TCState* s, void* coeffs, cudaStream_t st, StageTimer* T, std::string& err)
+int tc_refine_finish_group(TCState* s, void* coeffs, int terms, cudaStream_t st, StageTimer* T, std::string& err)
 {
     if (!s->refine || !s->d_coef2 || s->s2 || s->real) {
         err = "internal: group-major refinement is for complex SO(3) refined plans";
         return FFTSO3_ERR_CUDA;
     }
-    // the correction's GEMM into d_coef2 (group-major), then one permutation that adds it to F0 (d_fg).  One BF16
-    // term: the residual is ~5e-7 of the samples' spectrum, so the term's 2^-9 relative rounding leaves ~1e-9.
+    // the correction's GEMM into d_coef2 (group-major), then one permutation that adds it to F0 (d_fg).  terms = 1: the
+    // residual of a band-limited function is ~5e-7 of the samples' spectrum, so one BF16 term's 2^-9 relative rounding
+    // leaves ~1e-9; of other samples it keeps what F0 cannot represent (5 % of the samples: an error of 4e-6 at N = 160).
     T->begin(ST_GEMM_FWD, st);
-    int rc = launch_gemm(s, true, st, err, s->d_coef2, 1);
+    int rc = launch_gemm(s, true, st, err, s->d_coef2, terms);
     if (rc) return rc;
     T->end(st);
     // F0 + the correction, added as the permutation reads them
@@ -2049,19 +2050,18 @@ int tc_refine_finish_group(TCState* s, void* coeffs, cudaStream_t st, StageTimer
     return FFTSO3_SUCCESS;
 }
 
-int tc_refine_add_pencils(TCState* s, void* coeffs, cudaStream_t st, StageTimer* T, std::string& err)
+int tc_refine_add_pencils(TCState* s, void* coeffs, int terms, cudaStream_t st, StageTimer* T, std::string& err)
 {
     if (!s->refine || !s->d_coef2 || s->s2) {
         err = "internal: refinement buffers were not allocated";
         return FFTSO3_ERR_CUDA;
     }
-    // the correction in the coefficients' own element type: complex in d_coef2, real kinds in d_fc; its GEMM with
-    // one BF16 term (the residual is small: see tc_refine_finish_group)
+    // the correction in the coefficients' own element type: complex in d_coef2, real kinds in d_fc
     void* corr = s->real ? (void*)s->d_fc : (void*)s->d_coef2;
     if (s->real) {
         // tc_forward_finish writes the complex coefficients into d_fc first; route them through d_coef2
         T->begin(ST_GEMM_FWD, st);
-        int rc = launch_gemm(s, true, st, err, nullptr, 1);
+        int rc = launch_gemm(s, true, st, err, nullptr, terms);
         if (rc) return rc;
         T->end(st);
         T->begin(ST_BASIS, st);
@@ -2071,7 +2071,7 @@ int tc_refine_add_pencils(TCState* s, void* coeffs, cudaStream_t st, StageTimer*
         TCK(launch_so3_c2r(s->d_coef2, s->d_fc, false, s->L, s->batch, st));
         T->end(st);
     } else {
-        int rc = forward_from_pencils(s, s->d_coef2, st, T, err, 1);
+        int rc = forward_from_pencils(s, s->d_coef2, st, T, err, terms);
         if (rc) return rc;
     }
     const long long nc = (long long)s->batch * coeffs_per_fn(s);

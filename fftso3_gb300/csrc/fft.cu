@@ -1102,13 +1102,6 @@ cudaError_t launch_fft_df32_k_synth_pass(int pass, void* buf, int N, long long n
     return cudaGetLastError();
 }
 
-cudaError_t launch_fft_df32_k_synth(void* buf, int N, long long nb, void* out, bool real, const void* tw,
-                                    cudaStream_t st)
-{
-    cudaError_t e = launch_fft_df32_k_synth_pass(1, buf, N, nb, out, real, tw, st);
-    return e != cudaSuccess ? e : launch_fft_df32_k_synth_pass(2, buf, N, nb, out, real, tw, st);
-}
-
 void make_fft_factors(int N, FFTFactors& f)
 {
     f.N = N;

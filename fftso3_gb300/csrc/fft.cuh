@@ -51,11 +51,8 @@ cudaError_t launch_fft_df32_k(void* buf, int N, long long S, long long nouter, l
 // remainder); buf: nb double-float grids of work space.
 cudaError_t launch_fft_df32_k_forward(void* buf, int N, long long nb, const void* f, bool real, float2* hi,
                                       float2* lo, const void* tw, cudaStream_t st);
-// The double-float FFT of nb synthesis pencils buf [fn][p][q][k] (dfc32; overwritten) into the grids out
-// [fn][k][j1][j2], rounded once to complex64, or to the real part as float32 when real.
-cudaError_t launch_fft_df32_k_synth(void* buf, int N, long long nb, void* out, bool real, const void* tw,
-                                    cudaStream_t st);
-// One of its two passes (1: along p, in place; 2: along q into out), for pipelining pieces of functions.
+// One pass (1: along p, in place; 2: along q into out) of the double-float FFT of nb synthesis pencils buf [fn][p][q][k]
+// (dfc32; overwritten) into the grids out [fn][k][j1][j2], rounded once to complex64, or to the real part as float32 when real.
 cudaError_t launch_fft_df32_k_synth_pass(int pass, void* buf, int N, long long nb, void* out, bool real,
                                          const void* tw, cudaStream_t st);
 

@@ -25,10 +25,10 @@
 //  * the epilogue combines the four levels in double-float and scales by 2^E,
 //    giving H to about 2^-30 of its largest term (the dropped products
 //    i + j >= 4 and the digits below 2^-31), as double-float pencils.
-// Grid form (N not a power of two from 64 to 512): a double-float FFT over
+// Grid form (N > 222 but 256 and 512): a double-float FFT over
 // (p, q) then gives the grid g, and the residual r = f - g is formed against
 // the FP32 samples in the same arithmetic (f is exact there) and rounded to
-// FP32 only as the small difference.  Spectral form (N = 64..512): the
+// FP32 only as the small difference.  Spectral form (the other N): the
 // samples' FFT in double-float (pencils hi + lo), and the epilogue writes
 // r^ = (hi + lo) - N^2 H at the forward pencil place of each (m, n) instead
 // of H -- the FFT of the synthesised grid is N^2 H -- so neither g nor an
@@ -57,6 +57,7 @@
 #include "../../include/fftso3_gb300.h"
 #include "common.cuh"
 #include "df32.cuh"
+#include "dft_oz.cuh"
 #include "fft.cuh"
 #include "refine_oz.cuh"
 #include "tc.cuh"
@@ -102,10 +103,11 @@ struct Args {
     const signed char* et;  // exponents [group][k]
     float4* pout;           // double-float pencils [fn][p][q][k]
     // spectral residual (rhi non-null): instead of H, write r = (rhi + rlo) - N^2 H at the forward pencil place
-    // (-m, -n) of each (m, n), into rhi (complex64 pencils [fn][p][q][k]; rlo the remainders); e2n = log2 N^2
+    // (-m, -n) of each (m, n), into rhi (complex64 pencils [fn][p][q][k]; rlo the remainders); N^2 = n2 2^e2n, 1 <= n2 < 2
     float2* rhi;
     const float2* rlo;
     int e2n;
+    float n2;
     int* err;
 };
 
@@ -351,12 +353,15 @@ __global__ void __launch_bounds__(THREADS, 1)
                         const df32 im = combine_levels(__uint_as_float(v[0][cr + 1]), __uint_as_float(v[1][cr + 1]),
                                                        __uint_as_float(v[2][cr + 1]), __uint_as_float(v[3][cr + 1]));
                         if (spectral) {
-                            // N^2 H = FFT of the synthesised grid; hi - N^2 H.h is exact (close values)
+                            // N^2 H = FFT of the synthesised grid; hi - N^2 H.h is exact (close values), N^2 H.h itself
+                            // a product and its rounding error (zero for a power of two)
                             const int E2 = E + a.e2n;
                             const float2 h = sh[p], l = sl[p];
-                            __stcs(a.rhi + fo + poff[p],
-                                   make_float2((h.x - ldexpf(re.h, E2)) + (l.x - ldexpf(re.l, E2)),
-                                               (h.y - ldexpf(im.h, E2)) + (l.y - ldexpf(im.l, E2))));
+                            auto minus = [&](float x, float xl, df32 v) {
+                                const float vh = ldexpf(v.h, E2), ph = __fmul_rn(vh, a.n2), pl = __fmaf_rn(vh, a.n2, -ph);
+                                return (x - ph) + (xl - __fmaf_rn(ldexpf(v.l, E2), a.n2, pl));
+                            };
+                            __stcs(a.rhi + fo + poff[p], make_float2(minus(h.x, l.x, re), minus(h.y, l.y, im)));
                         } else {
                             a.pout[fo + poff[p]] =
                                 make_float4(ldexpf(re.h, E), ldexpf(re.l, E), ldexpf(im.h, E), ldexpf(im.l, E));
@@ -644,6 +649,7 @@ struct OZState {
     unsigned char* bimg = nullptr;  // [column tile][tile] x STAGE_B: their digit image (digit_image_kernel)
     int* gt0 = nullptr;             // first image tile of each group
     long long nbt = 0;              // image tiles per column tile
+    void* dft = nullptr;        // digit DFT matrices (dft_oz.cu), or null: N is a power of two, or the grid form
     float4* pen = nullptr;      // [chunk][N^3] double-float pencils / grid
     long long* goff2 = nullptr;
     int4* items = nullptr;      // work items of a full chunk (all column tiles)
@@ -682,7 +688,7 @@ void oz_destroy(OZState* o)
     if (!o) return;
     for (int p = 0; p < NS; ++p)
         if (o->planes[p]) cudaFree(o->planes[p]);
-    void* ptrs[] = {o->et, o->ey, o->bimg, o->gt0, o->pen, o->goff2, o->items, o->iaux, o->err};
+    void* ptrs[] = {o->et, o->ey, o->bimg, o->gt0, o->pen, o->dft, o->goff2, o->items, o->iaux, o->err};
     for (void* q : ptrs)
         if (q) cudaFree(q);
     for (void* q : o->items_z)
@@ -820,6 +826,11 @@ int oz_create(OZState** out, const double* d_table, const std::vector<long long>
     if ((rc = oz_alloc(o, (void**)&o->err, sizeof(int), err))) return bail(rc);
     cudaMemset(o->err, 0, sizeof(int));
     cudaError_t e = cudaFuncSetAttribute(oz_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    // powers of two from 64 have the double-float FFT (fft.cu); other N up to 222 the digit DFT
+    if (!fft_df32_k_supported(N) && dft_oz_supported(N)) {
+        if ((rc = oz_alloc(o, &o->dft, dft_oz_table_bytes(N), err))) return bail(rc);
+        if (e == cudaSuccess) e = dft_oz_build_table(o->dft, N, d_tw, 0);
+    }
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e != cudaSuccess) {
         err = std::string("refinement state: ") + cudaGetErrorString(e);
@@ -844,6 +855,13 @@ int oz_status(OZState* o)
             return FFTSO3_ERR_CUDA;                                            \
         }                                                                      \
     } while (0)
+
+// A chunk's synthesis FFT goes line by line: no other form, or too few samples for the digit DFT, whose CTAs take 64 lines
+// each (exact inverse of one complex function: N = 32 38 us against 57, N = 48 53 against 63, N = 62 109 against 70).
+static bool by_lines(const OZState* o)
+{
+    return !fft_df32_k_supported(o->N) && (!o->dft || (long long)o->chunk * o->N * o->N * o->N < 200000);
+}
 
 // coefficients -> double-float group-major runs and their exponents, then the exact contraction: H into the
 // double-float pencils (rhi null), or the spectral residual into rhi
@@ -872,7 +890,7 @@ static int oz_contract(OZState* o, const void* F, bool f64, int nb, float2* rhi,
             digit_image_kernel<float2, false><<<grid, 256, 0, st>>>((const float2*)F, o->C, o->ey, o->goff2, o->gt0,
                                                                     o->bimg, o->nbt, L, o->ngroups, nb);
         OZK(cudaGetLastError());
-        if (!rhi) {
+        if (!rhi && (!o->dft || by_lines(o))) {  // (the digit DFT does not read them)
             const long long tot = (long long)nb * 2 * NN;
             zero_nyquist_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(pen, N, nb);
             OZK(cudaGetLastError());
@@ -900,8 +918,9 @@ static int oz_contract(OZState* o, const void* F, bool f64, int nb, float2* rhi,
         a.rhi = rhi;
         a.rlo = rlo;
         int e2n = 0;
-        while ((1LL << e2n) < NN) ++e2n;
+        while ((2LL << e2n) <= NN) ++e2n;
         a.e2n = e2n;
+        a.n2 = ldexpf((float)NN, -e2n);
         a.err = o->err;
         const int nctas = o->nitems < o->nsm ? o->nitems : o->nsm;
         oz_inv_kernel<<<nctas, THREADS, SMEM_BYTES, st>>>(o->tm[0], o->tm[1], o->tm[2], o->tm[3], a);
@@ -911,7 +930,33 @@ static int oz_contract(OZState* o, const void* F, bool f64, int nb, float2* rhi,
     return FFTSO3_SUCCESS;
 }
 
-bool oz_spectral(const OZState* o) { return o && fft_df32_k_supported(o->N); }
+bool oz_spectral_supported(int N) { return fft_df32_k_supported(N) || dft_oz_supported(N); }
+
+bool oz_spectral(const OZState* o) { return o && oz_spectral_supported(o->N); }
+
+static int synth_fft_lines(OZState* o, float4* pen, int nb, cudaStream_t st, std::string& err);
+
+// One of the two steps of the synthesis of nb functions' double-float pencils pen (overwritten) into the grids out
+static int synth_step(OZState* o, int step, float4* pen, int nb, void* out, bool real, cudaStream_t st, std::string& err)
+{
+    const int N = o->N;
+    if (!by_lines(o)) {
+        OZK(o->dft ? launch_dft_oz_grid_pass(pen, step == 1 ? pen : out, nullptr, nb, N, step == 1 ? -2 : -1, real, o->dft,
+                                             o->err, st)
+                   : launch_fft_df32_k_synth_pass(step, pen, N, nb, out, real, o->d_tw, st));
+        return FFTSO3_SUCCESS;
+    }
+    if (step == 1) return synth_fft_lines(o, pen, nb, st, err);
+    const dim3 g((unsigned)((N + 31) / 32), (unsigned)((N + 31) / 32), (unsigned)((long long)nb * N));
+    if (real)
+        synth_out_kernel<true><<<g, 256, 0, st>>>(pen, out, N);
+    else
+        synth_out_kernel<false><<<g, 256, 0, st>>>(pen, out, N);
+    OZK(cudaGetLastError());
+    return FFTSO3_SUCCESS;
+}
+
+int oz_correction_terms(const OZState* o) { return o && o->dft ? 3 : 1; }
 
 int oz_fft_functions(const OZState* o) { return o ? o->pen_fns : 0; }
 
@@ -936,11 +981,16 @@ int oz_forward_fft(OZState* o, const void* fgrid, bool real, int nb, float2* hi,
                    StageTimer* T, std::string& err)
 {
     if (!oz_spectral(o) || nb < 1 || nb > o->pen_fns) {
-        err = "internal: double-float forward FFT needs N = 64..512 and nb <= its buffer's functions";
+        err = "internal: double-float forward FFT needs a spectral plan and nb <= its buffer's functions";
         return FFTSO3_ERR_CUDA;
     }
     T->begin(ST_REF_FFT, st);
-    OZK(launch_fft_df32_k_forward(o->pen, o->N, nb, fgrid, real, hi, lo, o->d_tw, st));
+    if (o->dft) {
+        OZK(launch_dft_oz_grid_pass(fgrid, o->pen, nullptr, nb, o->N, 1, real, o->dft, o->err, st));
+        OZK(launch_dft_oz_grid_pass(o->pen, hi, lo, nb, o->N, 2, real, o->dft, o->err, st));
+    } else {
+        OZK(launch_fft_df32_k_forward(o->pen, o->N, nb, fgrid, real, hi, lo, o->d_tw, st));
+    }
     T->end(st);
     return FFTSO3_SUCCESS;
 }
@@ -949,14 +999,14 @@ int oz_resid_pencils(OZState* o, const void* F, bool f64, int nb, float2* hi, co
                      StageTimer* T, std::string& err, bool group_major)
 {
     if (!oz_spectral(o) || (group_major && f64)) {
-        err = "internal: spectral residual needs N = 64..512 (group-major input: complex64)";
+        err = "internal: spectral residual needs a spectral plan (group-major input: complex64)";
         return FFTSO3_ERR_CUDA;
     }
     return oz_contract(o, F, f64, nb, hi, lo, st, T, err, group_major);
 }
 
 // double-float FFT of the synthesis pencils in o->pen over q (lines (fn, p, k)), then over p (lines (fn, q, k)),
-// in place, by the generic line kernels (any N)
+// in place, by the generic line kernels
 static int synth_fft_lines(OZState* o, float4* pen, int nb, cudaStream_t st, std::string& err)
 {
     const int N = o->N;
@@ -994,7 +1044,7 @@ int oz_inverse_resid(OZState* o, const void* F, bool f64, int nb, const void* fg
     int rc = oz_contract(o, F, f64, nb, nullptr, nullptr, st, T, err);
     if (rc) return rc;
     const int N = o->N;
-    // the grid form serves the sizes the spectral form does not (N not a power of two from 64 to 512)
+    // the grid form serves the sizes the spectral form does not (N > 222, not 256 or 512)
     T->begin(ST_REF_FFT, st);
     if ((rc = synth_fft_lines(o, o->pen, nb, st, err))) return rc;
     T->end(st);
@@ -1044,9 +1094,9 @@ int oz_inverse_exact(OZState* o, const void* F, bool f64, int nb, void* grid, bo
             const int np = nb - f0 < OZ_SYNTH_PIECE ? nb - f0 : OZ_SYNTH_PIECE, sl = (int)(o->ring_seq++ & 1);
             float4* pb = pen + (long long)f0 * G;
             char* rb = (char*)ring + (size_t)sl * OZ_SYNTH_PIECE * gbytes;
-            OZK(launch_fft_df32_k_synth_pass(1, pb, N, np, rb, real, o->d_tw, st));
+            if ((rc = synth_step(o, 1, pb, np, rb, real, st, err))) return rc;
             OZK(cudaStreamWaitEvent(st, o->ev_free[sl], 0));
-            OZK(launch_fft_df32_k_synth_pass(2, pb, N, np, rb, real, o->d_tw, st));
+            if ((rc = synth_step(o, 2, pb, np, rb, real, st, err))) return rc;
             OZK(cudaEventRecord(o->ev_ready[sl], st));
             OZK(cudaStreamWaitEvent(o->side, o->ev_ready[sl], 0));
             OZK(cudaMemcpyAsync((char*)host + (size_t)f0 * gbytes, rb, (size_t)np * gbytes, cudaMemcpyDeviceToHost,
@@ -1057,16 +1107,9 @@ int oz_inverse_exact(OZState* o, const void* F, bool f64, int nb, void* grid, bo
             OZK(cudaEventRecord(o->ev_join, o->side));
             OZK(cudaStreamWaitEvent(st, o->ev_join, 0));
         }
-    } else if (oz_spectral(o)) {
-        OZK(launch_fft_df32_k_synth(pen, N, nb, grid, real, o->d_tw, st));
     } else {
-        if ((rc = synth_fft_lines(o, pen, nb, st, err))) return rc;
-        dim3 g((unsigned)((N + 31) / 32), (unsigned)((N + 31) / 32), (unsigned)((long long)nb * N));
-        if (real)
-            synth_out_kernel<true><<<g, 256, 0, st>>>(pen, grid, N);
-        else
-            synth_out_kernel<false><<<g, 256, 0, st>>>(pen, grid, N);
-        OZK(cudaGetLastError());
+        if ((rc = synth_step(o, 1, pen, nb, grid, real, st, err)) || (rc = synth_step(o, 2, pen, nb, grid, real, st, err)))
+            return rc;
         if (host) OZK(cudaMemcpyAsync(host, grid, (size_t)nb * gbytes, cudaMemcpyDeviceToHost, st));
     }
     T->end(st);

@@ -31,7 +31,7 @@ int oz_inverse_resid(OZState* o, const void* F, bool f64, int nb, const void* fg
 // when real).  The double-float synthesis pencils go to pen (nb <= chunk functions of 16-byte elements), or,
 // when pen is null, to the state's own buffer (nb <= oz_fft_functions()).
 // host (non-null): the grids go to host memory instead; grid is then the device staging for all nb grids
-// (the generic FFT) and ring a device buffer of 2 OZ_SYNTH_PIECE grids (N = 64..512), whose copies to the host
+// (the grid form) and ring a device buffer of 2 OZ_SYNTH_PIECE grids (the spectral form), whose copies to the host
 // run under the FFT of the next pieces.
 constexpr int OZ_SYNTH_PIECE = 4;
 // join = false (host path): st does not wait for the last copies to the host (a later call's join, or the
@@ -47,12 +47,15 @@ int oz_chunk(const OZState* o);
 // Device bytes of the coefficients' digit image per column tile of 8 functions (the contraction's B operand).
 long long oz_image_bytes_per_column_tile(int L);
 
-// The spectral form of the residual step (N = 64..512): the forward's FFT in double-float and the residual in
+// The spectral form of the residual step (N <= 222, 256 or 512): the forward's FFT in double-float and the residual in
 // the pencil domain, r^ = FFT(f) - N^2 H(F), which is what the forward GEMM consumes -- no FP32 FFT of f or of
 // the residual.  oz_forward_fft: nb <= chunk sample grids f (complex64, or float32 when real) -> pencils
 // [fn][p][q][k] as hi (complex64) + lo (remainder).  oz_resid_pencils: hi := (hi + lo) - N^2 H(F) at every
 // pencil place the forward GEMM reads, for nb <= chunk coefficient sets F (as oz_inverse_resid).
+bool oz_spectral_supported(int N);
 bool oz_spectral(const OZState* o);
+// BF16 terms per operand of the correction's GEMM: 1 for powers of two, 3 for the other N, as their grid form has.
+int oz_correction_terms(const OZState* o);
 int oz_fft_functions(const OZState* o);
 int oz_forward_fft(OZState* o, const void* fgrid, bool real, int nb, float2* hi, float2* lo, cudaStream_t st,
                    StageTimer* T, std::string& err);

@@ -122,6 +122,12 @@ __host__ __device__ constexpr uint32_t idesc_bf16_mn(bool a_mn_major, int n, int
            ((uint32_t)(m >> 4) << 24);
 }
 
+// ... D = F32, A = B = FP16, both K-major.
+__host__ __device__ constexpr uint32_t idesc_f16_mn(int n, int m)
+{
+    return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+}
+
 // One thread of a converged warp.  The compiler then knows that a single thread issues the tcgen05 / TMA instructions behind
 // it, whose operands live in uniform registers: behind `lane == 0` it serialises each of them over the active threads, and an
 // MMA took 161 cycles to issue whatever its size, against 70 (N <= 128) to 129 (N = 256, the tensor pipe's rate) measured

@@ -64,7 +64,7 @@ extern "C" {
 /* plan flags */
 #define FFTSO3_FLAG_REFINE 0x1u /* FP32-data forward: one residual step F += forward(f - inverse(F)); the
                                    inverse of F and the difference f - inverse(F) are formed in FP64 or exactly
-                                   (SO(3), l_max <= 255: digit sums on the tensor cores; for N = 64..512 the
+                                   (SO(3), l_max <= 255: digit sums on the tensor cores; for N <= 222, 256, 512 the
                                    step runs in the pencil domain on a double-float FFT of the samples), so the
                                    correction removes the first forward's FP32 FFT and contraction errors.
                                    Environment at plan creation: FFTSO3_REFINE_FP64=1 keeps the FP64 inverse;
@@ -155,7 +155,7 @@ int fftso3_inverse(fftso3_plan* plan, const void* coeffs, void* grid, void* stre
  * coefficients to the device in bulk; its grids are copied out (or, for plain
  * plans and pinned buffers, written in place by the kernels over the host
  * link).  Refined forwards copy the samples in pieces of a few functions under
- * the FFT of the previous piece; exact inverses (SO(3), N = 64..512) run in
+ * the FFT of the previous piece; exact inverses (SO(3), N <= 222, 256, 512) run in
  * chunks of 8 functions whose grids stream out through a small device ring
  * on an internal copy stream while the next chunk is computed. */
 int fftso3_forward_host(fftso3_plan* plan, const void* grid_host, void* coeffs_host, void* stream);
