@@ -35,6 +35,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <cstddef>
 #include <cstdlib>
 #include <map>
 #include <mutex>
@@ -166,6 +167,10 @@ struct GemmArgs {
     float2* pout;              // inverse: output pencils H'[fn][p][q][k]
     const float* wf;           // forward: quadrature weights (FP32)
     int* err;
+    // real functions: the summed pairs have their pencils at q < N / 2 (by_q) or p < N / 2 (S^2: always); the FFT writes and
+    // reads those alone (half)
+    int by_q, half;
+    int half_coeffs;           // ... and forward: only the coefficients of pairs 0 and 2 (n0 < 0: 3), m >= 0, are written
 };
 
 // One plan's share of a fused launch over several plans (the l_max buckets of
@@ -232,6 +237,17 @@ __device__ __forceinline__ GroupPairs s2_pairs(int m)
     return p;
 }
 
+// Real functions: the pair that column pair j of a group sums (its partner, with the conjugate sum, is the pair ^ 1).
+template <bool FWD, bool S2>
+__device__ __forceinline__ int herm_pair(const GroupPairs& P, int n0, int j, int by_q)
+{
+    // forward pencils lie at (-m, -n) mod N, inverse ones at (m, n); S^2: forward bins at m for pair 0, inverse at m for pair 1
+    if (S2) return FWD || P.np == 1 ? 0 : 1;
+    if (by_q) return j == 0 ? ((FWD ? n0 > 0 : n0 < 0) ? 1 : 0) : FWD ? 3 : 2;
+    if (j == 0) return FWD && P.np > 1 ? 1 : 0;
+    return FWD ? (n0 > 0 ? 3 : 2) : (n0 >= 0 ? 2 : 3);
+}
+
 // FWD = true: A = table (K-major, rows l), B = X from pencils; D[l][c].
 // FWD = false: A = table^T (MN-major, rows k), B = Y from coefficients; D[k][c].
 // S2 = false: SO(3) Wigner-d groups, pencils [fn][p][q][k], 4 pairs per function;
@@ -247,7 +263,12 @@ __device__ __forceinline__ GroupPairs s2_pairs(int m)
 // done with it (multicast commits; empty barriers count C).
 // TERMS: BF16 terms per operand, 3 (split-BF16, six products) or 1 (one product: a refinement's correction,
 // whose input is small, needs no more)
-template <bool FWD, bool S2, bool FUSED, int TERMS = 3>
+// HERM: real functions: of each two pairs (m, n), (-m, -n), whose sums are conjugates, only one is summed, the one whose pencil
+// lies in the half that the FFT makes (args.by_q): half the columns, so twice the functions a tile.  Both coefficients are
+// written, and both pencils unless the FFT reads one half alone (args.half; of two pairs in q = 0 or p = 0 still both).
+// 1.60 ms against 3.03 (forward) and 1.86 against 3.01 (S^2, l_max 511, 512 functions), 0.24 against 0.43 and 0.22 against 0.27
+// (SO(3), l_max 63, 64 functions).
+template <bool FWD, bool S2, bool FUSED, int TERMS = 3, bool HERM = false>
 __global__ void __launch_bounds__(THREADS, 1)
     so3_tc_gemm_kernel(const __grid_constant__ CUtensorMap tA0, const __grid_constant__ CUtensorMap tA1,
                        const __grid_constant__ CUtensorMap tA2, const __grid_constant__ GemmArgs args,
@@ -264,7 +285,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     float* wsm = (float*)(smem + STAGES * STAGE_BYTES + 256);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    constexpr int PPF = S2 ? 2 : 4;        // pairs per function
+    constexpr int PPF = (S2 ? 2 : 4) / (HERM ? 2 : 1);  // pairs summed per function
     constexpr int FPTK = BN / (2 * PPF);   // functions per column tile
     // per-item arguments and column tile
     auto argsof = [&](const int4& it) -> const GemmArgs& { return FUSED ? segs[it.z >> 16].a : args; };
@@ -496,16 +517,17 @@ __global__ void __launch_bounds__(THREADS, 1)
             r.N = N;
             r.wf = A.wf;
             r.p = nullptr;
-            if (f >= A.batch || pp >= P.np) return r;
+            const int pr = HERM ? herm_pair<FWD, S2>(P, n0, pp, A.by_q) : pp;
+            if (f >= A.batch || pr >= P.np) return r;
             if (FWD && S2) {
-                const int bin = pp == 0 ? m0 : N - m0;
+                const int bin = pr == 0 ? m0 : N - m0;
                 r.p = A.pin + (long long)f * A.fstride + (long long)bin * N;
             } else if (FWD) {
-                int pi = (-P.m[pp]) % N; if (pi < 0) pi += N;
-                int qi = (-P.n[pp]) % N; if (qi < 0) qi += N;
+                int pi = (-P.m[pr]) % N; if (pi < 0) pi += N;
+                int qi = (-P.n[pr]) % N; if (qi < 0) qi += N;
                 r.p = A.pin + (long long)f * A.fstride + ((long long)pi * N + qi) * N;
             } else {
-                r.p = A.cin + (long long)f * A.cstride + aux.x + (long long)pp * r.lim;
+                r.p = A.cin + (long long)f * A.cstride + aux.x + (long long)pr * r.lim;
             }
             return r;
         };
@@ -648,6 +670,21 @@ __global__ void __launch_bounds__(THREADS, 1)
                     poff[p] = ((long long)pi * N + qi) * N;
                 }
             }
+            // HERM: where each summed pair's value goes, and its conjugate (-1: nowhere)
+            long long h1[PPF], h2[PPF];
+            float hs1[PPF], hs2[PPF];
+            if (HERM) {
+#pragma unroll
+                for (int p = 0; p < PPF; ++p) {
+                    const int pr = herm_pair<FWD, S2>(P, n0, p, A.by_q), pc = pr ^ 1;
+                    const bool in = pr < P.np, both = in && pc < P.np && (FWD || !A.half || (!S2 && (A.by_q ? P.n[pc] : P.m[pc]) == 0));
+                    const int kept = p == 0 ? 0 : n0 >= 0 ? 2 : 3;
+                    h1[p] = in && !(FWD && A.half_coeffs && pr != kept) ? poff[pr] : -1;
+                    h2[p] = both && !(FWD && A.half_coeffs && pc != kept) ? poff[pc] : -1;
+                    hs1[p] = in ? (float)P.sign[pr] : 0.f;
+                    hs2[p] = both ? (float)P.sign[pc] : 0.f;
+                }
+            }
             const int ab = t & 1;
             if (!mbar_wait(&accf[ab], (t >> 1) & 1, args.err, 5)) {
                 *abort_flag = 1;
@@ -668,6 +705,15 @@ __global__ void __launch_bounds__(THREADS, 1)
                         const int row = half ? item.y * BM + quarter * 16 + lane : item.y * BM + r;
                         if ((half && lane >= 16) || row >= nl) continue;
                         float2* Fo = A.cout + (long long)f * A.cstride + row;
+                        if (HERM) {
+#pragma unroll
+                            for (int p = 0; p < PPF; ++p) {
+                                const float x = v[fq * 2 * PPF + 2 * p], y = v[fq * 2 * PPF + 2 * p + 1];
+                                if (h1[p] >= 0) Fo[h1[p]] = make_float2(hs1[p] * x, hs1[p] * y);
+                                if (h2[p] >= 0) Fo[h2[p]] = make_float2(hs2[p] * x, -(hs2[p] * y));
+                            }
+                            continue;
+                        }
 #pragma unroll
                         for (int p = 0; p < 4; ++p) {
                             if (p >= P.np) break;
@@ -678,6 +724,15 @@ __global__ void __launch_bounds__(THREADS, 1)
                         const int k = item.y * BM + r;
                         if (k >= N) continue;
                         float2* Ho = A.pout + (long long)f * A.fstride + k;
+                        if (HERM) {
+#pragma unroll
+                            for (int p = 0; p < PPF; ++p) {
+                                const float x = v[fq * 2 * PPF + 2 * p], y = v[fq * 2 * PPF + 2 * p + 1];
+                                if (h1[p] >= 0) Ho[h1[p]] = make_float2(x, y);
+                                if (h2[p] >= 0) Ho[h2[p]] = make_float2(x, -y);
+                            }
+                            continue;
+                        }
 #pragma unroll
                         for (int p = 0; p < 4; ++p) {
                             if (p >= P.np) break;
@@ -1108,6 +1163,7 @@ struct TCState {
     int csize = 1;                 // CTAs per cluster of the tensor-core GEMM launches (shared table tiles)
     bool refine = false;
     bool real = false;            // real grids (FFTSO3_*_REAL): real samples in, real part out
+    bool herm = false;            // real functions on the tensor cores: one GEMM pair of two (see the kernel)
     bool s2 = false;              // S^2 (Legendre groups g = m, grids N^2) instead of SO(3)
     bool simt = false;            // FP32 CUDA-core beta-sum (FFTSO3_PREC_FP32) instead of tcgen05
     float* d_tab32 = nullptr;     // FP32 table [row][Kp] (simt)
@@ -1143,6 +1199,8 @@ struct TCState {
     int2* d_iaux_inv = nullptr;
     int nsm = 0;
     CUtensorMap tmA_fwd[3], tmA_inv[3];
+    // the FFT passes write and read half of the pencils (the generic line FFTs all of them)
+    bool half_pencils() const { return herm && (direct || fft_fast_supported(N)); }
     int* d_err = nullptr;
     long long bytes = 0;
 };
@@ -1309,10 +1367,12 @@ int tc_create(TCState** out, int L, int N, int batch, const double* d_table_fp64
         delete s;
         return FFTSO3_ERR_UNSUPPORTED;
     }
-    s->ntiles = s2 ? (batch + FPT_S2 - 1) / FPT_S2 : (batch + FPT - 1) / FPT;
     s->ngroups = s2 ? s->B : s->B * s->B;
     s->refine = refine;
     s->real = real;
+    s->herm = real && !simt;
+    const int fpt = (s2 ? FPT_S2 : FPT) * (s->herm ? 2 : 1);
+    s->ntiles = (batch + fpt - 1) / fpt;
     make_fft_factors_prime_first(N, s->fac);
     s->d_tw = d_tw;
     s->total_rows = table_elems / N;
@@ -1367,7 +1427,7 @@ int tc_create(TCState** out, int L, int N, int batch, const double* d_table_fp64
         s->dft_tc = s->direct && !s2 && !simt && dft_tc_supported(N);
     }
     if (s->fused_fft) {
-        s->ring_elems = fft_grid_fused_ring_elems(N);
+        s->ring_elems = fft_grid_fused_ring_elems(N, s->herm);
         if ((rc = tc_alloc(s, (void**)&s->d_ring, sizeof(float2) * s->ring_elems, err))) return bail(rc);
         if ((rc = tc_alloc(s, (void**)&s->d_fctl, sizeof(int) * fft_grid_fused_ctl_ints(batch, N), err)))
             return bail(rc);
@@ -1458,13 +1518,18 @@ int tc_create(TCState** out, int L, int N, int batch, const double* d_table_fp64
         }
     }
     cudaError_t e = cudaSuccess;
-    const void* kernels[9] = {
+    const void* kernels[18] = {
         (const void*)so3_tc_gemm_kernel<true, false, false>, (const void*)so3_tc_gemm_kernel<false, false, false>,
         (const void*)so3_tc_gemm_kernel<true, true, false>,  (const void*)so3_tc_gemm_kernel<false, true, false>,
         (const void*)so3_tc_gemm_kernel<true, false, true>,  (const void*)so3_tc_gemm_kernel<false, false, true>,
         (const void*)so3_tc_gemm_kernel<true, true, true>,   (const void*)so3_tc_gemm_kernel<false, true, true>,
-        (const void*)so3_tc_gemm_kernel<true, false, false, 1>};
-    for (int i = 0; i < 9 && e == cudaSuccess; ++i)
+        (const void*)so3_tc_gemm_kernel<true, false, false, 1>,
+        (const void*)so3_tc_gemm_kernel<true, false, false, 3, true>, (const void*)so3_tc_gemm_kernel<false, false, false, 3, true>,
+        (const void*)so3_tc_gemm_kernel<true, true, false, 3, true>,  (const void*)so3_tc_gemm_kernel<false, true, false, 3, true>,
+        (const void*)so3_tc_gemm_kernel<true, false, true, 3, true>,  (const void*)so3_tc_gemm_kernel<false, false, true, 3, true>,
+        (const void*)so3_tc_gemm_kernel<true, true, true, 3, true>,   (const void*)so3_tc_gemm_kernel<false, true, true, 3, true>,
+        (const void*)so3_tc_gemm_kernel<true, false, false, 1, true>};
+    for (int i = 0; i < 18 && e == cudaSuccess; ++i)
         e = cudaFuncSetAttribute(kernels[i], cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     if (e != cudaSuccess) {
         err = std::string("tensor-core kernel attributes: ") + cudaGetErrorString(e);
@@ -1698,7 +1763,25 @@ static GemmArgs gemm_args(const TCState* s)
     a.pout = nullptr;
     a.wf = s->d_wf;
     a.err = s->d_err;
+    a.half = s->half_pencils();
+    a.by_q = !s->dft_tc;
+    a.half_coeffs = 0;
     return a;
+}
+
+template <bool HERM>
+static auto gemm_kernel(bool fwd, bool s2, int terms)
+{
+    return fwd ? (s2 ? so3_tc_gemm_kernel<true, true, false, 3, HERM>
+                     : (terms == 1 ? so3_tc_gemm_kernel<true, false, false, 1, HERM>
+                                   : so3_tc_gemm_kernel<true, false, false, 3, HERM>))
+               : (s2 ? so3_tc_gemm_kernel<false, true, false, 3, HERM> : so3_tc_gemm_kernel<false, false, false, 3, HERM>);
+}
+template <bool HERM>
+static auto fused_gemm_kernel(bool fwd, bool s2)
+{
+    return fwd ? (s2 ? so3_tc_gemm_kernel<true, true, true, 3, HERM> : so3_tc_gemm_kernel<true, false, true, 3, HERM>)
+               : (s2 ? so3_tc_gemm_kernel<false, true, true, 3, HERM> : so3_tc_gemm_kernel<false, false, true, 3, HERM>);
 }
 
 // cout: the forward's group-major output (default: the plan's d_fg); terms: 1 selects the one-term kernel (SO(3)
@@ -1729,10 +1812,7 @@ static int launch_gemm(TCState* s, bool fwd, cudaStream_t st, std::string& err, 
         return FFTSO3_SUCCESS;
     }
     const CUtensorMap* tm = fwd ? s->tmA_fwd : s->tmA_inv;
-    auto kern = fwd ? (s->s2 ? so3_tc_gemm_kernel<true, true, false>
-                             : (terms == 1 ? so3_tc_gemm_kernel<true, false, false, 1>
-                                           : so3_tc_gemm_kernel<true, false, false>))
-                    : (s->s2 ? so3_tc_gemm_kernel<false, true, false> : so3_tc_gemm_kernel<false, false, false>);
+    auto kern = s->herm ? gemm_kernel<true>(fwd, s->s2, terms) : gemm_kernel<false>(fwd, s->s2, terms);
     if (s->csize == 1) {
         const int nctas = a.nitems < s->nsm ? a.nitems : s->nsm;
         kern<<<nctas, THREADS, SMEM_BYTES, st>>>(tm[0], tm[1], tm[2], a, nullptr);
@@ -1772,7 +1852,7 @@ static long long grid_per_fn(const TCState* s) { return (long long)s->N * s->N *
 static cudaError_t direct_pass(TCState* s, const void* in, void* out, int pass, cudaStream_t st)
 {
     return s->dft_tc ? launch_dft_tc_grid_pass(in, out, s->batch, s->N, pass, s->real, s->d_dft, s->d_err, st)
-                     : launch_direct_grid_pass(in, out, s->batch, s->N, pass, s->real, s->d_dft, st);
+                     : launch_direct_grid_pass(in, out, s->batch, s->N, pass, s->real, s->herm, s->d_dft, st);
 }
 
 // grid -> k-contiguous pencils (SO(3): [fn][p][q][k], S^2: [fn][p][k]); grid is
@@ -1785,19 +1865,19 @@ static int fft_forward(TCState* s, const void* grid, cudaStream_t st, StageTimer
         if (s->fused_fft) {
             T->begin(ST_FFT_2D, st);
             TCK(launch_fft_grid_fused(grid, s->d_pencil, s->d_ring, s->ring_elems, s->d_fctl, s->d_err, s->batch, s->N, 1, s->d_tw,
-                                      st, s->real));
+                                      st, s->real, s->herm));
             T->end(st);
             return FFTSO3_SUCCESS;
         }
         T->begin(ST_FFT_ROWS, st);
         if (s->s2)
-            TCK(launch_fft_s2_pass(grid, s->d_pencil, s->batch, s->N, 1, s->d_tw, st, s->real));
+            TCK(launch_fft_s2_pass(grid, s->d_pencil, s->batch, s->N, 1, s->d_tw, st, s->real, s->herm));
         else
-            TCK(launch_fft_grid_pass(grid, s->d_work, s->batch, s->N, 1, s->d_tw, st, s->real));
+            TCK(launch_fft_grid_pass(grid, s->d_work, s->batch, s->N, 1, s->d_tw, st, s->real, s->herm));
         T->end(st);
         if (!s->s2) {
             T->begin(ST_FFT_COLS, st);
-            TCK(launch_fft_grid_pass(s->d_work, s->d_pencil, s->batch, s->N, 2, s->d_tw, st));
+            TCK(launch_fft_grid_pass(s->d_work, s->d_pencil, s->batch, s->N, 2, s->d_tw, st, false, s->herm));
             T->end(st);
         }
         return FFTSO3_SUCCESS;
@@ -1805,7 +1885,7 @@ static int fft_forward(TCState* s, const void* grid, cudaStream_t st, StageTimer
     if (s->direct) {
         T->begin(ST_FFT_ROWS, st);
         if (s->s2)
-            TCK(launch_direct_s2_pass(grid, s->d_pencil, s->batch, s->N, 1, s->real, s->d_dft, st));
+            TCK(launch_direct_s2_pass(grid, s->d_pencil, s->batch, s->N, 1, s->real, s->herm, s->d_dft, st));
         else
             TCK(direct_pass(s, grid, s->d_work, 1, st));
         T->end(st);
@@ -1840,22 +1920,22 @@ static int fft_inverse(TCState* s, void* grid, cudaStream_t st, StageTimer* T, s
     if (fft_fast_supported(s->N)) {
         if (s->s2) {
             T->begin(ST_FFT_ROWS, st);
-            TCK(launch_fft_s2_pass(s->d_pencil, grid, s->batch, s->N, -1, s->d_tw, st, s->real));
+            TCK(launch_fft_s2_pass(s->d_pencil, grid, s->batch, s->N, -1, s->d_tw, st, s->real, s->herm));
             T->end(st);
             return FFTSO3_SUCCESS;
         }
         if (s->fused_fft) {
             T->begin(ST_FFT_2D, st);
             TCK(launch_fft_grid_fused(s->d_pencil, grid, s->d_ring, s->ring_elems, s->d_fctl, s->d_err, s->batch, s->N, -1, s->d_tw,
-                                      st, s->real));
+                                      st, s->real, s->herm));
             T->end(st);
             return FFTSO3_SUCCESS;
         }
         T->begin(ST_FFT_COLS, st);
-        TCK(launch_fft_grid_pass(s->d_pencil, s->d_work, s->batch, s->N, -2, s->d_tw, st));
+        TCK(launch_fft_grid_pass(s->d_pencil, s->d_work, s->batch, s->N, -2, s->d_tw, st, false, s->herm));
         T->end(st);
         T->begin(ST_FFT_ROWS, st);
-        TCK(launch_fft_grid_pass(s->d_work, grid, s->batch, s->N, -1, s->d_tw, st, s->real));
+        TCK(launch_fft_grid_pass(s->d_work, grid, s->batch, s->N, -1, s->d_tw, st, s->real, s->herm));
         T->end(st);
         return FFTSO3_SUCCESS;
     }
@@ -1867,7 +1947,7 @@ static int fft_inverse(TCState* s, void* grid, cudaStream_t st, StageTimer* T, s
         }
         T->begin(ST_FFT_ROWS, st);
         if (s->s2)
-            TCK(launch_direct_s2_pass(s->d_pencil, grid, s->batch, s->N, -1, s->real, s->d_dft, st));
+            TCK(launch_direct_s2_pass(s->d_pencil, grid, s->batch, s->N, -1, s->real, s->herm, s->d_dft, st));
         else
             TCK(direct_pass(s, s->d_work, grid, -1, st));
         T->end(st);
@@ -1923,7 +2003,7 @@ static int tc_forward_once(TCState* s, const void* grid, float2* F, cudaStream_t
 static cudaError_t zero_nyquist_pencils(TCState* s, cudaStream_t st)
 {
     const long long N = s->N;
-    if (s->direct) return cudaSuccess;
+    if (s->direct || (s->s2 && s->half_pencils())) return cudaSuccess;
     if (s->s2) {
         const long long tot = (long long)s->batch * N;
         s2_zero_nyquist_pencils_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(s->d_pencil, (int)N, s->batch);
@@ -1938,7 +2018,7 @@ static cudaError_t zero_nyquist_pencils(TCState* s, cudaStream_t st)
 static int tc_inverse_once(TCState* s, const float2* F, void* grid, cudaStream_t st, StageTimer* T,
                            std::string& err, const void* real_in = nullptr)
 {
-    if (!s->direct) {
+    if (!s->direct && !(s->s2 && s->half_pencils())) {
         T->begin(ST_NYQUIST, st);
         TCK(zero_nyquist_pencils(s, st));
         T->end(st);
@@ -2255,7 +2335,7 @@ int tc_fused_create(TCFused** out, const std::vector<TCState*>& parts, std::stri
         return FFTSO3_ERR_INVALID_ARG;
     }
     for (TCState* p : parts)
-        if (!p || p->simt || p->s2 != parts[0]->s2 || p->ntiles > 0xFFFF) {
+        if (!p || p->simt || p->s2 != parts[0]->s2 || p->herm != parts[0]->herm || p->ntiles > 0xFFFF) {
             err = "fused launch: all plans must be tensor-core plans of one family (SO(3) or S^2)";
             return FFTSO3_ERR_INVALID_ARG;
         }
@@ -2339,14 +2419,8 @@ int tc_fused_gemm(TCFused* f, bool fwd, cudaStream_t st, StageTimer* T, std::str
     const int nctas = a.nitems < f->nsm ? a.nitems : f->nsm;
     const CUtensorMap* tm = fwd ? f->parts[0]->tmA_fwd : f->parts[0]->tmA_inv;  // unused by fused kernels
     T->begin(fwd ? ST_GEMM_FWD : ST_GEMM_INV, st);
-    if (fwd && f->s2)
-        so3_tc_gemm_kernel<true, true, true><<<nctas, THREADS, SMEM_BYTES, st>>>(tm[0], tm[1], tm[2], a, f->d_segs[d]);
-    else if (fwd)
-        so3_tc_gemm_kernel<true, false, true><<<nctas, THREADS, SMEM_BYTES, st>>>(tm[0], tm[1], tm[2], a, f->d_segs[d]);
-    else if (f->s2)
-        so3_tc_gemm_kernel<false, true, true><<<nctas, THREADS, SMEM_BYTES, st>>>(tm[0], tm[1], tm[2], a, f->d_segs[d]);
-    else
-        so3_tc_gemm_kernel<false, false, true><<<nctas, THREADS, SMEM_BYTES, st>>>(tm[0], tm[1], tm[2], a, f->d_segs[d]);
+    auto kern = f->parts[0]->herm ? fused_gemm_kernel<true>(fwd, f->s2) : fused_gemm_kernel<false>(fwd, f->s2);
+    kern<<<nctas, THREADS, SMEM_BYTES, st>>>(tm[0], tm[1], tm[2], a, f->d_segs[d]);
     TCK(cudaGetLastError());
     T->end(st);
     return FFTSO3_SUCCESS;
@@ -2487,6 +2561,16 @@ int tc_fused_phases(TCFused* f, const std::vector<long long>& g0, const std::vec
             f->bytes = (long long)(tab + sizeof(float2) * work);
         }
     }
+    // these directions' pencils: the tensor-core DFT's p <= N / 2, or the slice FFT's, all of them; their conversions read and
+    // write the coefficients of m >= 0 alone
+    const int mode[3] = {0, f->dft.segs && f->parts[0]->herm, f->parts[0]->herm};
+    static_assert(offsetof(GemmArgs, half) == offsetof(GemmArgs, by_q) + sizeof(int) &&
+                      offsetof(GemmArgs, half_coeffs) == offsetof(GemmArgs, half) + sizeof(int), "copied together");
+    for (size_t i = 0; i < 2 * n; ++i)
+        if ((e = cudaMemcpy(&f->d_segs[i & 1][i / 2].a.by_q, mode, sizeof(mode), cudaMemcpyHostToDevice)) != cudaSuccess) {
+            err = std::string("fused phases: ") + cudaGetErrorString(e);
+            return FFTSO3_ERR_CUDA;
+        }
     f->nbseg = (int)segs.size();
     f->nblk = blk;
     f->ncblk = cblk;

@@ -67,7 +67,6 @@ struct Geo {
     long long i_f, i_a, i_e;  // input: function, o (or y), element strides
     long long o_f, o_a, o_e;  // output: function, o (or x), element strides
     int nyq;             // element P is taken as zero
-    int mirror;          // COMPLEX, straight: outputs of 0 < o < P also go conjugated to (N - o, N - q)
     int ext;             // batches: in (1) or out (2) is a byte offset into the caller's buffer
 };
 // A launch: one pass of one plan, or both passes of a direction of several plans (segments ascending in N and tile0).
@@ -285,18 +284,6 @@ __device__ __forceinline__ void finish(const Geo& a, void* dst, const Line& L, u
 #pragma unroll
     for (int i = 0; i < 16; ++i)
         if (FULL || (i >= h0 && i < h1)) *reinterpret_cast<float*>(hi + (unsigned long long)(15 - i) * step) = C[i] - S[i];
-    if (KIND == COMPLEX && !TR && a.mirror && L.o > 0 && L.o < P) {
-        // (o, q) -> (N - o, N - q) and (o, N - q) -> (N - o, q), conjugated
-        const long long mo = 8 * (long long)(N - 2 * L.o) * a.o_a;
-        const float sg = part ? -1.f : 1.f;
-#pragma unroll
-        for (int i = 0; i < 16; ++i)
-            if (FULL || (i >= h0 && i < nv))
-                *reinterpret_cast<float*>(hi + mo + (unsigned long long)(15 - i) * step) = sg * (C[i] + S[i]);
-#pragma unroll
-        for (int i = 0; i < 16; ++i)
-            if (FULL || i < h1) *reinterpret_cast<float*>(lo + mo + (unsigned long long)i * step) = sg * (C[i] - S[i]);
-    }
 }
 
 // What the roles of a CTA share.
@@ -729,7 +716,6 @@ static bool geometry(Geo& a, const void* in, void* out, long long nf, int N, int
             a.i_a = a.o_a = NN;
             a.i_e = a.o_e = n;
             a.nyq = pass < 0;
-            a.mirror = pass > 0 && real;
             if (pass > 0) {
                 a.no = real ? P + 1 : N;
             } else {

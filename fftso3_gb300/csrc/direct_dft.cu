@@ -386,7 +386,7 @@ cudaError_t launch_direct_dft(const DirectPass& p, const void* table, cudaStream
     return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_direct_grid_pass(const void* in, void* out, long long nf, int N, int pass, bool real,
+cudaError_t launch_direct_grid_pass(const void* in, void* out, long long nf, int N, int pass, bool real, bool half,
                                     const void* table, cudaStream_t st)
 {
     const long long n = N, NN = n * n, NNN = NN * n;
@@ -412,7 +412,7 @@ cudaError_t launch_direct_grid_pass(const void* in, void* out, long long nf, int
         case 2:  // o = q, units k
             p.no = real ? B + 1 : N;
             p.ni = N;
-            p.mirror = real;
+            p.mirror = real && !half;
             side_in(n, NN, 1);
             side_out(n, 1, NN);
             break;
@@ -443,8 +443,8 @@ cudaError_t launch_direct_grid_pass(const void* in, void* out, long long nf, int
     return launch_direct_dft(p, table, st);
 }
 
-cudaError_t launch_direct_s2_pass(const void* in, void* out, long long nf, int N, int dir, bool real, const void* table,
-                                  cudaStream_t st)
+cudaError_t launch_direct_s2_pass(const void* in, void* out, long long nf, int N, int dir, bool real, bool half,
+                                  const void* table, cudaStream_t st)
 {
     const long long n = N, NN = n * n;
     DirectPass p = {in, out, N, DIRECT_COMPLEX, nf, 1, N, NN, 0, 0, 0, 0, NN, 0, 0, 0, 0, false, false, false};
@@ -455,7 +455,7 @@ cudaError_t launch_direct_s2_pass(const void* in, void* out, long long nf, int N
         p.o_u = 1;
         if (real) {
             p.kind = DIRECT_REAL_IN;
-            p.full = true;
+            p.full = !half;
             p.ni = N / 2;
             p.i_l = n;
             p.i_u = 2 * n;

@@ -165,11 +165,12 @@ cudaError_t launch_direct_dft(const DirectPass& p, const void* table, cudaStream
 // The passes of the SO(3) grid transforms over nf grids of N^3, as launch_fft_grid_pass but with its own layout of
 // the work grid: pass 1 grid [nf][k][j1][j2] -> work [nf][k][q][j1]; 2 work -> pencils [nf][p][q][k]; -2 pencils ->
 // work [nf][j1][q][k]; -1 work -> grid.  real: real samples in / real part out; the work grid then holds q <= N/2
-// only.  The inverse passes take the Nyquist bins p = N/2, q = N/2 as zero without reading them.
-cudaError_t launch_direct_grid_pass(const void* in, void* out, long long nf, int N, int pass, bool real,
+// only, and with half the pencils too (else pass 2 writes the others' conjugates as well).  The inverse passes take the Nyquist bins p = N/2, q = N/2 as zero without reading them.
+cudaError_t launch_direct_grid_pass(const void* in, void* out, long long nf, int N, int pass, bool real, bool half,
                                     const void* table, cudaStream_t st);
 // ... and of nf S^2 grids of N^2: dir 1 grid [nf][k][j] -> pencils [nf][p][k], dir -1 pencils -> grid (bin N/2 zero).
-cudaError_t launch_direct_s2_pass(const void* in, void* out, long long nf, int N, int dir, bool real, const void* table,
-                                  cudaStream_t st);
+// half (real): the pencils p <= N/2 alone are written (the inverse reads those in any case).
+cudaError_t launch_direct_s2_pass(const void* in, void* out, long long nf, int N, int dir, bool real, bool half,
+                                  const void* table, cudaStream_t st);
 
 }  // namespace fftso3

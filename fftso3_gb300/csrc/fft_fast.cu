@@ -372,10 +372,12 @@ __device__ __forceinline__ void l2_discard(const void* p)
 // pass -1 writes the real part only).  IN / OUT: access modes (IO_*) of the
 // side read and the side written; an IO_SCRATCH input is dropped from L2
 // once the tile holds it (every line of the ring is read by exactly one tile).
+// HALF (with REAL_IO): the transposed side holds the elements j < N / 2 alone; those past N / 2 are the conjugates of
+// N - j, and j = N / 2 is zero (the Nyquist bin, which no coefficient maps to).
 // T: staged tile [TL][LP] in shared memory; Ws: twiddles (staged, synchronised).
 // mid(): run by every thread right after the barrier between the two halves of
 // the tile (the input is consumed, no output written yet).
-template <int R, bool C2T, bool REAL_IO, int IN, int OUT, typename MID>
+template <int R, bool C2T, bool REAL_IO, bool HALF, int IN, int OUT, typename MID>
 __device__ __forceinline__ void tile_body(const float2* __restrict__ in, float2* __restrict__ out, long long cbase,
                                           long long tbase, long long Ls, long long Js, float2* T,
                                           const float2* Ws, uint64_t pol_in, uint64_t pol_out, MID mid)
@@ -383,8 +385,8 @@ __device__ __forceinline__ void tile_body(const float2* __restrict__ in, float2*
     constexpr int N = 32 * R;
     constexpr int LP = tile_lp<R, REAL_IO>();  // padded staged line
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    constexpr int NV = TL * N / 2 / (32 * PWARPS);  // float4 accesses per thread on the transposed side
-    static_assert(TL * N / 2 % (32 * PWARPS) == 0, "tile must split evenly over the threads");
+    constexpr int NV = TL * N / (HALF ? 4 : 2) / (32 * PWARPS);  // float4 accesses per thread on the transposed side
+    static_assert(NV > 0 && TL * N / (HALF ? 4 : 2) % (32 * PWARPS) == 0, "tile must split evenly over the threads");
     static_assert(!(REAL_IO && IN == IO_SCRATCH && C2T), "the ring holds complex lines");
     // REAL_IO: real lines 2p and 2p+1 share one complex transform (staged row p):
     // forward z = x_{2p} + i x_{2p+1}, X = (Z[k] + conj Z[-k]) / 2, Y = (Z[k] - conj Z[-k]) / 2i;
@@ -455,8 +457,12 @@ __device__ __forceinline__ void tile_body(const float2* __restrict__ in, float2*
             for (int q = 0; q < VB; ++q) {
                 const int e2 = threadIdx.x + (u0 + q) * 32 * PWARPS;
                 const int l = (e2 % (TL / 2)) * 2, j = e2 / (TL / 2);
-                if (REAL_IO) {
+                if (REAL_IO && HALF && j == 0) {
+                    T[(l / 2) * LP + ppos<R>(0)] = make_float2(buf[q].x, buf[q].z);
+                    T[(l / 2) * LP + ppos<R>(N / 2)] = make_float2(0.f, 0.f);
+                } else if (REAL_IO) {
                     T[(l / 2) * LP + ppos<R>(j)] = make_float2(buf[q].x - buf[q].w, buf[q].y + buf[q].z);
+                    if (HALF) T[(l / 2) * LP + ppos<R>(N - j)] = make_float2(buf[q].x + buf[q].w, buf[q].z - buf[q].y);
                 } else {
                     T[l * LP + ppos<R>(j)] = make_float2(buf[q].x, buf[q].y);
                     T[(l + 1) * LP + ppos<R>(j)] = make_float2(buf[q].z, buf[q].w);
@@ -466,7 +472,7 @@ __device__ __forceinline__ void tile_body(const float2* __restrict__ in, float2*
         __syncthreads();
         mid();
         if (IN == IO_SCRATCH)
-            for (int j = threadIdx.x; j < N; j += 32 * PWARPS) l2_discard(in + tbase + (long long)j * Js);
+            for (int j = threadIdx.x; j < (HALF ? N / 2 : N); j += 32 * PWARPS) l2_discard(in + tbase + (long long)j * Js);
         // contiguous output straight from registers: runs of R consecutive outputs per lane group
         for (int row = warp; row < TLI; row += PWARPS) {
             float2* Tl = T + row * LP;
@@ -495,7 +501,7 @@ __device__ __forceinline__ void tile_body(const float2* __restrict__ in, float2*
 
 // One pass over nf functions: the CTA index splits into (f, o < NO, bb < N / TL),
 // cbase = f FS + o Oc + bb TL Ls, tbase = f FS + o Ot + bb TL.
-template <int R, bool C2T, bool REAL_IO>
+template <int R, bool C2T, bool REAL_IO, bool HALF>
 __global__ void __launch_bounds__(32 * PWARPS, 3) fft_tile(const float2* __restrict__ in, float2* __restrict__ out,
                                                         const TileGeo g, const double2* __restrict__ tw)
 {
@@ -512,7 +518,7 @@ __global__ void __launch_bounds__(32 * PWARPS, 3) fft_tile(const float2* __restr
     const long long cbase = f * g.FS + o * g.Oc + bb * TL * g.Ls;
     const long long tbase = f * g.FS + o * g.Ot + bb * TL;
     __syncthreads();  // twiddles staged
-    tile_body<R, C2T, REAL_IO, IO_PLAIN, IO_PLAIN>(in, out, cbase, tbase, g.Ls, g.Js, T, Ws, 0, 0, [] {});
+    tile_body<R, C2T, REAL_IO, HALF, IO_PLAIN, IO_PLAIN>(in, out, cbase, tbase, g.Ls, g.Js, T, Ws, 0, 0, [] {});
 }
 
 // ---------------------------------------------------------------------------
@@ -591,28 +597,33 @@ __device__ __forceinline__ void red_add(int* p, int v)
 }
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
-// Claim order -> (phase, chunk, tile within the phase).
-__device__ __forceinline__ void decode_task(int t, int N, int C, int D, bool& phaseA, int& c, int& u)
+// Claim order -> (phase, chunk, tile within the phase); NA, NB: tiles of a chunk's phases.
+template <int NA, int NB>
+__device__ __forceinline__ void decode_task(int t, int C, int D, bool& phaseA, int& c, int& u)
 {
-    const int bi = t / N;
-    u = t - bi * N;
-    const int P = D < C ? D : C;
-    if (bi < P) {
+    const int P = D < C ? D : C, Q = C > D ? C - D : 0;
+    if (t < P * NA) {
         phaseA = true;
-        c = bi;
+        c = t / NA;
+        u = t - c * NA;
         return;
     }
-    const int j = bi - P, Q = C > D ? C - D : 0;
-    if (j < 2 * Q) {
-        phaseA = (j & 1) == 0;
-        c = (j >> 1) + (phaseA ? D : 0);
+    t -= P * NA;
+    const int j = t / (NA + NB);
+    if (j < Q) {
+        u = t - j * (NA + NB);
+        phaseA = u < NA;
+        c = j + (phaseA ? D : 0);
+        if (!phaseA) u -= NA;
         return;
     }
+    t -= Q * (NA + NB);
     phaseA = false;
-    c = Q + (j - 2 * Q);
+    c = Q + t / NB;
+    u = t - (c - Q) * NB;
 }
 
-template <int R, bool FWD, bool REAL_IO>
+template <int R, bool FWD, bool REAL_IO, bool HALF>
 __global__ void __launch_bounds__(32 * PWARPS, 3) fft_grid2d(const Grid2DArgs a, const double2* __restrict__ tw)
 {
     constexpr int N = 32 * R;
@@ -626,14 +637,17 @@ __global__ void __launch_bounds__(32 * PWARPS, 3) fft_grid2d(const Grid2DArgs a,
     load_tile_twiddles<R>(Ws, tw);
     const uint64_t pol_stream = l2_policy_first(), pol_keep = l2_policy_last();
     const int C = a.nchunks, D = a.look, S = a.nslots;
-    const int total = 2 * C * N;
+    // HALF: phase B forward / phase A inverse has the tiles q < N / 2 alone
+    constexpr int TA = !FWD && HALF ? N / 2 : N, TB = FWD && HALF ? N / 2 : N;
+    const int total = C * (TA + TB);
     int* const abort_flag = a.ctl + 1;
     int* const doneA = a.ctl + 2;
     int* const doneB = a.ctl + 2 + C;
 
     // thread-0 control state
     int nxt = -1, pend = -1, prev = -1, dv = 0;
-    const int* dptr = nullptr;  // dependency counter of nxt (null: none)
+    const int* dptr = nullptr;  // dependency counter of nxt (null: none) ..
+    int need = 0;               // .. and the count it waits for
     bool ready = true;
     // raw claim (checked against total where it is used, so the atomic's latency hides behind a tile)
     auto claim = [&]() -> int { return atomicAdd(a.ctl, 1); };
@@ -641,26 +655,27 @@ __global__ void __launch_bounds__(32 * PWARPS, 3) fft_grid2d(const Grid2DArgs a,
     auto dep_of = [&](int t) -> const int* {
         bool pa;
         int c, u;
-        decode_task(t, N, C, D, pa, c, u);
+        decode_task<TA, TB>(t, C, D, pa, c, u);
+        need = pa ? TB : TA;
         if (pa) return c >= S ? doneB + (c - S) : nullptr;
         return doneA + c;
     };
     auto signal = [&](int t) {  // after a fence (release pattern)
         bool pa;
         int c, u;
-        decode_task(t, N, C, D, pa, c, u);
+        decode_task<TA, TB>(t, C, D, pa, c, u);
         red_add(pa ? doneA + c : doneB + c, 1);
     };
     auto signal_release = [&](int t) {  // one release reduction
         bool pa;
         int c, u;
-        decode_task(t, N, C, D, pa, c, u);
+        decode_task<TA, TB>(t, C, D, pa, c, u);
         red_add_release(pa ? doneA + c : doneB + c, 1);
     };
-    // bounded wait for *p >= N (relaxed reads; the caller fences)
+    // bounded wait for *p >= need (relaxed reads; the caller fences)
     auto spin = [&](const int* p) -> bool {
         const long long t0 = clock64();
-        while (ld_relaxed(p) < N) {
+        while (ld_relaxed(p) < need) {
             if (*(volatile int*)abort_flag) return false;
             if (clock64() - t0 > WAIT_LIMIT) {
                 atomicCAS(a.err, 0, 9);
@@ -688,7 +703,7 @@ __global__ void __launch_bounds__(32 * PWARPS, 3) fft_grid2d(const Grid2DArgs a,
         if (t < 0) break;
         if (threadIdx.x == 0) {
             pend = nxt >= 0 ? claim() : -1;  // the tile after next
-            dv = dptr ? ld_acquire(dptr) : N;  // acquire: the next tile's reads are ordered after it
+            dv = dptr ? ld_acquire(dptr) : need;  // acquire: the next tile's reads are ordered after it
             // The next tile's input, if it comes from HBM (phase A), is prefetched into L2 by every
             // thread after the middle barrier, a half tile ahead: its loads then wait on L2 instead of
             // HBM.  Phase-B inputs (the ring) are in L2 already.
@@ -696,7 +711,7 @@ __global__ void __launch_bounds__(32 * PWARPS, 3) fft_grid2d(const Grid2DArgs a,
             if (a.prefetch && nxt >= 0) {
                 bool pa;
                 int cn, un;
-                decode_task(nxt, N, C, D, pa, cn, un);
+                decode_task<TA, TB>(nxt, C, D, pa, cn, un);
                 const long long fb = (long long)(cn / NB) * N3, kbn = cn % NB;
                 if (pa && FWD)  // TL contiguous grid rows of slice kbn TL + un / NB (as tile_body reads them)
                     pf = reinterpret_cast<const char*>(a.in) +
@@ -712,7 +727,7 @@ __global__ void __launch_bounds__(32 * PWARPS, 3) fft_grid2d(const Grid2DArgs a,
                 // barriers) are released by the reduction
                 if (prev >= 0) signal_release(prev);
                 prev = -1;
-                ready = nxt < 0 || dv >= N;
+                ready = nxt < 0 || dv >= need;
                 s_cur[(it + 1) & 1] = nxt;
                 s_slow = !ready;
             }
@@ -727,27 +742,27 @@ __global__ void __launch_bounds__(32 * PWARPS, 3) fft_grid2d(const Grid2DArgs a,
         };
         bool phaseA;
         int c, u;
-        decode_task(t, N, C, D, phaseA, c, u);
+        decode_task<TA, TB>(t, C, D, phaseA, c, u);
         const long long f = c / NB, kb = c % NB;
         float2* slot = a.ring + (long long)(c % S) * TL * N2;
         const long long fbase = f * N3;
         const int kl = u / NB, bb = u % NB, q = u;  // slice-type tile (kl, bb), q-type tile q
         if (FWD) {
             if (phaseA)
-                tile_body<R, true, REAL_IO, IO_STREAM, IO_SCRATCH>(
+                tile_body<R, true, REAL_IO, HALF, IO_STREAM, IO_SCRATCH>(
                     a.in, slot, fbase + (kb * TL + kl) * N2 + (long long)bb * TL * N, kl * N2 + bb * TL, N, N, T,
                     Ws, pol_stream, pol_keep, mid);
             else
-                tile_body<R, true, false, IO_SCRATCH, IO_STREAM>(slot, a.out, (long long)q * N,
+                tile_body<R, true, false, false, IO_SCRATCH, IO_STREAM>(slot, a.out, (long long)q * N,
                                                                   fbase + (long long)q * N + kb * TL, N2, N2, T, Ws,
                                                                   0, pol_stream, mid);
         } else {
             if (phaseA)
-                tile_body<R, false, false, IO_STREAM, IO_SCRATCH>(a.in, slot, (long long)q * N,
+                tile_body<R, false, false, false, IO_STREAM, IO_SCRATCH>(a.in, slot, (long long)q * N,
                                                                    fbase + (long long)q * N + kb * TL, N2, N2, T,
                                                                    Ws, pol_stream, pol_keep, mid);
             else
-                tile_body<R, false, REAL_IO, IO_SCRATCH, IO_STREAM>(
+                tile_body<R, false, REAL_IO, HALF, IO_SCRATCH, IO_STREAM>(
                     slot, a.out, fbase + (kb * TL + kl) * N2 + (long long)bb * TL * N, kl * N2 + bb * TL, N, N, T,
                     Ws, 0, pol_stream, mid);
         }
@@ -758,7 +773,7 @@ __global__ void __launch_bounds__(32 * PWARPS, 3) fft_grid2d(const Grid2DArgs a,
             // next tile's middle barrier.  Otherwise publish t first (it may be one of them) and wait.
             if (threadIdx.x == 0) {
                 bool published = false, ok = true;
-                if (ld_relaxed(dptr) < N) {
+                if (ld_relaxed(dptr) < need) {
                     fence_gpu();
                     signal(t);
                     published = true;
@@ -784,14 +799,14 @@ __global__ void __launch_bounds__(32 * PWARPS, 3) fft_grid2d(const Grid2DArgs a,
     }
 }
 
-template <int R, bool C2T, bool REAL_IO>
+template <int R, bool C2T, bool REAL_IO, bool HALF>
 static cudaError_t tile_r(const void* in, void* out, long long nf, const TileGeo& g, const void* tw, cudaStream_t st)
 {
     constexpr int N = 32 * R;
     constexpr int LP = tile_lp<R, REAL_IO>();
     constexpr int TLI = REAL_IO ? TL / 2 : TL;  // staged rows (real lines go in pairs)
     const size_t smem = sizeof(float2) * ((size_t)tile_tw_elems<R>() + (size_t)TLI * LP);
-    auto k = fft_tile<R, C2T, REAL_IO>;
+    auto k = fft_tile<R, C2T, REAL_IO, HALF>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     const long long nblk = nf * (long long)g.NO * (N / TL);
@@ -799,26 +814,27 @@ static cudaError_t tile_r(const void* in, void* out, long long nf, const TileGeo
     return cudaGetLastError();
 }
 
-template <bool C2T, bool REAL_IO>
+template <bool C2T, bool REAL_IO, bool HALF>
 static cudaError_t tile_dispatch(const void* in, void* out, long long nf, int N, const TileGeo& g, const void* tw,
                                  cudaStream_t st)
 {
     switch (N) {
-        case 64: return tile_r<2, C2T, REAL_IO>(in, out, nf, g, tw, st);
-        case 128: return tile_r<4, C2T, REAL_IO>(in, out, nf, g, tw, st);
-        case 256: return tile_r<8, C2T, REAL_IO>(in, out, nf, g, tw, st);
-        case 512: return tile_r<16, C2T, REAL_IO>(in, out, nf, g, tw, st);
-        case 1024: return tile_r<32, C2T, REAL_IO>(in, out, nf, g, tw, st);
+        case 64: return tile_r<2, C2T, REAL_IO, HALF>(in, out, nf, g, tw, st);
+        case 128: return tile_r<4, C2T, REAL_IO, HALF>(in, out, nf, g, tw, st);
+        case 256: return tile_r<8, C2T, REAL_IO, HALF>(in, out, nf, g, tw, st);
+        case 512: return tile_r<16, C2T, REAL_IO, HALF>(in, out, nf, g, tw, st);
+        case 1024: return tile_r<32, C2T, REAL_IO, HALF>(in, out, nf, g, tw, st);
         default: return cudaErrorNotSupported;
     }
 }
 
 template <bool C2T>
 static cudaError_t tile_any(const void* in, void* out, long long nf, int N, const TileGeo& g, const void* tw,
-                            cudaStream_t st, bool real_io)
+                            cudaStream_t st, bool real_io, bool half = false)
 {
-    return real_io ? tile_dispatch<C2T, true>(in, out, nf, N, g, tw, st)
-                   : tile_dispatch<C2T, false>(in, out, nf, N, g, tw, st);
+    if (real_io && half) return tile_dispatch<C2T, true, true>(in, out, nf, N, g, tw, st);
+    return real_io ? tile_dispatch<C2T, true, false>(in, out, nf, N, g, tw, st)
+                   : tile_dispatch<C2T, false, false>(in, out, nf, N, g, tw, st);
 }
 
 // Lookahead D and ring slots S for N on a device of nsm SMs: about W = 12 nsm
@@ -827,15 +843,15 @@ static cudaError_t tile_any(const void* in, void* out, long long nf, int N, cons
 // every dependency at least W tiles back (2 D + 1 and 2 (S - D) - 1 blocks of
 // N tiles).  At N = 512 D stays 1 so that the live slots (D + 1, 32 MB each)
 // fit in L2; the rare incomplete dependency then takes the slow path.
-static void fused_geometry(int N, int nsm, int& D, int& S)
+static void fused_geometry(int N, int nsm, bool half, int& D, int& S)
 {
-    const int W = 12 * nsm;
-    D = N >= 512 ? 1 : std::max(1, (W - N + 2 * N - 1) / (2 * N));
+    const int W = 12 * nsm, pair = half ? N + N / 2 : 2 * N;  // tiles of a chunk
+    D = N >= 512 ? 1 : std::max(1, (W - N + pair - 1) / pair);
     if (const char* ev = getenv("FFTSO3_FFT_LOOKAHEAD")) {  // tuning override of D (1..16)
         const int d = atoi(ev);
         if (d >= 1 && d <= 16) D = d;
     }
-    S = D + std::max(2, (W + N + 2 * N - 1) / (2 * N));
+    S = D + std::max(2, (W + N + pair - 1) / pair);
 }
 
 static int device_sms()
@@ -846,13 +862,13 @@ static int device_sms()
     return nsm;
 }
 
-template <int R, bool FWD, bool REAL_IO>
+template <int R, bool FWD, bool REAL_IO, bool HALF>
 static cudaError_t grid2d_r(const Grid2DArgs& a, long long tiles, const void* tw, cudaStream_t st)
 {
     // staged tile: 16 complex lines, or 8 rows of real pairs (phase A forward / phase B inverse)
     constexpr size_t rows = std::max<size_t>((size_t)TL * tile_lp<R, false>(), (size_t)(TL / 2) * tile_lp<R, true>());
     const size_t smem = sizeof(float2) * ((size_t)tile_tw_elems<R>() + rows);
-    auto k = fft_grid2d<R, FWD, REAL_IO>;
+    auto k = fft_grid2d<R, FWD, REAL_IO, HALF>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int dev = 0, nsm = 0, occ = 0;
@@ -864,14 +880,14 @@ static cudaError_t grid2d_r(const Grid2DArgs& a, long long tiles, const void* tw
     return cudaGetLastError();
 }
 
-template <bool FWD, bool REAL_IO>
+template <bool FWD, bool REAL_IO, bool HALF>
 static cudaError_t grid2d_dispatch(const Grid2DArgs& a, long long tiles, int N, const void* tw, cudaStream_t st)
 {
     switch (N) {
-        case 64: return grid2d_r<2, FWD, REAL_IO>(a, tiles, tw, st);
-        case 128: return grid2d_r<4, FWD, REAL_IO>(a, tiles, tw, st);
-        case 256: return grid2d_r<8, FWD, REAL_IO>(a, tiles, tw, st);
-        case 512: return grid2d_r<16, FWD, REAL_IO>(a, tiles, tw, st);
+        case 64: return grid2d_r<2, FWD, REAL_IO, HALF>(a, tiles, tw, st);
+        case 128: return grid2d_r<4, FWD, REAL_IO, HALF>(a, tiles, tw, st);
+        case 256: return grid2d_r<8, FWD, REAL_IO, HALF>(a, tiles, tw, st);
+        case 512: return grid2d_r<16, FWD, REAL_IO, HALF>(a, tiles, tw, st);
         default: return cudaErrorNotSupported;
     }
 }
@@ -909,26 +925,26 @@ cudaError_t launch_fft_rows_fast(const void* in, void* out, long long nlines, in
 //   pass 2': pencils [f][p][q][k] -> FFT over p  -> T1 [f][k][q][j1]
 //   pass 1': T1 [f][k][q][j1]     -> FFT over q  -> grid [f][k][j1][j2]
 cudaError_t launch_fft_grid_pass(const void* in, void* out, long long nf, int N, int pass, const void* tw,
-                                 cudaStream_t st, bool real_io)
+                                 cudaStream_t st, bool real_io, bool half)
 {
     const long long N1 = N, N2 = (long long)N * N, N3 = N2 * N;
     if (real_io && pass != 1 && pass != -1) return cudaErrorInvalidValue;
     const ffast::TileGeo g1{N3, N, N2, N1, N2, N1};  // lines along j2 / q, transposed (q, j1)
-    const ffast::TileGeo g2{N3, N, N1, N2, N1, N2};  // lines along j1 / p, transposed (p.., k)
+    const ffast::TileGeo g2{N3, half ? N / 2 : N, N1, N2, N1, N2};  // lines along j1 / p of each q, transposed (p.., k)
     switch (pass) {
-        case 1: return ffast::tile_any<true>(in, out, nf, N, g1, tw, st, real_io);
+        case 1: return ffast::tile_any<true>(in, out, nf, N, g1, tw, st, real_io, half);
         case 2: return ffast::tile_any<true>(in, out, nf, N, g2, tw, st, false);
         case -2: return ffast::tile_any<false>(in, out, nf, N, g2, tw, st, false);
-        case -1: return ffast::tile_any<false>(in, out, nf, N, g1, tw, st, real_io);
+        case -1: return ffast::tile_any<false>(in, out, nf, N, g1, tw, st, real_io, half);
         default: return cudaErrorInvalidValue;
     }
 }
 
 bool fft_grid_fused_supported(int N) { return N == 64 || N == 128 || N == 256 || N == 512; }
-size_t fft_grid_fused_ring_elems(int N)
+size_t fft_grid_fused_ring_elems(int N, bool half)
 {
     int D, S;
-    ffast::fused_geometry(N, ffast::device_sms(), D, S);
+    ffast::fused_geometry(N, ffast::device_sms(), half, D, S);
     return (size_t)S * ffast::TL * N * N;
 }
 size_t fft_grid_fused_ctl_ints(long long nf, int N) { return 2 + 2 * (size_t)nf * (N / ffast::TL); }
@@ -936,34 +952,38 @@ size_t fft_grid_fused_ctl_ints(long long nf, int N) { return 2 + 2 * (size_t)nf 
 // Both passes of one direction (dir 1: grid -> pencils, dir -1: pencils ->
 // grid) in one persistent launch through the L2-resident ring (fft_grid2d).
 cudaError_t launch_fft_grid_fused(const void* in, void* out, void* ring, size_t ring_elems, int* ctl, int* err,
-                                  long long nf, int N, int dir, const void* tw, cudaStream_t st, bool real_io)
+                                  long long nf, int N, int dir, const void* tw, cudaStream_t st, bool real_io, bool half)
 {
+    if (half && !real_io) return cudaErrorInvalidValue;
     if (!fft_grid_fused_supported(N) || (dir != 1 && dir != -1) || nf < 1) return cudaErrorInvalidValue;
     const long long C = nf * (N / ffast::TL);
     if (C > (1LL << 29) / N) return cudaErrorInvalidValue;  // tile indices stay in int
     cudaError_t e = cudaMemsetAsync(ctl, 0, sizeof(int) * fft_grid_fused_ctl_ints(nf, N), st);
     if (e != cudaSuccess) return e;
     int D, S;
-    ffast::fused_geometry(N, ffast::device_sms(), D, S);
+    ffast::fused_geometry(N, ffast::device_sms(), half, D, S);
     if ((size_t)S * ffast::TL * N * N > ring_elems) return cudaErrorInvalidValue;  // ring sized for another device
     const char* pf = getenv("FFTSO3_FFT_PREFETCH");  // 0 turns the next-tile L2 prefetch off (tuning)
     ffast::Grid2DArgs a{(const float2*)in, (float2*)out, (float2*)ring, ctl, err, (int)C, D, S,
                         pf && atoi(pf) == 0 ? 0 : 1};
-    const long long tiles = 2 * C * N;
+    const long long tiles = C * (half ? N + N / 2 : 2 * N);
+    if (half)
+        return dir == 1 ? ffast::grid2d_dispatch<true, true, true>(a, tiles, N, tw, st)
+                        : ffast::grid2d_dispatch<false, true, true>(a, tiles, N, tw, st);
     if (dir == 1)
-        return real_io ? ffast::grid2d_dispatch<true, true>(a, tiles, N, tw, st)
-                       : ffast::grid2d_dispatch<true, false>(a, tiles, N, tw, st);
-    return real_io ? ffast::grid2d_dispatch<false, true>(a, tiles, N, tw, st)
-                   : ffast::grid2d_dispatch<false, false>(a, tiles, N, tw, st);
+        return real_io ? ffast::grid2d_dispatch<true, true, false>(a, tiles, N, tw, st)
+                       : ffast::grid2d_dispatch<true, false, false>(a, tiles, N, tw, st);
+    return real_io ? ffast::grid2d_dispatch<false, true, false>(a, tiles, N, tw, st)
+                   : ffast::grid2d_dispatch<false, false, false>(a, tiles, N, tw, st);
 }
 
 cudaError_t launch_fft_s2_pass(const void* in, void* out, long long nf, int N, int dir, const void* tw,
-                               cudaStream_t st, bool real_io)
+                               cudaStream_t st, bool real_io, bool half)
 {
     const long long N1 = N, N2 = (long long)N * N;
     const ffast::TileGeo g{N2, 1, 0, N1, 0, N1};  // lines along j (contiguous), transposed [p][k]
-    if (dir == 1) return ffast::tile_any<true>(in, out, nf, N, g, tw, st, real_io);
-    if (dir == -1) return ffast::tile_any<false>(in, out, nf, N, g, tw, st, real_io);
+    if (dir == 1) return ffast::tile_any<true>(in, out, nf, N, g, tw, st, real_io, half);
+    if (dir == -1) return ffast::tile_any<false>(in, out, nf, N, g, tw, st, real_io, half);
     return cudaErrorInvalidValue;
 }
 

@@ -4,10 +4,10 @@
 // permutations, then the real-basis change so3_c2r / so3_r2c of contract_fp64.cu, fdcl_FFTSO3.cpp:1107-1139
 // for matrix2rsph); here one thread forms one output coefficient of any bucket from the entries it needs,
 // with the same arithmetic in the same order, so the results are the bucket plans' bit for bit:
-//   forward: packed F(l, m, n) from the group-major GEMM output (real kinds: Re(T F T^H), the four
-//            entries (l, +-m, +-n));
+//   forward: packed F(l, m, n) from the group-major GEMM output (real kinds: Re(T F T^H), of the four entries
+//            (l, +-m, +-n) the two of m >= 0, the others being their conjugates up to sign);
 //   inverse: group-major (2l + 1) sign F(l, m, n) of the pair at that place (real kinds: F = T^H F_r T from
-//            the four real entries (l, +-m, +-n)).
+//            the four real entries (l, +-m, +-n), for the pairs of m >= 0, which the contraction reads).
 // The group-major place of (l, m, n) and its inverse are closed-form (no table lookups), each CTA serves one
 // bucket, and the gathers stay inside one function's coefficients (a few MB at l_max = 64), which the
 // neighbouring threads of the launch read at the same time, so they are served by L2.
@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(CONVERT_THREADS) fused_group_to_packed_kernel(
         reinterpret_cast<float2*>(out)[S.c0 + u] = fg[gm_offset(l, m, n, B)];
         return;
     }
-    const float acc = real_coefficient<float, false>(m, n, [&](int a, int c) {
+    const float acc = real_coefficient<float, true>(m, n, [&](int a, int c) {
         const float2 v = fg[gm_offset(l, a, c, B)];
         return c2t<float>{v.x, v.y};
     });
@@ -102,6 +102,8 @@ __global__ void __launch_bounds__(CONVERT_THREADS) fused_packed_to_group_kernel(
     else { n0 = -m0 + 1 + (ri - 2) / 4; pp = (ri - 2) & 3; }
     // pair pp of group_pairs(m0, n0), without its table (which a dynamic index would put in local memory)
     const int sgn = ((m0 + n0) & 1) ? -1 : 1;
+    // real functions: the contraction reads one of each two conjugate pairs (herm_pair of contract_tc.cu by p: m >= 0)
+    if (REAL && (pp == 1 || pp == (n0 >= 0 ? 3 : 2))) return;
     const int m = pp == 0 ? m0 : pp == 1 ? -m0 : pp == 2 ? n0 : -n0;
     const int n = pp == 0 ? n0 : pp == 1 ? -n0 : pp == 2 ? m0 : -m0;
     const int psign = (pp == 1 || pp == 2) ? sgn : 1;
