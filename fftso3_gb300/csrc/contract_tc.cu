@@ -1417,7 +1417,10 @@ int tc_create(TCState** out, int L, int N, int batch, const double* d_table_fp64
     // (FFTSO3_TWO_PASS_FFT=1 in the environment selects the two-launch form, for comparison)
     {
         const char* ev = getenv("FFTSO3_TWO_PASS_FFT");
-        s->fused_fft = !s2 && fft_grid_fused_supported(N) && !(ev && ev[0] == '1');
+        // below 10 M samples the work grid stays in L2 by itself, and two launches beat one with dependencies (both
+        // directions, us: l_max 31, 4 functions, 1 M, 34 against 46; 16 functions, 4.2 M, 61 against 81; l_max 63, 4 functions,
+        // 8.4 M, 108 against 113; 64 functions, 134 M, 1270 against 1086)
+        s->fused_fft = !s2 && fft_grid_fused_supported(N) && gridel > 10000000 && !(ev && ev[0] == '1');
         // the direct DFT from half a million samples (S^2: a million; smaller batches are bound by launch latencies, where
         // the line FFT's simpler kernels win: l_max 16, 4 functions, 0.16 M samples, 76 against 81 us both directions;
         // l_max 38, 0.47 M, 125 against 119 us; l_max 30, 32 functions, 7.6 M, 524 against 361 us; S^2 l_max 47, 8 signals,
@@ -1920,19 +1923,19 @@ static int fft_inverse(TCState* s, void* grid, cudaStream_t st, StageTimer* T, s
     if (fft_fast_supported(s->N)) {
         if (s->s2) {
             T->begin(ST_FFT_ROWS, st);
-            TCK(launch_fft_s2_pass(s->d_pencil, grid, s->batch, s->N, -1, s->d_tw, st, s->real, s->herm));
+            TCK(launch_fft_s2_pass(s->d_pencil, grid, s->batch, s->N, -1, s->d_tw, st, s->real, s->herm, true));
             T->end(st);
             return FFTSO3_SUCCESS;
         }
         if (s->fused_fft) {
             T->begin(ST_FFT_2D, st);
             TCK(launch_fft_grid_fused(s->d_pencil, grid, s->d_ring, s->ring_elems, s->d_fctl, s->d_err, s->batch, s->N, -1, s->d_tw,
-                                      st, s->real, s->herm));
+                                      st, s->real, s->herm, true));
             T->end(st);
             return FFTSO3_SUCCESS;
         }
         T->begin(ST_FFT_COLS, st);
-        TCK(launch_fft_grid_pass(s->d_pencil, s->d_work, s->batch, s->N, -2, s->d_tw, st, false, s->herm));
+        TCK(launch_fft_grid_pass(s->d_pencil, s->d_work, s->batch, s->N, -2, s->d_tw, st, false, s->herm, true));
         T->end(st);
         T->begin(ST_FFT_ROWS, st);
         TCK(launch_fft_grid_pass(s->d_work, grid, s->batch, s->N, -1, s->d_tw, st, s->real, s->herm));
@@ -1999,11 +2002,12 @@ static int tc_forward_once(TCState* s, const void* grid, float2* F, cudaStream_t
     return FFTSO3_SUCCESS;
 }
 
-// The pencils of the Nyquist bins, which no coefficient maps to (the direct DFT's passes take them as zero themselves).
+// The pencils of the Nyquist bins, which no coefficient maps to (the direct DFT's and the power-of-two FFT's passes take them
+// as zero themselves).
 static cudaError_t zero_nyquist_pencils(TCState* s, cudaStream_t st)
 {
     const long long N = s->N;
-    if (s->direct || (s->s2 && s->half_pencils())) return cudaSuccess;
+    if (s->direct || fft_fast_supported(s->N)) return cudaSuccess;
     if (s->s2) {
         const long long tot = (long long)s->batch * N;
         s2_zero_nyquist_pencils_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(s->d_pencil, (int)N, s->batch);
@@ -2018,7 +2022,7 @@ static cudaError_t zero_nyquist_pencils(TCState* s, cudaStream_t st)
 static int tc_inverse_once(TCState* s, const float2* F, void* grid, cudaStream_t st, StageTimer* T,
                            std::string& err, const void* real_in = nullptr)
 {
-    if (!s->direct && !(s->s2 && s->half_pencils())) {
+    if (!s->direct && !fft_fast_supported(s->N)) {
         T->begin(ST_NYQUIST, st);
         TCK(zero_nyquist_pencils(s, st));
         T->end(st);

@@ -66,9 +66,10 @@ cudaError_t launch_fft_rows_fast(const void* in, void* out, long long nlines, in
 //   pass -2: pencils [nf][p][q][k] -> FFT over p -> T1 [nf][k][q][j1]
 //   pass -1: T1 [nf][k][q][j1]     -> FFT over q -> grid [nf][k][j1][j2]
 // real_io: pass 1 reads real samples (float), pass -1 writes the real part only.  half (real grids, all four passes): T1 and
-// the pencils hold q < N / 2 alone, as in launch_fft_grid_fused.
+// the pencils hold q < N / 2 alone, as in launch_fft_grid_fused.  nyq (pass -2): the Nyquist bins p = N / 2 and q = N / 2 are
+// taken as zero without being read (no coefficient maps to them).
 cudaError_t launch_fft_grid_pass(const void* in, void* out, long long nf, int N, int pass, const void* tw,
-                                 cudaStream_t st, bool real_io = false, bool half = false);
+                                 cudaStream_t st, bool real_io = false, bool half = false, bool nyq = false);
 // Both passes of one direction in one persistent launch (N = 64..512): dir 1
 // grid -> pencils (passes 1, 2), dir -1 pencils -> grid (passes -2, -1), the
 // intermediate held in a ring of ring_elems >= fft_grid_fused_ring_elems(N)
@@ -83,13 +84,13 @@ size_t fft_grid_fused_ring_elems(int N, bool half = false);
 size_t fft_grid_fused_ctl_ints(long long nf, int N);
 cudaError_t launch_fft_grid_fused(const void* in, void* out, void* ring, size_t ring_elems, int* ctl, int* err,
                                   long long nf, int N, int dir, const void* tw, cudaStream_t st,
-                                  bool real_io = false, bool half = false);
+                                  bool real_io = false, bool half = false, bool nyq = false);
 // Tiled pass over nf S^2 grids of N^2 complex64 (in != out):
 //   dir  1: grid [nf][k][j]     -> FFT over j -> pencils [nf][p][k]
 //   dir -1: pencils [nf][p][k]  -> FFT over p -> grid [nf][k][j]
 // real_io: dir 1 reads real samples, dir -1 writes the real part only.  half (with real_io): the pencils of p < N / 2
 // alone are written or read (a real function's others are their conjugates, its Nyquist bin is taken as zero).
 cudaError_t launch_fft_s2_pass(const void* in, void* out, long long nf, int N, int dir, const void* tw,
-                               cudaStream_t st, bool real_io = false, bool half = false);
+                               cudaStream_t st, bool real_io = false, bool half = false, bool nyq = false);
 
 }  // namespace fftso3

@@ -1,23 +1,20 @@
 // Register-resident FP32 FFT kernels for the tensor-core path, N = 32 R
 // (R = 2..32, i.e. N = 64..1024, powers of two).
 //
-// One warp transforms one line of N points: lane t holds x[t + 32 i],
-// i < R.  With n = t + 32 i and K = k1 + R k2,
-//   X[K] = sum_t w_N^{t k1} w_32^{t k2} sum_i x[t + 32 i] w_R^{i k1},
-// so each lane runs an R-point radix-2 DIF in registers, multiplies by the
-// twiddles w_N^{t k1}, and the warp finishes with a 32-point radix-2 DIF across
-// lanes (shuffles).  Lane t then holds X[brR(r) + R br5(t)] in register r,
-// i.e. R consecutive outputs.  Twiddles come from the host FP64 table
-// W[j] = e^{-2 pi i j / N}, staged in shared memory as FP32.
-//
 // Kernels:
-//   fft_rows_reg  lines contiguous (one axis of a contiguous array);
-//   fft_tile      a tile of 16 lines staged in shared memory with one side
-//                 contiguous and the other transposed, so a 2-D transform of
-//                 the Euler grid is two passes that both read and write whole
-//                 128-byte runs, the second one producing the k-contiguous
-//                 pencils [fn][p][q][k] the beta-sum GEMM consumes (and the
-//                 reverse for the inverse).
+//   fft_rows_reg  lines contiguous (one axis of a contiguous array): one warp a line, lane t holds x[t + 32 i], an
+//                 R-point DFT in registers, twiddles, a 32-point one across the lanes by shuffles;
+//   fft_tile      a tile of 16 lines with one side contiguous and the other transposed, so a 2-D transform of
+//                 the Euler grid is two passes that both read and write whole 128-byte runs, the second one
+//                 producing the k-contiguous pencils [fn][p][q][k] the beta-sum GEMM consumes (and the reverse
+//                 for the inverse); each line in two in-register DFTs around one exchange through shared memory,
+//                 which also transposes the tile;
+//   fft_grid2d    both passes of the Euler grid in one persistent launch, through an L2-resident ring.
+// Bound: latency and the loads in flight (N = 256: 55 % of the L1's and 50 % of DRAM's rate).  With the line FFT over a warp's
+// lanes (radix-2 butterflies with loaded twiddles, two exchanges and a shuffle stage, the tile staged in shared memory besides)
+// a sample took 75 instructions a pass and the L1 was at 71 to 86 %: l_max 127, 16 functions, 1.61 and 1.72 ms a direction
+// against 1.05 and 1.04 (268 M samples; DRAM's floor 0.63), l_max 63, 64 real functions 0.65 and 0.71 against 0.33 and 0.37,
+// S^2 l_max 511, 512 real functions 0.94 and 0.97 against 0.84 and 0.82.
 #include <algorithm>
 #include <cstdlib>
 
@@ -76,20 +73,55 @@ __device__ __forceinline__ void reg_dif(float2 (&v)[R], const float2* __restrict
     reg_dif_t<R>(v, [&](int k, int h) { return W[k * (N / (2 * h))]; });
 }
 
-// Twiddles of the tile kernels in shared memory, laid out for their accesses:
-//   Wa[k1 * 32 + t] = w_N^{t k1}  (t < 32, k1 < R): step A's per-lane twiddles, consecutive
-//                                 lanes on consecutive entries (free of bank conflicts);
-//   W32[x] = w_N^{R x} = w_32^x   (x < 32, at Wa + N): every other twiddle of the line FFT
-//                                 (warp-uniform, or two values per warp: broadcast reads).
-template <int R>
-__host__ __device__ constexpr int tile_tw_elems() { return 32 * R + 32; }
-template <int R>
-__device__ __forceinline__ void load_tile_twiddles(float2* Wt, const double2* __restrict__ tw)
+// cos(2 pi k / 32)
+__host__ __device__ constexpr float cos32(int k)
 {
-    constexpr int N = 32 * R;
-    for (int i = threadIdx.x; i < N + 32; i += blockDim.x) {
-        const int j = i < N ? (i & 31) * (i >> 5) : (i - N) * R;
-        Wt[i] = make_float2((float)tw[j].x, (float)tw[j].y);
+    constexpr double c[9] = {1.0, 0.98078528040323044913, 0.92387953251128675613, 0.83146961230254523708,
+                             0.70710678118654752440, 0.55557023301960222474, 0.38268343236508977173,
+                             0.19509032201612826785, 0.0};
+    k &= 31;
+    if (k > 16) k = 32 - k;
+    return k <= 8 ? (float)c[k] : -(float)c[16 - k];
+}
+
+// d w, w = e^{-2 pi i e / 32} a literal
+__device__ __forceinline__ float2 twiddle32(float2 d, int e)
+{
+    if (e == 0) return d;
+    if (e == 8) return make_float2(d.y, -d.x);
+    return cmulf(d, make_float2(cos32(e), -cos32(e - 8)));
+}
+
+// P-point DIF in registers with literal twiddles (P <= 32; natural input, bit-reversed output): radix-4 stages, which round
+// once less between twiddles than pairs of radix-2 ones, and a last radix-2 one for P = 8, 32.
+template <int P>
+__device__ __forceinline__ void reg_dft(float2 (&v)[P])
+{
+#pragma unroll
+    for (int n = P; n >= 4; n >>= 2) {
+        const int q = n / 4;
+#pragma unroll
+        for (int j = 0; j < P; j += n) {
+#pragma unroll
+            for (int k = 0; k < q; ++k) {
+                const float2 a = v[j + k], b = v[j + k + q], c = v[j + k + 2 * q], d = v[j + k + 3 * q];
+                const float2 s = make_float2(a.x + c.x, a.y + c.y), t = make_float2(b.x + d.x, b.y + d.y);
+                const float2 m = make_float2(a.x - c.x, a.y - c.y), u = make_float2(b.x - d.x, b.y - d.y);
+                const int e = 32 * k / n;
+                v[j + k] = make_float2(s.x + t.x, s.y + t.y);
+                v[j + k + q] = twiddle32(make_float2(s.x - t.x, s.y - t.y), 2 * e);
+                v[j + k + 2 * q] = twiddle32(make_float2(m.x + u.y, m.y - u.x), e);
+                v[j + k + 3 * q] = twiddle32(make_float2(m.x - u.y, m.y + u.x), 3 * e);
+            }
+        }
+    }
+    if (P == 8 || P == 32 || P == 2) {
+#pragma unroll
+        for (int j = 0; j < P; j += 2) {
+            const float2 a = v[j], b = v[j + 1];
+            v[j] = make_float2(a.x + b.x, a.y + b.y);
+            v[j + 1] = make_float2(a.x - b.x, a.y - b.y);
+        }
     }
 }
 
@@ -122,84 +154,6 @@ __device__ __forceinline__ void warp_fft(float2 (&v)[R], const float2* __restric
             }
         }
     }
-}
-
-// Scratch row stride of the line FFT: 32 + P (P = 32 / R), so that step B's
-// reads (lane = (k1, h), h < P) fall in distinct banks for each half-warp of
-// 8-byte accesses ((32 + P) k1 + h is distinct mod 16).
-template <int R>
-__host__ __device__ constexpr int scratch_stride() { return 32 + 32 / R; }
-
-// Line FFT through shared memory (far fewer shuffles than warp_fft), in two
-// steps on a per-warp scratch line Tl (at least R * scratch_stride<R>() elements):
-//   step A: lane t holds x[t + 32 i] (i < R); R-point DFT over i, twiddle
-//           w_N^{t k1}, store Y[t][k1] at Tl[k1 * S + t], S = scratch_stride<R>();
-//   step B: lane (k1, h) (h < P = 32 / R) loads Y[P s + h][k1] (s < R), R-point
-//           DFT over s (index kappa), twiddle w_32^{h kappa}, then a P-point DFT
-//           across its P lanes (log2 P shuffle stages).  Register r then holds
-//           X[K(r)], K(r) = k1 + R kappa(r) + R^2 brP(h), kappa(r) = brR(r).
-// Wt: tile twiddles (load_tile_twiddles).
-template <int R>
-__device__ __forceinline__ void line_step_a(float2 (&v)[R], float2* Tl, const float2* __restrict__ Wt, int lane)
-{
-    constexpr int N = 32 * R;
-    constexpr int LR = ilog2(R);
-    const float2* W32 = Wt + N;
-    reg_dif_t<R>(v, [&](int k, int h) { return W32[16 * k / h]; });
-    __syncwarp();
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const int k1 = brev(r, LR);
-        Tl[k1 * scratch_stride<R>() + lane] = (r == 0) ? v[r] : cmulf(v[r], Wt[k1 * 32 + lane]);
-    }
-    __syncwarp();
-}
-
-template <int R>
-__device__ __forceinline__ void line_step_b(float2 (&v)[R], const float2* Tl, const float2* __restrict__ Wt,
-                                            int lane)
-{
-    constexpr int N = 32 * R;
-    constexpr int LR = ilog2(R);
-    constexpr int P = 32 / R;
-    const float2* W32 = Wt + N;
-    const int k1 = lane / P, h = lane % P;
-#pragma unroll
-    for (int s2 = 0; s2 < R; ++s2) v[s2] = Tl[k1 * scratch_stride<R>() + P * s2 + h];
-    reg_dif_t<R>(v, [&](int k, int hs) { return W32[16 * k / hs]; });
-    if (P > 1) {
-#pragma unroll
-        for (int r = 1; r < R; ++r) {
-            const int kappa = brev(r, LR);
-            if (h != 0) v[r] = cmulf(v[r], W32[h * kappa]);
-        }
-#pragma unroll
-        for (int hh = P / 2; hh >= 1; hh >>= 1) {
-            const bool upper = (h & hh) != 0;
-            const int kk = h & (hh - 1);
-            const float2 w = W32[16 * kk / hh];
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-                const float ox = __shfl_xor_sync(FULL, v[r].x, hh);
-                const float oy = __shfl_xor_sync(FULL, v[r].y, hh);
-                if (!upper) {
-                    v[r].x += ox;
-                    v[r].y += oy;
-                } else {
-                    v[r] = cmulf(make_float2(ox - v[r].x, oy - v[r].y), w);
-                }
-            }
-        }
-    }
-}
-
-template <int R>
-__device__ __forceinline__ int line_out_index(int lane, int r)
-{
-    constexpr int LR = ilog2(R);
-    constexpr int P = 32 / R;
-    const int k1 = lane / P, h = lane % P;
-    return k1 + R * brev(r, LR) + R * R * brev(h, ilog2(P));
 }
 
 template <int N>
@@ -238,40 +192,43 @@ __global__ void __launch_bounds__(32 * WPB) fft_rows_reg(const float2* __restric
 }
 
 constexpr int TL = 16;               // lines per CTA tile
-constexpr int PWARPS = 8;            // 2 lines per warp
+// Threads of a tile's CTA and CTAs an SM (a thread has 8 to 16 values of N <= 256 a step, one or two 32-point DFTs, 64
+// registers of values, of N >= 512).  Both directions, ms: N = 128, 64 real functions, 256 threads x 3 CTAs 1.19, 128 x 6 0.74;
+// N = 256, 16 real functions, 256 x 3 1.48, 128 x 5 1.18, 128 x 6 1.20 (complex 2.20, 2.11); N = 1024 (S^2, 512 real
+// functions) 256 x 2 1.65, 256 x 3 2.28, 128 x 3 1.94.
+__host__ __device__ constexpr int tile_threads(int R) { return R <= 8 ? 128 : 256; }
+__host__ __device__ constexpr int tile_ctas(int R) { return R <= 2 ? 8 : R <= 4 ? 6 : R <= 8 ? 5 : 2; }
 
-// Padded position of element j in a staged line:
-//   ppos(j) = j + PA floor(j / R) + PB floor(j / R^2).
-// The accesses to a staged line are the step-B stores of lane (k1, h) into
-// K = k1 + R brR(r) + R^2 brP(h), the row loads of element lane + 32 i, and the
-// transposed side's reads / writes of element j of 8 (real) or 16 (complex)
-// lines.  (PA, PB) = (1, R/2 - R^2 - R mod 16) for R >= 16 and (0, R/2) for
-// R = 4, 8 make every half-warp of 8-byte accesses touch 16 distinct banks
-// (R = 2: (0, 1), the row loads 2-way); checked for every R by a bank model on
-// the CPU.
-template <int R>
-__host__ __device__ constexpr int pad_a() { return R >= 16 ? 1 : 0; }
-template <int R>
-__host__ __device__ constexpr int pad_b()
+// The tile kernels' line FFT in two steps, N = A B, n = j2 + B j1, K = k1 + A k2:
+//   X[K] = sum_j2 w_B^{j2 k2} w_N^{j2 k1} sum_j1 w_A^{j1 k1} x[n],
+// an A-point DFT in a thread's registers per (line, j2), one exchange through shared memory, a B-point DFT per (line, k1).
+// Each step's threads run along whichever index makes its global accesses whole 128-byte runs, so the transposition of the
+// tile costs nothing beyond that exchange.
+template <int R, bool C2T>
+__host__ __device__ constexpr int rad_a() { return R == 2 ? 8 : R == 4 ? (C2T ? 8 : 16) : R == 32 ? 32 : 16; }
+template <int R, bool C2T>
+__host__ __device__ constexpr int rad_b() { return 32 * R / rad_a<R, C2T>(); }
+// The exchange: element (line, k1, j2) at line LS + k1 KS + j2, both strides odd: lanes along the line or along k1 hit
+// distinct banks.
+template <int R, bool C2T>
+__host__ __device__ constexpr int tile_ks() { return rad_b<R, C2T>() + 1; }
+template <int R, bool C2T>
+__host__ __device__ constexpr int tile_ls() { return (rad_a<R, C2T>() * tile_ks<R, C2T>()) | 1; }
+// Twiddles in shared memory: W[k1 B + j2] = w_N^{j2 k1}.
+template <int R, bool C2T>
+__device__ __forceinline__ void load_tile_twiddles(float2* W, const double2* __restrict__ tw)
 {
-    return R >= 32 ? 0 : R >= 16 ? (((R / 2 - R * R - R) % 16) + 16) % 16 : R >= 4 ? R / 2 : 1;
+    constexpr int N = 32 * R, B = rad_b<R, C2T>();
+    for (int i = threadIdx.x; i < N; i += blockDim.x) {
+        const int j = (i % B) * (i / B);
+        W[i] = make_float2((float)tw[j].x, (float)tw[j].y);
+    }
 }
-template <int R>
-__host__ __device__ constexpr int ppos(int j)
+// Places of 0 .. n - 1 in which x and n - x are neighbours (0 and n / 2 the first two).
+__device__ __forceinline__ int paired(int pos, int n)
 {
-    return j + pad_a<R>() * (j >> ilog2(R)) + pad_b<R>() * (j >> (2 * ilog2(R)));
-}
-// Staged line length: holds every padded position and the line-FFT scratch.
-// Complex tiles stage 16 lines read in pairs (l, l + 1): odd, so the pairs
-// spread over the banks.  Real tiles stage 8 lines (one per real pair), each
-// read by two lanes per element: = 2 (mod 16).
-template <int R, bool REAL>
-__host__ __device__ constexpr int tile_lp()
-{
-    constexpr int N = 32 * R;
-    constexpr int need = ppos<R>(N - 1) + 1;
-    constexpr int lp = need > R * scratch_stride<R>() ? need : R * scratch_stride<R>();
-    return REAL ? ((lp + 13) / 16) * 16 + 2 : (lp | 1);
+    const int u = pos >> 1;
+    return (pos & 1) ? (u ? n - u : n / 2) : u;
 }
 
 // Geometry of a tiled pass (element offsets).
@@ -374,127 +331,116 @@ __device__ __forceinline__ void l2_discard(const void* p)
 // once the tile holds it (every line of the ring is read by exactly one tile).
 // HALF (with REAL_IO): the transposed side holds the elements j < N / 2 alone; those past N / 2 are the conjugates of
 // N - j, and j = N / 2 is zero (the Nyquist bin, which no coefficient maps to).
-// T: staged tile [TL][LP] in shared memory; Ws: twiddles (staged, synchronised).
+// nyq (transposed input): the elements j = N / 2 are taken as zero without being read; zero: all of them (complex lines).
+// T: the exchange in shared memory; Ws: twiddles (staged, synchronised).
 // mid(): run by every thread right after the barrier between the two halves of
 // the tile (the input is consumed, no output written yet).
 template <int R, bool C2T, bool REAL_IO, bool HALF, int IN, int OUT, typename MID>
 __device__ __forceinline__ void tile_body(const float2* __restrict__ in, float2* __restrict__ out, long long cbase,
                                           long long tbase, long long Ls, long long Js, float2* T,
-                                          const float2* Ws, uint64_t pol_in, uint64_t pol_out, MID mid)
+                                          const float2* Ws, uint64_t pol_in, uint64_t pol_out, MID mid, bool nyq = false,
+                                          bool zero = false)
 {
-    constexpr int N = 32 * R;
-    constexpr int LP = tile_lp<R, REAL_IO>();  // padded staged line
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    constexpr int NV = TL * N / (HALF ? 4 : 2) / (32 * PWARPS);  // float4 accesses per thread on the transposed side
-    static_assert(NV > 0 && TL * N / (HALF ? 4 : 2) % (32 * PWARPS) == 0, "tile must split evenly over the threads");
+    constexpr int N = 32 * R, A = rad_a<R, C2T>(), B = rad_b<R, C2T>(), KS = tile_ks<R, C2T>(), LS = tile_ls<R, C2T>();
+    constexpr int LA = ilog2(A), LB = ilog2(B), NT = tile_threads(R);
     static_assert(!(REAL_IO && IN == IO_SCRATCH && C2T), "the ring holds complex lines");
-    // REAL_IO: real lines 2p and 2p+1 share one complex transform (staged row p):
+    static_assert(!HALF || REAL_IO, "half of a real line's spectrum");
+    // REAL_IO: real lines 2p and 2p+1 share one complex transform (row p):
     // forward z = x_{2p} + i x_{2p+1}, X = (Z[k] + conj Z[-k]) / 2, Y = (Z[k] - conj Z[-k]) / 2i;
     // inverse z = X_{2p} + i X_{2p+1} (spectra of real lines), lines = Re, Im of its transform.
-    constexpr int TLI = REAL_IO ? TL / 2 : TL;  // transforms (staged rows) per tile
-    if (C2T) {
-        // contiguous input: each warp loads its line(s) straight into registers
-        for (int row = warp; row < TLI; row += PWARPS) {
-            float2* Tl = T + row * LP;
-            float2 v[R];
-            if (REAL_IO) {
-                const float* s0 = reinterpret_cast<const float*>(in) + cbase + (2 * row) * Ls;
-                const float* s1 = s0 + Ls;
-#pragma unroll
-                for (int i = 0; i < R; ++i)
-                    v[i] = make_float2(ld1<IN>(s0 + lane + 32 * i, pol_in), ld1<IN>(s1 + lane + 32 * i, pol_in));
-            } else {
-                const float2* src = in + cbase + row * Ls;
-#pragma unroll
-                for (int i = 0; i < R; ++i) v[i] = ld2<IN>(src + lane + 32 * i, pol_in);
-            }
-            line_step_a<R>(v, Tl, Ws, lane);
-            line_step_b<R>(v, Tl, Ws, lane);
-            __syncwarp();
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-                const int K = line_out_index<R>(lane, r);
-                Tl[ppos<R>(K)] = v[r];
-            }
-        }
-        __syncthreads();
-        mid();
-        if (IN == IO_SCRATCH)
-            for (int i = threadIdx.x; i < TL * (N / 16); i += 32 * PWARPS)
-                l2_discard(in + cbase + (long long)(i / (N / 16)) * Ls + (i % (N / 16)) * 16);
-        // transposed output: pairs (l, l + 1) of element j as 16-byte stores
-        float4* out4 = reinterpret_cast<float4*>(out);
-#pragma unroll 4
-        for (int u = 0; u < NV; ++u) {
-            const int e2 = threadIdx.x + u * 32 * PWARPS;
-            const int l = (e2 % (TL / 2)) * 2, j = e2 / (TL / 2);
-            float2 a, b;
-            if (REAL_IO) {
-                const float2 z = T[(l / 2) * LP + ppos<R>(j)];
-                const float2 zm = T[(l / 2) * LP + ppos<R>((N - j) & (N - 1))];
-                a = make_float2(0.5f * (z.x + zm.x), 0.5f * (z.y - zm.y));
-                b = make_float2(0.5f * (z.y + zm.y), -0.5f * (z.x - zm.x));
-            } else {
-                a = T[l * LP + ppos<R>(j)];
-                b = T[(l + 1) * LP + ppos<R>(j)];
-            }
-            st4<OUT>(out4 + (tbase + (long long)j * Js + l) / 2, make_float4(a.x, a.y, b.x, b.y), pol_out);
-        }
-    } else {
-        // transposed input staged through shared memory (16-byte loads, all issued first)
-        constexpr int VB = NV < 8 ? NV : 8;
-        const float4* in4 = reinterpret_cast<const float4*>(in);
+    constexpr int ROWS = REAL_IO ? TL / 2 : TL;
 #pragma unroll 1
-        for (int u0 = 0; u0 < NV; u0 += VB) {
-            float4 buf[VB];
+    for (int u = threadIdx.x; u < ROWS * B; u += NT) {  // whole warps
+        const int l = C2T ? u / B : u % ROWS, j2 = C2T ? u % B : REAL_IO ? paired(u / ROWS, B) : u / ROWS;
+        float2 v[A];
+        if (C2T && REAL_IO) {
+            const float* s0 = reinterpret_cast<const float*>(in) + cbase + (2 * l) * Ls + j2;
+            const float* s1 = s0 + Ls;
 #pragma unroll
-            for (int q = 0; q < VB; ++q) {
-                const int e2 = threadIdx.x + (u0 + q) * 32 * PWARPS;
-                const int l = (e2 % (TL / 2)) * 2, j = e2 / (TL / 2);
-                buf[q] = ld4<IN>(in4 + (tbase + (long long)j * Js + l) / 2, pol_in);
-            }
+            for (int i = 0; i < A; ++i) v[i] = make_float2(ld1<IN>(s0 + B * i, pol_in), ld1<IN>(s1 + B * i, pol_in));
+        } else if (C2T) {
+            const float2* src = in + cbase + l * Ls + j2;
 #pragma unroll
-            for (int q = 0; q < VB; ++q) {
-                const int e2 = threadIdx.x + (u0 + q) * 32 * PWARPS;
-                const int l = (e2 % (TL / 2)) * 2, j = e2 / (TL / 2);
-                if (REAL_IO && HALF && j == 0) {
-                    T[(l / 2) * LP + ppos<R>(0)] = make_float2(buf[q].x, buf[q].z);
-                    T[(l / 2) * LP + ppos<R>(N / 2)] = make_float2(0.f, 0.f);
-                } else if (REAL_IO) {
-                    T[(l / 2) * LP + ppos<R>(j)] = make_float2(buf[q].x - buf[q].w, buf[q].y + buf[q].z);
-                    if (HALF) T[(l / 2) * LP + ppos<R>(N - j)] = make_float2(buf[q].x + buf[q].w, buf[q].z - buf[q].y);
-                } else {
-                    T[l * LP + ppos<R>(j)] = make_float2(buf[q].x, buf[q].y);
-                    T[(l + 1) * LP + ppos<R>(j)] = make_float2(buf[q].z, buf[q].w);
+            for (int i = 0; i < A; ++i) v[i] = ld2<IN>(src + B * i, pol_in);
+        } else if (!REAL_IO) {
+            const float2* src = in + tbase + j2 * Js + l;
+#pragma unroll
+            for (int i = 0; i < A; ++i)
+                v[i] = zero || (i == A / 2 && nyq && j2 == 0) ? make_float2(0.f, 0.f)
+                                                              : ld2<IN>(src + (long long)(B * i) * Js, pol_in);
+        } else {
+            constexpr int AL = HALF ? A / 2 : A;
+            const float4* src = reinterpret_cast<const float4*>(in) + (tbase + j2 * Js + 2 * l) / 2;
+            float4 x[AL];
+#pragma unroll
+            for (int i = 0; i < AL; ++i)
+                x[i] = i == A / 2 && nyq && j2 == 0 ? make_float4(0.f, 0.f, 0.f, 0.f)
+                                                    : ld4<IN>(src + (long long)(B * i) * Js / 2, pol_in);
+#pragma unroll
+            for (int i = 0; i < AL; ++i) v[i] = make_float2(x[i].x - x[i].w, x[i].y + x[i].z);
+            if (HALF) {
+                // elements past N / 2: those of N - j with conjugate spectra, held by the neighbour B - j2
+                if (j2 == 0) v[0] = make_float2(x[0].x, x[0].z);
+#pragma unroll
+                for (int i = A / 2; i < A; ++i) {
+                    const float4 o = x[A - 1 - i], q = i > A / 2 ? x[A - i] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    const float2 own = make_float2(o.x + o.w, o.z - o.y);
+                    const float2 oth = make_float2(__shfl_xor_sync(FULL, own.x, ROWS), __shfl_xor_sync(FULL, own.y, ROWS));
+                    v[i] = j2 == 0 ? make_float2(q.x + q.w, q.z - q.y) : 2 * j2 == B ? own : oth;
                 }
             }
         }
-        __syncthreads();
-        mid();
-        if (IN == IO_SCRATCH)
-            for (int j = threadIdx.x; j < (HALF ? N / 2 : N); j += 32 * PWARPS) l2_discard(in + tbase + (long long)j * Js);
-        // contiguous output straight from registers: runs of R consecutive outputs per lane group
-        for (int row = warp; row < TLI; row += PWARPS) {
-            float2* Tl = T + row * LP;
-            float2 v[R];
+        reg_dft<A>(v);
+        float2* S = T + l * LS + j2;
 #pragma unroll
-            for (int i = 0; i < R; ++i) v[i] = Tl[ppos<R>(lane + 32 * i)];
-            line_step_a<R>(v, Tl, Ws, lane);
-            line_step_b<R>(v, Tl, Ws, lane);
-            if (REAL_IO) {
-                float* d0 = reinterpret_cast<float*>(out) + cbase + (2 * row) * Ls;
-                float* d1 = d0 + Ls;
+        for (int r = 0; r < A; ++r) {
+            const int k1 = brev(r, LA);
+            S[k1 * KS] = r == 0 ? v[r] : cmulf(v[r], Ws[k1 * B + j2]);
+        }
+    }
+    __syncthreads();
+    mid();
+    if (IN == IO_SCRATCH && C2T)
+        for (int i = threadIdx.x; i < TL * (N / 16); i += NT)
+            l2_discard(in + cbase + (long long)(i / (N / 16)) * Ls + (i % (N / 16)) * 16);
+    if (IN == IO_SCRATCH && !C2T)
+        for (int j = threadIdx.x; j < (HALF ? N / 2 : N); j += NT) l2_discard(in + tbase + (long long)j * Js);
+#pragma unroll 1
+    for (int u = threadIdx.x; u < ROWS * A; u += NT) {
+        const int l = C2T ? u % ROWS : u / A, k1 = !C2T ? u % A : REAL_IO ? paired(u / ROWS, A) : u / ROWS;
+        float2 v[B];
+        const float2* S = T + l * LS + k1 * KS;
 #pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    const int K = line_out_index<R>(lane, r);
-                    st1<OUT>(d0 + K, v[r].x, pol_out);
-                    st1<OUT>(d1 + K, v[r].y, pol_out);
-                }
-            } else {
-                float2* dst = out + cbase + row * Ls;
+        for (int j = 0; j < B; ++j) v[j] = S[j];
+        reg_dft<B>(v);
+        if (C2T && REAL_IO) {
+            float4* dst = reinterpret_cast<float4*>(out) + (tbase + k1 * Js + 2 * l) / 2;
 #pragma unroll
-                for (int r = 0; r < R; ++r) st2<OUT>(dst + line_out_index<R>(lane, r), v[r], pol_out);
+            for (int k2 = 0; k2 < (HALF ? B / 2 : B); ++k2) {
+                // Z[N - K]: the neighbour A - k1's B - 1 - k2
+                const float2 z = v[brev(k2, LB)], own = v[brev(B - 1 - k2, LB)], own0 = v[brev((B - k2) % B, LB)];
+                const float2 oth = make_float2(__shfl_xor_sync(FULL, own.x, ROWS), __shfl_xor_sync(FULL, own.y, ROWS));
+                const float2 zm = k1 == 0 ? own0 : 2 * k1 == A ? own : oth;
+                st4<OUT>(dst + (long long)(A * k2) * Js / 2,
+                         make_float4(0.5f * (z.x + zm.x), 0.5f * (z.y - zm.y), 0.5f * (z.y + zm.y), -0.5f * (z.x - zm.x)),
+                         pol_out);
             }
+        } else if (C2T) {
+            float2* dst = out + tbase + k1 * Js + l;
+#pragma unroll
+            for (int k2 = 0; k2 < B; ++k2) st2<OUT>(dst + (long long)(A * k2) * Js, v[brev(k2, LB)], pol_out);
+        } else if (REAL_IO) {
+            float* d0 = reinterpret_cast<float*>(out) + cbase + (2 * l) * Ls + k1;
+            float* d1 = d0 + Ls;
+#pragma unroll
+            for (int k2 = 0; k2 < B; ++k2) {
+                st1<OUT>(d0 + A * k2, v[brev(k2, LB)].x, pol_out);
+                st1<OUT>(d1 + A * k2, v[brev(k2, LB)].y, pol_out);
+            }
+        } else {
+            float2* dst = out + cbase + l * Ls + k1;
+#pragma unroll
+            for (int k2 = 0; k2 < B; ++k2) st2<OUT>(dst + A * k2, v[brev(k2, LB)], pol_out);
         }
     }
 }
@@ -502,14 +448,14 @@ __device__ __forceinline__ void tile_body(const float2* __restrict__ in, float2*
 // One pass over nf functions: the CTA index splits into (f, o < NO, bb < N / TL),
 // cbase = f FS + o Oc + bb TL Ls, tbase = f FS + o Ot + bb TL.
 template <int R, bool C2T, bool REAL_IO, bool HALF>
-__global__ void __launch_bounds__(32 * PWARPS, 3) fft_tile(const float2* __restrict__ in, float2* __restrict__ out,
-                                                        const TileGeo g, const double2* __restrict__ tw)
+__global__ void __launch_bounds__(tile_threads(R), tile_ctas(R)) fft_tile(const float2* __restrict__ in, float2* __restrict__ out,
+                                                        const TileGeo g, bool nyq, const double2* __restrict__ tw)
 {
     constexpr int N = 32 * R;
     extern __shared__ float2 smem_f2[];
     float2* Ws = smem_f2;
-    float2* T = smem_f2 + tile_tw_elems<R>();  // [TL][LP]
-    load_tile_twiddles<R>(Ws, tw);
+    float2* T = smem_f2 + 32 * R;
+    load_tile_twiddles<R, C2T>(Ws, tw);
     constexpr int NB = N / TL;
     const long long b = blockIdx.x;
     const long long f = b / ((long long)g.NO * NB);
@@ -518,7 +464,8 @@ __global__ void __launch_bounds__(32 * PWARPS, 3) fft_tile(const float2* __restr
     const long long cbase = f * g.FS + o * g.Oc + bb * TL * g.Ls;
     const long long tbase = f * g.FS + o * g.Ot + bb * TL;
     __syncthreads();  // twiddles staged
-    tile_body<R, C2T, REAL_IO, HALF, IO_PLAIN, IO_PLAIN>(in, out, cbase, tbase, g.Ls, g.Js, T, Ws, 0, 0, [] {});
+    tile_body<R, C2T, REAL_IO, HALF, IO_PLAIN, IO_PLAIN>(in, out, cbase, tbase, g.Ls, g.Js, T, Ws, 0, 0, [] {}, nyq,
+                                                          nyq && g.NO > 1 && o == N / 2);
 }
 
 // ---------------------------------------------------------------------------
@@ -540,7 +487,7 @@ __global__ void __launch_bounds__(32 * PWARPS, 3) fft_tile(const float2* __restr
 //   A(0), ..., A(D-1), A(D), B(0), A(D+1), B(1), ..., B(C-1)
 // so a phase-B tile's producers were claimed at least D + 1 blocks earlier
 // and a slot is reused 2 (S - D) - 1 blocks after its last reader was claimed;
-// D and S are chosen from the number of resident CTAs (about 12 tiles per SM
+// D and S are chosen from the number of resident CTAs (several tiles per CTA
 // are claimed but not yet published at any time) so that dependencies are
 // normally complete when checked, while only about D + 1 slots hold live data
 // (the rest were dropped from L2 as they were read).  At N = 512 D stays 1 so
@@ -571,6 +518,7 @@ struct Grid2DArgs {
     int nchunks;     // C = nf * N / TL
     int look;        // D
     int nslots;      // S
+    int nyq;         // inverse: the Nyquist bins p = N / 2 and q = N / 2 are zero, not read
     int prefetch;    // 1: prefetch the next claimed phase-A tile's input into L2 at each middle barrier
 };
 
@@ -624,17 +572,17 @@ __device__ __forceinline__ void decode_task(int t, int C, int D, bool& phaseA, i
 }
 
 template <int R, bool FWD, bool REAL_IO, bool HALF>
-__global__ void __launch_bounds__(32 * PWARPS, 3) fft_grid2d(const Grid2DArgs a, const double2* __restrict__ tw)
+__global__ void __launch_bounds__(tile_threads(R), tile_ctas(R)) fft_grid2d(const Grid2DArgs a, const double2* __restrict__ tw)
 {
     constexpr int N = 32 * R;
     constexpr int NB = N / TL;
     constexpr long long N2 = (long long)N * N, N3 = N2 * N;
     extern __shared__ float2 smem_f2[];
     float2* Ws = smem_f2;
-    float2* T = smem_f2 + tile_tw_elems<R>();
+    float2* T = smem_f2 + 32 * R;
     __shared__ int s_cur[2], s_slow;
     __shared__ const char* s_pf;  // input of the next tile to prefetch into L2 (null: none)
-    load_tile_twiddles<R>(Ws, tw);
+    load_tile_twiddles<R, FWD>(Ws, tw);
     const uint64_t pol_stream = l2_policy_first(), pol_keep = l2_policy_last();
     const int C = a.nchunks, D = a.look, S = a.nslots;
     // HALF: phase B forward / phase A inverse has the tiles q < N / 2 alone
@@ -737,7 +685,7 @@ __global__ void __launch_bounds__(32 * PWARPS, 3) fft_grid2d(const Grid2DArgs a,
                 constexpr int NL = FWD ? TL * N * (REAL_IO ? 4 : 8) / 128 : N;
                 constexpr long long STEP = FWD ? 128 : 8 * N2;
 #pragma unroll
-                for (int i = threadIdx.x; i < NL; i += 32 * PWARPS) prefetch_l2(pf + STEP * i);
+                for (int i = threadIdx.x; i < NL; i += tile_threads(R)) prefetch_l2(pf + STEP * i);
             }
         };
         bool phaseA;
@@ -760,7 +708,8 @@ __global__ void __launch_bounds__(32 * PWARPS, 3) fft_grid2d(const Grid2DArgs a,
             if (phaseA)
                 tile_body<R, false, false, false, IO_STREAM, IO_SCRATCH>(a.in, slot, (long long)q * N,
                                                                    fbase + (long long)q * N + kb * TL, N2, N2, T,
-                                                                   Ws, pol_stream, pol_keep, mid);
+                                                                   Ws, pol_stream, pol_keep, mid, a.nyq,
+                                                                   a.nyq && q == N / 2);
             else
                 tile_body<R, false, REAL_IO, HALF, IO_SCRATCH, IO_STREAM>(
                     slot, a.out, fbase + (kb * TL + kl) * N2 + (long long)bb * TL * N, kl * N2 + bb * TL, N, N, T,
@@ -800,53 +749,57 @@ __global__ void __launch_bounds__(32 * PWARPS, 3) fft_grid2d(const Grid2DArgs a,
 }
 
 template <int R, bool C2T, bool REAL_IO, bool HALF>
-static cudaError_t tile_r(const void* in, void* out, long long nf, const TileGeo& g, const void* tw, cudaStream_t st)
+static cudaError_t tile_r(const void* in, void* out, long long nf, const TileGeo& g, bool nyq, const void* tw, cudaStream_t st)
 {
     constexpr int N = 32 * R;
-    constexpr int LP = tile_lp<R, REAL_IO>();
-    constexpr int TLI = REAL_IO ? TL / 2 : TL;  // staged rows (real lines go in pairs)
-    const size_t smem = sizeof(float2) * ((size_t)tile_tw_elems<R>() + (size_t)TLI * LP);
+    constexpr int ROWS = REAL_IO ? TL / 2 : TL;  // real lines go in pairs
+    const size_t smem = sizeof(float2) * (N + (size_t)ROWS * tile_ls<R, C2T>());
     auto k = fft_tile<R, C2T, REAL_IO, HALF>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     const long long nblk = nf * (long long)g.NO * (N / TL);
-    k<<<(unsigned)nblk, 32 * PWARPS, smem, st>>>((const float2*)in, (float2*)out, g, (const double2*)tw);
+    k<<<(unsigned)nblk, tile_threads(R), smem, st>>>((const float2*)in, (float2*)out, g, nyq, (const double2*)tw);
     return cudaGetLastError();
 }
 
 template <bool C2T, bool REAL_IO, bool HALF>
-static cudaError_t tile_dispatch(const void* in, void* out, long long nf, int N, const TileGeo& g, const void* tw,
+static cudaError_t tile_dispatch(const void* in, void* out, long long nf, int N, const TileGeo& g, bool nyq, const void* tw,
                                  cudaStream_t st)
 {
     switch (N) {
-        case 64: return tile_r<2, C2T, REAL_IO, HALF>(in, out, nf, g, tw, st);
-        case 128: return tile_r<4, C2T, REAL_IO, HALF>(in, out, nf, g, tw, st);
-        case 256: return tile_r<8, C2T, REAL_IO, HALF>(in, out, nf, g, tw, st);
-        case 512: return tile_r<16, C2T, REAL_IO, HALF>(in, out, nf, g, tw, st);
-        case 1024: return tile_r<32, C2T, REAL_IO, HALF>(in, out, nf, g, tw, st);
+        case 64: return tile_r<2, C2T, REAL_IO, HALF>(in, out, nf, g, nyq, tw, st);
+        case 128: return tile_r<4, C2T, REAL_IO, HALF>(in, out, nf, g, nyq, tw, st);
+        case 256: return tile_r<8, C2T, REAL_IO, HALF>(in, out, nf, g, nyq, tw, st);
+        case 512: return tile_r<16, C2T, REAL_IO, HALF>(in, out, nf, g, nyq, tw, st);
+        case 1024: return tile_r<32, C2T, REAL_IO, HALF>(in, out, nf, g, nyq, tw, st);
         default: return cudaErrorNotSupported;
     }
 }
 
 template <bool C2T>
 static cudaError_t tile_any(const void* in, void* out, long long nf, int N, const TileGeo& g, const void* tw,
-                            cudaStream_t st, bool real_io, bool half = false)
+                            cudaStream_t st, bool real_io, bool half, bool nyq)
 {
-    if (real_io && half) return tile_dispatch<C2T, true, true>(in, out, nf, N, g, tw, st);
-    return real_io ? tile_dispatch<C2T, true, false>(in, out, nf, N, g, tw, st)
-                   : tile_dispatch<C2T, false, false>(in, out, nf, N, g, tw, st);
+    if (real_io && half) return tile_dispatch<C2T, true, true>(in, out, nf, N, g, nyq, tw, st);
+    return real_io ? tile_dispatch<C2T, true, false>(in, out, nf, N, g, nyq, tw, st)
+                   : tile_dispatch<C2T, false, false>(in, out, nf, N, g, nyq, tw, st);
 }
 
-// Lookahead D and ring slots S for N on a device of nsm SMs: about W = 12 nsm
-// tiles are claimed and not yet published at any time (three resident CTAs per
-// SM, each holding up to three claims and one unpublished tile); D and S put
-// every dependency at least W tiles back (2 D + 1 and 2 (S - D) - 1 blocks of
-// N tiles).  At N = 512 D stays 1 so that the live slots (D + 1, 32 MB each)
-// fit in L2; the rare incomplete dependency then takes the slow path.
+// Lookahead D and ring slots S for N on a device of nsm SMs: about 4 nsm tile_ctas
+// tiles are claimed and not yet published at any time (the resident CTAs, each
+// holding up to three claims and one unpublished tile); D and S put every
+// dependency at least W = twice that many tiles back (a chunk is `pair` tiles),
+// where the live slots (D + 1) stay below 42 MB, a third of the L2.  Both bounds
+// measured (both directions, ms): N = 128, 64 functions 1.10 with W once, 1.08
+// twice, 1.08 three times; N = 64, 256 functions 0.83, 0.68, 0.68; N = 256, 16
+// functions D = 3 2.26, 4 2.11 (42 MB), 6 2.26, 10 2.53; N = 512 D = 1 2.58, 2
+// 2.91; the rare incomplete dependency takes the slow path.
 static void fused_geometry(int N, int nsm, bool half, int& D, int& S)
 {
-    const int W = 12 * nsm, pair = half ? N + N / 2 : 2 * N;  // tiles of a chunk
-    D = N >= 512 ? 1 : std::max(1, (W - N + pair - 1) / pair);
+    const int W = 8 * tile_ctas(N / 32) * nsm, pair = half ? N + N / 2 : 2 * N;  // tiles of a chunk
+    const long long slot = (long long)TL * N * N * sizeof(float2) / (half ? 2 : 1);  // its live bytes
+    D = std::max(1, (W - N + pair - 1) / pair);
+    D = std::max(1, std::min(D, (int)((42LL << 20) / slot) - 1));
     if (const char* ev = getenv("FFTSO3_FFT_LOOKAHEAD")) {  // tuning override of D (1..16)
         const int d = atoi(ev);
         if (d >= 1 && d <= 16) D = d;
@@ -865,18 +818,16 @@ static int device_sms()
 template <int R, bool FWD, bool REAL_IO, bool HALF>
 static cudaError_t grid2d_r(const Grid2DArgs& a, long long tiles, const void* tw, cudaStream_t st)
 {
-    // staged tile: 16 complex lines, or 8 rows of real pairs (phase A forward / phase B inverse)
-    constexpr size_t rows = std::max<size_t>((size_t)TL * tile_lp<R, false>(), (size_t)(TL / 2) * tile_lp<R, true>());
-    const size_t smem = sizeof(float2) * ((size_t)tile_tw_elems<R>() + rows);
+    const size_t smem = sizeof(float2) * (32 * R + (size_t)TL * tile_ls<R, FWD>());
     auto k = fft_grid2d<R, FWD, REAL_IO, HALF>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int dev = 0, nsm = 0, occ = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, 32 * PWARPS, smem)) != cudaSuccess) return e;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, tile_threads(R), smem)) != cudaSuccess) return e;
     const long long ctas = std::min<long long>(tiles, (long long)nsm * std::max(occ, 1));
-    k<<<(unsigned)ctas, 32 * PWARPS, smem, st>>>(a, (const double2*)tw);
+    k<<<(unsigned)ctas, tile_threads(R), smem, st>>>(a, (const double2*)tw);
     return cudaGetLastError();
 }
 
@@ -925,17 +876,17 @@ cudaError_t launch_fft_rows_fast(const void* in, void* out, long long nlines, in
 //   pass 2': pencils [f][p][q][k] -> FFT over p  -> T1 [f][k][q][j1]
 //   pass 1': T1 [f][k][q][j1]     -> FFT over q  -> grid [f][k][j1][j2]
 cudaError_t launch_fft_grid_pass(const void* in, void* out, long long nf, int N, int pass, const void* tw,
-                                 cudaStream_t st, bool real_io, bool half)
+                                 cudaStream_t st, bool real_io, bool half, bool nyq)
 {
     const long long N1 = N, N2 = (long long)N * N, N3 = N2 * N;
     if (real_io && pass != 1 && pass != -1) return cudaErrorInvalidValue;
     const ffast::TileGeo g1{N3, N, N2, N1, N2, N1};  // lines along j2 / q, transposed (q, j1)
     const ffast::TileGeo g2{N3, half ? N / 2 : N, N1, N2, N1, N2};  // lines along j1 / p of each q, transposed (p.., k)
     switch (pass) {
-        case 1: return ffast::tile_any<true>(in, out, nf, N, g1, tw, st, real_io, half);
-        case 2: return ffast::tile_any<true>(in, out, nf, N, g2, tw, st, false);
-        case -2: return ffast::tile_any<false>(in, out, nf, N, g2, tw, st, false);
-        case -1: return ffast::tile_any<false>(in, out, nf, N, g1, tw, st, real_io, half);
+        case 1: return ffast::tile_any<true>(in, out, nf, N, g1, tw, st, real_io, half, false);
+        case 2: return ffast::tile_any<true>(in, out, nf, N, g2, tw, st, false, false, false);
+        case -2: return ffast::tile_any<false>(in, out, nf, N, g2, tw, st, false, false, nyq);
+        case -1: return ffast::tile_any<false>(in, out, nf, N, g1, tw, st, real_io, half, false);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -952,7 +903,7 @@ size_t fft_grid_fused_ctl_ints(long long nf, int N) { return 2 + 2 * (size_t)nf 
 // Both passes of one direction (dir 1: grid -> pencils, dir -1: pencils ->
 // grid) in one persistent launch through the L2-resident ring (fft_grid2d).
 cudaError_t launch_fft_grid_fused(const void* in, void* out, void* ring, size_t ring_elems, int* ctl, int* err,
-                                  long long nf, int N, int dir, const void* tw, cudaStream_t st, bool real_io, bool half)
+                                  long long nf, int N, int dir, const void* tw, cudaStream_t st, bool real_io, bool half, bool nyq)
 {
     if (half && !real_io) return cudaErrorInvalidValue;
     if (!fft_grid_fused_supported(N) || (dir != 1 && dir != -1) || nf < 1) return cudaErrorInvalidValue;
@@ -964,7 +915,7 @@ cudaError_t launch_fft_grid_fused(const void* in, void* out, void* ring, size_t 
     ffast::fused_geometry(N, ffast::device_sms(), half, D, S);
     if ((size_t)S * ffast::TL * N * N > ring_elems) return cudaErrorInvalidValue;  // ring sized for another device
     const char* pf = getenv("FFTSO3_FFT_PREFETCH");  // 0 turns the next-tile L2 prefetch off (tuning)
-    ffast::Grid2DArgs a{(const float2*)in, (float2*)out, (float2*)ring, ctl, err, (int)C, D, S,
+    ffast::Grid2DArgs a{(const float2*)in, (float2*)out, (float2*)ring, ctl, err, (int)C, D, S, nyq,
                         pf && atoi(pf) == 0 ? 0 : 1};
     const long long tiles = C * (half ? N + N / 2 : 2 * N);
     if (half)
@@ -978,12 +929,12 @@ cudaError_t launch_fft_grid_fused(const void* in, void* out, void* ring, size_t 
 }
 
 cudaError_t launch_fft_s2_pass(const void* in, void* out, long long nf, int N, int dir, const void* tw,
-                               cudaStream_t st, bool real_io, bool half)
+                               cudaStream_t st, bool real_io, bool half, bool nyq)
 {
     const long long N1 = N, N2 = (long long)N * N;
     const ffast::TileGeo g{N2, 1, 0, N1, 0, N1};  // lines along j (contiguous), transposed [p][k]
-    if (dir == 1) return ffast::tile_any<true>(in, out, nf, N, g, tw, st, real_io, half);
-    if (dir == -1) return ffast::tile_any<false>(in, out, nf, N, g, tw, st, real_io, half);
+    if (dir == 1) return ffast::tile_any<true>(in, out, nf, N, g, tw, st, real_io, half, nyq);
+    if (dir == -1) return ffast::tile_any<false>(in, out, nf, N, g, tw, st, real_io, half, nyq);
     return cudaErrorInvalidValue;
 }
 
