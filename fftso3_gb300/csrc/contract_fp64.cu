@@ -463,7 +463,7 @@ constexpr int S2T = 32;
 
 __global__ void __launch_bounds__(256) s2_group_to_real_kernel(const float2* __restrict__ Fg, float* __restrict__ Fr,
                                                               const long long* __restrict__ goff2, int L,
-                                                              long long cstride)
+                                                              long long cstride, bool half)
 {
     __shared__ float2 tp[S2T][S2T + 1];  // F_c(l0 + li, +(mb + mi)) as [mi][li]
     __shared__ float2 tn[S2T][S2T + 1];  // F_c(l0 + li, -(mb + mi))
@@ -475,8 +475,12 @@ __global__ void __launch_bounds__(256) s2_group_to_real_kernel(const float2* __r
         const int mi = e / S2T, li = e % S2T, g = mb + mi, l = l0 + li;
         if (g > L || l > L || l < g) continue;
         const long long o = goff2[g] + (l - g);
-        tp[mi][li] = fg[o];
-        tn[mi][li] = g > 0 ? fg[o + (B - g)] : fg[o];
+        const float2 v = fg[o];
+        tp[mi][li] = v;
+        if (half)
+            tn[mi][li] = g > 0 ? (g & 1 ? make_float2(-v.x, v.y) : make_float2(v.x, -v.y)) : v;
+        else
+            tn[mi][li] = g > 0 ? fg[o + (B - g)] : v;
     }
     __syncthreads();
     float* fr = Fr + (long long)b * cstride;
@@ -499,6 +503,7 @@ __global__ void __launch_bounds__(256) s2_group_to_real_kernel(const float2* __r
     }
 }
 
+// (half, in both: of the pairs of m > 0 the GEMM writes pair 0 alone, and reads pair 1 alone: the others are their conjugates.)
 // S^2 real coefficients straight into the scaled group-major layout of the
 // inverse GEMM (pair 0: F_c(l, m), pair 1: (-1)^m F_c(l, -m), m >= 0):
 // s2_r2c_kernel and the packed -> group-major permutation in one pass, with
@@ -506,7 +511,7 @@ __global__ void __launch_bounds__(256) s2_group_to_real_kernel(const float2* __r
 // read along m (packed) and written along l (group-major).
 __global__ void __launch_bounds__(256) s2_real_to_group_kernel(const float* __restrict__ Fr, float2* __restrict__ Y,
                                                               const long long* __restrict__ goff2, int L,
-                                                              long long cstride)
+                                                              long long cstride, bool half)
 {
     __shared__ float tp[S2T][S2T + 1];  // F_r(l0 + li, +(mb + mi)) as [li][mi]
     __shared__ float tn[S2T][S2T + 1];  // F_r(l0 + li, -(mb + mi))
@@ -526,7 +531,7 @@ __global__ void __launch_bounds__(256) s2_real_to_group_kernel(const float* __re
     for (int e = threadIdx.x; e < 2 * S2T * S2T; e += 256) {
         const int p = e / (S2T * S2T), r = e % (S2T * S2T), mi = r / S2T, li = r % S2T;
         const int m = mb + mi, l = l0 + li;
-        if (m > L || l > L || l < m || (p == 1 && m == 0)) continue;
+        if (m > L || l > L || l < m || (p == 1 && m == 0) || (half && p == 0 && m > 0)) continue;
         const int c = p == 0 ? m : -m;
         const int as[2] = {c, -c};
         const int na = (c == 0) ? 1 : 2;
@@ -644,21 +649,21 @@ cudaError_t launch_s2_c2r(const void* Fc, void* Fr, bool fp64, int L, int batch,
     return cudaGetLastError();
 }
 
-cudaError_t launch_s2_group_to_real(const void* Fg, void* Fr, const long long* goff2, int L, int batch,
+cudaError_t launch_s2_group_to_real(const void* Fg, void* Fr, const long long* goff2, int L, int batch, bool half,
                                    cudaStream_t st)
 {
     const long long C = (long long)(L + 1) * (L + 1);
     const unsigned nt = (unsigned)((L + 1 + S2T - 1) / S2T);
-    s2_group_to_real_kernel<<<dim3(nt, nt, batch), 256, 0, st>>>((const float2*)Fg, (float*)Fr, goff2, L, C);
+    s2_group_to_real_kernel<<<dim3(nt, nt, batch), 256, 0, st>>>((const float2*)Fg, (float*)Fr, goff2, L, C, half);
     return cudaGetLastError();
 }
 
-cudaError_t launch_s2_real_to_group(const void* Fr, void* Y, const long long* goff2, int L, int batch,
+cudaError_t launch_s2_real_to_group(const void* Fr, void* Y, const long long* goff2, int L, int batch, bool half,
                                    cudaStream_t st)
 {
     const long long C = (long long)(L + 1) * (L + 1);
     const unsigned nt = (unsigned)((L + 1 + S2T - 1) / S2T);
-    s2_real_to_group_kernel<<<dim3(nt, nt, batch), 256, 0, st>>>((const float*)Fr, (float2*)Y, goff2, L, C);
+    s2_real_to_group_kernel<<<dim3(nt, nt, batch), 256, 0, st>>>((const float*)Fr, (float2*)Y, goff2, L, C, half);
     return cudaGetLastError();
 }
 

@@ -48,6 +48,7 @@
 #include "dft_tc.cuh"
 #include "direct_dft.cuh"
 #include "fused.cuh"
+#include "rsph.cuh"
 #include "tc.cuh"
 #include "tc_ptx.cuh"
 
@@ -1112,6 +1113,135 @@ static dim3 ptile_grid(int L, int batch)
     return dim3((unsigned)(2 * L + 1), (unsigned)((L + 1 + PT - 1) / PT), (unsigned)(mtiles * fgroups));
 }
 
+// Real SO(3) functions: the group-major coefficients of one of each two conjugate pairs <-> the packed real ones, in one pass
+// (as two, through packed complex coefficients, 0.148 and 0.141 ms a direction at l_max 63, 64 functions).  A CTA takes the
+// quadruples (+-mu, +-nu) of one nu >= 0, 32 mu and 32 l: group-major runs along l on one side, packed runs along mu on the
+// other: 0.108 and 0.103 ms.  Arithmetic as so3_c2r / so3_r2c and the permutations (rsph.cuh).
+constexpr int RFPC = 4;  // functions per CTA
+struct RTileIdx {
+    long long gbase[2][PT];  // of the two group-major entries of mu, relative to l
+    float gsign[2][PT];
+    long long pbase[2][PT];  // packed place of (l, 0, +-nu)
+    int an[PT];              // max(mu, nu)
+};
+__device__ __forceinline__ bool rtile_coords(int L, int& nu, int& l0, int& mb, int& fg)
+{
+    const int mtiles = (L + 1 + PT - 1) / PT;
+    nu = (int)blockIdx.x;
+    l0 = (int)blockIdx.y * PT;
+    fg = (int)(blockIdx.z / mtiles);
+    mb = (int)(blockIdx.z % mtiles) * PT;
+    return mb <= l0 + PT - 1 && nu <= l0 + PT - 1;
+}
+// entries [0]: (mu, nu); [1]: (-mu, nu) when neg_m, else (mu, -nu)
+__device__ __forceinline__ void rtile_index(RTileIdx& t, int L, int nu, int l0, int mb, bool neg_m, const long long* goff2)
+{
+    if (threadIdx.x < 2 * PT) {
+        const int i = threadIdx.x / PT, mi = threadIdx.x % PT, mu = mb + mi;
+        if (mu > L) {
+            t.an[mi] = 0x7fffffff;
+        } else {
+            int g, pp, m0, sg;
+            pair_m0(i && neg_m ? -mu : mu, i && !neg_m ? -nu : nu, g, pp, m0, sg);
+            t.gbase[i][mi] = goff2[g] + (long long)pp * (L + 1 - m0) - m0;
+            t.gsign[i][mi] = (float)sg;
+            t.an[mi] = m0;
+        }
+    } else if (threadIdx.x < 4 * PT) {
+        const int i = (threadIdx.x - 2 * PT) / PT, li = threadIdx.x % PT, l = l0 + li;
+        t.pbase[i][li] = so3_idx(l, 0, i ? -nu : nu);
+    }
+    __syncthreads();
+}
+
+// add: the real coefficients are added to (the refinement's correction)
+__global__ void __launch_bounds__(256) group_to_real_tiled(const float2* __restrict__ Fg, float* __restrict__ Fr,
+                                                           const long long* __restrict__ goff2, int L, long long cstride,
+                                                           int batch, bool add)
+{
+    __shared__ float2 tile[2][PT][PT + 1];  // F(l, mu, +-nu): [nu < 0][mu - mb][l - l0]
+    __shared__ RTileIdx ix;
+    int nu, l0, mb, fg;
+    if (!rtile_coords(L, nu, l0, mb, fg)) return;
+    rtile_index(ix, L, nu, l0, mb, false, goff2);
+    const int fend = min(batch, (fg + 1) * RFPC);
+    for (int f = fg * RFPC; f < fend; ++f) {
+        const float2* src = Fg + (long long)f * cstride;
+        float* dst = Fr + (long long)f * cstride;
+#pragma unroll
+        for (int u = 0; u < PT * PT / 256; ++u) {
+            const int e = threadIdx.x + u * 256, mi = e / PT, li = e % PT, l = l0 + li;
+            if (l < ix.an[mi] || l > L) continue;
+            tile[0][mi][li] = src[ix.gbase[0][mi] + l];
+            if (nu > 0 && mb + mi > 0) tile[1][mi][li] = src[ix.gbase[1][mi] + l];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < PT * PT / 256; ++u) {
+            const int e = threadIdx.x + u * 256, li = e / PT, mi = e % PT, l = l0 + li, mu = mb + mi;
+            if (l < ix.an[mi] || l > L) continue;
+            auto at = [&](int, int b) {
+                const float2 v = tile[b < 0][mi][li];
+                return c2t<float>{v.x, v.y};
+            };
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if (((q & 1) && mu == 0) || ((q & 2) && nu == 0)) continue;
+                const int m = q & 1 ? -mu : mu, n = q & 2 ? -nu : nu;
+                float* o = dst + ix.pbase[q >> 1][li] + m;
+                const float x = real_coefficient<float, true>(m, n, at);
+                *o = add ? *o + x : x;
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// neg_m: the pairs of n >= 0 are wanted (GemmArgs.by_q), else those of m >= 0
+__global__ void __launch_bounds__(256) real_to_group_tiled(const float* __restrict__ Fr, float2* __restrict__ Y,
+                                                           const long long* __restrict__ goff2, int L, long long cstride,
+                                                           int batch, bool neg_m)
+{
+    __shared__ float tile[4][PT][PT + 1];  // F_r(l, +-mu, +-nu): [m < 0 | 2 (n < 0)][l - l0][mu - mb]
+    __shared__ RTileIdx ix;
+    int nu, l0, mb, fg;
+    if (!rtile_coords(L, nu, l0, mb, fg)) return;
+    rtile_index(ix, L, nu, l0, mb, neg_m, goff2);
+    const int fend = min(batch, (fg + 1) * RFPC);
+    for (int f = fg * RFPC; f < fend; ++f) {
+        const float* src = Fr + (long long)f * cstride;
+        float2* dst = Y + (long long)f * cstride;
+#pragma unroll
+        for (int u = 0; u < PT * PT / 256; ++u) {
+            const int e = threadIdx.x + u * 256, li = e / PT, mi = e % PT, l = l0 + li, mu = mb + mi;
+            if (l < ix.an[mi] || l > L) continue;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) tile[q][li][mi] = src[ix.pbase[q >> 1][li] + (q & 1 ? -mu : mu)];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < PT * PT / 256; ++u) {
+            const int e = threadIdx.x + u * 256, mi = e / PT, li = e % PT, l = l0 + li, mu = mb + mi;
+            if (l < ix.an[mi] || l > L) continue;
+            auto at = [&](int a, int b) { return tile[(a < 0 ? 1 : 0) + (b < 0 ? 2 : 0)][li][mi]; };
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                if (i && (neg_m ? mu : nu) == 0) continue;
+                const c2t<float> v = complex_coefficient<float>(i && neg_m ? -mu : mu, i && !neg_m ? -nu : nu, at);
+                const float sc = (float)(2 * l + 1) * ix.gsign[i][mi];
+                dst[ix.gbase[i][mi] + l] = make_float2(sc * v.x, sc * v.y);
+            }
+        }
+        __syncthreads();
+    }
+}
+
+static dim3 rtile_grid(int L, int batch)
+{
+    const unsigned t = (unsigned)((L + 1 + PT - 1) / PT);
+    return dim3((unsigned)(L + 1), t, t * (unsigned)((batch + RFPC - 1) / RFPC));
+}
+
 // S^2: group-major forward output -> packed F(l, m) at l^2 + m + l (one CTA per (l, function)).
 __global__ void s2_group_to_packed_kernel(const float2* __restrict__ Fg, float2* __restrict__ F,
                                           const long long* __restrict__ goff2, int L, long long cstride)
@@ -1768,7 +1898,7 @@ static GemmArgs gemm_args(const TCState* s)
     a.err = s->d_err;
     a.half = s->half_pencils();
     a.by_q = !s->dft_tc;
-    a.half_coeffs = 0;
+    a.half_coeffs = s->herm;
     return a;
 }
 
@@ -1979,9 +2109,27 @@ static int fft_inverse(TCState* s, void* grid, cudaStream_t st, StageTimer* T, s
     return FFTSO3_SUCCESS;
 }
 
-// real_out (S^2 real kinds): write the real coefficients straight from the GEMM output instead of F.
+// real_out (S^2 real kinds, and SO(3) ones whose GEMM sums half of the pairs): write the real coefficients straight from the
+// GEMM output instead of F (add, SO(3): add them).
+// the direct conversions of the real kinds (see real_out of tc_forward_once)
+static bool direct_real(const TCState* s) { return s->real && (s->s2 || s->herm); }
+static cudaError_t real_from_group(TCState* s, void* out, bool add, cudaStream_t st)
+{
+    if (s->s2) return launch_s2_group_to_real(s->d_fg, out, s->d_goff2, s->L, s->batch, s->herm, st);
+    group_to_real_tiled<<<rtile_grid(s->L, s->batch), 256, 0, st>>>(s->d_fg, (float*)out, s->d_goff2, s->L, coeffs_per_fn(s),
+                                                                    s->batch, add);
+    return cudaGetLastError();
+}
+static cudaError_t real_to_group(TCState* s, const void* in, cudaStream_t st)
+{
+    if (s->s2) return launch_s2_real_to_group(in, s->d_fg, s->d_goff2, s->L, s->batch, s->herm, st);
+    real_to_group_tiled<<<rtile_grid(s->L, s->batch), 256, 0, st>>>((const float*)in, s->d_fg, s->d_goff2, s->L,
+                                                                    coeffs_per_fn(s), s->batch, !s->dft_tc);
+    return cudaGetLastError();
+}
+
 static int tc_forward_once(TCState* s, const void* grid, float2* F, cudaStream_t st, StageTimer* T,
-                           std::string& err, void* real_out = nullptr)
+                           std::string& err, void* real_out = nullptr, bool add = false)
 {
     int rc = fft_forward(s, grid, st, T, err);
     if (rc) return rc;
@@ -1990,7 +2138,7 @@ static int tc_forward_once(TCState* s, const void* grid, float2* F, cudaStream_t
     T->end(st);
     T->begin(ST_BASIS, st);
     if (real_out)
-        TCK(launch_s2_group_to_real(s->d_fg, real_out, s->d_goff2, s->L, s->batch, st));
+        TCK(real_from_group(s, real_out, add, st));
     else if (s->s2)
         s2_group_to_packed_kernel<<<dim3(s->B, s->batch), 256, 0, st>>>(s->d_fg, F, s->d_goff2, s->L,
                                                                        coeffs_per_fn(s));
@@ -2018,7 +2166,7 @@ static cudaError_t zero_nyquist_pencils(TCState* s, cudaStream_t st)
     return cudaGetLastError();
 }
 
-// real_in (S^2 real kinds): read the real coefficients straight into the GEMM input instead of F.
+// real_in (as real_out of tc_forward_once): read the real coefficients straight into the GEMM input instead of F.
 static int tc_inverse_once(TCState* s, const float2* F, void* grid, cudaStream_t st, StageTimer* T,
                            std::string& err, const void* real_in = nullptr)
 {
@@ -2029,7 +2177,7 @@ static int tc_inverse_once(TCState* s, const float2* F, void* grid, cudaStream_t
     }
     T->begin(ST_BASIS, st);
     if (real_in)
-        TCK(launch_s2_real_to_group(real_in, s->d_fg, s->d_goff2, s->L, s->batch, st));
+        TCK(real_to_group(s, real_in, st));
     else if (s->s2)
         s2_packed_to_group_kernel<<<dim3(s->ngroups, s->batch), 128, 0, st>>>(F, s->d_fg, s->d_goff2, s->L,
                                                                              coeffs_per_fn(s));
@@ -2047,10 +2195,9 @@ static int tc_inverse_once(TCState* s, const float2* F, void* grid, cudaStream_t
 
 int tc_forward(TCState* s, const void* grid, void* coeffs, cudaStream_t st, StageTimer* T, std::string& err)
 {
-    // real kinds: complex coefficients in d_fc, then the real basis
-    // (fdcl_FFTSO3.cpp:1169-1181, fdcl_FFTS2.cpp:424-436); the S^2 real kinds
-    // write the real coefficients straight from the GEMM output
-    if (s->real && s->s2) return tc_forward_once(s, grid, nullptr, st, T, err, coeffs);
+    // real kinds (fdcl_FFTSO3.cpp:1169-1181, fdcl_FFTS2.cpp:424-436): the real coefficients straight from the GEMM output, or,
+    // of the FP32 beta-sum on SO(3), complex coefficients in d_fc, then the real basis
+    if (direct_real(s)) return tc_forward_once(s, grid, nullptr, st, T, err, coeffs);
     float2* Fc = s->real ? s->d_fc : (float2*)coeffs;
     int rc = tc_forward_once(s, grid, Fc, st, T, err);
     if (rc) return rc;
@@ -2149,6 +2296,11 @@ int tc_refine_add_pencils(TCState* s, void* coeffs, int terms, cudaStream_t st, 
         if (rc) return rc;
         T->end(st);
         T->begin(ST_BASIS, st);
+        if (s->herm) {
+            TCK(real_from_group(s, coeffs, true, st));
+            T->end(st);
+            return FFTSO3_SUCCESS;
+        }
         group_to_packed_tiled<<<ptile_grid(s->L, s->batch), 256, 0, st>>>(s->d_fg, s->d_coef2, s->d_goff2, s->L,
                                                                           coeffs_per_fn(s), s->batch);
         TCK(cudaGetLastError());
@@ -2174,6 +2326,7 @@ int tc_refine_add(TCState* s, const void* resid, void* coeffs, cudaStream_t st, 
     const long long nc = (long long)s->batch * coeffs_per_fn(s);
     int rc;
     float* corr;  // the correction in the coefficients' own element type
+    if (s->herm && !s->s2) return tc_forward_once(s, resid, nullptr, st, T, err, coeffs, true);
     if (s->real && s->s2) {
         rc = tc_forward_once(s, resid, nullptr, st, T, err, s->d_coef2);
         corr = (float*)s->d_coef2;
@@ -2200,7 +2353,7 @@ int tc_refine_add(TCState* s, const void* resid, void* coeffs, cudaStream_t st, 
 
 int tc_inverse(TCState* s, const void* coeffs, void* grid, cudaStream_t st, StageTimer* T, std::string& err)
 {
-    if (s->real && s->s2) return tc_inverse_once(s, nullptr, grid, st, T, err, coeffs);
+    if (direct_real(s)) return tc_inverse_once(s, nullptr, grid, st, T, err, coeffs);
     const float2* Fc = (const float2*)coeffs;
     if (s->real) {
         T->begin(ST_BASIS, st);
@@ -2225,8 +2378,8 @@ int tc_forward_finish(TCState* s, void* coeffs, cudaStream_t st, StageTimer* T, 
 {
     float2* Fc = s->real ? s->d_fc : (float2*)coeffs;
     T->begin(ST_BASIS, st);
-    if (s->real && s->s2) {
-        TCK(launch_s2_group_to_real(s->d_fg, coeffs, s->d_goff2, s->L, s->batch, st));
+    if (direct_real(s)) {
+        TCK(real_from_group(s, coeffs, false, st));
         T->end(st);
         return FFTSO3_SUCCESS;
     }
@@ -2251,9 +2404,9 @@ int tc_inverse_prepare(TCState* s, const void* coeffs, cudaStream_t st, StageTim
 {
     const float2* Fc = (const float2*)coeffs;
     T->begin(ST_BASIS, st);
-    if (s->real && s->s2) {
+    if (direct_real(s)) {
         TCK(zero_nyquist_pencils(s, st));
-        TCK(launch_s2_real_to_group(coeffs, s->d_fg, s->d_goff2, s->L, s->batch, st));
+        TCK(real_to_group(s, coeffs, st));
         T->end(st);
         return FFTSO3_SUCCESS;
     }
