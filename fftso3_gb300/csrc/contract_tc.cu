@@ -172,6 +172,9 @@ struct GemmArgs {
     // reads those alone (half)
     int by_q, half;
     int half_coeffs;           // ... and forward: only the coefficients of pairs 0 and 2 (n0 < 0: 3), m >= 0, are written
+    // SO(3), at most half a column tile of functions: items of n0 >= 0, the second half of the columns holds the group
+    // (m0, -n0) against the same table rows, d^l_{m0, -n0}(beta) = (-1)^(l + m0) d^l_{m0, n0}(pi - beta)
+    int paired;
 };
 
 // One plan's share of a fused launch over several plans (the l_max buckets of
@@ -269,7 +272,10 @@ __device__ __forceinline__ int herm_pair(const GroupPairs& P, int n0, int j, int
 // written, and both pencils unless the FFT reads one half alone (args.half; of two pairs in q = 0 or p = 0 still both).
 // 1.60 ms against 3.03 (forward) and 1.86 against 3.01 (S^2, l_max 511, 512 functions), 0.24 against 0.43 and 0.22 against 0.27
 // (SO(3), l_max 63, 64 functions).
-template <bool FWD, bool S2, bool FUSED, int TERMS = 3, bool HERM = false>
+// PAIR: args.paired may be set (a kernel of its own: the other's forward took 0.99 ms instead of 0.75 with it, l_max 127, 16
+// functions).  Forward and inverse, without and with: l_max 127, 4 functions 0.61 and 0.48 ms, 0.48 and 0.26; l_max 255, one
+// function 6.0 and 4.9, 4.2 and 2.3.
+template <bool FWD, bool S2, bool FUSED, int TERMS = 3, bool HERM = false, bool PAIR = false>
 __global__ void __launch_bounds__(THREADS, 1)
     so3_tc_gemm_kernel(const __grid_constant__ CUtensorMap tA0, const __grid_constant__ CUtensorMap tA1,
                        const __grid_constant__ CUtensorMap tA2, const __grid_constant__ GemmArgs args,
@@ -505,21 +511,25 @@ __global__ void __launch_bounds__(THREADS, 1)
             int lim;          // valid extent of the run (N, or nl)
             int N;            // the item's grid size (weights are zero beyond it)
             const float* wf;  // the item's quadrature weights (fused launches)
+            bool second;      // the paired group: forward runs backwards, inverse signs alternate
         };
         auto source = [&](const int4& item, const int2& aux) -> Src {
             const GemmArgs& A = argsof(item);
             const int N = A.N;
             int m0, n0;
             item_mn(item, m0, n0);
-            const GroupPairs P = S2 ? s2_pairs(m0) : group_pairs(m0, n0);
-            const int f = ctile(item) * FPTK + fl;
             Src r;
+            r.second = PAIR && A.paired && fl >= FPTK / 2;
+            const bool none = r.second && n0 == 0;
+            if (r.second) n0 = -n0;
+            const GroupPairs P = S2 ? s2_pairs(m0) : group_pairs(m0, n0);
+            const int f = PAIR && A.paired ? fl & (FPTK / 2 - 1) : ctile(item) * FPTK + fl;
             r.lim = FWD ? N : A.L + 1 - m0;
             r.N = N;
             r.wf = A.wf;
             r.p = nullptr;
             const int pr = HERM ? herm_pair<FWD, S2>(P, n0, pp, A.by_q) : pp;
-            if (f >= A.batch || pr >= P.np) return r;
+            if (f >= A.batch || pr >= P.np || none) return r;
             if (FWD && S2) {
                 const int bin = pr == 0 ? m0 : N - m0;
                 r.p = A.pin + (long long)f * A.fstride + (long long)bin * N;
@@ -528,7 +538,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                 int qi = (-P.n[pr]) % N; if (qi < 0) qi += N;
                 r.p = A.pin + (long long)f * A.fstride + ((long long)pi * N + qi) * N;
             } else {
-                r.p = A.cin + (long long)f * A.cstride + aux.x + (long long)pr * r.lim;
+                r.p = A.cin + (long long)f * A.cstride + (r.second ? A.goff2[m0 * m0 + m0 + n0] : aux.x) + (long long)pr * r.lim;
             }
             return r;
         };
@@ -536,7 +546,23 @@ __global__ void __launch_bounds__(THREADS, 1)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int k = i * BK + (q4 + 4 * (h ^ hs)) * 8;
-                if (FWD && sr.p && k + 8 <= sr.lim) {
+                if (PAIR && FWD && sr.second) {
+                    // a paired group's run backwards: element k + j at e - j (N is even: e - 7 on 16 bytes)
+                    const float2* e = sr.p + sr.lim - 1 - k;
+                    if (sr.p && k + 8 <= sr.lim) {
+                        const float4* s4 = reinterpret_cast<const float4*>(e - 7);
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const float4 t = __ldg(s4 + 3 - j);
+                            v[8 * h + 2 * j] = make_float2(t.z, t.w);
+                            v[8 * h + 2 * j + 1] = make_float2(t.x, t.y);
+                        }
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j)
+                            v[8 * h + j] = (sr.p && k + j < sr.lim) ? __ldg(e - j) : make_float2(0.f, 0.f);
+                    }
+                } else if (FWD && sr.p && k + 8 <= sr.lim) {
                     const float4* s4 = reinterpret_cast<const float4*>(sr.p + k);
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
@@ -591,7 +617,8 @@ __global__ void __launch_bounds__(THREADS, 1)
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const int k = (i2 + 2) * BK + (q4 + 4 * h) * 8;
-                    if (k < snxt.lim) asm volatile("prefetch.global.L2 [%0];" ::"l"(snxt.p + k) : "memory");
+                    if (k < snxt.lim)
+                        asm volatile("prefetch.global.L2 [%0];" ::"l"(snxt.p + (PAIR && snxt.second ? snxt.lim - 1 - k : k)) : "memory");
                 }
             }
             const int s = kc % STAGES;
@@ -608,8 +635,9 @@ __global__ void __launch_bounds__(THREADS, 1)
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
                     const float2 v = cur[h * 8 + j];
-                    const float wk =
-                        FWD ? ((k + j < scur.N) ? (FUSED ? __ldg(scur.wf + k + j) : wsm[k + j]) : 0.f) : 1.f;
+                    const int kw = PAIR && scur.second ? scur.N - 1 - k - j : k + j;
+                    const float wk = FWD ? ((k + j < scur.N) ? (FUSED ? __ldg(scur.wf + kw) : wsm[kw]) : 0.f)
+                                         : PAIR && (j & 1) && scur.second ? -1.f : 1.f;
                     re[j] = v.x * wk;
                     im[j] = v.y * wk;
                 }
@@ -654,14 +682,20 @@ __global__ void __launch_bounds__(THREADS, 1)
             const int N = A.N;
             int m0, n0;
             item_mn(item, m0, n0);
-            const GroupPairs P = S2 ? s2_pairs(m0) : group_pairs(m0, n0);
             const int nl = A.L + 1 - m0;
             const bool half = FWD && FFTSO3_MMA_M64 && (nl - item.y * BM) <= BM / 2;  // M = 64 item (see MMA)
+            const int ab = t & 1;
+            const int nhalf = PAIR && A.paired ? 2 : 1;
+            for (int hf = 0; hf < (PAIR ? nhalf : 1); ++hf) {
+            if (hf && n0 == 0) break;
+            if (hf) n0 = -n0;
+            const GroupPairs P = S2 ? s2_pairs(m0) : group_pairs(m0, n0);
+            const long long co = hf ? A.goff2[m0 * m0 + m0 + n0] : aux.x;
             long long poff[4];
 #pragma unroll
             for (int p = 0; p < 4; ++p) {
                 if (FWD) {
-                    poff[p] = aux.x + (long long)p * nl;
+                    poff[p] = co + (long long)p * nl;
                 } else if (S2) {
                     int bin = (p == 0 ? -m0 : m0) % N; if (bin < 0) bin += N;
                     poff[p] = (long long)bin * N;
@@ -686,30 +720,30 @@ __global__ void __launch_bounds__(THREADS, 1)
                     hs2[p] = both ? (float)P.sign[pc] : 0.f;
                 }
             }
-            const int ab = t & 1;
-            if (!mbar_wait(&accf[ab], (t >> 1) & 1, args.err, 5)) {
+            if (hf == 0 && !mbar_wait(&accf[ab], (t >> 1) & 1, args.err, 5)) {
                 *abort_flag = 1;
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(ab * 256);
-            for (int chunk = 0; chunk < BN / 32; ++chunk) {
+            for (int chunk = hf * (BN / 64); chunk < (nhalf == 2 ? (hf + 1) * (BN / 64) : BN / 32); ++chunk) {
                 float v[32];
                 if constexpr (TERMS == 3) tmem_ld32_sum(trow + chunk * 32, trow + 128 + chunk * 32, v);
                 else tmem_ld32_one(trow + chunk * 32, v);
 #pragma unroll
                 for (int fq = 0; fq < 32 / (2 * PPF); ++fq) {
-                    const int f = ctile(item) * FPTK + chunk * (32 / (2 * PPF)) + fq;
+                    const int f = ctile(item) * FPTK + chunk * (32 / (2 * PPF)) + fq - hf * (FPTK / 2);
                     if (f >= A.batch) continue;
                     if (FWD) {
                         // M = 64 tiles: rows 16 quarter + lane (lanes 0..15 of each quarter)
                         const int row = half ? item.y * BM + quarter * 16 + lane : item.y * BM + r;
                         if ((half && lane >= 16) || row >= nl) continue;
                         float2* Fo = A.cout + (long long)f * A.cstride + row;
+                        const float flip = hf && (row & 1) ? -1.f : 1.f;
                         if (HERM) {
 #pragma unroll
                             for (int p = 0; p < PPF; ++p) {
-                                const float x = v[fq * 2 * PPF + 2 * p], y = v[fq * 2 * PPF + 2 * p + 1];
+                                const float x = flip * v[fq * 2 * PPF + 2 * p], y = flip * v[fq * 2 * PPF + 2 * p + 1];
                                 if (h1[p] >= 0) Fo[h1[p]] = make_float2(hs1[p] * x, hs1[p] * y);
                                 if (h2[p] >= 0) Fo[h2[p]] = make_float2(hs2[p] * x, -(hs2[p] * y));
                             }
@@ -718,13 +752,13 @@ __global__ void __launch_bounds__(THREADS, 1)
 #pragma unroll
                         for (int p = 0; p < 4; ++p) {
                             if (p >= P.np) break;
-                            const float sg = (float)P.sign[p];
+                            const float sg = flip * (float)P.sign[p];
                             Fo[poff[p]] = make_float2(sg * v[fq * 2 * PPF + 2 * p], sg * v[fq * 2 * PPF + 2 * p + 1]);
                         }
                     } else {
                         const int k = item.y * BM + r;
                         if (k >= N) continue;
-                        float2* Ho = A.pout + (long long)f * A.fstride + k;
+                        float2* Ho = A.pout + (long long)f * A.fstride + (hf ? N - 1 - k : k);
                         if (HERM) {
 #pragma unroll
                             for (int p = 0; p < PPF; ++p) {
@@ -742,6 +776,8 @@ __global__ void __launch_bounds__(THREADS, 1)
                     }
                 }
             }
+            }
+            if (*abort_flag) break;
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(&acce[ab]);
@@ -1294,6 +1330,7 @@ struct TCState {
     bool refine = false;
     bool real = false;            // real grids (FFTSO3_*_REAL): real samples in, real part out
     bool herm = false;            // real functions on the tensor cores: one GEMM pair of two (see the kernel)
+    bool paired = false;          // at most half a column tile of functions: groups +-n0 share the tiles (GemmArgs::paired)
     bool s2 = false;              // S^2 (Legendre groups g = m, grids N^2) instead of SO(3)
     bool simt = false;            // FP32 CUDA-core beta-sum (FFTSO3_PREC_FP32) instead of tcgen05
     float* d_tab32 = nullptr;     // FP32 table [row][Kp] (simt)
@@ -1395,6 +1432,25 @@ void tc_destroy(TCState* s)
 }
 
 long long tc_device_bytes(const TCState* s) { return s ? s->bytes : 0; }
+
+template <bool HERM, bool PAIR>
+static auto so3_kernel(bool fwd, bool fused, int terms)
+{
+    if (fused) return fwd ? so3_tc_gemm_kernel<true, false, true, 3, HERM, PAIR> : so3_tc_gemm_kernel<false, false, true, 3, HERM, PAIR>;
+    if (!fwd) return so3_tc_gemm_kernel<false, false, false, 3, HERM, PAIR>;
+    return terms == 1 ? so3_tc_gemm_kernel<true, false, false, 1, HERM, PAIR> : so3_tc_gemm_kernel<true, false, false, 3, HERM, PAIR>;
+}
+template <bool HERM>
+static auto gemm_kernel(bool fwd, bool s2, bool fused, int terms, bool paired)
+{
+    if (!s2) return paired ? so3_kernel<HERM, true>(fwd, fused, terms) : so3_kernel<HERM, false>(fwd, fused, terms);
+    if (fused) return fwd ? so3_tc_gemm_kernel<true, true, true, 3, HERM> : so3_tc_gemm_kernel<false, true, true, 3, HERM>;
+    return fwd ? so3_tc_gemm_kernel<true, true, false, 3, HERM> : so3_tc_gemm_kernel<false, true, false, 3, HERM>;
+}
+static auto gemm_kernel(bool herm, bool fwd, bool s2, bool fused, int terms, bool paired)
+{
+    return herm ? gemm_kernel<true>(fwd, s2, fused, terms, paired) : gemm_kernel<false>(fwd, s2, fused, terms, paired);
+}
 
 static int autotune_fft(TCState* s, std::string& err);
 static int autotune_cluster(TCState* s, std::string& err);
@@ -1503,6 +1559,7 @@ int tc_create(TCState** out, int L, int N, int batch, const double* d_table_fp64
     s->herm = real && !simt;
     const int fpt = (s2 ? FPT_S2 : FPT) * (s->herm ? 2 : 1);
     s->ntiles = (batch + fpt - 1) / fpt;
+    s->paired = !s2 && !simt && batch <= fpt / 2;
     make_fft_factors_prime_first(N, s->fac);
     s->d_tw = d_tw;
     s->total_rows = table_elems / N;
@@ -1595,6 +1652,7 @@ int tc_create(TCState** out, int L, int N, int batch, const double* d_table_fp64
         const int nl = s->B - m0;
         goff2[g] = acc2;
         acc2 += (long long)(s2 ? (m0 > 0 ? 2 : 1) : group_pairs(m0, n0).np) * nl;
+        if (s->paired && n0 < 0) continue;
         for (int nt = 0; nt < s->ntiles; ++nt) {
             for (int mt = 0; mt * BM < nl; ++mt) itf.push_back(make_int4(g, mt, nt, item_w(m0, n0)));
             for (int mt = 0; mt * BM < N; ++mt) iti.push_back(make_int4(g, mt, nt, item_w(m0, n0)));
@@ -1651,19 +1709,9 @@ int tc_create(TCState** out, int L, int N, int batch, const double* d_table_fp64
         }
     }
     cudaError_t e = cudaSuccess;
-    const void* kernels[18] = {
-        (const void*)so3_tc_gemm_kernel<true, false, false>, (const void*)so3_tc_gemm_kernel<false, false, false>,
-        (const void*)so3_tc_gemm_kernel<true, true, false>,  (const void*)so3_tc_gemm_kernel<false, true, false>,
-        (const void*)so3_tc_gemm_kernel<true, false, true>,  (const void*)so3_tc_gemm_kernel<false, false, true>,
-        (const void*)so3_tc_gemm_kernel<true, true, true>,   (const void*)so3_tc_gemm_kernel<false, true, true>,
-        (const void*)so3_tc_gemm_kernel<true, false, false, 1>,
-        (const void*)so3_tc_gemm_kernel<true, false, false, 3, true>, (const void*)so3_tc_gemm_kernel<false, false, false, 3, true>,
-        (const void*)so3_tc_gemm_kernel<true, true, false, 3, true>,  (const void*)so3_tc_gemm_kernel<false, true, false, 3, true>,
-        (const void*)so3_tc_gemm_kernel<true, false, true, 3, true>,  (const void*)so3_tc_gemm_kernel<false, false, true, 3, true>,
-        (const void*)so3_tc_gemm_kernel<true, true, true, 3, true>,   (const void*)so3_tc_gemm_kernel<false, true, true, 3, true>,
-        (const void*)so3_tc_gemm_kernel<true, false, false, 1, true>};
-    for (int i = 0; i < 18 && e == cudaSuccess; ++i)
-        e = cudaFuncSetAttribute(kernels[i], cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    for (int i = 0; i < 8 && !simt && e == cudaSuccess; ++i)
+        e = cudaFuncSetAttribute((const void*)gemm_kernel(s->herm, i & 1, s2, i & 2, i & 4 ? 1 : 3, s->paired),
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     if (e != cudaSuccess) {
         err = std::string("tensor-core kernel attributes: ") + cudaGetErrorString(e);
         return bail(FFTSO3_ERR_CUDA);
@@ -1899,22 +1947,8 @@ static GemmArgs gemm_args(const TCState* s)
     a.half = s->half_pencils();
     a.by_q = !s->dft_tc;
     a.half_coeffs = s->herm;
+    a.paired = s->paired;
     return a;
-}
-
-template <bool HERM>
-static auto gemm_kernel(bool fwd, bool s2, int terms)
-{
-    return fwd ? (s2 ? so3_tc_gemm_kernel<true, true, false, 3, HERM>
-                     : (terms == 1 ? so3_tc_gemm_kernel<true, false, false, 1, HERM>
-                                   : so3_tc_gemm_kernel<true, false, false, 3, HERM>))
-               : (s2 ? so3_tc_gemm_kernel<false, true, false, 3, HERM> : so3_tc_gemm_kernel<false, false, false, 3, HERM>);
-}
-template <bool HERM>
-static auto fused_gemm_kernel(bool fwd, bool s2)
-{
-    return fwd ? (s2 ? so3_tc_gemm_kernel<true, true, true, 3, HERM> : so3_tc_gemm_kernel<true, false, true, 3, HERM>)
-               : (s2 ? so3_tc_gemm_kernel<false, true, true, 3, HERM> : so3_tc_gemm_kernel<false, false, true, 3, HERM>);
 }
 
 // cout: the forward's group-major output (default: the plan's d_fg); terms: 1 selects the one-term kernel (SO(3)
@@ -1945,7 +1979,7 @@ static int launch_gemm(TCState* s, bool fwd, cudaStream_t st, std::string& err, 
         return FFTSO3_SUCCESS;
     }
     const CUtensorMap* tm = fwd ? s->tmA_fwd : s->tmA_inv;
-    auto kern = s->herm ? gemm_kernel<true>(fwd, s->s2, terms) : gemm_kernel<false>(fwd, s->s2, terms);
+    auto kern = gemm_kernel(s->herm, fwd, s->s2, false, terms, s->paired);
     if (s->csize == 1) {
         const int nctas = a.nitems < s->nsm ? a.nitems : s->nsm;
         kern<<<nctas, THREADS, SMEM_BYTES, st>>>(tm[0], tm[1], tm[2], a, nullptr);
@@ -2576,7 +2610,9 @@ int tc_fused_gemm(TCFused* f, bool fwd, cudaStream_t st, StageTimer* T, std::str
     const int nctas = a.nitems < f->nsm ? a.nitems : f->nsm;
     const CUtensorMap* tm = fwd ? f->parts[0]->tmA_fwd : f->parts[0]->tmA_inv;  // unused by fused kernels
     T->begin(fwd ? ST_GEMM_FWD : ST_GEMM_INV, st);
-    auto kern = f->parts[0]->herm ? fused_gemm_kernel<true>(fwd, f->s2) : fused_gemm_kernel<false>(fwd, f->s2);
+    bool paired = false;
+    for (TCState* p : f->parts) paired = paired || p->paired;
+    auto kern = gemm_kernel(f->parts[0]->herm, fwd, f->s2, true, 3, paired);
     kern<<<nctas, THREADS, SMEM_BYTES, st>>>(tm[0], tm[1], tm[2], a, f->d_segs[d]);
     TCK(cudaGetLastError());
     T->end(st);
