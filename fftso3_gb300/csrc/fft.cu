@@ -559,10 +559,27 @@ __device__ __forceinline__ void synth_rows_out(const qc32* sm, long long o, long
     }
 }
 
+// The stage tables: radix-8 stages with Ns = 8, 64 (when present), then the last radix-4 / 2 stage with Ns = 64, N - 8 entries.
+// Made once per plan: built by every CTA from the FP64 table, their FP64 loads and conversions took
+// 8 to 11 % of a pass at N = 64 and 128, 2 % at N = 512.
+__global__ void df32_k_table_kernel(dfc32* __restrict__ w, const double2* __restrict__ tw, int N)
+{
+    int off = 0;
+    for (int Ns = 8; Ns < N; Ns *= 8) {
+        const int R = Ns * 8 <= N ? 8 : N / Ns;
+        for (int i = threadIdx.x; i < (R - 1) * Ns; i += blockDim.x) {
+            const int r = i / Ns + 1, kt = i % Ns;
+            const double2 v = tw[r * kt * (N / (R * Ns))];
+            w[off + i] = dfc32{df32(v.x), df32(v.y)};
+        }
+        off += (R - 1) * Ns;
+    }
+}
+
 template <int N, int LOAD, int STORE>
 __global__ void __launch_bounds__(256, 4) fft_df32_k_kernel(dfc32* __restrict__ buf, long long S, long long oinner,
                                                              long long oouter, long long oistride,
-                                                             const double2* __restrict__ twg, const void* fin,
+                                                             const dfc32* __restrict__ twg, const void* fin,
                                                              float2* __restrict__ hi, float2* __restrict__ lo)
 {
     constexpr int TK = 2048 / N;         // lines per CTA
@@ -575,19 +592,7 @@ __global__ void __launch_bounds__(256, 4) fft_df32_k_kernel(dfc32* __restrict__ 
     const int tid = threadIdx.x;
     const long long o = blockIdx.y;
     const long long obase = (o / oinner) * oouter + (o % oinner) * oistride + (long long)blockIdx.x * TK;
-    // stage tables: radix-8 stages with Ns = 8, 64 (when present) and the last radix-4 / 2 stage with Ns = 64
-    {
-        int off = 0;
-        for (int Ns = 8; Ns < N; Ns *= 8) {
-            const int R = Ns * 8 <= N ? 8 : N / Ns;
-            for (int i = tid; i < (R - 1) * Ns; i += 256) {
-                const int r = i / Ns + 1, kt = i % Ns;
-                const double2 v = twg[r * kt * (N / (R * Ns))];
-                w[off + i] = dfc32{df32(v.x), df32(v.y)};
-            }
-            off += (R - 1) * Ns;
-        }
-    }
+    for (int i = tid; i < N - 8; i += 256) w[i] = twg[i];
     const int kq = tid % TK, tq = tid / TK;  // k-fastest thread of the first / last stage
     const int kk = tid / TPL, t = tid % TPL;  // line-major thread of the middle stages
     // the CTA's block of TK lines: loaded as double-float, then put on the block's quantum
@@ -1033,7 +1038,7 @@ bool fft_df32_k_supported(int N) { return N == 64 || N == 128 || N == 256 || N =
 
 template <int LOAD, int STORE>
 static void df32_k_launch(int N, dim3 grid, dfc32* b, long long S, long long oinner, long long oouter,
-                          long long oistride, const double2* t, const void* fin, float2* hi, float2* lo,
+                          long long oistride, const dfc32* t, const void* fin, float2* hi, float2* lo,
                           cudaStream_t st)
 {
     switch (N) {
@@ -1052,13 +1057,11 @@ static void df32_k_launch(int N, dim3 grid, dfc32* b, long long S, long long oin
     }
 }
 
-cudaError_t launch_fft_df32_k(void* buf, int N, long long S, long long nouter, long long oinner, long long oouter,
-                              long long oistride, const void* tw, cudaStream_t st)
+size_t fft_df32_k_table_bytes(int N) { return sizeof(dfc32) * (size_t)N; }
+
+cudaError_t fft_df32_k_build_table(void* table, int N, const void* tw, cudaStream_t st)
 {
-    if (!fft_df32_k_supported(N) || nouter < 1 || nouter > 65535 || oinner < 1) return cudaErrorInvalidValue;
-    const dim3 grid((unsigned)(N / (2048 / N)), (unsigned)nouter);
-    df32_k_launch<0, 0>(N, grid, (dfc32*)buf, S, oinner, oouter, oistride, (const double2*)tw, nullptr, nullptr,
-                        nullptr, st);
+    df32_k_table_kernel<<<1, 256, 0, st>>>((dfc32*)table, (const double2*)tw, N);
     return cudaGetLastError();
 }
 
@@ -1068,7 +1071,7 @@ cudaError_t launch_fft_df32_k_forward(void* buf, int N, long long nb, const void
     if (!fft_df32_k_supported(N) || nb < 1 || nb * N > 65535) return cudaErrorInvalidValue;
     const dim3 grid((unsigned)(N / (2048 / N)), (unsigned)(nb * N));
     const long long NN = (long long)N * N;
-    const double2* t = (const double2*)tw;
+    const dfc32* t = (const dfc32*)tw;
     dfc32* b = (dfc32*)buf;
     // along j2, from the grid rows, into buf [fn][j1][q][k]
     if (real)
@@ -1088,7 +1091,7 @@ cudaError_t launch_fft_df32_k_synth_pass(int pass, void* buf, int N, long long n
     if (!fft_df32_k_supported(N) || nb < 1 || nb * N > 65535 || (pass != 1 && pass != 2)) return cudaErrorInvalidValue;
     const dim3 grid((unsigned)(N / (2048 / N)), (unsigned)(nb * N));
     const long long NN = (long long)N * N;
-    const double2* t = (const double2*)tw;
+    const dfc32* t = (const dfc32*)tw;
     dfc32* b = (dfc32*)buf;
     if (pass == 1) {
         // along p (stride N^2), lines (fn, q), in place

@@ -40,26 +40,23 @@ cudaError_t launch_fft_lines(const FFTLaunch& L, cudaStream_t st);
 bool dft64_supported(int N);
 cudaError_t launch_dft64(const FFTLaunch& L, cudaStream_t st);
 
-// Double-float (dfc32) FFT along a strided axis of arrays whose innermost index k (N values) is contiguous,
-// in place: line (o, k), o < nouter, has element j at obase(o) + k + j S, obase(o) = (o / oinner) oouter +
-// (o % oinner) oistride.  N = 64..512, powers of two (fft.cu).
+// Double-float (dfc32) FFTs of N = 64..512, powers of two, along a strided axis of arrays whose innermost index k (N values)
+// is contiguous (fft.cu).  table: the stage twiddles in double-float, made once per plan from its twiddle table tw.
 bool fft_df32_k_supported(int N);
-cudaError_t launch_fft_df32_k(void* buf, int N, long long S, long long nouter, long long oinner, long long oouter,
-                              long long oistride, const void* tw, cudaStream_t st);
+size_t fft_df32_k_table_bytes(int N);
+cudaError_t fft_df32_k_build_table(void* table, int N, const void* tw, cudaStream_t st);
 // Double-float forward FFT of nb sample grids f [fn][k][j1][j2] (complex64, or float32 when real) into the
 // k-contiguous pencils [fn][p][q][k], written renormalised as hi (complex64, the FP32 rounding) + lo (the
 // remainder); buf: nb double-float grids of work space.
 cudaError_t launch_fft_df32_k_forward(void* buf, int N, long long nb, const void* f, bool real, float2* hi,
-                                      float2* lo, const void* tw, cudaStream_t st);
+                                      float2* lo, const void* table, cudaStream_t st);
 // One pass (1: along p, in place; 2: along q into out) of the double-float FFT of nb synthesis pencils buf [fn][p][q][k]
 // (dfc32; overwritten) into the grids out [fn][k][j1][j2], rounded once to complex64, or to the real part as float32 when real.
 cudaError_t launch_fft_df32_k_synth_pass(int pass, void* buf, int N, long long nb, void* out, bool real,
-                                         const void* tw, cudaStream_t st);
+                                         const void* table, cudaStream_t st);
 
 // Register-resident FP32 kernels for N = 64..1024, powers of two (fft_fast.cu).
 bool fft_fast_supported(int N);
-// nlines contiguous lines of N complex64: out[line][K] = FFT(in[line])[K] (in may equal out)
-cudaError_t launch_fft_rows_fast(const void* in, void* out, long long nlines, int N, const void* tw, cudaStream_t st);
 // Tiled transposing passes over nf grids of N^3 complex64 (in != out):
 //   pass  1: grid [nf][k][j1][j2] -> FFT over j2 -> T1 [nf][k][q][j1]
 //   pass  2: T1 [nf][k][q][j1]    -> FFT over j1 -> pencils [nf][p][q][k]

@@ -2,8 +2,6 @@
 // (R = 2..32, i.e. N = 64..1024, powers of two).
 //
 // Kernels:
-//   fft_rows_reg  lines contiguous (one axis of a contiguous array): one warp a line, lane t holds x[t + 32 i], an
-//                 R-point DFT in registers, twiddles, a 32-point one across the lanes by shuffles;
 //   fft_tile      a tile of 16 lines with one side contiguous and the other transposed, so a 2-D transform of
 //                 the Euler grid is two passes that both read and write whole 128-byte runs, the second one
 //                 producing the k-contiguous pencils [fn][p][q][k] the beta-sum GEMM consumes (and the reverse
@@ -39,38 +37,6 @@ __host__ __device__ constexpr int ilog2(int x) { return x <= 1 ? 0 : 1 + ilog2(x
 __device__ __forceinline__ float2 cmulf(float2 a, float2 b)
 {
     return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-
-// R-point radix-2 DIF in registers (natural input, bit-reversed output);
-// tw(k, h) = e^{-2 pi i k / (2h)}, the twiddle of butterfly k of the stage of span h.
-template <int R, typename TW>
-__device__ __forceinline__ void reg_dif_t(float2 (&v)[R], TW tw)
-{
-#pragma unroll
-    for (int h = R / 2; h >= 1; h >>= 1) {
-#pragma unroll
-        for (int j = 0; j < R; j += 2 * h) {
-#pragma unroll
-            for (int k = 0; k < h; ++k) {
-                const float2 a = v[j + k], b = v[j + k + h];
-                v[j + k] = make_float2(a.x + b.x, a.y + b.y);
-                const float2 d = make_float2(a.x - b.x, a.y - b.y);
-                if (k == 0)
-                    v[j + k + h] = d;
-                else if (4 * k == 2 * h)
-                    v[j + k + h] = make_float2(d.y, -d.x);  // w = -i
-                else
-                    v[j + k + h] = cmulf(d, tw(k, h));
-            }
-        }
-    }
-}
-
-// ... with the full table W[j] = e^{-2 pi i j / N}
-template <int R>
-__device__ __forceinline__ void reg_dif(float2 (&v)[R], const float2* __restrict__ W, int N)
-{
-    reg_dif_t<R>(v, [&](int k, int h) { return W[k * (N / (2 * h))]; });
 }
 
 // cos(2 pi k / 32)
@@ -121,72 +87,6 @@ __device__ __forceinline__ void reg_dft(float2 (&v)[P])
             const float2 a = v[j], b = v[j + 1];
             v[j] = make_float2(a.x + b.x, a.y + b.y);
             v[j + 1] = make_float2(a.x - b.x, a.y - b.y);
-        }
-    }
-}
-
-// Full N = 32 R point FFT of the line held by the warp (see the file comment).
-template <int R>
-__device__ __forceinline__ void warp_fft(float2 (&v)[R], const float2* __restrict__ W, int lane)
-{
-    constexpr int N = 32 * R;
-    constexpr int LR = ilog2(R);
-    reg_dif<R>(v, W, N);
-#pragma unroll
-    for (int r = 1; r < R; ++r) {
-        const int k1 = brev(r, LR);
-        v[r] = cmulf(v[r], W[lane * k1]);
-    }
-#pragma unroll
-    for (int h = 16; h >= 1; h >>= 1) {
-        const bool upper = (lane & h) != 0;
-        const int kk = lane & (h - 1);
-        const float2 w = W[kk * (N / (2 * h))];
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const float ox = __shfl_xor_sync(FULL, v[r].x, h);
-            const float oy = __shfl_xor_sync(FULL, v[r].y, h);
-            if (!upper) {
-                v[r].x += ox;
-                v[r].y += oy;
-            } else {
-                v[r] = cmulf(make_float2(ox - v[r].x, oy - v[r].y), w);
-            }
-        }
-    }
-}
-
-template <int N>
-__device__ __forceinline__ void load_twiddles(float2* Ws, const double2* __restrict__ tw)
-{
-    for (int i = threadIdx.x; i < N; i += blockDim.x) Ws[i] = make_float2((float)tw[i].x, (float)tw[i].y);
-}
-
-// Contiguous lines: in[line * N + j] -> out[line * N + K].
-template <int R, int WPB, int LPW>
-__global__ void __launch_bounds__(32 * WPB) fft_rows_reg(const float2* __restrict__ in, float2* __restrict__ out,
-                                                         long long nlines, const double2* __restrict__ tw)
-{
-    constexpr int N = 32 * R;
-    constexpr int LR = ilog2(R);
-    __shared__ float2 Ws[N];
-    load_twiddles<N>(Ws, tw);
-    __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int t5 = brev(lane, 5);
-    for (int u = 0; u < LPW; ++u) {
-        const long long line = ((long long)blockIdx.x * LPW + u) * WPB + warp;
-        if (line >= nlines) return;
-        const float2* src = in + line * N;
-        float2 v[R];
-#pragma unroll
-        for (int i = 0; i < R; ++i) v[i] = src[lane + 32 * i];
-        warp_fft<R>(v, Ws, lane);
-        float2* dst = out + line * N + R * t5;
-#pragma unroll
-        for (int k1 = 0; k1 < R; k1 += 2) {
-            const float2 a = v[brev(k1, LR)], b = v[brev(k1 + 1, LR)];
-            reinterpret_cast<float4*>(dst)[k1 / 2] = make_float4(a.x, a.y, b.x, b.y);
         }
     }
 }
@@ -843,31 +743,9 @@ static cudaError_t grid2d_dispatch(const Grid2DArgs& a, long long tiles, int N, 
     }
 }
 
-template <int R>
-static cudaError_t rows_r(const void* in, void* out, long long nlines, const void* tw, cudaStream_t st)
-{
-    constexpr int WPB = 8, LPW = 4;
-    const long long per = (long long)WPB * LPW;
-    fft_rows_reg<R, WPB, LPW><<<(unsigned)((nlines + per - 1) / per), 32 * WPB, 0, st>>>(
-        (const float2*)in, (float2*)out, nlines, (const double2*)tw);
-    return cudaGetLastError();
-}
-
 }  // namespace ffast
 
 bool fft_fast_supported(int N) { return N == 64 || N == 128 || N == 256 || N == 512 || N == 1024; }
-
-cudaError_t launch_fft_rows_fast(const void* in, void* out, long long nlines, int N, const void* tw, cudaStream_t st)
-{
-    switch (N) {
-        case 64: return ffast::rows_r<2>(in, out, nlines, tw, st);
-        case 128: return ffast::rows_r<4>(in, out, nlines, tw, st);
-        case 256: return ffast::rows_r<8>(in, out, nlines, tw, st);
-        case 512: return ffast::rows_r<16>(in, out, nlines, tw, st);
-        case 1024: return ffast::rows_r<32>(in, out, nlines, tw, st);
-        default: return cudaErrorNotSupported;
-    }
-}
 
 // Forward passes of one batch of N^3 grids (see fft.cuh):
 //   pass 1: grid [f][k][j1][j2] -> FFT over j2 -> T1 [f][k][q][j1]

@@ -668,6 +668,7 @@ struct OZState {
     unsigned char* bimg = nullptr;  // [column tile][tile] x STAGE_B: their digit image (digit_image_kernel)
     int* gt0 = nullptr;             // first image tile of each group
     long long nbt = 0;              // image tiles per column tile
+    void* wk = nullptr;         // stage twiddles of the double-float FFT (fft.cu), or null: N is not one of its
     void* dft = nullptr;        // digit DFT matrices (dft_oz.cu), or null: N is a power of two, or the grid form
     float4* pen = nullptr;      // [chunk][N^3] double-float pencils / grid
     long long* goff2 = nullptr;
@@ -711,7 +712,7 @@ void oz_destroy(OZState* o)
     if (!o) return;
     for (int p = 0; p < NS; ++p)
         if (o->planes[p]) cudaFree(o->planes[p]);
-    void* ptrs[] = {o->et, o->ey, o->bimg, o->gt0, o->pen, o->dft, o->goff2, o->items, o->iaux, o->items_p, o->iaux_p, o->err};
+    void* ptrs[] = {o->et, o->ey, o->bimg, o->gt0, o->pen, o->wk, o->dft, o->goff2, o->items, o->iaux, o->items_p, o->iaux_p, o->err};
     for (void* q : ptrs)
         if (q) cudaFree(q);
     for (void* q : o->items_z)
@@ -864,7 +865,10 @@ int oz_create(OZState** out, const double* d_table, const std::vector<long long>
     cudaMemset(o->err, 0, sizeof(int));
     cudaError_t e = cudaFuncSetAttribute(oz_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     // powers of two from 64 have the double-float FFT (fft.cu); other N up to 222 the digit DFT
-    if (!fft_df32_k_supported(N) && dft_oz_supported(N)) {
+    if (fft_df32_k_supported(N)) {
+        if ((rc = oz_alloc(o, &o->wk, fft_df32_k_table_bytes(N), err))) return bail(rc);
+        if (e == cudaSuccess) e = fft_df32_k_build_table(o->wk, N, d_tw, 0);
+    } else if (dft_oz_supported(N)) {
         if ((rc = oz_alloc(o, &o->dft, dft_oz_table_bytes(N), err))) return bail(rc);
         if (e == cudaSuccess) e = dft_oz_build_table(o->dft, N, d_tw, 0);
     }
@@ -987,7 +991,7 @@ static int synth_step(OZState* o, int step, float4* pen, int nb, void* out, bool
     if (!by_lines(o)) {
         OZK(o->dft ? launch_dft_oz_grid_pass(pen, step == 1 ? pen : out, nullptr, nb, N, step == 1 ? -2 : -1, real, o->dft,
                                              o->err, st)
-                   : launch_fft_df32_k_synth_pass(step, pen, N, nb, out, real, o->d_tw, st));
+                   : launch_fft_df32_k_synth_pass(step, pen, N, nb, out, real, o->wk, st));
         return FFTSO3_SUCCESS;
     }
     if (step == 1) return synth_fft_lines(o, pen, nb, st, err);
@@ -1033,7 +1037,7 @@ int oz_forward_fft(OZState* o, const void* fgrid, bool real, int nb, float2* hi,
         OZK(launch_dft_oz_grid_pass(fgrid, o->pen, nullptr, nb, o->N, 1, real, o->dft, o->err, st));
         OZK(launch_dft_oz_grid_pass(o->pen, hi, lo, nb, o->N, 2, real, o->dft, o->err, st));
     } else {
-        OZK(launch_fft_df32_k_forward(o->pen, o->N, nb, fgrid, real, hi, lo, o->d_tw, st));
+        OZK(launch_fft_df32_k_forward(o->pen, o->N, nb, fgrid, real, hi, lo, o->wk, st));
     }
     T->end(st);
     return FFTSO3_SUCCESS;
