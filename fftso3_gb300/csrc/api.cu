@@ -281,7 +281,6 @@ int fp64_inverse(fftso3_plan* p, const void* Fin_, void* gout, int nb, void* wor
         }
         FFTLaunch rows = fft_rows(p, work, gout, (long long)nb * N, false, p->real, true);
         rows.nyq = 1;
-        if (!dft64_supported(N)) STAGE(ST_NYQUIST, launch_zero_nyquist_s2(work, true, N, (long long)nb * N, st));
         STAGE(s_con, launch_s2_inv_fp64(p->d_table, p->d_goff, Fin, (double2*)work, L, N, nb, st));
         STAGE(s_rows, fft64(rows, st));
     }

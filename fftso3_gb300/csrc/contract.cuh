@@ -17,7 +17,6 @@ cudaError_t launch_s2_fwd_fp64(const double* table, const long long* moff, const
                                double2* F, int L, int N, int batch, bool is_real, cudaStream_t st);
 cudaError_t launch_s2_inv_fp64(const double* table, const long long* moff, const double2* F, double2* H, int L,
                                int N, int batch, cudaStream_t st);
-cudaError_t launch_zero_nyquist_s2(void* H, bool fp64, int N, long long nrows, cudaStream_t st);
 cudaError_t launch_s2_c2r(const void* Fc, void* Fr, bool fp64, int L, int batch, cudaStream_t st);
 cudaError_t launch_s2_r2c(const void* Fr, void* Fc, bool fp64, int L, int batch, cudaStream_t st);
 // tensor-core S^2 real kinds: group-major GEMM output -> real coefficients, and real coefficients ->
