@@ -170,12 +170,13 @@ struct GemmArgs {
     int* err;
     // real functions: the summed pairs have their pencils at q < N / 2 (by_q) or p < N / 2 (S^2: always); the FFT writes and
     // reads those alone (half)
-    int by_q, half;
-    int half_coeffs;           // ... and forward: only the coefficients of pairs 0 and 2 (n0 < 0: 3), m >= 0, are written
+    unsigned char by_q, half;
+    unsigned char half_coeffs;           // ... and forward: only the coefficients of pairs 0 and 2 (n0 < 0: 3), m >= 0, are written
     // SO(3), at most half a column tile of functions: items of n0 >= 0, the second half of the columns holds the group
     // (m0, -n0) against the same table rows, d^l_{m0, -n0}(beta) = (-1)^(l + m0) d^l_{m0, n0}(pi - beta)
-    int paired;
+    unsigned char paired;
 };
+static_assert(sizeof(GemmArgs) <= 128, "small launches took 4 us more with larger arguments (FP32, S^2, l_max 90)");
 
 // One plan's share of a fused launch over several plans (the l_max buckets of
 // an uneven batch): its table maps and arguments.  Work items of a fused launch
@@ -241,14 +242,31 @@ __device__ __forceinline__ GroupPairs s2_pairs(int m)
     return p;
 }
 
+// Pair p of a group as group_pairs / s2_pairs have it, without their tables (a dynamic index would put those in local memory).
+struct Pair {
+    int m, n, sign;
+};
+template <bool S2>
+__device__ __forceinline__ Pair pair_member(int m0, int n0, int p)
+{
+    if (S2) return {p ? -m0 : m0, 0, p && (m0 & 1) ? -1 : 1};
+    const int a = p < 2 ? m0 : n0, b = p < 2 ? n0 : m0;
+    return {p & 1 ? -a : a, p & 1 ? -b : b, (p == 1 || p == 2) && ((m0 + n0) & 1) ? -1 : 1};
+}
+template <bool S2>
+__device__ __forceinline__ int pair_count(int m0, int n0)
+{
+    return m0 == 0 ? 1 : S2 || n0 == m0 || n0 == -m0 ? 2 : 4;
+}
+
 // Real functions: the pair that column pair j of a group sums (its partner, with the conjugate sum, is the pair ^ 1).
 template <bool FWD, bool S2>
-__device__ __forceinline__ int herm_pair(const GroupPairs& P, int n0, int j, int by_q)
+__device__ __forceinline__ int herm_pair(int m0, int n0, int j, int by_q)
 {
     // forward pencils lie at (-m, -n) mod N, inverse ones at (m, n); S^2: forward bins at m for pair 0, inverse at m for pair 1
-    if (S2) return FWD || P.np == 1 ? 0 : 1;
+    if (S2) return FWD || m0 == 0 ? 0 : 1;
     if (by_q) return j == 0 ? ((FWD ? n0 > 0 : n0 < 0) ? 1 : 0) : FWD ? 3 : 2;
-    if (j == 0) return FWD && P.np > 1 ? 1 : 0;
+    if (j == 0) return FWD && m0 > 0 ? 1 : 0;
     return FWD ? (n0 > 0 ? 3 : 2) : (n0 >= 0 ? 2 : 3);
 }
 
@@ -522,20 +540,19 @@ __global__ void __launch_bounds__(THREADS, 1)
             r.second = PAIR && A.paired && fl >= FPTK / 2;
             const bool none = r.second && n0 == 0;
             if (r.second) n0 = -n0;
-            const GroupPairs P = S2 ? s2_pairs(m0) : group_pairs(m0, n0);
             const int f = PAIR && A.paired ? fl & (FPTK / 2 - 1) : ctile(item) * FPTK + fl;
             r.lim = FWD ? N : A.L + 1 - m0;
             r.N = N;
             r.wf = A.wf;
             r.p = nullptr;
-            const int pr = HERM ? herm_pair<FWD, S2>(P, n0, pp, A.by_q) : pp;
-            if (f >= A.batch || pr >= P.np || none) return r;
+            const int pr = HERM ? herm_pair<FWD, S2>(m0, n0, pp, A.by_q) : pp;
+            if (f >= A.batch || pr >= pair_count<S2>(m0, n0) || none) return r;
             if (FWD && S2) {
                 const int bin = pr == 0 ? m0 : N - m0;
                 r.p = A.pin + (long long)f * A.fstride + (long long)bin * N;
             } else if (FWD) {
-                int pi = (-P.m[pr]) % N; if (pi < 0) pi += N;
-                int qi = (-P.n[pr]) % N; if (qi < 0) qi += N;
+                const Pair q = pair_member<S2>(m0, n0, pr);  // |m|, |n| < N
+                const int pi = q.m > 0 ? N - q.m : -q.m, qi = q.n > 0 ? N - q.n : -q.n;
                 r.p = A.pin + (long long)f * A.fstride + ((long long)pi * N + qi) * N;
             } else {
                 r.p = A.cin + (long long)f * A.cstride + (r.second ? A.goff2[m0 * m0 + m0 + n0] : aux.x) + (long long)pr * r.lim;
@@ -693,7 +710,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             const long long co = hf ? A.goff2[m0 * m0 + m0 + n0] : aux.x;
             long long poff[4];
 #pragma unroll
-            for (int p = 0; p < 4; ++p) {
+            for (int p = 0; p < (HERM ? 0 : 4); ++p) {
                 if (FWD) {
                     poff[p] = co + (long long)p * nl;
                 } else if (S2) {
@@ -709,15 +726,21 @@ __global__ void __launch_bounds__(THREADS, 1)
             long long h1[PPF], h2[PPF];
             float hs1[PPF], hs2[PPF];
             if (HERM) {
+                const int cnt = pair_count<S2>(m0, n0);
+                auto place = [&](int p, const Pair& q) -> long long {
+                    if (FWD) return co + (long long)p * nl;
+                    if (S2) return (long long)(q.m > 0 ? N - q.m : -q.m) * N;
+                    return ((long long)(q.m < 0 ? N + q.m : q.m) * N + (q.n < 0 ? N + q.n : q.n)) * N;
+                };
 #pragma unroll
                 for (int p = 0; p < PPF; ++p) {
-                    const int pr = herm_pair<FWD, S2>(P, n0, p, A.by_q), pc = pr ^ 1;
-                    const bool in = pr < P.np, both = in && pc < P.np && (FWD || !A.half || (!S2 && (A.by_q ? P.n[pc] : P.m[pc]) == 0));
-                    const int kept = p == 0 ? 0 : n0 >= 0 ? 2 : 3;
-                    h1[p] = in && !(FWD && A.half_coeffs && pr != kept) ? poff[pr] : -1;
-                    h2[p] = both && !(FWD && A.half_coeffs && pc != kept) ? poff[pc] : -1;
-                    hs1[p] = in ? (float)P.sign[pr] : 0.f;
-                    hs2[p] = both ? (float)P.sign[pc] : 0.f;
+                    const int pr = herm_pair<FWD, S2>(m0, n0, p, A.by_q), pc = pr ^ 1, kept = p == 0 ? 0 : n0 >= 0 ? 2 : 3;
+                    const Pair q = pair_member<S2>(m0, n0, pr), c = pair_member<S2>(m0, n0, pc);
+                    const bool in = pr < cnt, both = in && pc < cnt && (FWD || !A.half || (!S2 && (A.by_q ? c.n : c.m) == 0));
+                    h1[p] = in && !(FWD && A.half_coeffs && pr != kept) ? place(pr, q) : -1;
+                    h2[p] = both && !(FWD && A.half_coeffs && pc != kept) ? place(pc, c) : -1;
+                    hs1[p] = (float)q.sign;
+                    hs2[p] = (float)c.sign;
                 }
             }
             if (hf == 0 && !mbar_wait(&accf[ab], (t >> 1) & 1, args.err, 5)) {
@@ -727,6 +750,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(ab * 256);
             for (int chunk = hf * (BN / 64); chunk < (nhalf == 2 ? (hf + 1) * (BN / 64) : BN / 32); ++chunk) {
+                if (ctile(item) * FPTK + chunk * (32 / (2 * PPF)) - hf * (FPTK / 2) >= A.batch) break;  // no functions left
                 float v[32];
                 if constexpr (TERMS == 3) tmem_ld32_sum(trow + chunk * 32, trow + 128 + chunk * 32, v);
                 else tmem_ld32_one(trow + chunk * 32, v);
@@ -1153,7 +1177,13 @@ static dim3 ptile_grid(int L, int batch)
 // (as two, through packed complex coefficients, 0.148 and 0.141 ms a direction at l_max 63, 64 functions).  A CTA takes the
 // quadruples (+-mu, +-nu) of one nu >= 0, 32 mu and 32 l: group-major runs along l on one side, packed runs along mu on the
 // other: 0.108 and 0.103 ms.  Arithmetic as so3_c2r / so3_r2c and the permutations (rsph.cuh).
-constexpr int RFPC = 4;  // functions per CTA
+// Functions per CTA: 4, which share the index tables, where that leaves enough CTAs (l_max 16, 4 functions: 17 CTAs of 4
+// functions 2 us more than 68 of one).
+static int rtile_functions(int L, int batch)
+{
+    const long long t = (L + 1 + PT - 1) / PT;
+    return (L + 1) * t * t * batch >= 4096 ? 4 : 1;
+}
 struct RTileIdx {
     long long gbase[2][PT];  // of the two group-major entries of mu, relative to l
     float gsign[2][PT];
@@ -1193,15 +1223,15 @@ __device__ __forceinline__ void rtile_index(RTileIdx& t, int L, int nu, int l0, 
 // add: the real coefficients are added to (the refinement's correction)
 __global__ void __launch_bounds__(256) group_to_real_tiled(const float2* __restrict__ Fg, float* __restrict__ Fr,
                                                            const long long* __restrict__ goff2, int L, long long cstride,
-                                                           int batch, bool add)
+                                                           int batch, int fpc, bool add)
 {
     __shared__ float2 tile[2][PT][PT + 1];  // F(l, mu, +-nu): [nu < 0][mu - mb][l - l0]
     __shared__ RTileIdx ix;
     int nu, l0, mb, fg;
     if (!rtile_coords(L, nu, l0, mb, fg)) return;
     rtile_index(ix, L, nu, l0, mb, false, goff2);
-    const int fend = min(batch, (fg + 1) * RFPC);
-    for (int f = fg * RFPC; f < fend; ++f) {
+    const int fend = min(batch, (fg + 1) * fpc);
+    for (int f = fg * fpc; f < fend; ++f) {
         const float2* src = Fg + (long long)f * cstride;
         float* dst = Fr + (long long)f * cstride;
 #pragma unroll
@@ -1236,15 +1266,15 @@ __global__ void __launch_bounds__(256) group_to_real_tiled(const float2* __restr
 // neg_m: the pairs of n >= 0 are wanted (GemmArgs.by_q), else those of m >= 0
 __global__ void __launch_bounds__(256) real_to_group_tiled(const float* __restrict__ Fr, float2* __restrict__ Y,
                                                            const long long* __restrict__ goff2, int L, long long cstride,
-                                                           int batch, bool neg_m)
+                                                           int batch, int fpc, bool neg_m)
 {
     __shared__ float tile[4][PT][PT + 1];  // F_r(l, +-mu, +-nu): [m < 0 | 2 (n < 0)][l - l0][mu - mb]
     __shared__ RTileIdx ix;
     int nu, l0, mb, fg;
     if (!rtile_coords(L, nu, l0, mb, fg)) return;
     rtile_index(ix, L, nu, l0, mb, neg_m, goff2);
-    const int fend = min(batch, (fg + 1) * RFPC);
-    for (int f = fg * RFPC; f < fend; ++f) {
+    const int fend = min(batch, (fg + 1) * fpc);
+    for (int f = fg * fpc; f < fend; ++f) {
         const float* src = Fr + (long long)f * cstride;
         float2* dst = Y + (long long)f * cstride;
 #pragma unroll
@@ -1272,10 +1302,10 @@ __global__ void __launch_bounds__(256) real_to_group_tiled(const float* __restri
     }
 }
 
-static dim3 rtile_grid(int L, int batch)
+static dim3 rtile_grid(int L, int batch, int fpc)
 {
     const unsigned t = (unsigned)((L + 1 + PT - 1) / PT);
-    return dim3((unsigned)(L + 1), t, t * (unsigned)((batch + RFPC - 1) / RFPC));
+    return dim3((unsigned)(L + 1), t, t * (unsigned)((batch + fpc - 1) / fpc));
 }
 
 // S^2: group-major forward output -> packed F(l, m) at l^2 + m + l (one CTA per (l, function)).
@@ -2150,15 +2180,17 @@ static bool direct_real(const TCState* s) { return s->real && (s->s2 || s->herm)
 static cudaError_t real_from_group(TCState* s, void* out, bool add, cudaStream_t st)
 {
     if (s->s2) return launch_s2_group_to_real(s->d_fg, out, s->d_goff2, s->L, s->batch, s->herm, st);
-    group_to_real_tiled<<<rtile_grid(s->L, s->batch), 256, 0, st>>>(s->d_fg, (float*)out, s->d_goff2, s->L, coeffs_per_fn(s),
-                                                                    s->batch, add);
+    const int fpc = rtile_functions(s->L, s->batch);
+    group_to_real_tiled<<<rtile_grid(s->L, s->batch, fpc), 256, 0, st>>>(s->d_fg, (float*)out, s->d_goff2, s->L, coeffs_per_fn(s),
+                                                                    s->batch, fpc, add);
     return cudaGetLastError();
 }
 static cudaError_t real_to_group(TCState* s, const void* in, cudaStream_t st)
 {
     if (s->s2) return launch_s2_real_to_group(in, s->d_fg, s->d_goff2, s->L, s->batch, s->herm, st);
-    real_to_group_tiled<<<rtile_grid(s->L, s->batch), 256, 0, st>>>((const float*)in, s->d_fg, s->d_goff2, s->L,
-                                                                    coeffs_per_fn(s), s->batch, !s->dft_tc);
+    const int fpc = rtile_functions(s->L, s->batch);
+    real_to_group_tiled<<<rtile_grid(s->L, s->batch, fpc), 256, 0, st>>>((const float*)in, s->d_fg, s->d_goff2, s->L,
+                                                                    coeffs_per_fn(s), s->batch, fpc, !s->dft_tc);
     return cudaGetLastError();
 }
 
@@ -2756,9 +2788,9 @@ int tc_fused_phases(TCFused* f, const std::vector<long long>& g0, const std::vec
     }
     // these directions' pencils: the tensor-core DFT's p <= N / 2, or the slice FFT's, all of them; their conversions read and
     // write the coefficients of m >= 0 alone
-    const int mode[3] = {0, f->dft.segs && f->parts[0]->herm, f->parts[0]->herm};
-    static_assert(offsetof(GemmArgs, half) == offsetof(GemmArgs, by_q) + sizeof(int) &&
-                      offsetof(GemmArgs, half_coeffs) == offsetof(GemmArgs, half) + sizeof(int), "copied together");
+    const unsigned char herm = f->parts[0]->herm, mode[3] = {0, (unsigned char)(f->dft.segs && herm), herm};
+    static_assert(offsetof(GemmArgs, half) == offsetof(GemmArgs, by_q) + 1 &&
+                      offsetof(GemmArgs, half_coeffs) == offsetof(GemmArgs, half) + 1, "copied together");
     for (size_t i = 0; i < 2 * n; ++i)
         if ((e = cudaMemcpy(&f->d_segs[i & 1][i / 2].a.by_q, mode, sizeof(mode), cudaMemcpyHostToDevice)) != cudaSuccess) {
             err = std::string("fused phases: ") + cudaGetErrorString(e);
