@@ -21,8 +21,9 @@
 //    fork / per-bucket FFTs / join / fused GEMM / fork / per-bucket coefficient
 //    permutations / join, inverse the mirror image;
 //  * SO(3) tensor-core batches without refinement go further: each direction is
-//    three launches over all buckets (fused.cuh) -- one slice-FFT launch (every
-//    bucket's beta slices, a CTA per slice or per few slices), the fused GEMM,
+//    three launches over all buckets (fused.cuh) -- the DFT passes (large batches:
+//    both on the tensor cores, dft_tc.cu; small ones: the slice FFT, a CTA per
+//    beta slice or per few slices), the fused GEMM,
 //    one coefficient-conversion launch -- on the caller's stream, no fork/join;
 //  * with FFTSO3_FLAG_GRAPH the whole fork / bucket launches / join sequence
 //    is captured once per (direction, input, output) into a CUDA graph and

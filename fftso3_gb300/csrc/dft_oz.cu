@@ -13,7 +13,8 @@
 // Not-a-number and infinite inputs make their line's outputs not-a-number.
 //
 // Bound: the producers' instructions (about 30 a value read: two sweeps' fixed-point splits, folds, carries and digit fields)
-// and the epilogue's 20 a level sum, not the MMAs.  In double-float arithmetic on the CUDA cores the mixed-radix line kernels
+// and the epilogue's 20 a level sum, with 19 warps to hide their latency (0.38 to 0.50 issued a scheduler and cycle), not the
+// MMAs or memory (DRAM 12 to 27 %).  In double-float arithmetic on the CUDA cores the mixed-radix line kernels
 // took 5.9 ms for the forward passes of 16 real functions of N = 160 and 6.1 ms for the inverse ones; these take 1.13 and
 // 0.98 (65.5 M samples).  Powers of two from 64 keep the line FFT along k runs, which is faster still: N = 126 30 G complex
 // samples/s here, N = 128 76 there (two passes).  Folding in 32-bit words instead (four base-256 digits, one sweep) took 0.80 ms,

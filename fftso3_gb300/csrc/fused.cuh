@@ -1,5 +1,6 @@
 // Launches that span every l_max bucket of an uneven SO(3) tensor-core batch (fftso3_batch_*): with the fused
 // beta-sum GEMM (contract_tc.cu) a direction is three launches,
+//   (large batches run both DFT passes on the tensor cores instead, dft_tc.cu)
 //   forward: slice FFT (grid slabs -> pencils), GEMM, group-major -> packed coefficients (+ real basis);
 //   inverse: packed (+ real basis) -> scaled group-major, GEMM, slice FFT (pencils -> grid slabs).
 #pragma once
