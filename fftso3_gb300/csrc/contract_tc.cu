@@ -644,6 +644,9 @@ __global__ void __launch_bounds__(THREADS, 1)
                 break;
             }
             const uint32_t bpl = smem_u32(smem + s * STAGE_BYTES + STAGE_A);
+            // columns without a function or pair keep whatever the stage holds: no other column sees it, and their sums are
+            // not read
+            if (scur.p)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int chunk = q4 + 4 * (h ^ hs);
@@ -750,7 +753,8 @@ __global__ void __launch_bounds__(THREADS, 1)
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(ab * 256);
             for (int chunk = hf * (BN / 64); chunk < (nhalf == 2 ? (hf + 1) * (BN / 64) : BN / 32); ++chunk) {
-                if (ctile(item) * FPTK + chunk * (32 / (2 * PPF)) - hf * (FPTK / 2) >= A.batch) break;  // no functions left
+                // no functions left (the kernels of full tiles lose 1 % by the test)
+                if ((HERM || PAIR) && ctile(item) * FPTK + chunk * (32 / (2 * PPF)) - hf * (FPTK / 2) >= A.batch) break;
                 float v[32];
                 if constexpr (TERMS == 3) tmem_ld32_sum(trow + chunk * 32, trow + 128 + chunk * 32, v);
                 else tmem_ld32_one(trow + chunk * 32, v);
