@@ -669,11 +669,13 @@ int fftso3_plan_create(fftso3_plan** out, int kind, int l_max, int batch, int pr
         if (p->real)
             if ((rc = plan_alloc(p, &p->d_fc, 16 * (size_t)batch * p->coeff_elems))) return bail(rc);
     } else {
+        // the groups (m0, +-n0) may share table rows
+        const bool mirrored = p->so3 && wigner_table_mirrored(recursion == FFTSO3_RECURSION_STABLE, L, N);
         std::string err;
         rc = tc_create(&p->tc, p->L, p->N, batch, p->d_table, goff, p->table_elems, p->d_tw, p->d_w,
                        (flags & (FFTSO3_FLAG_REFINE | FFTSO3_FLAG_EXACT_INVERSE)) != 0, p->real, !p->so3,
                        (flags & FFTSO3_FLAG_AUTOTUNE) != 0,
-                       precision == FFTSO3_PREC_FP32, err);
+                       precision == FFTSO3_PREC_FP32, mirrored, err);
         if (rc) {
             g_err = err;
             return bail(rc);
@@ -712,7 +714,7 @@ int fftso3_plan_create(fftso3_plan** out, int kind, int l_max, int batch, int pr
             p->rchunk = (int)(nch < (size_t)batch ? nch : (size_t)batch);
             const int pen_fns = spectral ? std::min(p->rchunk, 8) : p->rchunk;
             std::string err;
-            if ((rc = oz_create(&p->oz, p->d_table, goff, L, N, p->rchunk, pen_fns, p->d_tw, err))) {
+            if ((rc = oz_create(&p->oz, p->d_table, goff, L, N, p->rchunk, pen_fns, p->d_tw, mirrored, err))) {
                 g_err = err;
                 return bail(rc);
             }

@@ -173,7 +173,8 @@ struct GemmArgs {
     unsigned char by_q, half;
     unsigned char half_coeffs;           // ... and forward: only the coefficients of pairs 0 and 2 (n0 < 0: 3), m >= 0, are written
     // SO(3), at most half a column tile of functions: items of n0 >= 0, the second half of the columns holds the group
-    // (m0, -n0) against the same table rows, d^l_{m0, -n0}(beta) = (-1)^(l + m0) d^l_{m0, n0}(pi - beta)
+    // (m0, -n0) against the same table rows, d^l_{m0, -n0}(beta) = (-1)^(l + m0) d^l_{m0, n0}(pi - beta), where the table has
+    // that to rounding (wigner_table_mirrored)
     unsigned char paired;
 };
 static_assert(sizeof(GemmArgs) <= 128, "small launches took 4 us more with larger arguments (FP32, S^2, l_max 90)");
@@ -1364,7 +1365,7 @@ struct TCState {
     bool refine = false;
     bool real = false;            // real grids (FFTSO3_*_REAL): real samples in, real part out
     bool herm = false;            // real functions on the tensor cores: one GEMM pair of two (see the kernel)
-    bool paired = false;          // at most half a column tile of functions: groups +-n0 share the tiles (GemmArgs::paired)
+    bool paired = false;          // at most half a column tile of functions, mirrored table: groups +-n0 share the tiles (GemmArgs::paired)
     bool s2 = false;              // S^2 (Legendre groups g = m, grids N^2) instead of SO(3)
     bool simt = false;            // FP32 CUDA-core beta-sum (FFTSO3_PREC_FP32) instead of tcgen05
     float* d_tab32 = nullptr;     // FP32 table [row][Kp] (simt)
@@ -1564,7 +1565,7 @@ static int set_launch_lists(TCState* s, int csize, std::string& err)
 
 int tc_create(TCState** out, int L, int N, int batch, const double* d_table_fp64, const std::vector<long long>& goff,
               long long table_elems, const double* d_tw, const double* d_w, bool refine, bool real, bool s2,
-              bool autotune, bool simt, std::string& err)
+              bool autotune, bool simt, bool mirrored, std::string& err)
 {
     *out = nullptr;
     if (N > MAXN) {
@@ -1593,7 +1594,7 @@ int tc_create(TCState** out, int L, int N, int batch, const double* d_table_fp64
     s->herm = real && !simt;
     const int fpt = (s2 ? FPT_S2 : FPT) * (s->herm ? 2 : 1);
     s->ntiles = (batch + fpt - 1) / fpt;
-    s->paired = !s2 && !simt && batch <= fpt / 2;
+    s->paired = !s2 && !simt && mirrored && batch <= fpt / 2;
     make_fft_factors_prime_first(N, s->fac);
     s->d_tw = d_tw;
     s->total_rows = table_elems / N;

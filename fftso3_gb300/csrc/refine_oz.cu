@@ -112,7 +112,8 @@ struct Args {
     int* err;
 };
 
-// d^l_{m0, -n0}(beta) = (-1)^(l + m0) d^l_{m0, n0}(pi - beta): with at most FPT / 2 functions, the second half of a column
+// d^l_{m0, -n0}(beta) = (-1)^(l + m0) d^l_{m0, n0}(pi - beta), where the table has that to rounding
+// (wigner_table_mirrored): with at most FPT / 2 functions, the second half of a column
 // tile takes the group (m0, -n0) against the table rows of (m0, n0), its coefficients' signs alternating with l, its results
 // at N - 1 - k.  Half of the table is read (which bounds small batches) and half of the tiles contracted: l_max 255, 4
 // functions, 8.4 -> 4.6 ms in the refined forward, 6.2 -> 3.8 ms in the exact inverse.
@@ -675,6 +676,7 @@ struct OZState {
     int4* items = nullptr;      // work items of a full chunk (all column tiles)
     int2* iaux = nullptr;
     int nitems = 0;
+    bool mirrored = false;      // the table pairs the groups (m0, +-n0) (wigner_table_mirrored)
     // ... of the groups n0 >= 0 of the first column tile, for paired groups
     int4* items_p = nullptr;
     int2* iaux_p = nullptr;
@@ -728,7 +730,7 @@ void oz_destroy(OZState* o)
 long long oz_device_bytes(const OZState* o) { return o ? o->bytes : 0; }
 
 int oz_create(OZState** out, const double* d_table, const std::vector<long long>& goff, int L, int N, int chunk,
-              int pen_fns, const double* d_tw, std::string& err)
+              int pen_fns, const double* d_tw, bool mirrored, std::string& err)
 {
     *out = nullptr;
     if (!oz_supported(L, N) || chunk < 1 || pen_fns < 1) {
@@ -747,6 +749,7 @@ int oz_create(OZState** out, const double* d_table, const std::vector<long long>
     o->C = so3_off(o->B);
     o->total_rows = goff[o->ngroups] / N;
     o->d_tw = d_tw;
+    o->mirrored = mirrored;
     make_fft_factors(N, o->fac);
     int dev = 0;
     cudaGetDevice(&dev);
@@ -918,7 +921,7 @@ static int oz_contract(OZState* o, const void* F, bool f64, int nb, float2* rhi,
     }
     const int N = o->N, L = o->L;
     const long long NN = (long long)N * N;
-    const bool paired = nb <= FPT / 2;
+    const bool paired = o->mirrored && nb <= FPT / 2;
     T->begin(ST_REFINE, st);
     {
         const dim3 grid((unsigned)o->ngroups, (unsigned)((nb + FPT - 1) / FPT));

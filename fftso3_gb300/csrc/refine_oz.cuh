@@ -16,8 +16,9 @@ bool oz_supported(int L, int N);
 // Builds the table's digit planes and exponents from the plan's FP64 Wigner-d table (goff: group offsets into
 // it), coefficient buffers for `chunk` functions per contraction and a double-float pencil buffer for pen_fns
 // functions (the grid form's synthesis needs pen_fns >= chunk; the spectral form's FFT runs pen_fns at a time).
+// mirrored: wigner_table_mirrored of the table.
 int oz_create(OZState** out, const double* d_table, const std::vector<long long>& goff, int L, int N, int chunk,
-              int pen_fns, const double* d_tw, std::string& err);
+              int pen_fns, const double* d_tw, bool mirrored, std::string& err);
 void oz_destroy(OZState* o);
 long long oz_device_bytes(const OZState* o);
 // Error word of the exact contraction kernel (a bounded wait that gave up); synchronising read.

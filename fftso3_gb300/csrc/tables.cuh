@@ -2,6 +2,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <cmath>
+
 namespace fftso3 {
 
 // Per-angle seeds, computed on the host with the C library exactly as
@@ -19,6 +21,14 @@ struct WignerSeeds {
     double s2;     // sin(beta/2)          (stable mode, sign)
 };
 
+// d^l_{m,-n}(beta) = (-1)^(l + m) d^l_{m,n}(pi - beta) holds for a table to rounding where no seed leaves the normal range.  The
+// stable recursion keeps its seeds' exponents apart.  The reference's start at cos(beta / 2)^(2 l), which the last angle of the
+// grid, pi - pi / (2 N), makes subnormal from l_max = 69: up to 68 its tables are mirrored to 7e-14, at 70 to 2e-8, and from 72
+// on entries of 1.0 stand against zero (what the mode is to reproduce).
+inline bool wigner_table_mirrored(bool stable, int L, int N)
+{
+    return stable || 2.0 * L * log2(sin(M_PI / (4.0 * N))) > -1022.0;
+}
 cudaError_t launch_wigner_table(double* table, const long long* goff, const WignerSeeds* seeds, const double* lfact,
                                 int L, int N, int ngroups, bool stable, cudaStream_t st);
 cudaError_t launch_legendre_table(double* table, const long long* moff, const double* xs, int L, int N,

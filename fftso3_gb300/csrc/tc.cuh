@@ -13,9 +13,10 @@ namespace fftso3 {
 
 struct TCState;
 
+// mirrored: wigner_table_mirrored of the table (SO(3))
 int tc_create(TCState** out, int L, int N, int batch, const double* d_table_fp64, const std::vector<long long>& goff,
               long long table_elems, const double* d_tw, const double* d_w, bool refine, bool real, bool s2,
-              bool autotune, bool simt, std::string& err);
+              bool autotune, bool simt, bool mirrored, std::string& err);
 void tc_destroy(TCState* s);
 long long tc_device_bytes(const TCState* s);
 int tc_forward(TCState* s, const void* grid, void* coeffs, cudaStream_t st, StageTimer* T, std::string& err);
