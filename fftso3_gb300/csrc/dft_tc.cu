@@ -5,9 +5,14 @@
 //   C[q] = sum_t u_t cos(2 pi t q / N), S[q] = sum_t v_t sin(2 pi t q / N), for the even and the odd q <= P,
 //   X[q], X[N - q] = C[q] -/+ i S[q].
 // Each is a product of 128 rows (64 complex lines x re / im, or 128 real lines) with a constant matrix of the plan's N: the
-// lines' folded terms are the A operand (128 x H, K-major), the matrix the B operand, both as three BF16 terms (24
-// significant bits) with the six products of weight >= 2^-16 accumulated in FP32 (the leading one apart from the five
-// small ones), as the beta-sum does it.
+// lines' folded terms are the A operand (128 x H, K-major), the matrix the B operand, both as three BF16 terms with the six
+// products of weight >= 2^-16 accumulated in FP32 (the leading one apart from the five small ones), as the beta-sum does it.
+//
+// The leading terms are in fixed point, 8 bits under the line's largest folded value and 8 under 1 for the matrix, so that
+// their products are whole multiples of one unit, at most 56 2^16 of it, and their sums exact.  The tensor cores cut a sum
+// off where they cannot hold it; with floating-point leading terms that shrank every bin by the same 1e-8 to 2e-8 of itself,
+// which the beta-sum, unlike rounding, does not average (forward of l_max 96, one complex function: off by 1.79e-7 of its 2-norm,
+// now 1.53e-7, of which the beta-sum alone makes most; inverse 1.82e-7 and 1.28e-7; 4 to 8 % more time).  The two other terms hold the remainder to 2^-26 of the line's largest value.
 //
 // Why: as FP32 register tiles (direct_dft.cu) the products and the loads take turns on the same warps: 1.1 to 1.2 ms a pass
 // at N = 194 (16 complex functions).  Here one thread issues them and the warps only move data: 0.43 ms (0.55 ms the
@@ -45,6 +50,7 @@ constexpr int THREADS = 32 * (MMAW + 1);
 constexpr int PLANE = 128 * 128;      // 128 rows x 64 BF16
 constexpr int SLOT = 3 * PLANE;
 constexpr int MAXH = 56;              // folded terms: 7 chunks of 8 (a 64-line tile is 14 items, one a producer warp)
+constexpr int MX = 3 * 128 * 4;       // bytes of the lines' largest values (a ring of three tiles)
 
 // Below, the FP32 kernel: with few terms a tile's fixed latencies outweigh its products (all four passes, complex / real, ms:
 // N = 66, 64 functions 0.52 / 0.40 here, 0.53 / 0.32 there; N = 160, 16 functions 1.00 / 0.70 here, 2.44 / 1.33 there).
@@ -81,7 +87,7 @@ struct Args {
     int* err;
 };
 
-__host__ __device__ constexpr size_t smem_bytes(int KC) { return 2 * SLOT + 12 * 16 * KC * 128 + 128 + 1024; }
+__host__ __device__ constexpr size_t smem_bytes(int KC) { return 2 * SLOT + 12 * 16 * KC * 128 + 128 + MX + 1024; }
 
 // Loads: data of an earlier launch through the read-only path; the work grid of the same launch's first pass at L2.
 template <bool COH, typename T>
@@ -98,19 +104,34 @@ __device__ __forceinline__ uint32_t bf2(float a, float b)
     const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
     return *reinterpret_cast<const uint32_t*>(&v);
 }
-// eight values into one 16-byte chunk of each of the three BF16 planes
-__device__ __forceinline__ void store_split(uint32_t dst, const float* x)
+// The unit of a line's leading terms, 2^(e - 8) for its largest folded value m < 2^e (as bits; not finite: any), and its
+// inverse.
+struct Unit {
+    float u, inv;
+};
+__device__ __forceinline__ Unit unit_of(unsigned m)
 {
+    const int e = min(max((int)(m >> 23) - 126, -118), 128);
+    return {__uint_as_float((unsigned)(127 + e - 8) << 23), __uint_as_float((unsigned)(127 + 8 - e) << 23)};
+}
+
+// eight values into one 16-byte chunk of each of the three BF16 planes
+__device__ __forceinline__ void store_split(uint32_t dst, const float* x, Unit s)
+{
+    constexpr float MAGIC = 12582912.f;  // 1.5 2^23
     uint32_t w[3][4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        float a = x[2 * j], b = x[2 * j + 1];
+        float v[2];
+        float q[2];
 #pragma unroll
-        for (int p = 0; p < 3; ++p) {
-            w[p][j] = bf2(a, b);
-            a -= __uint_as_float(w[p][j] << 16);
-            b -= __uint_as_float(w[p][j] & 0xffff0000u);
+        for (int h = 0; h < 2; ++h) {
+            q[h] = __fsub_rn(__fmaf_rn(x[2 * j + h], s.inv, MAGIC), MAGIC);
+            v[h] = __fmaf_rn(-q[h], s.u, x[2 * j + h]);  // exact
         }
+        w[0][j] = bf2(q[0] * s.u, q[1] * s.u);  // |q| <= 256
+        w[1][j] = bf2(v[0], v[1]);
+        w[2][j] = bf2(v[0] - __uint_as_float(w[1][j] << 16), v[1] - __uint_as_float(w[1][j] & 0xffff0000u));
     }
 #pragma unroll
     for (int p = 0; p < 3; ++p)
@@ -118,6 +139,7 @@ __device__ __forceinline__ void store_split(uint32_t dst, const float* x)
                      "r"(w[p][2]), "r"(w[p][3])
                      : "memory");
 }
+__device__ __forceinline__ void producers_sync() { asm volatile("bar.sync 1, %0;" ::"n"(32 * NPROD) : "memory"); }
 
 // A line of a tile: its place in the input and the output (elements of the side's type), and whether it exists.
 struct Line {
@@ -292,6 +314,7 @@ struct Ctx {
     unsigned char* bmat;
     uint64_t *full, *empty, *accf, *acce, *bfull;
     volatile int* abort_flag;
+    unsigned* mx;  // [tile mod 3][line]: bits of the largest folded value
     uint32_t tmem;
     int warp, lane;
 };
@@ -299,6 +322,7 @@ struct Ctx {
 struct Counts {
     unsigned s = 0;   // problems produced / issued, or accumulator buffers finished
     unsigned nb = 0;  // matrices loaded
+    int tp = 0;       // producers: tiles mod 3
 };
 
 // The segment a role's next tile is in (tiles ascend).
@@ -319,7 +343,7 @@ __device__ __forceinline__ void produce(const Args& a, int pass, const Ctx& c, C
     constexpr int IPW = KIND == COMPLEX ? 1 : 2;   // items of a warp
     constexpr int LB = KIND == COMPLEX ? 2 : 4;    // blocks of 32 lines in a tile
     const int lane = c.lane;
-    int lx[IPW], ly[IPW], ch[IPW], row[IPW];
+    int lx[IPW], ly[IPW], ch[IPW], row[IPW], ln[IPW];
 #pragma unroll
     for (int w = 0; w < IPW; ++w) {
         const int it = c.warp + w * NPROD, lb = it % LB;
@@ -338,10 +362,13 @@ __device__ __forceinline__ void produce(const Args& a, int pass, const Ctx& c, C
             ly[w] = (lane >> 3) + 4 * lb;
             row[w] = lx[w] * 16 + (ly[w] ^ lx[w]);
         }
+        ln[w] = lane + 32 * lb;
     }
     int seg = 0;
     const unsigned ntiles = a.ntiles[pass];
-    for (unsigned tile = blockIdx.x; tile < ntiles && !*c.abort_flag; tile += gridDim.x) {
+    // a failed wait (every producer meets it in its turn) ends the stores; the tiles' barriers go on, so that no warp waits
+    // for one that left
+    for (unsigned tile = blockIdx.x; tile < ntiles; tile += gridDim.x, n.tp = n.tp == 2 ? 0 : n.tp + 1) {
         const Geo& g = seek<BATCH>(a, pass, tile, seg);
         const int H = g.H, N = g.N, P = N / 2;
         const void* src = BATCH && g.ext == 1 ? a.ext + (size_t)g.in : g.in;
@@ -360,6 +387,12 @@ __device__ __forceinline__ void produce(const Args& a, int pass, const Ctx& c, C
             } else {
                 load_fold<KIND, true, COH>(g, src, L.in, t0, H, N, x);
             }
+            unsigned m = 0;
+#pragma unroll
+            for (int k = 0; k < VPL; ++k)
+#pragma unroll
+                for (int pr = 0; pr < 4; ++pr) m = max(m, __float_as_uint(x[pr][k]) & 0x7fffffffu);
+            atomicMax(&c.mx[n.tp * 128 + ln[w]], m);
         }
         // the next tile's elements into L2 while this one's problems are stored and multiplied: lane k of a run of
         // eight lines requests the run's element t0 + k (and its three images)
@@ -381,28 +414,30 @@ __device__ __forceinline__ void produce(const Args& a, int pass, const Ctx& c, C
                 }
             }
         }
-        bool ok = true;
+        // the next tile's maxima: last read before the last tile's barrier
+        if (threadIdx.x < 128) c.mx[(n.tp == 2 ? 0 : n.tp + 1) * 128 + threadIdx.x] = 0;
+        producers_sync();
+        Unit un[IPW];
+#pragma unroll
+        for (int w = 0; w < IPW; ++w) un[w] = unit_of(c.mx[n.tp * 128 + ln[w]]);
 #pragma unroll
         for (int pr = 0; pr < 4; ++pr, ++n.s) {
             const int sl = n.s & 1;
-            if (n.s >= 2 && !mbar_wait(&c.empty[sl], ((n.s >> 1) - 1) & 1, a.err, 31)) {
-                ok = false;
-                break;
+            const bool stop = *c.abort_flag || (n.s >= 2 && !mbar_wait(&c.empty[sl], ((n.s >> 1) - 1) & 1, a.err, 31));
+            if (__any_sync(0xffffffffu, stop)) {
+                *c.abort_flag = 1;
+                continue;
             }
 #pragma unroll
             for (int w = 0; w < IPW; ++w) {
                 if (8 * ch[w] >= H) continue;
                 const uint32_t d = smem_u32(c.smem + sl * SLOT) + row[w] * 128 + ((ch[w] ^ (row[w] & 7)) << 4);
-                store_split(d, v[w][pr]);
-                if (KIND == COMPLEX) store_split(d + 8 * 128, v[w][pr] + 8);
+                store_split(d, v[w][pr], un[w]);
+                if (KIND == COMPLEX) store_split(d + 8 * 128, v[w][pr] + 8, un[w]);
             }
             fence_proxy_async();
             __syncwarp();
             if (lane == 0) mbar_arrive(&c.full[sl]);
-        }
-        if (!ok) {
-            *c.abort_flag = 1;
-            break;
         }
     }
 }
@@ -579,6 +614,7 @@ __global__ void __launch_bounds__(THREADS, 1) dft_tc_kernel(const __grid_constan
     c.bfull = c.acce + 2;
     uint32_t* tmem_slot = (uint32_t*)(c.bfull + 1);
     c.abort_flag = (volatile int*)(tmem_slot + 1);
+    c.mx = (unsigned*)((unsigned char*)c.full + 128);
     c.warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);
     c.lane = threadIdx.x & 31;
 
@@ -598,6 +634,7 @@ __global__ void __launch_bounds__(THREADS, 1) dft_tc_kernel(const __grid_constan
                      "r"(512));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
+    for (int i = threadIdx.x; i < MX / 4; i += THREADS) c.mx[i] = 0;
     // the slots' columns past the folded terms stay zero (segments ascend in N, so a pass never leaves longer rows behind)
     clear_slots(c.smem);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -627,7 +664,7 @@ __global__ void __launch_bounds__(THREADS, 1) dft_tc_kernel(const __grid_constan
 }
 
 // [problem: cos even, sin even, cos odd, sin odd][plane][q][t] BF16, rows of 128 bytes, their 16-byte chunks swizzled; one
-// thread a chunk (eight t of the three planes).  The terms are split from the FP64 values.
+// thread a chunk (eight t of the three planes).  The terms are split from the FP64 values, the first to multiples of 2^-8.
 __global__ void build_table_kernel(unsigned char* table, int N, int H, int NQ, const double2* __restrict__ tw)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -648,7 +685,7 @@ __global__ void build_table_kernel(unsigned char* table, int N, int H, int NQ, c
         }
 #pragma unroll
         for (int p = 0; p < 3; ++p) {
-            w[p][j] = bf2((float)v[0], (float)v[1]);
+            w[p][j] = p ? bf2((float)v[0], (float)v[1]) : bf2((float)(rint(v[0] * 256.) / 256.), (float)(rint(v[1] * 256.) / 256.));
             v[0] -= (double)__uint_as_float(w[p][j] << 16);
             v[1] -= (double)__uint_as_float(w[p][j] & 0xffff0000u);
         }
