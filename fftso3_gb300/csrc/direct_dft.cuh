@@ -8,7 +8,8 @@
 // N^2 / 2 FMAs a complex line (P / 2 a real one) whatever N's factors are, all of them independent register-tile work
 // with every operand in shared memory.  A mixed-radix Stockham FFT has fewer operations, but its stages each cross
 // shared memory and a barrier, and a prime factor R costs it R FMAs an element anyway.  Measured on one GB300 (all four
-// passes, 64 complex functions, N = 194): 38.9 ms with the separate transposes as a mixed-radix FFT, 18.5 ms here.
+// passes, 64 complex functions, N = 194): 38.9 ms with the separate transposes as a mixed-radix FFT, 18.5 ms here (with one
+// accumulator a sum, see CHUNK).
 //
 // A unit is a complex line, or two real lines x, y.  Its folded terms are held as the pairs (a.x, b.y), (a.y, b.x) (real
 // lines: (a.x, b.x), (a.y, b.y)) and the matrices as the pairs (cos, sin), so that one packed FMA advances a cosine sum
@@ -25,6 +26,12 @@ __device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c)
 {
     u64 r;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ u64 add2(u64 a, u64 b)
+{
+    u64 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
 __device__ __forceinline__ float2 unpack2(u64 a)
@@ -96,38 +103,64 @@ __device__ __forceinline__ Folded fold_line(int t, int P, float2 x, float2 xn, f
 // A thread's register tile: four outputs q of one parity of four units.  Lanes: QL blocks of outputs fastest, then 32 / QL
 // units.  Adjacent lanes then read the same units: a 16-byte shared-memory read costs max(2, distinct bytes / 128) cycles
 // (measured: 2 for a warp-uniform one, 4 for 32 lanes side by side or for eight lanes' addresses repeated in each quarter
-// warp), so a step t costs 12 cycles of the shared-memory pipe for 32 packed FMAs, 48 against the 64 that four warps' FMAs
-// take.
+// warp), so reads are shared by as many lanes as possible.
 struct Tile {
     u64 A[4][4], B[4][4];  // [output][unit]: the accumulators of the unit's two pairs
 };
+// A sum goes in chunks of at most CHUNK terms that are added up apart, each an even sample of the line (every C-th term, C
+// chunks), from its last term to its first: one accumulator over all terms rounds at the size of its partial sums, which
+// spectra (largest at t = 0) reach with their first term and smooth samples grow through and beyond
+// (inverse of l_max 135 and 143, one function: off by 2.70e-7 and 2.79e-7 of the 2-norm, now 1.86e-7 and 1.94e-7; S^2 l_max 99
+// 2.17e-7 and 1.63e-7).
+// The chunks' totals take the registers of two units' accumulators, so a tile's units go two by two: 16 cycles of the
+// shared-memory pipe a step instead of 12 (64 against the 64 of the FMAs).
+constexpr int CHUNK = 12;
 // m: the block's pairs at t = 0 (next t 2 QS further on); v: the thread's first unit of the parity at t = 0 (next t TS
-// further on), the others 32 / QL, HU, HU + 32 / QL further on.
+// further on), the others HU, 32 / QL, HU + 32 / QL further on.
 template <int QL>
 __device__ __forceinline__ void product(const float2* m, const float4* v, int H, int QS, int HU, int TS, Tile& a)
 {
     constexpr int G = 32 / QL;
+    const int C = (H + CHUNK - 1) / CHUNK, sm = 2 * QS * C, sv = TS * C;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int h = 0; h < 2; ++h) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) a.A[i][j] = a.B[i][j] = 0;
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) a.A[i][2 * h + j] = a.B[i][2 * h + j] = 0;
+        for (int c0 = C - 1; c0 >= 0; --c0) {
+            u64 A[4][2], B[4][2];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) A[i][j] = B[i][j] = 0;
+            const int t0 = H - 1 - (H - 1 - c0) % C;  // the chunk's last term
+            const float2* mt = m + t0 * 2 * QS;
+            const float4* vt = v + t0 * TS + h * G;
 #pragma unroll 2
-    for (int t = 0; t < H; ++t) {
-        const ulonglong2 m0 = *reinterpret_cast<const ulonglong2*>(m);
-        const ulonglong2 m1 = *reinterpret_cast<const ulonglong2*>(m + 2);
-        const u64 c[4] = {m0.x, m0.y, m1.x, m1.y};
-        const ulonglong2 x[4] = {
-            *reinterpret_cast<const ulonglong2*>(v), *reinterpret_cast<const ulonglong2*>(v + HU),
-            *reinterpret_cast<const ulonglong2*>(v + G), *reinterpret_cast<const ulonglong2*>(v + HU + G)};
-        m += 2 * QS;
-        v += TS;
+            for (int t = t0; t >= 0; t -= C) {
+                const ulonglong2 m0 = *reinterpret_cast<const ulonglong2*>(mt);
+                const ulonglong2 m1 = *reinterpret_cast<const ulonglong2*>(mt + 2);
+                const u64 c[4] = {m0.x, m0.y, m1.x, m1.y};
+                const ulonglong2 x[2] = {*reinterpret_cast<const ulonglong2*>(vt), *reinterpret_cast<const ulonglong2*>(vt + HU)};
+                mt -= sm;
+                vt -= sv;
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
+                for (int j = 0; j < 2; ++j)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                a.A[i][j] = fma2(c[i], x[j].x, a.A[i][j]);
-                a.B[i][j] = fma2(c[i], x[j].y, a.B[i][j]);
+                    for (int i = 0; i < 4; ++i) {
+                        A[i][j] = fma2(c[i], x[j].x, A[i][j]);
+                        B[i][j] = fma2(c[i], x[j].y, B[i][j]);
+                    }
             }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    a.A[i][2 * h + j] = add2(a.A[i][2 * h + j], A[i][j]);
+                    a.B[i][2 * h + j] = add2(a.B[i][2 * h + j], B[i][j]);
+                }
+        }
     }
 }
 

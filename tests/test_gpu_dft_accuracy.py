@@ -31,6 +31,9 @@ def samples(N, b, real, seed):
 # (l_max, batch, real, forward, inverse)
 TENSOR_CORES = [(96, 1, False, 4.836e-8, 2.387e-7), (96, 1, True, 4.699e-8, 2.691e-7), (59, 1, False, 1.579e-7, 1.495e-7)]
 
+PACKED_FP32 = [(38, 2, False, 9.860e-8, 1.432e-7), (38, 2, True, 1.053e-7, 1.747e-7), (119, 1, False, 2.052e-7, 2.033e-7),
+               (119, 1, True, 2.128e-7, 2.532e-7), (159, 1, False, 2.600e-7, 2.222e-7), (159, 1, True, 3.710e-7, 2.747e-7)]
+
 
 def errors(gblib, L, real, smp, F):
     import torch
@@ -51,7 +54,7 @@ def errors(gblib, L, real, smp, F):
     return [float(torch.linalg.vector_norm(y.to(x.dtype) - x) / torch.linalg.vector_norm(x)) for x, y in zip(*out)]
 
 
-@pytest.mark.parametrize("L,b,real,fwd,inv", TENSOR_CORES)
+@pytest.mark.parametrize("L,b,real,fwd,inv", TENSOR_CORES + PACKED_FP32)
 def test_errors(gblib, L, b, real, fwd, inv):
     F = np.concatenate([so3_coeffs(L, seed=L + i, complex_=not real, decay="pow") for i in range(b)])
     e = errors(gblib, L, real, samples(2 * L + 2, b, real, L), F)
