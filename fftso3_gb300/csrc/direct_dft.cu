@@ -11,6 +11,7 @@
 // functions, a pass takes 1.1 to 1.2 ms, 0.3 of it the bytes, 0.5 the products (0.35 at the FMA rate), the rest loading and
 // folding.  SO(3) passes of N = 80 to 222 run on the tensor cores instead (dft_tc.cu).
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 #include "direct_dft.cuh"
@@ -307,21 +308,34 @@ __global__ void __launch_bounds__(MAXT, 1) direct_dft_kernel(const __grid_consta
                 }
             }
             __syncthreads();
-            if (KIND == DIRECT_REAL_OUT) {
-                const float* r = reinterpret_cast<const float*>(V);
-                for (int i = warp; i < 2 * LT; i += nw) {
-                    if (ib[i >> 1] < 0) continue;
-                    float* o = reinterpret_cast<float*>(p.out) + ob[i >> 1] + (i & 1) * p.o_l;
+            using E = std::conditional_t<KIND == DIRECT_REAL_OUT, float, float2>;
+            const E* r = reinterpret_cast<const E*>(V);
+            const int rows = KIND == DIRECT_REAL_OUT ? 2 * LT : LT;
+            auto row = [&](int i) {  // its place, or null: past the last unit
+                const int u = KIND == DIRECT_REAL_OUT ? i >> 1 : i;
+                return ib[u] < 0 ? nullptr : reinterpret_cast<E*>(p.out) + ob[u] + (KIND == DIRECT_REAL_OUT ? (i & 1) * p.o_l : 0);
+            };
+            if (N < 64) {
+                // threads over all rows (a warp a row left most lanes idle: inverse of l_max 6, 200 real functions, 62 us, now
+                // 44; from N = 78 on the rows are up to 8 % faster)
+                const int ri = blockDim.x / N, ji = blockDim.x - ri * N;
+                int i = tid / N, j = tid - i * N;
 #pragma unroll 4
-                    for (int j = lane; j < N; j += 32) o[j] = r[i * (N + 1) + j];
+                while (i < rows) {
+                    if (E* o = row(i)) o[j] = r[i * (N + 1) + j];
+                    j += ji;
+                    i += ri;
+                    if (j >= N) {
+                        j -= N;
+                        ++i;
+                    }
                 }
             } else {
-                const float2* r = reinterpret_cast<const float2*>(V);
-                for (int u = warp; u < LT; u += nw) {
-                    if (ib[u] < 0) continue;
-                    float2* o = reinterpret_cast<float2*>(p.out) + ob[u];
+                for (int i = warp; i < rows; i += nw) {
+                    E* o = row(i);
+                    if (!o) continue;
 #pragma unroll 4
-                    for (int j = lane; j < N; j += 32) o[j] = r[u * (N + 1) + j];
+                    for (int j = lane; j < N; j += 32) o[j] = r[i * (N + 1) + j];
                 }
             }
             __syncthreads();
