@@ -347,7 +347,7 @@ int refine_forward_spectral(fftso3_plan* p, const void* grid, void* coeffs, cuda
     float2* lo = (float2*)tc_resid_buffer(p->tc);
     const int per = p->real ? 1 : 2;  // floats per sample
     const int fftn = oz_fft_functions(p->oz);
-    const int piece = host ? (fftn < 4 ? fftn : 4) : fftn;
+    const int piece = host ? std::min(fftn, oz_piece(p->N, 4)) : fftn;
     if (host) {
         if (!p->copy_stream) {
             CK(cudaStreamCreateWithFlags(&p->copy_stream, cudaStreamNonBlocking));
@@ -452,11 +452,11 @@ int exact_inverse(fftso3_plan* p, const void* coeffs, void* grid, cudaStream_t s
     const int per = p->real ? 1 : 2;  // floats per element
     if (p->oz) {
         void* pen = tc_exact_buffer(p->tc);
-        const int fftn = pen ? p->rchunk : oz_fft_functions(p->oz);
+        const int fftn = pen ? p->rchunk : std::min(p->rchunk, oz_fft_functions(p->oz));
         void* ring = nullptr;
         if (host && oz_spectral(p->oz)) {
             const size_t fn_bytes = (size_t)G * per * sizeof(float);
-            int rc = p->d_io_ring ? FFTSO3_SUCCESS : plan_alloc(p, &p->d_io_ring, 2 * (size_t)OZ_SYNTH_PIECE * fn_bytes);
+            int rc = p->d_io_ring ? FFTSO3_SUCCESS : plan_alloc(p, &p->d_io_ring, 2 * (size_t)oz_piece(p->N, OZ_SYNTH_PIECE) * fn_bytes);
             if (rc) return rc;
             ring = p->d_io_ring;
         }
@@ -690,7 +690,7 @@ int fftso3_plan_create(fftso3_plan** out, int kind, int l_max, int batch, int pr
             // digit planes are read once per 16 functions) when the device has room for them with 16 GB to
             // spare after the FP64 table is freed, else 8 (one column tile), else fewer
             // The spectral form (N <= 222, 256 or 512) needs the double-float pencils only as its FFT's work space
-            // (pen_fns = up to 8 functions at a time), so its contraction chunks grow to 32 functions (four column
+            // (pen_fns = up to 8 functions at a time, of small grids more), so its contraction chunks grow to 32 functions (four column
             // tiles sharing each table tile; the digit planes read once per 32 functions).
             const bool spectral = oz_spectral_supported(N);
             const size_t pen_fn = 16 * (size_t)p->grid_elems;
@@ -712,7 +712,7 @@ int fftso3_plan_create(fftso3_plan** out, int kind, int l_max, int batch, int pr
                 if (c >= 1 && (size_t)c < nch) nch = (size_t)c;
             }
             p->rchunk = (int)(nch < (size_t)batch ? nch : (size_t)batch);
-            const int pen_fns = spectral ? std::min(p->rchunk, 8) : p->rchunk;
+            const int pen_fns = !spectral ? p->rchunk : p->rchunk < 8 ? p->rchunk : std::min(batch, oz_piece(N, 8));
             std::string err;
             if ((rc = oz_create(&p->oz, p->d_table, goff, L, N, p->rchunk, pen_fns, p->d_tw, mirrored, err))) {
                 g_err = err;
@@ -895,7 +895,7 @@ int fftso3_forward_host(fftso3_plan* plan, const void* grid_host, void* coeffs_h
 }
 
 // The exact inverse into host memory (SO(3), N <= 222, 256 or 512), pipelined in chunks of up to 8 functions (one column
-// tile of the exact contraction): each chunk's coefficients are copied in, contracted and transformed, and its
+// tile of the exact contraction; of small grids more, oz_piece): each chunk's coefficients are copied in, contracted and transformed, and its
 // grids stream out through the device ring on the copy stream, so the copies out (the host link bounds the call)
 // start after the first chunk instead of after the whole batch.
 static int exact_inverse_host(fftso3_plan* p, const void* coeffs_host, void* grid_host, cudaStream_t st)
@@ -904,10 +904,10 @@ static int exact_inverse_host(fftso3_plan* p, const void* coeffs_host, void* gri
     const long long C = p->coeff_elems, G = p->grid_elems;
     const int per = p->real ? 1 : 2;  // floats per element
     const size_t fn_bytes = (size_t)G * per * sizeof(float), cf_bytes = (size_t)C * per * sizeof(float);
-    int rc = p->d_io_ring ? FFTSO3_SUCCESS : plan_alloc(p, &p->d_io_ring, 2 * (size_t)OZ_SYNTH_PIECE * fn_bytes);
+    int rc = p->d_io_ring ? FFTSO3_SUCCESS : plan_alloc(p, &p->d_io_ring, 2 * (size_t)oz_piece(p->N, OZ_SYNTH_PIECE) * fn_bytes);
     if (rc) return rc;
     void* pen = tc_exact_buffer(p->tc);
-    const int cf = std::min(p->rchunk, 8);
+    const int cf = std::min(p->rchunk, oz_piece(p->N, 8));
     for (int f0 = 0; f0 < p->batch; f0 += cf) {
         const int nb = p->batch - f0 < cf ? p->batch - f0 : cf;
         float* cd = (float*)p->d_io_coeff + (long long)f0 * C * per;

@@ -1129,7 +1129,7 @@ int oz_inverse_exact(OZState* o, const void* F, bool f64, int nb, void* grid, bo
     const size_t gbytes = (size_t)G * (real ? sizeof(float) : sizeof(float2));  // one function's grid
     T->begin(ST_INV_FFT, st);
     if (oz_spectral(o) && host) {
-        // into host memory: both passes of each piece of OZ_SYNTH_PIECE functions on st into a slot of the
+        // into host memory: both passes of each piece of functions (oz_piece) on st into a slot of the
         // two-slot device ring, then the slot's copy to the host on the copy stream, so the copies (the host link
         // bounds them) run under the FFT of the next pieces; a slot is rewritten once its copy is done
         if (!o->side) {
@@ -1140,11 +1140,12 @@ int oz_inverse_exact(OZState* o, const void* F, bool f64, int nb, void* grid, bo
             }
             OZK(cudaEventCreateWithFlags(&o->ev_join, cudaEventDisableTiming));
         }
-        for (int f0 = 0; f0 < nb; f0 += OZ_SYNTH_PIECE) {
+        const int piece = oz_piece(N, OZ_SYNTH_PIECE);
+        for (int f0 = 0; f0 < nb; f0 += piece) {
             // the ring's slots alternate across calls; a slot's last copy (if any) must be done before it is rewritten
-            const int np = nb - f0 < OZ_SYNTH_PIECE ? nb - f0 : OZ_SYNTH_PIECE, sl = (int)(o->ring_seq++ & 1);
+            const int np = nb - f0 < piece ? nb - f0 : piece, sl = (int)(o->ring_seq++ & 1);
             float4* pb = pen + (long long)f0 * G;
-            char* rb = (char*)ring + (size_t)sl * OZ_SYNTH_PIECE * gbytes;
+            char* rb = (char*)ring + (size_t)sl * piece * gbytes;
             if ((rc = synth_step(o, 1, pb, np, rb, real, st, err))) return rc;
             OZK(cudaStreamWaitEvent(st, o->ev_free[sl], 0));
             if ((rc = synth_step(o, 2, pb, np, rb, real, st, err))) return rc;

@@ -27,14 +27,22 @@ int oz_status(OZState* o);
 // f the FP32 samples (complex64, or float32 when real), r written like f.
 int oz_inverse_resid(OZState* o, const void* F, bool f64, int nb, const void* fgrid, bool real, float* resid,
                      cudaStream_t st, StageTimer* T, std::string& err);
+// Functions of a piece: `least`, or of grids below N = 64 `least` times as many as make 2^18 samples (a launch or copy of 8
+// small grids is all latency: refined forward of l_max 3, 3906 functions, 14.5 ms with pieces of 8, 2.4 with pieces of 4096;
+// host-buffer forward and inverse 28 and 29 ms with 4 and 8 functions, 2.5 and 6.4).
+constexpr int OZ_SYNTH_PIECE = 4;
+inline int oz_piece(int N, int least)
+{
+    const int m = (1 << 18) / (N * N * N);
+    return m > 1 ? m * least : least;
+}
 // The exact inverse (FFTSO3_FLAG_EXACT_INVERSE): for nb coefficient sets F (as oz_inverse_resid), the synthesis
 // with exact digit sums and a double-float FFT, rounded once into grid (complex64, or the real part as float32
 // when real).  The double-float synthesis pencils go to pen (nb <= chunk functions of 16-byte elements), or,
 // when pen is null, to the state's own buffer (nb <= oz_fft_functions()).
 // host (non-null): the grids go to host memory instead; grid is then the device staging for all nb grids
-// (the grid form) and ring a device buffer of 2 OZ_SYNTH_PIECE grids (the spectral form), whose copies to the host
+// (the grid form) and ring a device buffer of 2 oz_piece(N, OZ_SYNTH_PIECE) grids (the spectral form), whose copies to the host
 // run under the FFT of the next pieces.
-constexpr int OZ_SYNTH_PIECE = 4;
 // join = false (host path): st does not wait for the last copies to the host (a later call's join, or the
 // caller's synchronisation of the copy stream through oz_host_join, covers them).  group_major: F (complex64) is
 // in the tensor-core path's group-major order, unscaled (tc_group_from_packed), read as runs.
