@@ -109,18 +109,20 @@ __global__ void __launch_bounds__(T64) dft64_kernel(const D64 a)
 
 }  // namespace
 
-// The direct form where it takes fewer FP64 operations than the mixed radices, or N is short enough for latency to count
-// (N <= 64: 0.5 N^2 against about 12 log2 N an element is equal there).  By N alone: batches keep a single plan's bits.
+// The direct form below N = 64 and where it takes less than 0.72 of the mixed radices' FP64 operations.  Both directions of
+// complex functions, direct over mixed radices (ratio of the operations): N = 56 (0.77) 0.82, 60 (0.79) 0.92, 62 (0.12) 0.26; 64
+// (1.33) 1.12; 70 (0.71) 0.86, 154 (0.64) 0.97, 238 (0.71) 0.79, 286 (0.719) 0.93; 266 (0.725) 1.04, 176 (0.82) 1.14, 198
+// (0.85) 1.15, 98 (0.88) 1.20, 84 (0.93) 1.15, 90 (0.99) 1.22, 260 (0.99) 1.25.  By N alone: batches keep a single plan's bits.
 bool dft64_supported(int N)
 {
     if (N < 2 || N % 2) return false;
-    if (N <= 64) return true;
+    if (N < 64) return true;
     if (N > 512) return false;
     FFTFactors f;
     make_fft_factors(N, f);
     double cost = 0;
     for (int i = 0; i < f.n; ++i) cost += f.r[i] > 8 ? 8.0 * f.r[i] : f.r[i] == 8 ? 12 : f.r[i] == 4 ? 10 : f.r[i] == 2 ? 7 : 3.5 * f.r[i];
-    return 0.5 * N < cost;
+    return 0.5 * N < 0.72 * cost;
 }
 
 cudaError_t launch_dft64(const FFTLaunch& L, cudaStream_t st)
