@@ -179,6 +179,9 @@ struct GemmArgs {
 };
 static_assert(sizeof(GemmArgs) <= 128, "small launches took 4 us more with larger arguments (FP32, S^2, l_max 90)");
 
+// An item of a group (m0, n0), n0 >= 0, which takes the group (m0, -n0) along in paired launches.
+inline bool leads_pair(const int4& item) { return (item.w & 0xFFFF) >= 32768; }
+
 // One plan's share of a fused launch over several plans (the l_max buckets of
 // an uneven batch): its table maps and arguments.  Work items of a fused launch
 // carry (segment << 16 | column tile) in .z.
@@ -1394,7 +1397,7 @@ struct TCState {
     int4* d_items_fwd = nullptr;
     int4* d_items_inv = nullptr;
     int n_items_fwd = 0, n_items_inv = 0;
-    std::vector<int4> items_h[2];  // host copies (forward, inverse), for fused launches
+    std::vector<int4> items_h[2];  // host copies (forward, inverse) of all groups' items, for fused launches
     std::vector<int2> iaux_h[2];   // per item (goff2[g], grow0[g]), same order
     std::vector<long long> h_goff2, h_grow0;  // host copies (the launch lists are rebuilt by the cluster tuner)
     int2* d_iaux_fwd = nullptr;
@@ -1503,8 +1506,9 @@ static int set_launch_lists(TCState* s, int csize, std::string& err)
     const int N = s->N;
     std::vector<int4> itf, iti;
     if (csize <= 1) {
-        itf = s->items_h[0];
-        iti = s->items_h[1];
+        for (int d = 0; d < 2; ++d)
+            for (const int4& it : s->items_h[d])
+                if (!s->paired || leads_pair(it)) (d ? iti : itf).push_back(it);
         csize = 1;
     } else {
         const int CLs = csize, ntb = (s->ntiles + CLs - 1) / CLs;
@@ -1687,7 +1691,6 @@ int tc_create(TCState** out, int L, int N, int batch, const double* d_table_fp64
         const int nl = s->B - m0;
         goff2[g] = acc2;
         acc2 += (long long)(s2 ? (m0 > 0 ? 2 : 1) : group_pairs(m0, n0).np) * nl;
-        if (s->paired && n0 < 0) continue;
         for (int nt = 0; nt < s->ntiles; ++nt) {
             for (int mt = 0; mt * BM < nl; ++mt) itf.push_back(make_int4(g, mt, nt, item_w(m0, n0)));
             for (int mt = 0; mt * BM < N; ++mt) iti.push_back(make_int4(g, mt, nt, item_w(m0, n0)));
@@ -1744,8 +1747,8 @@ int tc_create(TCState** out, int L, int N, int batch, const double* d_table_fp64
         }
     }
     cudaError_t e = cudaSuccess;
-    for (int i = 0; i < 8 && !simt && e == cudaSuccess; ++i)
-        e = cudaFuncSetAttribute((const void*)gemm_kernel(s->herm, i & 1, s2, i & 2, i & 4 ? 1 : 3, s->paired),
+    for (int i = 0; i < 4 && !simt && e == cudaSuccess; ++i)  // (the fused kernels': tc_fused_create)
+        e = cudaFuncSetAttribute((const void*)gemm_kernel(s->herm, i & 1, s2, false, i & 2 ? 1 : 3, s->paired),
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     if (e != cudaSuccess) {
         err = std::string("tensor-core kernel attributes: ") + cudaGetErrorString(e);
@@ -2519,6 +2522,7 @@ struct TCFused {
     int* d_err = nullptr;
     int nsm = 0;
     bool s2 = false;
+    bool paired[2] = {false, false};  // the PAIR kernel, and paired items of the plans that can (pairing_pays)
     // three-launch directions (SO(3) batches, tc_fused_phases): the bucket table of the slice FFT and the
     // coefficient conversions
     BucketSeg* d_bseg = nullptr;
@@ -2552,6 +2556,21 @@ void tc_fused_destroy(TCFused* f)
     delete f;
 }
 
+// Whether a fused launch pairs the groups (m0, +-n0) of its plans of at most half a column tile: all of its items then go
+// through the PAIR kernel, which is slower on the others.  Times with pairing over those without, by the ratio of the other
+// plans' work (items times K steps) to those plans':
+//   complex forward 0.10 0.87, 0.23 0.96, 0.44 1.02, 0.65 1.01, 0.98 1.10, 74 1.21; inverse 0.65 0.87, 0.98 0.92, 4.4 1.00, 7.1 1.02, 37 1.04
+//   real forward 0 0.80, 0.3 0.88, 1.38 1.08, 2.2 0.93, 37 0.95; inverse 0 0.94, 0.3 0.93, 1.33 1.02, 2.2 1.02, 3.6 1.04
+// (1.38, 1.33: 1024 functions of l_max 8 to 64; 74, 37: 64 functions of l_max 63 and one of 20).
+static bool pairing_pays(const std::vector<TCState*>& parts, bool fwd)
+{
+    double can = 0, cannot = 0;
+    for (const TCState* p : parts)
+        for (const int4& it : p->items_h[fwd ? 0 : 1])
+            (p->paired ? can : cannot) += fwd ? p->Kp / BK : (p->B - (it.w >> 16) + BK - 1) / BK;
+    return cannot < (parts[0]->herm ? 1.0 : fwd ? 0.35 : 3.0) * can;
+}
+
 // One work list over the tensor-core plans `parts` (same kind, at most 32768
 // plans): items of plan i carry segment i; sorted by decreasing k-steps so the
 // longest items start first on the persistent CTAs.
@@ -2579,6 +2598,7 @@ int tc_fused_create(TCFused** out, const std::vector<TCState*>& parts, std::stri
     cudaError_t e;
     for (int d = 0; d < 2; ++d) {
         const bool fwd = d == 0;
+        f->paired[d] = pairing_pays(parts, fwd);
         std::vector<GemmSeg> segs(parts.size());
         struct FItem {
             int nk;
@@ -2589,6 +2609,7 @@ int tc_fused_create(TCFused** out, const std::vector<TCState*>& parts, std::stri
         for (size_t i = 0; i < parts.size(); ++i) {
             TCState* p = parts[i];
             GemmArgs a = gemm_args(p);
+            a.paired = p->paired && f->paired[d];
             if (fwd) {
                 a.pin = p->d_pencil;
                 a.cout = p->d_fg;
@@ -2600,6 +2621,7 @@ int tc_fused_create(TCFused** out, const std::vector<TCState*>& parts, std::stri
             for (int q = 0; q < 3; ++q) segs[i].tm[q] = fwd ? p->tmA_fwd[q] : p->tmA_inv[q];
             for (size_t j = 0; j < p->items_h[d].size(); ++j) {
                 const int4& it = p->items_h[d][j];
+                if (a.paired && !leads_pair(it)) continue;
                 const int m0 = it.w >> 16;
                 const int nk = fwd ? p->Kp / BK : (p->B - m0 + BK - 1) / BK;
                 items.push_back({nk, make_int4(it.x, it.y, ((int)i << 16) | it.z, it.w), p->iaux_h[d][j]});
@@ -2613,6 +2635,9 @@ int tc_fused_create(TCFused** out, const std::vector<TCState*>& parts, std::stri
             faux[i] = items[i].aux;
         }
         f->nitems[d] = (int)flat.size();
+        if ((e = cudaFuncSetAttribute((const void*)gemm_kernel(parts[0]->herm, fwd, f->s2, true, 3, f->paired[d]),
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES)) != cudaSuccess)
+            return fail(e, "tensor-core kernel attributes");
         if ((e = cudaMalloc(&f->d_segs[d], sizeof(GemmSeg) * segs.size())) != cudaSuccess) return fail(e, "cudaMalloc");
         if ((e = cudaMalloc(&f->d_items[d], sizeof(int4) * std::max<size_t>(flat.size(), 1))) != cudaSuccess)
             return fail(e, "cudaMalloc");
@@ -2647,9 +2672,7 @@ int tc_fused_gemm(TCFused* f, bool fwd, cudaStream_t st, StageTimer* T, std::str
     const int nctas = a.nitems < f->nsm ? a.nitems : f->nsm;
     const CUtensorMap* tm = fwd ? f->parts[0]->tmA_fwd : f->parts[0]->tmA_inv;  // unused by fused kernels
     T->begin(fwd ? ST_GEMM_FWD : ST_GEMM_INV, st);
-    bool paired = false;
-    for (TCState* p : f->parts) paired = paired || p->paired;
-    auto kern = gemm_kernel(f->parts[0]->herm, fwd, f->s2, true, 3, paired);
+    auto kern = gemm_kernel(f->parts[0]->herm, fwd, f->s2, true, 3, f->paired[d]);
     kern<<<nctas, THREADS, SMEM_BYTES, st>>>(tm[0], tm[1], tm[2], a, f->d_segs[d]);
     TCK(cudaGetLastError());
     T->end(st);
