@@ -1661,7 +1661,8 @@ int tc_create(TCState** out, int L, int N, int batch, const double* d_table_fp64
         if ((rc = tc_alloc(s, (void**)&s->d_fctl, sizeof(int) * fft_grid_fused_ctl_ints(batch, N), err)))
             return bail(rc);
     } else if (!(s2 && (fft_fast_supported(N) || s->direct))) {
-        if ((rc = tc_alloc(s, (void**)&s->d_work, sizeof(float2) * gridel, err))) return bail(rc);
+        const size_t el = s->dft_tc ? batch * dft_tc_work_elems(N, real) : gridel;
+        if ((rc = tc_alloc(s, (void**)&s->d_work, sizeof(float2) * el, err))) return bail(rc);
     }
     if (s->direct) {
         if ((rc = tc_alloc(s, &s->d_dft, s->dft_tc ? dft_tc_table_bytes(N) : direct_dft_table_bytes(N), err))) return bail(rc);
@@ -2766,12 +2767,13 @@ int tc_fused_phases(TCFused* f, const std::vector<long long>& g0, const std::vec
     }
     // the DFT on the tensor cores
     long long samples = 0;
-    size_t tab = 0, work = 0;
+    size_t tab = 0, work = 0, io = (size_t)1 << 30;  // io: the caller's grids and coefficients, and some room
     bool dft = true;
     for (TCState* p : f->parts) {
         samples += (long long)p->batch * p->N * p->N * p->N;
         tab += (dft_tc_table_bytes(p->N) + 255) & ~(size_t)255;
-        if (!p->d_work) work += (size_t)p->batch * p->N * p->N * p->N;
+        if (!p->d_work) work += p->batch * dft_tc_work_elems(p->N, real);
+        io += (size_t)p->batch * ((size_t)p->N * p->N * p->N + coeffs_per_fn(p)) * (real ? sizeof(float) : sizeof(float2));
         dft = dft && dft_tc_batch_supported(p->N);
     }
     auto drop_dft = [&] {
@@ -2783,8 +2785,10 @@ int tc_fused_phases(TCFused* f, const std::vector<long long>& g0, const std::vec
         f->bytes = 0;
     };
     drop_dft();
-    if (dft && samples >= DFT_BATCH_SAMPLES) {
-        // (no memory for the work grids: the slice FFT, which needs none)
+    size_t freeb = 0, totb = 0;
+    cudaMemGetInfo(&freeb, &totb);
+    // (no memory for the work grids, or none left for the caller's buffers: the slice FFT, which needs none)
+    if (dft && samples >= DFT_BATCH_SAMPLES && tab + sizeof(float2) * work + io <= freeb) {
         e = cudaMalloc(&f->d_dft, tab);
         if (e == cudaSuccess && work) e = cudaMalloc(&f->d_dwork, sizeof(float2) * work);
         std::vector<DftTcBucket> buckets;
@@ -2798,7 +2802,7 @@ int tc_fused_phases(TCFused* f, const std::vector<long long>& g0, const std::vec
             float2* w = p->d_work;
             if (!w) {
                 w = f->d_dwork + wo;
-                wo += (size_t)p->batch * p->N * p->N * p->N;
+                wo += p->batch * dft_tc_work_elems(p->N, real);
             }
             buckets.push_back({p->N, p->batch, p->d_pencil, w, t, g0[i]});
         }

@@ -737,6 +737,7 @@ static bool geometry(Geo& a, const void* in, void* out, long long nf, int N, int
     a.H = folded_terms(N);
     a.KC = (a.H + 15) / 16;
     a.i_f = a.o_f = NN * n;
+    (pass == 1 || pass == -2 ? a.o_f : a.i_f) = (long long)dft_tc_work_elems(N, real);
     a.skip = -1;
     auto blocks = [&](int b) { return (unsigned)((N + b - 1) / b); };
     switch (pass) {
@@ -782,6 +783,8 @@ using namespace dtc;
 
 bool dft_tc_supported(int N) { return N >= MINN && dft_tc_batch_supported(N); }
 bool dft_tc_batch_supported(int N) { return N >= 2 && N % 2 == 0 && folded_terms(N) <= MAXH; }
+
+size_t dft_tc_work_elems(int N, bool real) { return (size_t)(real ? N / 2 + 1 : N) * N * N; }
 
 size_t dft_tc_table_bytes(int N) { return (size_t)12 * 16 * ((folded_terms(N) + 15) / 16) * 128; }
 
