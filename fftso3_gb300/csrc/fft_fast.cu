@@ -18,6 +18,7 @@
 
 #include "common.cuh"
 #include "fft.cuh"
+#include "fft_tile_layout.h"
 
 namespace fftso3 {
 
@@ -91,7 +92,6 @@ __device__ __forceinline__ void reg_dft(float2 (&v)[P])
     }
 }
 
-constexpr int TL = 16;               // lines per CTA tile
 // Threads of a tile's CTA and CTAs an SM (a thread has 8 to 16 values of N <= 256 a step, one or two 32-point DFTs, 64
 // registers of values, of N >= 512).  Both directions, ms: N = 128, 64 real functions, 256 threads x 3 CTAs 1.19, 128 x 6 0.74;
 // N = 256, 16 real functions, 256 x 3 1.48, 128 x 5 1.18, 128 x 6 1.20 (complex 2.20, 2.11); N = 1024 (S^2, 512 real
@@ -99,21 +99,6 @@ constexpr int TL = 16;               // lines per CTA tile
 __host__ __device__ constexpr int tile_threads(int R) { return R <= 8 ? 128 : 256; }
 __host__ __device__ constexpr int tile_ctas(int R) { return R <= 2 ? 8 : R <= 4 ? 6 : R <= 8 ? 5 : 2; }
 
-// The tile kernels' line FFT in two steps, N = A B, n = j2 + B j1, K = k1 + A k2:
-//   X[K] = sum_j2 w_B^{j2 k2} w_N^{j2 k1} sum_j1 w_A^{j1 k1} x[n],
-// an A-point DFT in a thread's registers per (line, j2), one exchange through shared memory, a B-point DFT per (line, k1).
-// Each step's threads run along whichever index makes its global accesses whole 128-byte runs, so the transposition of the
-// tile costs nothing beyond that exchange.
-template <int R, bool C2T>
-__host__ __device__ constexpr int rad_a() { return R == 2 ? 8 : R == 4 ? (C2T ? 8 : 16) : R == 32 ? 32 : 16; }
-template <int R, bool C2T>
-__host__ __device__ constexpr int rad_b() { return 32 * R / rad_a<R, C2T>(); }
-// The exchange: element (line, k1, j2) at line LS + k1 KS + j2, both strides odd: lanes along the line or along k1 hit
-// distinct banks.
-template <int R, bool C2T>
-__host__ __device__ constexpr int tile_ks() { return rad_b<R, C2T>() + 1; }
-template <int R, bool C2T>
-__host__ __device__ constexpr int tile_ls() { return (rad_a<R, C2T>() * tile_ks<R, C2T>()) | 1; }
 // Twiddles in shared memory: W[k1 B + j2] = w_N^{j2 k1}.
 template <int R, bool C2T>
 __device__ __forceinline__ void load_tile_twiddles(float2* W, const double2* __restrict__ tw)
@@ -124,13 +109,6 @@ __device__ __forceinline__ void load_tile_twiddles(float2* W, const double2* __r
         W[i] = make_float2((float)tw[j].x, (float)tw[j].y);
     }
 }
-// Places of 0 .. n - 1 in which x and n - x are neighbours (0 and n / 2 the first two).
-__device__ __forceinline__ int paired(int pos, int n)
-{
-    const int u = pos >> 1;
-    return (pos & 1) ? (u ? n - u : n / 2) : u;
-}
-
 // Geometry of a tiled pass (element offsets).
 struct TileGeo {
     long long FS;  // per function (N^3 for SO(3) grids, N^2 for S^2 grids)
@@ -241,7 +219,7 @@ __device__ __forceinline__ void tile_body(const float2* __restrict__ in, float2*
                                           const float2* Ws, uint64_t pol_in, uint64_t pol_out, MID mid, bool nyq = false,
                                           bool zero = false)
 {
-    constexpr int N = 32 * R, A = rad_a<R, C2T>(), B = rad_b<R, C2T>(), KS = tile_ks<R, C2T>(), LS = tile_ls<R, C2T>();
+    constexpr int N = 32 * R, A = rad_a<R, C2T>(), B = rad_b<R, C2T>(), KS = tile_ks<R, C2T>();
     constexpr int LA = ilog2(A), LB = ilog2(B), NT = tile_threads(R);
     static_assert(!(REAL_IO && IN == IO_SCRATCH && C2T), "the ring holds complex lines");
     static_assert(!HALF || REAL_IO, "half of a real line's spectrum");
@@ -251,7 +229,8 @@ __device__ __forceinline__ void tile_body(const float2* __restrict__ in, float2*
     constexpr int ROWS = REAL_IO ? TL / 2 : TL;
 #pragma unroll 1
     for (int u = threadIdx.x; u < ROWS * B; u += NT) {  // whole warps
-        const int l = C2T ? u / B : u % ROWS, j2 = C2T ? u % B : REAL_IO ? paired(u / ROWS, B) : u / ROWS;
+        const TilePlace at = step1_place<R, C2T, REAL_IO>(u);
+        const int l = at.l, j2 = at.x;
         float2 v[A];
         if (C2T && REAL_IO) {
             const float* s0 = reinterpret_cast<const float*>(in) + cbase + (2 * l) * Ls + j2;
@@ -291,7 +270,7 @@ __device__ __forceinline__ void tile_body(const float2* __restrict__ in, float2*
             }
         }
         reg_dft<A>(v);
-        float2* S = T + l * LS + j2;
+        float2* S = T + step1_slot<R, C2T>(at, 0);
 #pragma unroll
         for (int r = 0; r < A; ++r) {
             const int k1 = brev(r, LA);
@@ -307,9 +286,10 @@ __device__ __forceinline__ void tile_body(const float2* __restrict__ in, float2*
         for (int j = threadIdx.x; j < (HALF ? N / 2 : N); j += NT) l2_discard(in + tbase + (long long)j * Js);
 #pragma unroll 1
     for (int u = threadIdx.x; u < ROWS * A; u += NT) {
-        const int l = C2T ? u % ROWS : u / A, k1 = !C2T ? u % A : REAL_IO ? paired(u / ROWS, A) : u / ROWS;
+        const TilePlace at = step2_place<R, C2T, REAL_IO>(u);
+        const int l = at.l, k1 = at.x;
         float2 v[B];
-        const float2* S = T + l * LS + k1 * KS;
+        const float2* S = T + step2_slot<R, C2T>(at, 0);
 #pragma unroll
         for (int j = 0; j < B; ++j) v[j] = S[j];
         reg_dft<B>(v);
