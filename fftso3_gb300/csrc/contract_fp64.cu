@@ -6,8 +6,8 @@
 // where G_k is the unscaled 2-D DFT of the beta_k slice.  One CTA per
 // (symmetry group, function): the group's <= 4 (m,n) pairs share one table
 // block d_g[l][k], so X[p][k] = w_k G_k(pair p) is staged in shared memory and
-// each warp walks one row l with its lanes over k (coalesced table reads),
-// finishing with a shuffle reduction.
+// each warp takes four rows l at a time, eight lanes a row over k, finishing
+// with a shuffle reduction over the eight.
 //
 // SO(3) inverse (grid form of fdcl_FFTSO3.cpp:498-531):
 //   H_k(m,n) = sum_l (2l+1) F(l,m,n) d^l_mn(beta_k), placed at bin
@@ -16,7 +16,8 @@
 //   Threads over k (coalesced table reads), (2l+1) F staged in shared memory.
 //
 // S^2 is the same pattern with the Legendre table and groups m >= 0 serving
-// the pairs (m, -m) (fdcl_FFTS2.cpp:157-173 forward, :194-230 inverse).
+// the pairs (m, -m) (fdcl_FFTS2.cpp:157-173 forward, :194-230 inverse), its
+// sums folded by parity.
 #include "common.cuh"
 #include "contract.cuh"
 #include "rsph.cuh"
@@ -24,13 +25,6 @@
 namespace fftso3 {
 
 __device__ __forceinline__ int mod_n(int a, int N) { int r = a % N; return r < 0 ? r + N : r; }
-
-__device__ __forceinline__ double warp_sum(double v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
 
 // Reduce-scatter of 8 (4) per-lane partial sums over eight neighbouring lanes: lane `sub` of them gets the full sum of value
 // sub (sub >> 1); each level halves the values a lane carries.  The forward sums take eight lanes a degree, four degrees a
@@ -195,17 +189,6 @@ __global__ void zero_nyquist_so3_kernel(C* __restrict__ H, int N, long long nsli
     else
         slice[(long long)(r - N) * N + B] = z;
 }
-
-__device__ __forceinline__ double2 tmat(int a, int c)
-{
-    c2t<double> t = tmat_t<double>(a, c);
-    return make_double2(t.x, t.y);
-}
-__device__ __forceinline__ double2 cmul2(double2 a, double2 b)
-{
-    return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-__device__ __forceinline__ double2 conj2(double2 a) { return make_double2(a.x, -a.y); }
 
 // The basis changes, F_r = Re(T F_c T^H) per l (fdcl_FFTSO3.cpp:1169-1181) and back, F_c = T^H F_r T (the complex
 // coefficients whose synthesis equals the real synthesis of F_r).  One thread a quadruple (l, +-mu, +-nu), which is closed

@@ -79,7 +79,10 @@ extern "C" {
                                           sums on the tensor cores and a double-float FFT, otherwise in FP64, in
                                           chunks of functions (the refinement's buffers, shared with
                                           FFTSO3_FLAG_REFINE).  The grid values are the FP64 synthesis of the
-                                          coefficients up to that one rounding. */
+                                          coefficients up to that one rounding and an error relative to the
+                                          function's largest values: the digit sums keep 2^-30 of a sum's largest
+                                          term, the DFTs 2^-33 of a line's largest value for N <= 222 that are no
+                                          power of two from 64 (the refined forward likewise). */
 
 typedef struct fftso3_plan fftso3_plan;
 typedef struct fftso3_batch fftso3_batch;
