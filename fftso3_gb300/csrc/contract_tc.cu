@@ -1368,7 +1368,8 @@ struct TCState {
     bool refine = false;
     bool real = false;            // real grids (FFTSO3_*_REAL): real samples in, real part out
     bool herm = false;            // real functions on the tensor cores: one GEMM pair of two (see the kernel)
-    bool paired = false;          // at most half a column tile of functions, mirrored table: groups +-n0 share the tiles (GemmArgs::paired)
+    bool pairable = false;        // at most half a column tile of functions, mirrored table: groups +-n0 may share the tiles
+    bool paired = false;          // ... and do in the plan's own launches (GemmArgs::paired)
     bool s2 = false;              // S^2 (Legendre groups g = m, grids N^2) instead of SO(3)
     bool simt = false;            // FP32 CUDA-core beta-sum (FFTSO3_PREC_FP32) instead of tcgen05
     float* d_tab32 = nullptr;     // FP32 table [row][Kp] (simt)
@@ -1598,13 +1599,15 @@ int tc_create(TCState** out, int L, int N, int batch, const double* d_table_fp64
     s->herm = real && !simt;
     const int fpt = (s2 ? FPT_S2 : FPT) * (s->herm ? 2 : 1);
     s->ntiles = (batch + fpt - 1) / fpt;
-    s->paired = !s2 && !simt && mirrored && batch <= fpt / 2;
+    s->pairable = !s2 && !simt && mirrored && batch <= fpt / 2;
     make_fft_factors_prime_first(N, s->fac);
     s->d_tw = d_tw;
     s->total_rows = table_elems / N;
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&s->nsm, cudaDevAttrMultiProcessorCount, dev);
+    // a launch whose items all run at once gains nothing by fewer, longer ones (l_max 7, 8 functions, forward 37 us against 35)
+    s->paired = s->pairable && s->ngroups > s->nsm;
     int rc;
     auto bail = [&](int code) {
         tc_destroy(s);
@@ -2566,9 +2569,12 @@ void tc_fused_destroy(TCFused* f)
 static bool pairing_pays(const std::vector<TCState*>& parts, bool fwd)
 {
     double can = 0, cannot = 0;
+    size_t items = 0;
+    for (const TCState* p : parts) items += p->items_h[fwd ? 0 : 1].size();
+    if (items <= (size_t)parts[0]->nsm) return false;  // they all run at once
     for (const TCState* p : parts)
         for (const int4& it : p->items_h[fwd ? 0 : 1])
-            (p->paired ? can : cannot) += fwd ? p->Kp / BK : (p->B - (it.w >> 16) + BK - 1) / BK;
+            (p->pairable ? can : cannot) += fwd ? p->Kp / BK : (p->B - (it.w >> 16) + BK - 1) / BK;
     return cannot < (parts[0]->herm ? 1.0 : fwd ? 0.35 : 3.0) * can;
 }
 
@@ -2610,7 +2616,7 @@ int tc_fused_create(TCFused** out, const std::vector<TCState*>& parts, std::stri
         for (size_t i = 0; i < parts.size(); ++i) {
             TCState* p = parts[i];
             GemmArgs a = gemm_args(p);
-            a.paired = p->paired && f->paired[d];
+            a.paired = p->pairable && f->paired[d];
             if (fwd) {
                 a.pin = p->d_pencil;
                 a.cout = p->d_fg;
