@@ -1491,6 +1491,15 @@ static auto gemm_kernel(bool herm, bool fwd, bool s2, bool fused, int terms, boo
     return herm ? gemm_kernel<true>(fwd, s2, fused, terms, paired) : gemm_kernel<false>(fwd, s2, fused, terms, paired);
 }
 
+static int largest_prime(int n)
+{
+    int p = 2;
+    while (p < n)
+        if (n % p == 0) n /= p;
+        else ++p;
+    return n;
+}
+
 static int autotune_fft(TCState* s, std::string& err);
 static int autotune_cluster(TCState* s, std::string& err);
 static int launch_gemm(TCState* s, bool fwd, cudaStream_t st, std::string& err, float2* cout = nullptr,
@@ -1653,9 +1662,14 @@ int tc_create(TCState** out, int L, int N, int batch, const double* d_table_fp64
         // the direct DFT from half a million samples (S^2: a million; smaller batches are bound by launch latencies, where
         // the line FFT's simpler kernels win: l_max 16, 4 functions, 0.16 M samples, 76 against 81 us both directions;
         // l_max 38, 0.47 M, 125 against 119 us; l_max 30, 32 functions, 7.6 M, 524 against 361 us; S^2 l_max 47, 8 signals,
-        // 51 against 53 us, l_max 200, 8 signals, 1.3 M, equal, l_max 100, 64 signals, 2.6 M, 219 against 124 us;
-        // l_max 39, 0.51 M, on the tensor cores 125 against 107 us)
-        s->direct = !fft_fast_supported(N) && direct_dft_supported(N) && gridel >= (s2 ? 1000000 : 500000);
+        // 51 against 53 us, l_max 200, 8 signals, 1.3 M, equal, l_max 100, 64 signals, 2.6 M, 219 against 124 us, l_max
+        // 159, 11 real signals, 1.1 M, 92 against 97; l_max 39, 0.51 M, on the tensor cores 125 against 107 us)
+        s->direct = !fft_fast_supported(N) && direct_dft_supported(N) && gridel >= (!s2 ? 500000 : N > 288 ? 1200000 : 1000000);
+        // complex signals above N = 222, where an SM holds one CTA, and with small prime factors, which the line FFT is good at:
+        // from waves four fifths full on (N = 320, both directions, direct over line FFT: fill 0.99 0.88, 0.92 0.90, 0.88 1.01,
+        // 0.72 1.11, 0.56 1.20; N = 240: 0.94 0.82, 0.87 0.81, 0.82 0.92, 0.72 0.99, 0.52 1.08)
+        if (s->direct && s2 && !s->herm && N > 222 && largest_prime(N) < 32)
+            s->direct = direct_dft_fill(N, (long long)batch * N) >= 0.8;
         s->dft_tc = s->direct && !s2 && !simt && dft_tc_supported(N);
     }
     if (s->fused_fft) {

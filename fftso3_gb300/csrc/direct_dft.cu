@@ -66,6 +66,19 @@ static Shape shape_of(int N, unsigned nu = 0x7fffffffu, int nsm = 1)
     return s;
 }
 
+// CTAs an SM holds (the runtime's occupancy query costs more than a small pass): shared memory, and 128 registers a thread
+static int ctas_per_sm(const Shape& s)
+{
+    return std::max(1, std::min((int)(228 * 1024 / (s.smem + 1024)), 512 / s.threads));
+}
+static int device_sms()
+{
+    int dev = 0, nsm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    return nsm;
+}
+
 struct Args {
     DirectPass p;
     const float4* table;
@@ -349,9 +362,7 @@ static cudaError_t run_ql(const Args& a, const Shape& s, cudaStream_t st)
     auto kern = direct_dft_kernel<KIND, LC, SC, MIR, QL>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
     if (e != cudaSuccess) return e;
-    // CTAs an SM holds (the runtime's occupancy query costs more than a small pass): shared memory, and 128 registers a thread
-    const int per = std::max(1, std::min((int)(228 * 1024 / (s.smem + 1024)), 512 / s.threads));
-    const unsigned nblk = std::min(a.ntiles, (unsigned)(a.nsm * per));
+    const unsigned nblk = std::min(a.ntiles, (unsigned)(a.nsm * ctas_per_sm(s)));
     kern<<<nblk, s.threads, s.smem, st>>>(a);
     return cudaGetLastError();
 }
@@ -381,6 +392,15 @@ bool direct_dft_supported(int N)
     return s.QL > 0;
 }
 
+double direct_dft_fill(int N, long long units)
+{
+    const int nsm = device_sms();
+    const Shape s = shape_of(N, (unsigned)std::min(units, 0x7fffffffLL), nsm);
+    if (!s.QL || nsm < 1) return 0;
+    const long long tiles = (units + s.LT - 1) / s.LT, slots = (long long)nsm * ctas_per_sm(s);
+    return (double)tiles / (double)((tiles + slots - 1) / slots * slots);
+}
+
 cudaError_t launch_direct_dft(const DirectPass& p, const void* table, cudaStream_t st)
 {
     if (!direct_dft_supported(p.N) || p.nf < 1 || p.no < 1 || p.ni < 1) return cudaErrorInvalidValue;
@@ -388,9 +408,7 @@ cudaError_t launch_direct_dft(const DirectPass& p, const void* table, cudaStream
     Args a;
     a.p = p;
     a.nu = (unsigned)(p.nf * p.no * p.ni);
-    int dev = 0, nsm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    const int nsm = device_sms();
     const Shape s = shape_of(p.N, a.nu, nsm);
     a.table = (const float4*)table;
     a.LT = s.LT;

@@ -190,6 +190,8 @@ struct DirectPass {
 };
 // Even N whose matrices and one tile fit a CTA's shared memory (N <= 400 or so).
 bool direct_dft_supported(int N);
+// Share of the SMs' CTAs that a pass of so many units keeps busy in its waves of tiles.
+double direct_dft_fill(int N, long long units);
 // The matrices of length N in device memory, made once per plan from its twiddle table tw (N double2): built by every CTA
 // of every pass, the FP64 loads and conversions took 10 to 25 us of small passes.
 size_t direct_dft_table_bytes(int N);
