@@ -12,7 +12,7 @@
 // their products are whole multiples of one unit, at most 56 2^16 of it, and their sums exact.  The tensor cores cut a sum
 // off where they cannot hold it; with floating-point leading terms that shrank every bin by the same 1e-8 to 2e-8 of itself,
 // which the beta-sum, unlike rounding, does not average (forward of l_max 96, one complex function: off by 1.79e-7 of its 2-norm,
-// now 1.53e-7, of which the beta-sum alone makes most; inverse 1.82e-7 and 1.28e-7; 4 to 8 % more time).  The two other terms hold the remainder to 2^-26 of the line's largest value.
+// now 1.53e-7, of which the beta-sum alone makes most; inverse 1.82e-7 and 1.28e-7; 0 to 7 % more time a direction).  The two other terms hold the remainder to 2^-26 of the line's largest value.
 //
 // Why: as FP32 register tiles (direct_dft.cu) the products and the loads take turns on the same warps: 1.1 to 1.2 ms a pass
 // at N = 194 (16 complex functions).  Here one thread issues them and the warps only move data: 0.43 ms (0.55 ms the
@@ -115,23 +115,56 @@ __device__ __forceinline__ Unit unit_of(unsigned m)
     return {__uint_as_float((unsigned)(127 + e - 8) << 23), __uint_as_float((unsigned)(127 + 8 - e) << 23)};
 }
 
+// Packed FP32 pairs: half the instructions of the splits (19 warps' producers are short of issue slots).
+typedef unsigned long long u64;
+__device__ __forceinline__ u64 pack2(float a, float b)
+{
+    u64 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(u64 a)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+    return r;
+}
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c)
+{
+    u64 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ u64 add2(u64 a, u64 b)
+{
+    u64 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ u64 mul2(u64 a, u64 b)
+{
+    u64 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
 // eight values into one 16-byte chunk of each of the three BF16 planes
 __device__ __forceinline__ void store_split(uint32_t dst, const float* x, Unit s)
 {
-    constexpr float MAGIC = 12582912.f;  // 1.5 2^23
+    const u64 magic = pack2(12582912.f, 12582912.f), minus = pack2(-12582912.f, -12582912.f);  // 1.5 2^23
+    const u64 inv = pack2(s.inv, s.inv), u = pack2(s.u, s.u), nu = pack2(-s.u, -s.u), n1 = pack2(-1.f, -1.f);
     uint32_t w[3][4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        float v[2];
-        float q[2];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            q[h] = __fsub_rn(__fmaf_rn(x[2 * j + h], s.inv, MAGIC), MAGIC);
-            v[h] = __fmaf_rn(-q[h], s.u, x[2 * j + h]);  // exact
-        }
-        w[0][j] = bf2(q[0] * s.u, q[1] * s.u);  // |q| <= 256
-        w[1][j] = bf2(v[0], v[1]);
-        w[2][j] = bf2(v[0] - __uint_as_float(w[1][j] << 16), v[1] - __uint_as_float(w[1][j] & 0xffff0000u));
+        const u64 v = pack2(x[2 * j], x[2 * j + 1]);
+        const u64 q = add2(fma2(v, inv, magic), minus);  // |q| <= 256
+        const u64 r = fma2(q, nu, v);                    // exact
+        const float2 lead = unpack2(mul2(q, u)), rest = unpack2(r);
+        w[0][j] = bf2(lead.x, lead.y);
+        w[1][j] = bf2(rest.x, rest.y);
+        const u64 t = pack2(__uint_as_float(w[1][j] << 16), __uint_as_float(w[1][j] & 0xffff0000u));
+        const float2 last = unpack2(fma2(t, n1, r));
+        w[2][j] = bf2(last.x, last.y);
     }
 #pragma unroll
     for (int p = 0; p < 3; ++p)
@@ -139,7 +172,11 @@ __device__ __forceinline__ void store_split(uint32_t dst, const float* x, Unit s
                      "r"(w[p][2]), "r"(w[p][3])
                      : "memory");
 }
-__device__ __forceinline__ void producers_sync() { asm volatile("bar.sync 1, %0;" ::"n"(32 * NPROD) : "memory"); }
+// A line's warps: those of the same parity (their items' blocks of 32 lines have it).
+__device__ __forceinline__ void producers_sync(int warp)
+{
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + (warp & 1)), "n"(16 * NPROD) : "memory");
+}
 
 // A line of a tile: its place in the input and the output (elements of the side's type), and whether it exists.
 struct Line {
@@ -414,18 +451,24 @@ __device__ __forceinline__ void produce(const Args& a, int pass, const Ctx& c, C
                 }
             }
         }
-        // the next tile's maxima: last read before the last tile's barrier
-        if (threadIdx.x < 128) c.mx[(n.tp == 2 ? 0 : n.tp + 1) * 128 + threadIdx.x] = 0;
-        producers_sync();
+        // the next tile's maxima (of this parity's lines): last read before the last tile's barrier
+        if (c.warp < 2) {
+            unsigned* next = c.mx + (n.tp == 2 ? 0 : n.tp + 1) * 128 + 32 * c.warp + lane;
+            next[0] = 0;
+            if (LB == 4) next[64] = 0;
+        }
+        producers_sync(c.warp);
+        bool dead = __any_sync(0xffffffffu, *c.abort_flag);
         Unit un[IPW];
 #pragma unroll
         for (int w = 0; w < IPW; ++w) un[w] = unit_of(c.mx[n.tp * 128 + ln[w]]);
 #pragma unroll
         for (int pr = 0; pr < 4; ++pr, ++n.s) {
             const int sl = n.s & 1;
-            const bool stop = *c.abort_flag || (n.s >= 2 && !mbar_wait(&c.empty[sl], ((n.s >> 1) - 1) & 1, a.err, 31));
-            if (__any_sync(0xffffffffu, stop)) {
+            if (dead) continue;
+            if (__any_sync(0xffffffffu, n.s >= 2 && !mbar_wait(&c.empty[sl], ((n.s >> 1) - 1) & 1, a.err, 31))) {
                 *c.abort_flag = 1;
+                dead = true;
                 continue;
             }
 #pragma unroll
