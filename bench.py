@@ -135,7 +135,8 @@ def measured_peaks() -> dict:
 def profiled_traffic(stage: str, l_max: int, batch: int):
     """DRAM bytes per launch of `stage` from the committed ncu capture figures
     (profiles/traffic.json: stage, l_max, batch, bytes per launch), scaled to
-    this workload: by batch (functions per launch) at the same l_max, and for
+    this workload: by batch (functions per launch) at the same l_max (from the
+    capture of the nearest batch), and for
     the FFT stages (whose traffic is one read and one write of every sample) by
     batch * N^3 across l_max."""
     path = os.path.join(ROOT, "profiles", "traffic.json")
@@ -143,9 +144,10 @@ def profiled_traffic(stage: str, l_max: int, batch: int):
         return None
     found = [(r["l_max"], r["batch"], r["bytes_per_launch"]) for r in json.load(open(path))["captures"]
              if r["stage"] == stage]
-    for L0, b0, byts in found:
-        if L0 == l_max:
-            return byts * batch / b0
+    same = [(abs(b0 - batch), b0, byts) for L0, b0, byts in found if L0 == l_max]
+    if same:
+        _, b0, byts = min(same)
+        return byts * batch / b0
     for L0, b0, byts in found:
         if "fft" in stage:
             return byts * batch / b0 * ((l_max + 1) / (L0 + 1)) ** 3
@@ -429,7 +431,7 @@ def uneven_line(args) -> dict:
                                "N(0,1)/(2l+1), FP32 samples; fftso3_batch, tensor-core buckets, CUDA graph",
                    "functions": n, "buckets": bt.buckets, "streams": bt.streams, "samples": int(G),
                    "coefficients": int(Ctot),
-                   "form": ("three launches per direction over all buckets (slice FFT, fused GEMM, conversion)"
+                   "form": ("three launches per direction over all buckets (FFT, fused GEMM, conversion)"
                             if bt.graph_kernels(0) == 3 else "per-bucket phases around one fused GEMM launch"),
                    "l2": "inputs larger than L2"},
         "io_gbs": io_bytes / (ms / 1000.0) / 1e9, "io_frac_of_hbm": io_bytes / (ms / 1000.0) / 1e9 / peaks["hbm_gbs"],

@@ -686,12 +686,11 @@ int fftso3_plan_create(fftso3_plan** out, int kind, int l_max, int batch, int pr
         const bool use_oz = (flags & exact_flags) && p->so3 && oz_supported(L, N) && !(ev_ref && ev_ref[0] == '1');
         if (use_oz) {
             // SO(3) refinement on the tensor cores: digit planes of the FP64 table, then the table is freed.
-            // Chunks of 16 functions (two column tiles, whose items share each table tile through L2, so the
-            // digit planes are read once per 16 functions) when the device has room for them with 16 GB to
-            // spare after the FP64 table is freed, else 8 (one column tile), else fewer
-            // The spectral form (N <= 222, 256 or 512) needs the double-float pencils only as its FFT's work space
-            // (pen_fns = up to 8 functions at a time, of small grids more), so its contraction chunks grow to 32 functions (four column
-            // tiles sharing each table tile; the digit planes read once per 32 functions).
+            // The contraction's chunks: as many functions as the device has room for with 16 GB to spare after
+            // the FP64 table is freed.  A chunk's column tiles (8 functions each) share each table tile through
+            // L2, so the digit planes are read once per chunk.  The spectral form (N <= 222, 256 or 512) needs the
+            // double-float pencils only as its FFT's work space (pen_fns = up to 8 functions at a time, of small
+            // grids more) and takes up to 32 functions, the grid form, whose pencils cover the chunk, up to 16.
             const bool spectral = oz_spectral_supported(N);
             const size_t pen_fn = 16 * (size_t)p->grid_elems;
             const size_t planes = 4 * 2 * (size_t)(p->table_elems / N) * (size_t)((N + 63) / 64 * 64);
@@ -707,7 +706,7 @@ int fftso3_plan_create(fftso3_plan** out, int kind, int l_max, int batch, int pr
             size_t nch = spectral ? 32 : 16;
             while (nch > 1 && (need(nch) + slack > freeb || freeb + tab64 < need(nch) + spare))
                 nch = nch > 16 ? 16 : nch > 8 ? 8 : nch - 1;
-            if (const char* ev = getenv("FFTSO3_REFINE_CHUNK")) {  // cap (1..16), e.g. to exercise several chunks
+            if (const char* ev = getenv("FFTSO3_REFINE_CHUNK")) {  // a cap, e.g. to exercise several chunks
                 const int c = atoi(ev);
                 if (c >= 1 && (size_t)c < nch) nch = (size_t)c;
             }

@@ -2528,7 +2528,7 @@ int tc_inverse_fft(TCState* s, void* grid, cudaStream_t st, StageTimer* T, std::
 }
 
 // Samples from which a batch's DFT passes run on the tensor cores (both directions, complex / real, us, slice FFT -> tensor
-// cores: 0.9 M samples 177 / 163 -> 187 / 172, 5.4 M 472 / 397 -> 404 / 315, 82 M 9297 / 5708 -> 4417 / 3883).
+// cores: 0.9 M samples 142 / 129 -> 126 / 129, 4.9 M 533 / 431 -> 388 / 347, 90 M 9239 / 5297 -> 3947 / 3320).
 constexpr long long DFT_BATCH_SAMPLES = 2000000;
 
 struct TCFused {

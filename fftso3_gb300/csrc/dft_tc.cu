@@ -11,12 +11,13 @@
 // The leading terms are in fixed point, 8 bits under the line's largest folded value and 8 under 1 for the matrix, so that
 // their products are whole multiples of one unit, at most 56 2^16 of it, and their sums exact.  The tensor cores cut a sum
 // off where they cannot hold it; with floating-point leading terms that shrank every bin by the same 1e-8 to 2e-8 of itself,
-// which the beta-sum, unlike rounding, does not average (forward of l_max 96, one complex function: off by 1.79e-7 of its 2-norm,
-// now 1.53e-7, of which the beta-sum alone makes most; inverse 1.82e-7 and 1.28e-7; 0 to 7 % more time a direction).  The two other terms hold the remainder to 2^-26 of the line's largest value.
+// which the beta-sum, unlike rounding, does not average (forward of l_max 96, one complex function: off by 1.79e-7 of its
+// 2-norm, now 1.53e-7, of which the beta-sum alone makes most; inverse 1.82e-7 and 1.28e-7; 0 to 7 % more time a
+// direction).  The two other terms hold the remainder to 2^-26 of the line's largest value.
 //
-// Why: as FP32 register tiles (direct_dft.cu) the products and the loads take turns on the same warps: 1.1 to 1.2 ms a pass
-// at N = 194 (16 complex functions).  Here one thread issues them and the warps only move data: 0.43 ms (0.55 ms the
-// transposing passes), 0.24 to 0.38 ms real.  Roles of the one CTA an SM holds:
+// Why: as FP32 register tiles (direct_dft.cu) the products and the loads take turns on the same warps: 1.0 to 1.2 ms a pass
+// at N = 194 (16 complex functions).  Here one thread issues them and the warps only move data: 0.39 ms (0.49 and 0.63 the
+// transposing passes), 0.21 to 0.29 ms real.  Roles of the one CTA an SM holds:
 //   warps 0-13   producers: load a line's elements t, N - t, P - t, P + t for eight t, fold, split, store the K-major
 //                swizzled rows, one problem at a time into a ring of two 48 KB slots (the folded values wait in registers);
 //   warps 14-17  epilogue, one TMEM lane quarter each: C and S -> X[q], X[N - q] -> global memory;
@@ -24,7 +25,7 @@
 // The matrices (at most 96 KB) stay in shared memory.  Accumulators: two buffers (even and odd q) of C and S, hi and lo.
 // Bound: a 64-line tile takes 12 k cycles at N = 194, of which its bytes need 8.6 k (16 a complex sample and pass at
 // 6.8 TB/s) and its 80 MMAs 6 k; the rest is the producers' load latency, which 96 registers a thread cannot cover further
-// (64 hold the folded values), and instruction issue (53% of the slots).  Eight epilogue warps with a register split
+// (64 hold the folded values), and instruction issue (45 to 55% of the slots).  Eight epilogue warps with a register split
 // (setmaxnreg 88 / 64) measured the same.
 
 // Layouts: both sides of a pass are contiguous along a line index, never along the transformed one, so every global access
@@ -53,7 +54,7 @@ constexpr int MAXH = 56;              // folded terms: 7 chunks of 8 (a 64-line 
 constexpr int MX = 3 * 128 * 4;       // bytes of the lines' largest values (a ring of three tiles)
 
 // Below, the FP32 kernel: with few terms a tile's fixed latencies outweigh its products (all four passes, complex / real, ms:
-// N = 66, 64 functions 0.52 / 0.40 here, 0.53 / 0.32 there; N = 160, 16 functions 1.00 / 0.70 here, 2.44 / 1.33 there).
+// N = 66, 64 functions 0.51 / 0.28 here, 0.42 / 0.26 there; N = 160, 16 functions 0.92 / 0.52 here, 2.32 / 1.24 there).
 constexpr int MINN = 80;
 
 enum { COMPLEX = 0, REAL_IN = 1, REAL_OUT = 2 };

@@ -8,7 +8,7 @@
 // run, and two CTAs share an SM where the shared memory allows, so one loads while the other multiplies.
 // What bounds it: N / 2 packed FMAs a complex sample (35 T FMA/s measured with fma.rn.f32x2; 25 T with scalar fma, whose
 // three register operands meet in the register banks), and that a CTA's loads and products take turns: at N = 194, 16
-// functions, a pass takes 1.1 to 1.2 ms, 0.3 of it the bytes, 0.5 the products (0.35 at the FMA rate), the rest loading and
+// functions, a pass takes 1.0 to 1.2 ms, 0.3 of it the bytes, 0.5 the products (0.35 at the FMA rate), the rest loading and
 // folding.  SO(3) passes of N = 80 to 222 run on the tensor cores instead (dft_tc.cu).
 #include <algorithm>
 #include <type_traits>

@@ -8,8 +8,7 @@
 // N^2 / 2 FMAs a complex line (P / 2 a real one) whatever N's factors are, all of them independent register-tile work
 // with every operand in shared memory.  A mixed-radix Stockham FFT has fewer operations, but its stages each cross
 // shared memory and a barrier, and a prime factor R costs it R FMAs an element anyway.  Measured on one GB300 (all four
-// passes, 64 complex functions, N = 194): 38.9 ms with the separate transposes as a mixed-radix FFT, 18.5 ms here (with one
-// accumulator a sum, see CHUNK).
+// passes, 64 complex functions, N = 194): 38.9 ms with the separate transposes as a mixed-radix FFT, 18.2 ms here.
 //
 // A unit is a complex line, or two real lines x, y.  Its folded terms are held as the pairs (a.x, b.y), (a.y, b.x) (real
 // lines: (a.x, b.x), (a.y, b.y)) and the matrices as the pairs (cos, sin), so that one packed FMA advances a cosine sum
